@@ -111,7 +111,7 @@ struct forge_ctx {
     double last_residual = INFINITY;
     DevBuf oaws, w_all;
     // group solve led by this context (forge_gpu_solve_group): padded H slots, eigenpairs, workspaces
-    DevBuf g_H, g_X, g_w, g_eigws, g_mixws, g_tmp, g_rows, g_sig, g_rr;
+    DevBuf g_H, g_X, g_w, g_eigws, g_mixws, g_tmp, g_rows, g_sig, g_rr, g_lim;
     int64_t eig_batch = 0;
     int64_t k_begin = 0, k_end = 0;  // local k range (k_end = 0: all k)
     // mixing: FORGE_MIX_ODA (OptimalStep, the reference), FORGE_MIX_PULAY (Anderson / Pulay) or
@@ -310,7 +310,10 @@ int project_k(forge_ctx* x, int64_t k, int64_t K, const double2* ph, double2* ou
     const int64_t N = c.N, iu = c.nUpper;
     const double2* Xk = c.X.as<double2>() + (size_t)k * N * iu;
     if (c.precision == FORGE_PREC_MIXED) {
-        FORGE_TRY(x->tcerr.ensure(sizeof(int)));
+        if (!x->tcerr.ptr) {
+            FORGE_TRY(x->tcerr.ensure(sizeof(int)));
+            FORGE_CUDA(cudaMemsetAsync(x->tcerr.ptr, 0, sizeof(int), c.stream));
+        }
         if (x->oa_active) {
             // refined eigenvectors: the projector keeps their FP64 accuracy (exact sliced products)
             FORGE_TRY(x->projws.ensure(proj_tc_exact_workspace_bytes(N, iu)));
@@ -884,6 +887,8 @@ int solve_group_device(forge_ctx** xs, int64_t nctx, int* infos) {
     FORGE_TRY(x0->g_tmp.ensure(slot * sizeof(double2)));
     FORGE_TRY(x0->g_rows.ensure(nmax * sizeof(double)));
     FORGE_TRY(x0->g_sig.ensure(sizeof(double)));
+    FORGE_TRY(x0->g_lim.ensure((size_t)B * sizeof(int)));
+    std::vector<int> lims(B);
     if (mixed && x0->rr_width > 0) FORGE_TRY(x0->g_rr.ensure(rr_window_workspace_bytes(nmax, 1)));
     double2* gH = x0->g_H.as<double2>();
     double2* gX = x0->g_X.as<double2>();
@@ -913,6 +918,11 @@ int solve_group_device(forge_ctx** xs, int64_t nctx, int* infos) {
         g.strideX = nmax * iumax;
         g.w = gw;
         g.ortol_rel = 1e-7;
+        // each slot solves for its own system's nUpper eigenpairs: the padding's eigenvalues, all
+        // equal, would otherwise form one large cluster when nUpper of the largest exceeds N of a small one
+        for (int64_t q = 0; q < nb; ++q) lims[q] = (int)xs[items[q0 + q].first]->c.nUpper;
+        FORGE_CUDA(cudaMemcpyAsync(x0->g_lim.ptr, lims.data(), nb * sizeof(int), cudaMemcpyHostToDevice, st));
+        g.iu_lim = x0->g_lim.as<int>();
         eig_bind_workspace(g, x0->g_eigws.ptr);
         FORGE_TRY(mixed ? eig_mixed(st, g, x0->g_mixws.ptr) : eig_fp64(st, g));
         if (mixed && x0->rr_width > 0)
@@ -1160,7 +1170,7 @@ int forge_gpu_finalize(forge_ctx* x) {
                       &x->c3_Xr, &x->c3_wr, &x->c3_tab, &x->c3_perm, &x->c3_phase, &x->c2_perm,
                       &x->v_rowp, &x->v_col, &x->v_coef, &x->v_code, &x->v_ph, &x->v_W, &x->v_G, &x->v_S,
                       &x->v_Xv, &x->v_st, &x->oaws, &x->w_all, &x->g_H, &x->g_X, &x->g_w, &x->g_eigws,
-                      &x->g_mixws, &x->g_tmp, &x->g_rows, &x->g_sig, &x->g_rr};
+                      &x->g_mixws, &x->g_tmp, &x->g_rows, &x->g_sig, &x->g_rr, &x->g_lim};
     for (DevBuf* b : bufs) b->release();
     if (c.stream) cudaStreamDestroy(c.stream);
     delete x;

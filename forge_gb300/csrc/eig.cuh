@@ -34,9 +34,12 @@ struct EigArgs {
     int64_t scr_stride;         // >= iu
     int* fail;                  // batch
     double2 *G, *T, *Wb, *W2b;  // back-transform: NB x NB, NB x NB, NB x iu, NB x iu per batch
-    float* tf;                  // batch x 2n: FP32 copies of d and e^2 (FP32 bisection)
+    float2* tf;                 // batch x n: T scaled to |T| <= 1, (d_i, e_{i-1}^2) in FP32 (FP32 bisection)
+    double2* de;                // the same in FP64
+    float* tq;                  // batch x 2n: unscaled T in FP32, d and e^2 (mixed precision)
+    int replay = 0;             // 1 (mixed precision): eigenvalues as the quotient-form bisection gives them
     double ortol_rel;
-    int bisect_f32 = 0;         // 1: FP32 bisection first, FP64 bisection from its bracket
+    const int* iu_lim = nullptr;  // device: eigenpairs wanted of each matrix (nullptr: iu of every one)
     int64_t iu_out = 0;         // mixed solver: FP64 columns written to X (0: all iu)
 };
 

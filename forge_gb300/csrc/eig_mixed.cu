@@ -611,9 +611,9 @@ int eig_mixed(cudaStream_t st, EigArgs& g, void* mixed_ws) {
     a.her2k_user = &ws;
     FORGE_CUDA(cudaMemsetAsync(ws.cnt, 0, sizeof(unsigned) * 4 * batch, st));
     FORGE_TRY(tridiagonalize<float>(st, a, batch));
-    // eigenvalues of T: FP32 bisection, then FP64 bisection from the FP32 bracket
+    // eigenpairs of T in FP64
     EigArgs ge = g;
-    ge.bisect_f32 = 1;
+    ge.replay = 1;
     FORGE_TRY(tridiag_eigvecs(st, ge));
     dim3 gz((unsigned)((ws.n4 + 31) / 32), (unsigned)((iu + 31) / 32), (unsigned)batch);
     k_z_to_planes<<<gz, dim3(32, 8), 0, st>>>(g.Z, n, ws.n4, iu, ws.Xs);
