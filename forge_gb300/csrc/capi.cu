@@ -304,37 +304,55 @@ int eig_batch_run(forge_ctx* x, int64_t k0, int64_t nb, int* info, double2* Xdst
     return 0;
 }
 
-// bulk_c += ph_c(k) conj(X_k) X_k^T over the first K columns (precision of the context)
-int project_k(forge_ctx* x, int64_t k, int64_t K, const double2* ph, double2* out) {
+// appends the projector of k's first K columns to a batch; at a C3-invariant k the average of Solve_C3 /
+// GetFock_C3: the projectors of k's eigenvectors and of their two rotated copies, each with a third of the phases
+void add_projector(forge_ctx* x, int64_t k, int64_t K, const double2* ph, std::vector<ProjItem>& items) {
+    ProjItem p{k, K, {ph[0], ph[1], ph[2], ph[3]}};
+    if (!x->c3 || x->c3t.extra[k] < 0) {
+        items.push_back(p);
+        return;
+    }
+    for (int t = 0; t < 4; ++t) p.ph[t] = cscale(ph[t], 1.0 / 3.0);
+    items.push_back(p);
+    p.slot = x->c3t.extra[k];
+    items.push_back(p);
+    ++p.slot;
+    items.push_back(p);
+}
+
+// out_c += sum over the batch of ph_c conj(X) X^T over the items' first K columns (precision of the context)
+int project_items(forge_ctx* x, const std::vector<ProjItem>& items, double2* out) {
     Context& c = x->c;
-    const int64_t N = c.N, iu = c.nUpper;
-    const double2* Xk = c.X.as<double2>() + (size_t)k * N * iu;
-    if (c.precision == FORGE_PREC_MIXED) {
-        if (!x->tcerr.ptr) {
-            FORGE_TRY(x->tcerr.ensure(sizeof(int)));
-            FORGE_CUDA(cudaMemsetAsync(x->tcerr.ptr, 0, sizeof(int), c.stream));
-        }
+    const int64_t N = c.N, iu = c.nUpper, nit = (int64_t)items.size();
+    if (!x->tcerr.ptr) {
+        FORGE_TRY(x->tcerr.ensure(sizeof(int)));
+        FORGE_CUDA(cudaMemsetAsync(x->tcerr.ptr, 0, sizeof(int), c.stream));
+    }
+    if (c.precision != FORGE_PREC_MIXED) {
+        FORGE_TRY(x->projws.ensure(proj_oz_workspace_bytes(N, iu, nit)));
+        return projectors_oz(c.stream, c.X.as<double2>(), N, N * iu, N, iu, items.data(), nit, out, x->projws.ptr,
+                             x->tcerr.as<int>());
+    }
+    for (const ProjItem& p : items) {
+        const double2* Xk = c.X.as<double2>() + (size_t)p.slot * N * iu;
         if (x->oa_active) {
             // refined eigenvectors: the projector keeps their FP64 accuracy (exact sliced products)
             FORGE_TRY(x->projws.ensure(proj_tc_exact_workspace_bytes(N, iu)));
-            return bulk_projector_tc_exact(c.stream, Xk, N, N, K, iu, ph, out, x->projws.ptr, x->tcerr.as<int>());
+            FORGE_TRY(bulk_projector_tc_exact(c.stream, Xk, N, N, p.K, iu, p.ph, out, x->projws.ptr, x->tcerr.as<int>()));
+        } else {
+            FORGE_TRY(x->projws.ensure(proj_tc_workspace_floats(N, iu) * sizeof(float)));
+            FORGE_TRY(bulk_projector_tc(c.stream, Xk, N, N, p.K, iu, p.ph, out, x->projws.as<float>(), x->tcerr.as<int>()));
         }
-        FORGE_TRY(x->projws.ensure(proj_tc_workspace_floats(N, iu) * sizeof(float)));
-        return bulk_projector_tc(c.stream, Xk, N, N, K, iu, ph, out, x->projws.as<float>(), x->tcerr.as<int>());
     }
-    return bulk_projector_fp64(c.stream, Xk, N, N, K, ph, out);
+    return 0;
 }
 
-// project_k, with the average of Solve_C3 / GetFock_C3 at a C3-invariant k: the projector of k's
-// eigenvectors and of their two rotated copies, each with a third of the phases
-int project_k_c3(forge_ctx* x, int64_t k, int64_t K, const double2* ph, double2* out) {
-    if (!x->c3 || x->c3t.extra[k] < 0) return project_k(x, k, K, ph, out);
-    double2 ph3[4];
-    for (int t = 0; t < 4; ++t) ph3[t] = cscale(ph[t], 1.0 / 3.0);
-    const int64_t e = x->c3t.extra[k];
-    FORGE_TRY(project_k(x, k, K, ph3, out));
-    FORGE_TRY(project_k(x, e, K, ph3, out));
-    return project_k(x, e + 1, K, ph3, out);
+// the zFockBulk sum over the local k points: bands 1..nLower-1 of every k
+int project_bulk(forge_ctx* x, double2* out) {
+    const int64_t kb = x->k_begin, ke = (x->k_end > 0) ? x->k_end : x->c.Nk;
+    std::vector<ProjItem> items;
+    for (int64_t k = kb; k < ke; ++k) add_projector(x, k, x->c.nLower - 1, &x->h_bph[k * 4], items);
+    return project_items(x, items, out);
 }
 
 // window states with the C3 average: a state at a C3-invariant k becomes itself and its two
@@ -404,9 +422,7 @@ int solve_device(forge_ctx* x, int* info, bool with_projector = true) {
         FORGE_TRY(launch_c3_rotate(c.stream, x->c3_Xr.as<double2>(), x->c3_wr.as<double>(), N_, iu, x->c3t.nslots,
                                    x->c3_tab.as<int64_t>(), x->c3_perm.as<int64_t>(), x->c3_phase.as<double2>(),
                                    c.X.as<double2>(), x->w.as<double>()));
-        if (with_projector)
-            for (int64_t k = 0; k < Nk; ++k)
-                FORGE_TRY(project_k_c3(x, k, c.nLower - 1, &x->h_bph[k * 4], c.bulk.as<double2>()));
+        if (with_projector) FORGE_TRY(project_bulk(x, c.bulk.as<double2>()));
         x->have_solve = true;
         x->have_sort = false;
         x->bulk_is_fused = !with_projector;
@@ -416,10 +432,8 @@ int solve_device(forge_ctx* x, int* info, bool with_projector = true) {
         const int64_t nb = (ke - k0 < B) ? ke - k0 : B;
         FORGE_TRY(launch_assemble(c, c.V.as<double>(), c.P.as<double2>(), k0, nb, c.H.as<double2>()));
         FORGE_TRY(eig_batch_run(x, k0, nb, info));
-        if (with_projector)
-            for (int64_t k = k0; k < k0 + nb; ++k)
-                FORGE_TRY(project_k(x, k, c.nLower - 1, &x->h_bph[k * 4], c.bulk.as<double2>()));
     }
+    if (with_projector) FORGE_TRY(project_bulk(x, c.bulk.as<double2>()));
     x->have_solve = true;
     x->have_sort = false;
     x->bulk_is_fused = !with_projector;
@@ -460,8 +474,9 @@ int project_fused_once(forge_ctx* x) {
     FORGE_CUDA(cudaMemsetAsync(x->Pn.ptr, 0, 4 * NN * sizeof(double2), c.stream));
     if (x->tcerr.ptr) FORGE_CUDA(cudaMemsetAsync(x->tcerr.ptr, 0, sizeof(int), c.stream));
     const int64_t kb = x->k_begin, ke = (x->k_end > 0) ? x->k_end : Nk;
-    for (int64_t k = kb; k < ke; ++k)
-        FORGE_TRY(project_k_c3(x, k, c.nLower - 1 + fk[k], &x->h_bph[k * 4], x->Pn.as<double2>()));
+    std::vector<ProjItem> items;
+    for (int64_t k = kb; k < ke; ++k) add_projector(x, k, c.nLower - 1 + fk[k], &x->h_bph[k * 4], items);
+    FORGE_TRY(project_items(x, items, x->Pn.as<double2>()));
     // partially occupied states of local k points (complex weight zdeg in reference mode)
     std::vector<WinState> part;
     for (int64_t q = nocc - npart; q < nocc; ++q)
@@ -580,8 +595,7 @@ int project_valley_once(forge_ctx* x) {
     FORGE_TRY(x->Pn.ensure(4 * NN * sizeof(double2)));
     FORGE_CUDA(cudaMemsetAsync(x->Pn.ptr, 0, 4 * NN * sizeof(double2), c.stream));
     if (x->tcerr.ptr) FORGE_CUDA(cudaMemsetAsync(x->tcerr.ptr, 0, sizeof(int), c.stream));
-    for (int64_t k = 0; k < Nk; ++k)
-        FORGE_TRY(project_k(x, k, c.nLower - 1, &x->h_bph[k * 4], x->Pn.as<double2>()));
+    FORGE_TRY(project_bulk(x, x->Pn.as<double2>()));
     FORGE_TRY(valley_window(x, st));
     FORGE_CUDA(cudaMemsetAsync(c.bulk.ptr, 0, 4 * NN * sizeof(double2), c.stream));
     FORGE_TRY(scf_combine(c, x->Pn.as<double2>(), c.bulk.as<double2>()));
@@ -773,9 +787,7 @@ int ensure_bulk(forge_ctx* x) {
     FORGE_TRY(c.bulk.ensure(4 * (size_t)c.N * c.N * sizeof(double2)));
     FORGE_CUDA(cudaMemsetAsync(c.bulk.ptr, 0, 4 * (size_t)c.N * c.N * sizeof(double2), c.stream));
     if (x->tcerr.ptr) FORGE_CUDA(cudaMemsetAsync(x->tcerr.ptr, 0, sizeof(int), c.stream));
-    const int64_t kb = x->k_begin, ke = (x->k_end > 0) ? x->k_end : c.Nk;
-    for (int64_t k = kb; k < ke; ++k)
-        FORGE_TRY(project_k_c3(x, k, c.nLower - 1, &x->h_bph[k * 4], c.bulk.as<double2>()));
+    FORGE_TRY(project_bulk(x, c.bulk.as<double2>()));
     x->bulk_is_fused = false;
     return 0;
 }

@@ -33,7 +33,12 @@ struct EigArgs {
     unsigned char* pivs;        // n x (scr_stride * batch)
     int64_t scr_stride;         // >= iu
     int* fail;                  // batch
-    double2 *G, *T, *Wb, *W2b;  // back-transform: NB x NB, NB x NB, NB x iu, NB x iu per batch
+    // FP64 products on the tensor cores (oz_fp64.cu): slices of X (and U, Z of the rank-2k update), V, V^H, W
+    // and T; W and W2, the Gram matrices and T in FP64; row scales; error flag of the bounded waits
+    void *oz_xs, *oz_vr, *oz_vh, *oz_ws, *oz_ts;
+    double2 *oz_wp, *oz_g, *oz_t;
+    int* oz_ex;
+    int* oz_err;
     float2* tf;                 // batch x n: T scaled to |T| <= 1, (d_i, e_{i-1}^2) in FP32 (FP32 bisection)
     double2* de;                // the same in FP64
     float* tq;                  // batch x 2n: unscaled T in FP32, d and e^2 (mixed precision)
@@ -50,8 +55,14 @@ void eig_bind_workspace(EigArgs& g, void* base);
 
 int eig_fp64(cudaStream_t st, EigArgs& g);
 int tridiag_eigvecs(cudaStream_t st, EigArgs& g);
-int backtransform_fp64(cudaStream_t st, const double2* A, int64_t lda, int64_t strideA, const double2* tau, int64_t n,
-                       double2* X, int64_t ldx, int64_t strideX, int64_t iu, int64_t batch, double2* Gws,
-                       double2* Tws, double2* Wws, double2* W2ws);
+
+// workspace of the FP64 products (elements of each array)
+struct OzSizes {
+    int64_t NB, nblk, mb, ks, ldx;        // block width, blocks, blocks per chunk, K splits of V^H X, slice pitch
+    int64_t xs, vr, vh, uz, wp, ws, g, ts, ex;
+};
+void oz_sizes(int64_t n, int64_t iu, int64_t batch, OzSizes& z);
+int her2k_oz(cudaStream_t st, TrdArgs<double>& a, int64_t p, int64_t w, int64_t batch, void* user);
+int backtransform_oz(cudaStream_t st, EigArgs& g);
 
 }  // namespace forge

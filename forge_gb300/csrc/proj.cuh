@@ -12,8 +12,14 @@ struct WinState {
     double2 wph[4];
 };
 
-int bulk_projector_fp64(cudaStream_t st, const double2* X, int64_t ldx, int64_t N, int64_t K, const double2 ph[4],
-                        double2* P);
+// One projector of a batch: the first K columns at X's slot, weighted by ph in the four cells.
+struct ProjItem {
+    int64_t slot, K;
+    double2 ph[4];
+};
+size_t proj_oz_workspace_bytes(int64_t n, int64_t iu, int64_t nit);
+int projectors_oz(cudaStream_t st, const double2* X, int64_t ldx, int64_t strideX, int64_t n, int64_t iu,
+                  const ProjItem* items, int64_t nit, double2* P, void* ws, int* err);
 int window_projector_fp64(cudaStream_t st, const WinState* states, int64_t nstates, const double2* X, int64_t ldx,
                           int64_t strideX, int64_t N, double2* P);
 size_t proj_tc_workspace_floats(int64_t n, int64_t iu);

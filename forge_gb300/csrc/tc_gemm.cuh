@@ -71,6 +71,9 @@ __host__ __device__ inline TcKMap tc_kmap_plain(int64_t K) {
 
 // Builds the 3D TMA descriptor {K, rows, planes} with a 32 x box_rows box and 128B swizzle.
 int tc_make_tmap(CUtensorMap* map, const TcOperand& op, int64_t batch, int box_rows);
+// The same for bf16 planes {cols, rows, planes} with a box_cols x box_rows box.
+int tc_make_tmap_bf16(CUtensorMap* map, const void* ptr, int64_t cols, int64_t rows, int64_t planes, int64_t ld,
+                      int64_t plane, int box_cols, int box_rows);
 
 __device__ inline uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

@@ -10,8 +10,8 @@
 //   k_invit     : one thread per cluster: LU of T - lambda I with partial pivoting
 //                 (dlagtf), perturbed back-substitution (dlagts, job=-1), modified
 //                 Gram-Schmidt against the earlier members of the cluster;
-//   back-transform: Q applied in compact-WY blocks (zlarft forward/columnwise), two
-//                 GEMMs per block on the chosen engine.
+//   back-transform: Q applied in compact-WY blocks (zlarft forward/columnwise) on the tensor
+//                 cores (oz_fp64.cu; eig_mixed.cu for the mixed path).
 // ortol is tighter than zstein's 1e-3*||T||_1 (which groups a whole dense spectrum
 // into one serial cluster); with ortol = 1e-7*||T||_1 the vector error bound
 // eps*||T||/gap stays below 1e-8 outside clusters.
@@ -19,7 +19,6 @@
 #include <cfloat>
 #include "cvec.cuh"
 #include "eig.cuh"
-#include "zgemm_engine.cuh"
 
 namespace forge {
 
@@ -792,165 +791,6 @@ __global__ void k_z_to_x(const double* __restrict__ Z, int64_t n, int64_t iu, do
     }
 }
 
-// ---------------------------------------------------------------- back-transformation (FP64)
-// Compact-WY blocks of BT64 reflectors; the two long-K products (the Gram matrix V^H V and
-// W = V^H X) are split over K so that their few output tiles still fill the GPU.
-constexpr int BT64 = 64;
-constexpr int64_t BT64_CTA_TARGET = 2 * 152;
-
-// upper bounds of the K splits (they size the workspace): enough CTAs for the GPU, no split
-// shorter than 256 rows
-inline void bt64_split_caps(int64_t n, int64_t iu, int64_t batch, int64_t& ksg, int64_t& ksw) {
-    const int64_t kmax = std::max<int64_t>(1, (n + 255) / 256);
-    ksg = std::min<int64_t>(std::min<int64_t>(32, (BT64_CTA_TARGET + batch - 1) / batch), kmax);
-    const int64_t wt = (iu + ZG_BN - 1) / ZG_BN * batch;
-    ksw = std::min<int64_t>(std::min<int64_t>(16, (BT64_CTA_TARGET + wt - 1) / wt), kmax);
-}
-
-struct BtV {  // V(r, l) of block j0: reflector j0+l, rows >= j0+1 (r relative to j0+1)
-    const double2* A;
-    int64_t lda, strideA, n, j0, nbk;
-    __device__ double2 at(int64_t rr, int64_t l) const {
-        const int64_t r = j0 + 1 + rr, j = j0 + l;
-        if (l >= nbk || r >= n || r < j + 1) return make_double2(0.0, 0.0);
-        if (r == j + 1) return make_double2(1.0, 0.0);
-        return A[blockIdx.z * strideA + r + j * lda];
-    }
-};
-struct BtGramA {  // a(l, k) = conj(V(k, l))
-    BtV v;
-    __device__ double2 operator()(int64_t l, int64_t k) const { return cconj(v.at(k, l)); }
-};
-struct BtGramB {  // b(i, k) = V(k, i)
-    BtV v;
-    __device__ double2 operator()(int64_t i, int64_t k) const { return v.at(k, i); }
-};
-struct BtStoreSmall {  // G(l, i) or W(l, c) stored column-major with leading dim ld
-    double2* G;
-    int64_t ld, stride;
-    __device__ void operator()(int64_t i, int64_t j, double2 c) const { G[blockIdx.z * stride + i + j * ld] = c; }
-};
-struct BtXk {  // b(c, k) = X(j0+1+k, c)
-    const double2* X;
-    int64_t ldx, strideX, n, j0, iu;
-    __device__ double2 operator()(int64_t c, int64_t k) const {
-        const int64_t r = j0 + 1 + k;
-        if (c >= iu || r >= n) return make_double2(0.0, 0.0);
-        return X[blockIdx.z * strideX + r + c * ldx];
-    }
-};
-struct BtTW_A {  // a(l, q) = T(l, q) upper triangular, BT64 x BT64 column-major
-    const double2* T;
-    int64_t nbk, stride;
-    __device__ double2 operator()(int64_t l, int64_t q) const {
-        if (l >= nbk || q >= nbk || q < l) return make_double2(0.0, 0.0);
-        return T[blockIdx.z * stride + l + q * BT64];
-    }
-};
-struct BtTW_B {  // b(c, q) = W(q, c), W column-major with leading dimension BT64
-    const double2* W;
-    int64_t nbk, iu, stride;
-    __device__ double2 operator()(int64_t c, int64_t q) const {
-        if (q >= nbk || c >= iu) return make_double2(0.0, 0.0);
-        return W[blockIdx.z * stride + q + c * BT64];
-    }
-};
-struct BtTW_Bsum {  // b(c, q) = W(q, c) summed over ks K-split partials (partial s at (s * batch + b))
-    const double2* W;
-    int64_t nbk, iu, ks, batch;
-    __device__ double2 operator()(int64_t c, int64_t q) const {
-        if (q >= nbk || c >= iu) return make_double2(0.0, 0.0);
-        const double2* p = W + blockIdx.z * BT64 * iu + q + c * BT64;
-        double2 acc = p[0];
-        for (int64_t s = 1; s < ks; ++s) acc = cadd(acc, p[s * batch * BT64 * iu]);
-        return acc;
-    }
-};
-struct BtStoreSplit {  // partial s of batch item b at P + (s * batch + b) * stride, leading dimension BT64
-    double2* P;
-    int64_t stride, batch;
-    __device__ void operator()(int64_t s, int64_t i, int64_t j, double2 c) const {
-        P[(s * batch + blockIdx.z) * stride + i + j * BT64] = c;
-    }
-};
-struct BtVa {  // a(rr, l) = V(rr, l)
-    BtV v;
-    __device__ double2 operator()(int64_t rr, int64_t l) const { return v.at(rr, l); }
-};
-struct BtXUpd {
-    double2* X;
-    int64_t ldx, strideX, j0;
-    __device__ void operator()(int64_t rr, int64_t c, double2 val) const {
-        double2* x = X + blockIdx.z * strideX + (j0 + 1 + rr) + c * ldx;
-        *x = csub(*x, val);
-    }
-};
-
-// zlarft (forward, columnwise) from the Gram matrix G = V^H V given as ks K-split partials
-// (partial s of batch item b at G + (s * batch + b) BT64^2):
-// T(0:i, i) = T(0:i, 0:i) (-tau_i G(0:i, i)), T(i, i) = tau_i.  blockDim.x = BT64, thread l owns row l.
-__global__ void k_larft(const double2* __restrict__ G, int64_t ks, int64_t batch, const double2* __restrict__ tau,
-                        int64_t n, int64_t j0, int64_t nbk, double2* __restrict__ T) {
-    const int64_t b = blockIdx.x;
-    double2* Tb = T + b * BT64 * BT64;
-    const double2* tb = tau + b * n;
-    __shared__ double2 tmp[BT64];
-    const int l = threadIdx.x;
-    for (int q = l; q < BT64 * BT64; q += blockDim.x) Tb[q] = make_double2(0.0, 0.0);
-    __syncthreads();
-    for (int64_t i = 0; i < nbk; ++i) {
-        const double2 ti = tb[j0 + i];
-        if (l < i) {
-            double2 g = make_double2(0.0, 0.0);
-            for (int64_t s = 0; s < ks; ++s) g = cadd(g, G[(s * batch + b) * BT64 * BT64 + l + i * BT64]);
-            tmp[l] = cmul(cmake(-ti.x, -ti.y), g);
-        }
-        __syncthreads();
-        if (l < i) {
-            double2 acc = make_double2(0.0, 0.0);
-            for (int64_t q = l; q < i; ++q) acc = cadd(acc, cmul(Tb[l + q * BT64], tmp[q]));
-            Tb[l + i * BT64] = acc;
-        }
-        if (l == 0) Tb[i + i * BT64] = ti;
-        __syncthreads();
-    }
-}
-
-int backtransform_fp64(cudaStream_t st, const double2* A, int64_t lda, int64_t strideA, const double2* tau, int64_t n,
-                       double2* X, int64_t ldx, int64_t strideX, int64_t iu, int64_t batch, double2* Gws,
-                       double2* Tws, double2* Wws, double2* W2ws) {
-    const int64_t nrefl = n - 1;
-    const int64_t nblocks = (nrefl + BT64 - 1) / BT64;
-    int64_t ksg_cap, ksw_cap;
-    bt64_split_caps(n, iu, batch, ksg_cap, ksw_cap);
-    for (int64_t blk = nblocks - 1; blk >= 0; --blk) {
-        const int64_t j0 = blk * BT64;
-        const int64_t nbk = (nrefl - j0 < BT64) ? (nrefl - j0) : BT64;
-        const int64_t K = n - j0 - 1;
-        BtV v{A, lda, strideA, n, j0, nbk};
-        // G = V^H V (nbk x nbk), split over K
-        const int64_t ksg = zg_ksplit_count(K, std::min<int64_t>(ksg_cap, (K + 255) / 256));
-        FORGE_TRY((zgemm_launch_splitk<double2, KMAJOR, KMAJOR>(st, nbk, nbk, K, batch, ksg, BtGramA{v},
-                                                                BtGramB{v}, BtStoreSplit{Gws, BT64 * BT64, batch})));
-        k_larft<<<(unsigned)batch, BT64, 0, st>>>(Gws, ksg, batch, tau, n, j0, nbk, Tws);
-        FORGE_LAUNCH_CHECK();
-        // W = V^H X (nbk x iu), split over K
-        const int64_t ksw = zg_ksplit_count(K, std::min<int64_t>(ksw_cap, (K + 255) / 256));
-        FORGE_TRY((zgemm_launch_splitk<double2, KMAJOR, KMAJOR>(st, nbk, iu, K, batch, ksw, BtGramA{v},
-                                                                BtXk{X, ldx, strideX, n, j0, iu},
-                                                                BtStoreSplit{Wws, BT64 * iu, batch})));
-        // W2 = T W
-        FORGE_TRY((zgemm_launch<double2, KMAJOR, KMAJOR, false>(
-            st, nbk, iu, nbk, batch, BtTW_A{Tws, nbk, BT64 * BT64}, BtTW_Bsum{Wws, nbk, iu, ksw, batch},
-            BtStoreSmall{W2ws, BT64, BT64 * iu})));
-        // X(j0+1:, :) -= V W2
-        FORGE_TRY((zgemm_launch<double2, IMAJOR, KMAJOR, false>(st, K, iu, nbk, batch, BtVa{v},
-                                                                 BtTW_B{W2ws, nbk, iu, BT64 * iu},
-                                                                 BtXUpd{X, ldx, strideX, j0})));
-    }
-    return 0;
-}
-
 // ---------------------------------------------------------------- FP64 eigen-solver driver
 int eig_fp64(cudaStream_t st, EigArgs& g) {
     const int64_t n = g.n, iu = g.iu, batch = g.batch;
@@ -972,6 +812,9 @@ int eig_fp64(cudaStream_t st, EigArgs& g) {
     a.pstride = g.pstride;
     a.scal = g.scal;
     a.cnt = g.cnt;
+    a.her2k = her2k_oz;
+    a.her2k_user = &g;
+    FORGE_CUDA(cudaMemsetAsync(g.oz_err, 0, sizeof(int), st));
     FORGE_CUDA(cudaMemsetAsync(g.cnt, 0, sizeof(unsigned) * 4 * batch, st));
     FORGE_TRY(tridiagonalize<double>(st, a, batch));
     FORGE_TRY(tridiag_eigvecs(st, g));
@@ -979,10 +822,16 @@ int eig_fp64(cudaStream_t st, EigArgs& g) {
     k_z_to_x<<<gz, dim3(32, 8), 0, st>>>(g.Z, n, iu, g.X, g.ldx, g.strideX);
     FORGE_LAUNCH_CHECK();
     prof_begin(ST_BACKTRANSFORM);
-    FORGE_TRY(backtransform_fp64(st, g.A, g.lda, g.strideA, g.tau, n, g.X, g.ldx, g.strideX, iu, batch, g.G, g.T,
-                                 g.Wb, g.W2b));
+    FORGE_TRY(backtransform_oz(st, g));
     prof_end(ST_BACKTRANSFORM, batch * (double)n * iu * 16.0 * 2.0 + batch * 0.5 * n * (double)n * 16.0,
              batch * 8.0 * (double)n * n * iu);
+    int herr = 0;
+    FORGE_CUDA(cudaMemcpyAsync(&herr, g.oz_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    FORGE_CUDA(cudaStreamSynchronize(st));
+    if (herr) {
+        set_error(FORGE_ERR_TIMEOUT, "tcgen05 GEMM (FP64 slices): a bounded mbarrier wait gave up");
+        return FORGE_ERR_TIMEOUT;
+    }
     return 0;
 }
 
@@ -1080,16 +929,24 @@ void carve(EigArgs& g, Carve& c) {
     g.cnt = c.take<unsigned>(B * 4);
     g.info = c.take<double>(B * 8);
     g.clus = c.take<int>(B * (iu + 2));
-    g.Z = c.take<double>(B * n * iu);
-    g.scr = c.take<double>(4 * n * iu * B);
+    OzSizes z;
+    oz_sizes(n, iu, B, z);
+    // the slices of X (and of the rank-2k update) share the scratch of the inverse iteration, those of V its
+    // vectors: both are free before it, and again once Z has been copied to X
+    g.Z = (double*)c.take<char>(std::max<size_t>(sizeof(double) * B * n * iu, 2 * z.vr));
+    g.oz_vr = g.Z;
+    g.scr = (double*)c.take<char>(std::max<size_t>(sizeof(double) * 4 * n * iu * B, 2 * std::max(z.xs, z.uz)));
+    g.oz_xs = g.scr;
     g.pivs = c.take<unsigned char>(n * iu * B);
     g.fail = c.take<int>(B);
-    int64_t ksg, ksw;
-    bt64_split_caps(n, iu, B, ksg, ksw);
-    g.G = c.take<double2>(ksg * B * BT64 * BT64);
-    g.T = c.take<double2>(B * BT64 * BT64);
-    g.Wb = c.take<double2>(ksw * B * BT64 * iu);
-    g.W2b = c.take<double2>(B * BT64 * iu);
+    g.oz_vh = c.take<char>(2 * z.vh);
+    g.oz_ws = c.take<char>(2 * z.ws);
+    g.oz_ts = c.take<char>(2 * z.ts);
+    g.oz_wp = c.take<double2>(z.wp);
+    g.oz_g = c.take<double2>(z.g);
+    g.oz_t = c.take<double2>(z.g);
+    g.oz_ex = c.take<int>(z.ex);
+    g.oz_err = c.take<int>(1);
     g.tf = c.take<float2>(B * n);
     g.de = c.take<double2>(B * n);
     g.tq = c.take<float>(B * 2 * n);

@@ -3,7 +3,6 @@
 // Bytes per column step (algorithmic): the trailing lower triangle, (n-col)^2/2
 // complex elements, read once by trd_hemv; the rank-2k update is GEMM-shaped.
 #include "tridiag.cuh"
-#include "zgemm_engine.cuh"
 
 namespace forge {
 
@@ -342,54 +341,6 @@ __global__ void __launch_bounds__(TRD_ROWS) k_trd_fix(TrdArgs<T> a, int ii, int6
     if (r < n) W[r + ii * n] = vadd(W[r + ii * n], vmul(al, A[r + col * lda]));
 }
 
-// ---------------------------------------------------------------- rank-2k trailing update
-template <class V>
-struct Her2kA {
-    const V* A;
-    const V* W;
-    int64_t lda, strideA, n, strideW, r0, p, w;
-    __device__ V operator()(int64_t i, int64_t k) const {
-        const int64_t r = r0 + i, b = blockIdx.z;
-        if (r >= n || k >= 2 * w) return vzero<V>();
-        if (k < w) return A[b * strideA + r + (p + k) * lda];
-        return W[b * strideW + r + (k - w) * n];
-    }
-};
-template <class V>
-struct Her2kB {
-    const V* A;
-    const V* W;
-    int64_t lda, strideA, n, strideW, r0, p, w;
-    __device__ V operator()(int64_t j, int64_t k) const {
-        const int64_t r = r0 + j, b = blockIdx.z;
-        if (r >= n || k >= 2 * w) return vzero<V>();
-        if (k < w) return vconj(W[b * strideW + r + k * n]);
-        return vconj(A[b * strideA + r + (p + k - w) * lda]);
-    }
-};
-template <class V>
-struct Her2kEpi {
-    V* A;
-    int64_t lda, strideA, r0;
-    __device__ void operator()(int64_t i, int64_t j, V c) const {
-        V* x = A + blockIdx.z * strideA + (r0 + i) + (r0 + j) * lda;
-        V y = vsub(*x, c);
-        if (i == j) y.y = 0;
-        *x = y;
-    }
-};
-
-template <class T>
-int her2k_update(cudaStream_t st, TrdArgs<T>& a, int64_t p, int64_t w, int64_t batch) {
-    using V = typename CV<T>::type;
-    const int64_t r0 = p + w, m = a.n - r0;
-    if (m <= 0) return 0;
-    Her2kA<V> fa{a.A, a.W, a.lda, a.strideA, a.n, a.n * TRD_NB, r0, p, w};
-    Her2kB<V> fb{a.A, a.W, a.lda, a.strideA, a.n, a.n * TRD_NB, r0, p, w};
-    Her2kEpi<V> ep{a.A, a.lda, a.strideA, r0};
-    return zgemm_launch<V, IMAJOR, IMAJOR, true>(st, m, m, 2 * w, batch, fa, fb, ep);
-}
-
 // ---------------------------------------------------------------- driver
 template <class T>
 int tridiagonalize(cudaStream_t st, TrdArgs<T>& a, int64_t batch) {
@@ -430,10 +381,7 @@ int tridiagonalize(cudaStream_t st, TrdArgs<T>& a, int64_t batch) {
         if (nrefl > 0 && p + w < n) {
             const double m2 = (double)(n - p - w);
             prof_begin(ST_HER2K);
-            if (a.her2k)
-                FORGE_TRY(a.her2k(st, a, p, nrefl, batch, a.her2k_user));
-            else
-                FORGE_TRY(her2k_update<T>(st, a, p, nrefl, batch));
+            FORGE_TRY(a.her2k(st, a, p, nrefl, batch, a.her2k_user));
             prof_end(ST_HER2K, batch * m2 * m2 * (double)sizeof(typename CV<T>::type),
                      batch * 8.0 * m2 * m2 * (double)nrefl);  // lower half of 2*nrefl complex MACs
         }

@@ -13,7 +13,7 @@
 //   trd_finish: y -= V s1 + W s2, W(:,i) = tau y, v written back, alpha2 in the last CTA;
 //   trd_fix   : W(:,i) += alpha2 v.
 // After each panel of NB columns, the trailing matrix gets A22 -= V W^H + W V^H
-// (a rank-2k update on the GEMM engine of the chosen precision).
+// (a rank-2k update on the tensor cores in the chosen precision).
 #pragma once
 #include "cvec.cuh"
 #include "forge_internal.cuh"
@@ -44,7 +44,7 @@ struct TrdArgs {
     int64_t pstride;
     double* scal;       // batch x 16
     unsigned* cnt;      // batch x 4
-    // optional trailing-update override (the tensor-core rank-2k update of the mixed path):
+    // trailing update on the tensor cores (her2k_oz in FP64, her2k_tc in the mixed path):
     // A(p+w:n, p+w:n) -= V W^H + W V^H for the panel [p, p+w)
     int (*her2k)(cudaStream_t st, TrdArgs<T>& a, int64_t p, int64_t w, int64_t batch, void* user) = nullptr;
     void* her2k_user = nullptr;
