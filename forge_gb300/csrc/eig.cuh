@@ -18,6 +18,7 @@ struct EigArgs {
     double *d, *e;              // batch x n
     double2* tau;               // batch x n
     double2* Wp;                // batch x n x NB (panel W)
+    double2* w0;                // batch x n
     double2 *Yrow, *Ycol;       // batch x ystride
     int64_t ystride;
     double2* Spart;

@@ -610,7 +610,7 @@ int eig_mixed(cudaStream_t st, EigArgs& g, void* mixed_ws) {
     a.her2k = her2k_tc;
     a.her2k_user = &ws;
     FORGE_CUDA(cudaMemsetAsync(ws.cnt, 0, sizeof(unsigned) * 4 * batch, st));
-    FORGE_TRY(tridiagonalize<float>(st, a, batch));
+    FORGE_TRY(tridiagonalize_f32(st, a, batch));
     // eigenpairs of T in FP64
     EigArgs ge = g;
     ge.replay = 1;

@@ -812,11 +812,11 @@ int eig_fp64(cudaStream_t st, EigArgs& g) {
     a.pstride = g.pstride;
     a.scal = g.scal;
     a.cnt = g.cnt;
+    a.w0 = g.w0;
     a.her2k = her2k_oz;
     a.her2k_user = &g;
     FORGE_CUDA(cudaMemsetAsync(g.oz_err, 0, sizeof(int), st));
-    FORGE_CUDA(cudaMemsetAsync(g.cnt, 0, sizeof(unsigned) * 4 * batch, st));
-    FORGE_TRY(tridiagonalize<double>(st, a, batch));
+    FORGE_TRY(tridiagonalize_fp64(st, a, batch));
     FORGE_TRY(tridiag_eigvecs(st, g));
     dim3 gz((unsigned)((n + 31) / 32), (unsigned)((iu + 31) / 32), (unsigned)batch);
     k_z_to_x<<<gz, dim3(32, 8), 0, st>>>(g.Z, n, iu, g.X, g.ldx, g.strideX);
@@ -912,15 +912,16 @@ struct Carve {
 void carve(EigArgs& g, Carve& c) {
     const int64_t n = g.n, iu = g.iu, B = g.batch;
     const int64_t nblk = (n + TRD_TILE - 1) / TRD_TILE;
-    const int64_t nrb = (n + 255) / 256;
+    const int64_t nrb = (n + 127) / 128;   // slots of the panel dots
     g.ystride = nblk * n;
     g.sstride = nrb * 2 * TRD_NB;
-    g.pstride = 2 * ((n + 31) / 32) + 2;  // per-CTA partials of trd_col / trd_finish
+    g.pstride = 3 * ((n + 31) / 32) + 1;  // per-CTA partials of k_col64 and k_finish64
     g.scr_stride = iu;
     g.d = c.take<double>(B * n);
     g.e = c.take<double>(B * n);
     g.tau = c.take<double2>(B * n);
     g.Wp = c.take<double2>(B * n * TRD_NB);
+    g.w0 = c.take<double2>(B * n);
     g.Yrow = c.take<double2>(B * g.ystride);
     g.Ycol = c.take<double2>(B * g.ystride);
     g.Spart = c.take<double2>(B * g.sstride);

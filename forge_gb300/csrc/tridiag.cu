@@ -342,8 +342,8 @@ __global__ void __launch_bounds__(TRD_ROWS) k_trd_fix(TrdArgs<T> a, int ii, int6
 }
 
 // ---------------------------------------------------------------- driver
-template <class T>
-int tridiagonalize(cudaStream_t st, TrdArgs<T>& a, int64_t batch) {
+int tridiagonalize_f32(cudaStream_t st, TrdArgs<float>& a, int64_t batch) {
+    using T = float;
     const int64_t n = a.n;
     for (int64_t p = 0; p < n; p += TRD_NB) {
         const int64_t w = (n - p < TRD_NB) ? (n - p) : TRD_NB;
@@ -388,8 +388,5 @@ int tridiagonalize(cudaStream_t st, TrdArgs<T>& a, int64_t batch) {
     }
     return 0;
 }
-
-template int tridiagonalize<double>(cudaStream_t, TrdArgs<double>&, int64_t);
-template int tridiagonalize<float>(cudaStream_t, TrdArgs<float>&, int64_t);
 
 }  // namespace forge

@@ -44,13 +44,14 @@ struct TrdArgs {
     int64_t pstride;
     double* scal;       // batch x 16
     unsigned* cnt;      // batch x 4
+    V* w0 = nullptr;    // batch x n: the last column's w before the alpha2 correction (FP64)
     // trailing update on the tensor cores (her2k_oz in FP64, her2k_tc in the mixed path):
     // A(p+w:n, p+w:n) -= V W^H + W V^H for the panel [p, p+w)
     int (*her2k)(cudaStream_t st, TrdArgs<T>& a, int64_t p, int64_t w, int64_t batch, void* user) = nullptr;
     void* her2k_user = nullptr;
 };
 
-template <class T>
-int tridiagonalize(cudaStream_t st, TrdArgs<T>& a, int64_t batch);
+int tridiagonalize_f32(cudaStream_t st, TrdArgs<float>& a, int64_t batch);     // tridiag.cu
+int tridiagonalize_fp64(cudaStream_t st, TrdArgs<double>& a, int64_t batch);   // tridiag_fp64.cu
 
 }  // namespace forge
