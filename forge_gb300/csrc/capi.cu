@@ -79,7 +79,7 @@ int rr_window(cudaStream_t st, const double2* H, int64_t strideH, double2* X, in
               int64_t iu, int64_t n, int64_t c0, int64_t nw, int64_t batch, void* ws);
 size_t rr_window_workspace_bytes(int64_t n, int64_t batch);
 const float* eig_mixed_planes(void* mixed_ws, int64_t n, int64_t iu, int64_t batch, int64_t* n4);
-size_t oa_workspace_bytes(int64_t n, int64_t iu);
+size_t oa_workspace_bytes(int64_t n, int64_t iu, int64_t batch);
 int launch_pad_slot(cudaStream_t st, const double2* src, int64_t nb, double2* dst, int64_t n, double* rowsum,
                     double* sigma);
 int oa_refine(cudaStream_t st, double2* H, int64_t strideH, const float* Xs, int64_t n4, int64_t nall,
@@ -172,7 +172,7 @@ int choose_batch(forge_ctx* x) {
     // cells) is allocated at the first mixing step, after this choice
     const size_t diis = x->mix_mode == FORGE_MIX_PULAY ? ((size_t)(2 * (x->diis_depth + 1) + 1) * 4 * N * N * 8) : 0;
     const size_t reserve = ((size_t)8 << 30) + (size_t)xslots * N * iu * 16 + (size_t)10 * N * N * 16 +
-                           (oa ? oa_workspace_bytes(N, iu) : 0) + diis;
+                           (oa ? oa_workspace_bytes(N, iu, c.Nk) : 0) + diis;
     const size_t budget = freeb > reserve ? freeb - reserve : freeb / 4;
     int64_t b = (int64_t)(budget / per_k);
     // FORGE_EIG_BATCH caps the number of k points solved per launch (memory control)
@@ -210,7 +210,7 @@ int ensure_solve_buffers(forge_ctx* x) {
     if (c.precision == FORGE_PREC_MIXED) FORGE_TRY(x->mixws.ensure(eig_mixed_workspace_bytes(N, iu_solve, B)));
     if (oa) {
         FORGE_TRY(x->w_all.ensure((size_t)B * N * sizeof(double)));
-        FORGE_TRY(x->oaws.ensure(oa_workspace_bytes(N, iu)));
+        FORGE_TRY(x->oaws.ensure(oa_workspace_bytes(N, iu, B)));
         FORGE_TRY(x->tcerr.ensure(sizeof(int)));
     }
     FORGE_TRY(c.bulk.ensure(4 * NN * sizeof(double2)));
@@ -328,21 +328,16 @@ int project_items(forge_ctx* x, const std::vector<ProjItem>& items, double2* out
         FORGE_TRY(x->tcerr.ensure(sizeof(int)));
         FORGE_CUDA(cudaMemsetAsync(x->tcerr.ptr, 0, sizeof(int), c.stream));
     }
-    if (c.precision != FORGE_PREC_MIXED) {
-        FORGE_TRY(x->projws.ensure(proj_oz_workspace_bytes(N, iu, nit)));
+    const bool refined = c.precision == FORGE_PREC_MIXED && x->oa_active;
+    if (c.precision != FORGE_PREC_MIXED || refined) {
+        FORGE_TRY(x->projws.ensure(proj_oz_workspace_bytes(N, iu, nit, refined)));
         return projectors_oz(c.stream, c.X.as<double2>(), N, N * iu, N, iu, items.data(), nit, out, x->projws.ptr,
-                             x->tcerr.as<int>());
+                             x->tcerr.as<int>(), refined);
     }
     for (const ProjItem& p : items) {
         const double2* Xk = c.X.as<double2>() + (size_t)p.slot * N * iu;
-        if (x->oa_active) {
-            // refined eigenvectors: the projector keeps their FP64 accuracy (exact sliced products)
-            FORGE_TRY(x->projws.ensure(proj_tc_exact_workspace_bytes(N, iu)));
-            FORGE_TRY(bulk_projector_tc_exact(c.stream, Xk, N, N, p.K, iu, p.ph, out, x->projws.ptr, x->tcerr.as<int>()));
-        } else {
-            FORGE_TRY(x->projws.ensure(proj_tc_workspace_floats(N, iu) * sizeof(float)));
-            FORGE_TRY(bulk_projector_tc(c.stream, Xk, N, N, p.K, iu, p.ph, out, x->projws.as<float>(), x->tcerr.as<int>()));
-        }
+        FORGE_TRY(x->projws.ensure(proj_tc_workspace_floats(N, iu) * sizeof(float)));
+        FORGE_TRY(bulk_projector_tc(c.stream, Xk, N, N, p.K, iu, p.ph, out, x->projws.as<float>(), x->tcerr.as<int>()));
     }
     return 0;
 }
@@ -1591,7 +1586,7 @@ int forge_gpu_zheevr_batch(forge_ctx* x, int64_t nb, const double* A, int64_t iu
         (rc = dw.ensure(nb * iu * sizeof(double))) || (rc = ws.ensure(eig_workspace_bytes(N, iu_solve, nb))))
         return rc;
     if (c.precision == FORGE_PREC_MIXED && (rc = mws.ensure(eig_mixed_workspace_bytes(N, iu_solve, nb)))) return rc;
-    if (oa && ((rc = wall.ensure(nb * N * sizeof(double))) || (rc = ows.ensure(oa_workspace_bytes(N, iu))) ||
+    if (oa && ((rc = wall.ensure(nb * N * sizeof(double))) || (rc = ows.ensure(oa_workspace_bytes(N, iu, nb))) ||
                (rc = oerr.ensure(sizeof(int)))))
         return rc;
     FORGE_CUDA(cudaMemcpyAsync(dA.ptr, A, nb * NN * sizeof(double2), cudaMemcpyHostToDevice, c.stream));
@@ -1652,6 +1647,7 @@ int forge_gpu_zheevr_batch(forge_ctx* x, int64_t nb, const double* A, int64_t iu
     wall.release();
     ows.release();
     oerr.release();
+    rws.release();
     if (rc) return rc;
     int bad = 0;
     for (int64_t b = 0; b < nb; ++b) bad += fails[b] ? 1 : 0;

@@ -19,17 +19,18 @@
 // mixing (both occupied: no effect on the density matrix; around the Fermi level the FP64
 // window Rayleigh-Ritz that follows resolves them).
 //
-// The residual product H X runs as real GEMMs over integer slices (Ozaki et al., Numer.
-// Algorithms 59 (2012)): every row of H and column of X is scaled by a power of two to |v| < 1
-// and cut into slices v = sum_s v_s 2^-(8 + 9 s) with integer |v_s| <= 256; slice products with
-// s + t <= depth are summed by the exact-block mode of the tcgen05 GEMM (integer blocks of 256
-// products, double-float accumulation), which keeps ~2^-(16 + 9 (depth + 1)) of |H||X|.
+// The residual product H X runs on the bf16 tensor cores as exact integer slices (oz_gemm.cuh) of five slices
+// per operand; the blocks of the slice products with s + t <= depth are summed in double-float, which keeps
+// ~2^-(16 + 9 (depth + 1)) of |H||X|.  The matrices of a batch are refined together (one matrix of N = 364 has
+// nine tiles).  Measured per refinement (TF32 slices, one matrix at a time before; residual product / the
+// rest, ms): N = 364, 36 k 18.7 / 12.7 -> 0.5 / 1.1; N = 1324, 16 k 23.1 / 17.1 -> 5.3 / 7.2; N = 5044
+// 49.8 / 21.3 -> 13.7 / 18.0.
 #include <algorithm>
 #include <cmath>
-#include <vector>
 
 #include "cvec.cuh"
 #include "forge_internal.cuh"
+#include "oz_gemm.cuh"
 #include "tc_gemm.cuh"
 
 namespace forge {
@@ -49,9 +50,10 @@ __device__ inline float tf32_rna(float x) {
 
 // Fills the strict upper triangle of every H(k) with the conjugate of its lower triangle.
 // 32 x 32 tiles (tr, tc), tc >= tr; reads and writes are coalesced along rows.
-__global__ void k_herm_fill(double2* __restrict__ H, int64_t n) {
+__global__ void k_herm_fill(double2* __restrict__ H, int64_t strideH, int64_t n) {
     const int64_t tr = blockIdx.y, tc = blockIdx.x;
     if (tc < tr) return;
+    H += blockIdx.z * strideH;
     __shared__ double2 t[32][33];
     for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
         const int64_t r = tc * 32 + threadIdx.x, c = tr * 32 + yy;   // source (lower): row r, column c
@@ -67,80 +69,54 @@ __global__ void k_herm_fill(double2* __restrict__ H, int64_t n) {
     }
 }
 
-// Slices of one column per CTA.  mode 0 (H -> rows of the A operand): column i of the full
-// Hermitian H is conj(row i), so planes 0..S-1 hold the slices of Re H(i, k) = Re H(k, i) and
-// planes S..2S-1 those of Im H(i, k) = -Im H(k, i).  mode 1 (X -> rows of the B operand):
-// planes Re (0..S-1), Im (S..2S-1), -Im (2S..3S-1).  Plane p of the output:
-// out + p * pstride + col * pitch + row; the column's power-of-two scale goes to expo[col].
-__global__ void __launch_bounds__(256) k_oa_slice(const double2* __restrict__ src, int64_t ld, int64_t nrows,
-                                                  int mode, float* __restrict__ out, int64_t pitch, int64_t pstride,
-                                                  int* __restrict__ expo) {
-    const int64_t col = blockIdx.x;
-    const double2* s = src + col * ld;
-    double m = 0.0;
-    for (int64_t r = threadIdx.x; r < nrows; r += blockDim.x) m = fmax(m, fmax(fabs(s[r].x), fabs(s[r].y)));
-    __shared__ double red[8];
-    m = warp_max_d(m);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double t = threadIdx.x < 8 ? red[threadIdx.x] : 0.0;
-        t = warp_max_d(t);
-        if (threadIdx.x == 0) red[0] = t;
+// Rows of the operands of H X: row i of H is the conjugate of its (filled) column i; row j of X^T is column j.
+struct LdOaH {
+    const double2* H;
+    int64_t n, strideH;
+    __device__ double2 operator()(int64_t b, int64_t i, int64_t k) const {
+        const double2 h = H[b * strideH + i * n + k];
+        return make_double2(h.x, -h.y);
     }
-    __syncthreads();
-    int e = 0;
-    if (red[0] > 0.0) frexp(red[0], &e);   // red[0] < 2^e
-    if (threadIdx.x == 0) expo[col] = e;
-    constexpr int S = OA_SLICES;
-    for (int64_t r = threadIdx.x; r < nrows; r += blockDim.x) {
-        double a[2] = {ldexp(s[r].x, -e), ldexp(s[r].y, -e)};   // |a| < 1, exact
-        if (mode == 0) a[1] = -a[1];                            // row i of H = conj(column i)
-        for (int part = 0; part < 2; ++part) {
-            double t = a[part] * 256.0;
-            for (int q = 0; q < S; ++q) {
-                const double v = rint(t);                        // |v| <= 256
-                t = (t - v) * 512.0;                             // exact: the remainder has <= 53 bits
-                const int64_t o = col * pitch + r;
-                const float fv = (float)v;
-                out[(part * S + q) * pstride + o] = fv;
-                if (mode == 1 && part == 1) out[(2 * S + q) * pstride + o] = -fv;
-            }
-        }
-    }
-}
+};
+struct LdOaX {
+    const double2* X;
+    int64_t ldx, strideX;
+    __device__ double2 operator()(int64_t b, int64_t j, int64_t k) const { return X[b * strideX + j * ldx + k]; }
+};
 
-// W = H X - X lam (one part per launch), written as TF32 hi/lo planes of the B operand of C:
-// plane 0 Re hi, 1 Re lo, 2 Im hi, 3 Im lo, 4 -Re hi, 5 -Re lo; element (k, j) at j * pitch + k.
+// W = H X - X lam, written as TF32 hi/lo planes of the B operand of C: plane 0 Re hi, 1 Re lo, 2 Im hi,
+// 3 Im lo, 4 -Re hi, 5 -Re lo of matrix b from plane 6 b on; element (k, j) at j * pitch + k.
 struct OaWEpi {
     const int *eA, *eB;
     const double2* X;
-    int64_t ldx;
+    int64_t ldx, strideX;
     const double* lam;
     float* Wp;
-    int64_t pitch, pstride;
-    int part;
-    __device__ void operator()(int64_t, int64_t row, int64_t col0, const double* v, int64_t M, int64_t N) const {
+    int64_t pitch, pstride, n, iu, nall;
+    __device__ void operator()(int64_t b, int part, int64_t row, int64_t col0, const double* v, int64_t M,
+                               int64_t N) const {
         if (row >= M) return;
-        const int ea = eA[row];
+        const int ea = eA[b * n + row];
+        float* W = Wp + b * 6 * pstride;
+        const double2* Xb = X + b * strideX;
 #pragma unroll
-        for (int q = 0; q < 32; ++q) {
+        for (int q = 0; q < 16; ++q) {
             const int64_t j = col0 + q;
             if (j >= N) continue;
-            const double y = ldexp(v[q], ea + eB[j]);
-            const double2 x = X[row + j * ldx];
-            const double w = y - (part ? x.y : x.x) * lam[j];
+            const double y = __dmul_rn(v[q], oz_pow2(ea + eB[b * iu + j]));   // exact
+            const double2 x = Xb[row + j * ldx];
+            const double w = fma(-(part ? x.y : x.x), lam[b * nall + j], y);
             const float hi = tf32_rna((float)w);
             const float lo = (float)(w - (double)hi);
             const int64_t o = j * pitch + row;
             if (part == 0) {
-                Wp[o] = hi;
-                Wp[pstride + o] = lo;
-                Wp[4 * pstride + o] = -hi;
-                Wp[5 * pstride + o] = -lo;
+                W[o] = hi;
+                W[pstride + o] = lo;
+                W[4 * pstride + o] = -hi;
+                W[5 * pstride + o] = -lo;
             } else {
-                Wp[2 * pstride + o] = hi;
-                Wp[3 * pstride + o] = lo;
+                W[2 * pstride + o] = hi;
+                W[3 * pstride + o] = lo;
             }
         }
     }
@@ -150,13 +126,15 @@ struct OaWEpi {
 // k_oa_cluster); TF32 hi/lo planes of the B operand of the update: 0 Re hi, 1 Re lo, 2 Im hi,
 // 3 Im lo, 4 -Im hi, 5 -Im lo; element (i, j) at j * pitch + i.
 struct OaCEpi {
-    const double* lam;
+    const double* lams;
     double delta;
-    float* Ep;
-    int64_t pitch, pstride;
+    float* Es;
+    int64_t pitch, pstride, nall;
     int part;
-    __device__ void operator()(int64_t, int64_t row, int64_t col0, const float* v, int64_t M, int64_t N) const {
+    __device__ void operator()(int64_t b, int64_t row, int64_t col0, const float* v, int64_t M, int64_t N) const {
         if (row >= M) return;
+        const double* lam = lams + b * nall;
+        float* Ep = Es + b * 6 * pstride;
         const double li = lam[row];
 #pragma unroll
         for (int q = 0; q < 32; ++q) {
@@ -183,15 +161,15 @@ struct OaCEpi {
 // X(r, j) += the update of one part
 struct OaUEpi {
     double2* X;
-    int64_t ldx;
+    int64_t ldx, strideX;
     int part;
-    __device__ void operator()(int64_t, int64_t row, int64_t col0, const float* v, int64_t M, int64_t N) const {
+    __device__ void operator()(int64_t b, int64_t row, int64_t col0, const float* v, int64_t M, int64_t N) const {
         if (row >= M) return;
 #pragma unroll
         for (int q = 0; q < 32; ++q) {
             const int64_t j = col0 + q;
             if (j >= N) continue;
-            double2* p = X + row + j * ldx;
+            double2* p = X + b * strideX + row + j * ldx;
             if (part == 0)
                 p->x += (double)v[q];
             else
@@ -211,6 +189,9 @@ __global__ void __launch_bounds__(256) k_oa_cluster(const float* __restrict__ Xs
                                                     float* __restrict__ Ep, int64_t pitch, int64_t pstride) {
     const int64_t j = blockIdx.x;
     const int64_t P = n4 * nall;
+    Xs += blockIdx.y * 4 * P;
+    lam += blockIdx.y * nall;
+    Ep += blockIdx.y * 6 * pstride;
     int64_t lo = j, hi = j;
     while (lo > 0 && j - lo < OA_CLUSTER_RADIUS && lam[j] - lam[lo - 1] <= delta) --lo;
     while (hi + 1 < nall && hi - j < OA_CLUSTER_RADIUS && lam[hi + 1] - lam[j] <= delta) ++hi;
@@ -243,8 +224,13 @@ __global__ void __launch_bounds__(256) k_oa_cluster(const float* __restrict__ Xs
 // lam_out(j) = lam(j) + Re(x_j^H w_j) in FP64 (x_j unit-normalised).  One CTA per column.
 __global__ void __launch_bounds__(256) k_oa_diag(const double2* __restrict__ X, int64_t ldx, int64_t n,
                                                  const float* __restrict__ Wp, int64_t pitch, int64_t pstride,
-                                                 const double* __restrict__ lam, double* __restrict__ lam_out) {
+                                                 const double* __restrict__ lam, double* __restrict__ lam_out,
+                                                 int64_t strideX, int64_t nall, int64_t w_stride) {
     const int64_t j = blockIdx.x;
+    X += blockIdx.y * strideX;
+    Wp += blockIdx.y * 6 * pstride;
+    lam += blockIdx.y * nall;
+    lam_out += blockIdx.y * w_stride;
     double s = 0.0;
     for (int64_t r = threadIdx.x; r < n; r += blockDim.x) {
         const int64_t o = j * pitch + r;
@@ -271,6 +257,8 @@ __global__ void k_oa_transpose(const float* __restrict__ Xs, int64_t n4, int64_t
     __shared__ float t[4][32][33];
     const int64_t i0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
     const int64_t P = n4 * nall, PT = n * pitchT;
+    Xs += blockIdx.z * 4 * P;
+    XT += blockIdx.z * 4 * PT;
     for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
         const int64_t i = i0 + yy, r = r0 + threadIdx.x;
 #pragma unroll
@@ -286,9 +274,9 @@ __global__ void k_oa_transpose(const float* __restrict__ Xs, int64_t n4, int64_t
     }
 }
 
-__global__ void k_normalize(double2* __restrict__ X, int64_t n, int64_t ldx) {
+__global__ void k_normalize(double2* __restrict__ X, int64_t n, int64_t ldx, int64_t strideX) {
     const int64_t c = blockIdx.x;
-    double2* x = X + c * ldx;
+    double2* x = X + blockIdx.y * strideX + c * ldx;
     double s = 0.0;
     for (int64_t r = threadIdx.x; r < n; r += blockDim.x) s += x[r].x * x[r].x + x[r].y * x[r].y;
     __shared__ double red[8];
@@ -306,41 +294,47 @@ __global__ void k_normalize(double2* __restrict__ X, int64_t n, int64_t ldx) {
 }
 
 struct OaLayout {
-    int64_t pitch, K256, nslab, nA, nB, nW, nE, nT;
-    float *A, *B, *W, *E, *T;
+    int64_t pitch, pz;
+    unsigned short *A, *B;   // bf16 slices of H and X
+    float *W, *E, *T;
     int *eA, *eB;
+    size_t bytes;
 };
 
-OaLayout oa_layout(int64_t n, int64_t iu, void* base) {
+// workspace of nb matrices
+OaLayout oa_layout(int64_t n, int64_t iu, int64_t nb, void* base) {
     OaLayout L{};
     L.pitch = round_up(n, 4);
-    L.K256 = round_up(n, 256);
+    L.pz = round_up(n, 8);
     constexpr int S = OA_SLICES;
-    L.nA = 2 * S * n * L.pitch;
-    L.nB = 3 * S * iu * L.pitch;
-    L.nW = 6 * iu * L.pitch;
-    L.nE = 6 * iu * L.pitch;
-    L.nT = 4 * n * L.pitch;
     char* p = static_cast<char*>(base);
-    auto take = [&](size_t bytes) {
+    auto take = [&](int64_t bytes) {
         char* q = p;
-        p += round_up((int64_t)bytes, 256);
+        p += round_up(nb * bytes, 256);
         return q;
     };
-    L.A = (float*)take(L.nA * 4);
-    L.B = (float*)take(L.nB * 4);
-    L.W = (float*)take(L.nW * 4);
-    L.E = (float*)take(L.nE * 4);
-    L.T = (float*)take(L.nT * 4);
+    L.A = (unsigned short*)take(2 * S * n * L.pz * 2);
+    L.B = (unsigned short*)take(2 * S * iu * L.pz * 2);
+    L.W = (float*)take(6 * iu * L.pitch * 4);
+    L.E = (float*)take(6 * iu * L.pitch * 4);
+    L.T = (float*)take(4 * n * L.pitch * 4);
     L.eA = (int*)take(n * 4);
     L.eB = (int*)take(iu * 4);
-    L.nslab = (int64_t)(p - static_cast<char*>(base));
+    L.bytes = (size_t)(p - static_cast<char*>(base));
     return L;
+}
+
+// matrices refined together: what fits in 4 GB, at least one (one matrix of N = 364 has nine tiles)
+int64_t oa_chunk(int64_t n, int64_t iu, int64_t batch) {
+    const int64_t per = (int64_t)oa_layout(n, iu, 1, nullptr).bytes;
+    return std::max<int64_t>(1, std::min<int64_t>(batch, ((int64_t)4 << 30) / per));
 }
 
 }  // namespace
 
-size_t oa_workspace_bytes(int64_t n, int64_t iu) { return (size_t)oa_layout(n, iu, nullptr).nslab + 256; }
+size_t oa_workspace_bytes(int64_t n, int64_t iu, int64_t batch) {
+    return oa_layout(n, iu, oa_chunk(n, iu, batch), nullptr).bytes + 256;
+}
 
 // Refines columns 0..iu-1 of X (FP64, unit-normalised, ldx, strideX per matrix) and their eigenvalues
 // for each of the batch matrices: H (FP64, lower triangles; the upper triangles are filled here), Xs
@@ -356,48 +350,25 @@ int oa_refine(cudaStream_t st, double2* H, int64_t strideH, const float* Xs, int
                   (long long)nall, (long long)n, OA_SLICES - 1);
         return FORGE_ERR_ARG;
     }
-    OaLayout L = oa_layout(n, iu, ws);
     constexpr int S = OA_SLICES;
-    // slice pairs (s, t), s + t <= depth, and their scale 2^-(16 + 9 (s + t))
-    std::vector<std::pair<int, int>> pairs;
-    for (int d = 0; d <= depth; ++d)
-        for (int s = 0; s <= d; ++s) pairs.push_back({s, d - s});
-    const int nseg = 2 * (int)pairs.size();
-    if (nseg > TC_MAXSEG) {
-        set_error(FORGE_ERR_ARG, "oa_refine: %d segments exceed %d", nseg, TC_MAXSEG);
-        return FORGE_ERR_ARG;
-    }
-    const int32_t nkp256 = (int32_t)(L.K256 / 32);
-    auto wmap = [&](int part, TcKMap& ka, TcKMap& kb) {
-        ka = TcKMap{};
-        kb = TcKMap{};
-        ka.nkp = kb.nkp = nkp256;
-        ka.nseg = kb.nseg = nseg;
-        ka.zbatch = kb.zbatch = 0;
-        int q = 0;
-        for (auto [s, t] : pairs) {
-            const int8_t sc = (int8_t)(16 + 9 * (s + t));
-            // part 0: Re(HX) = Re H Re X - Im H Im X; part 1: Im(HX) = Re H Im X + Im H Re X
-            ka.zsel[q] = s;
-            kb.zsel[q] = part == 0 ? t : S + t;
-            ka.sexp[q++] = sc;
-            ka.zsel[q] = S + s;
-            kb.zsel[q] = part == 0 ? 2 * S + t : t;
-            ka.sexp[q++] = sc;
-        }
-    };
+    const int64_t chunk = oa_chunk(n, iu, batch);
+    const OaLayout L = oa_layout(n, iu, chunk, ws);
     auto cmap = [&](const int32_t* za, const int32_t* zb, int64_t K, TcKMap& ka, TcKMap& kb) {
         ka = TcKMap{};
         kb = TcKMap{};
         ka.nkp = kb.nkp = (int32_t)((K + 31) / 32);
         ka.nseg = kb.nseg = 6;
+        ka.zbatch = 4;
+        kb.zbatch = 6;
         for (int q = 0; q < 6; ++q) {
             ka.zsel[q] = za[q];
             kb.zsel[q] = zb[q];
         }
     };
     const double nd = (double)n, iud = (double)iu;
-    for (int64_t b = 0; b < batch; ++b) {
+    for (int64_t b = 0; b < batch; b += chunk) {
+        const int64_t nb = std::min(chunk, batch - b);
+        const unsigned nbu = (unsigned)nb;
         double2* Hb = H + b * strideH;
         const float* Xsb = Xs + b * 4 * n4 * nall;
         const double* lamb = lam + b * nall;
@@ -405,63 +376,64 @@ int oa_refine(cudaStream_t st, double2* H, int64_t strideH, const float* Xs, int
         double* wb = w_out + b * w_stride;
         prof_begin(ST_OA);
         const unsigned nt = (unsigned)((n + 31) / 32);
-        k_herm_fill<<<dim3(nt, nt), dim3(32, 8), 0, st>>>(Hb, n);
+        k_herm_fill<<<dim3(nt, nt, nbu), dim3(32, 8), 0, st>>>(Hb, strideH, n);
         FORGE_LAUNCH_CHECK();
-        k_oa_slice<<<(unsigned)n, 256, 0, st>>>(Hb, n, n, 0, L.A, L.pitch, n * L.pitch, L.eA);
+        k_oz_cols<S, true><<<dim3((unsigned)n, nbu), 256, 0, st>>>(LdOaH{Hb, n, strideH}, n, L.pz, L.A, L.pz, n * L.pz, L.eA, n);
         FORGE_LAUNCH_CHECK();
-        k_oa_slice<<<(unsigned)iu, 256, 0, st>>>(Xb, ldx, n, 1, L.B, L.pitch, iu * L.pitch, L.eB);
+        k_oz_cols<S, true><<<dim3((unsigned)iu, nbu), 256, 0, st>>>(LdOaX{Xb, ldx, strideX}, n, L.pz, L.B, L.pz, iu * L.pz, L.eB,
+                                                              iu);
         FORGE_LAUNCH_CHECK();
-        prof_end(ST_OA, nd * nd * 16.0 * 2.0 + nd * nd * 4.0 * 2 * S + nd * iud * (16.0 + 4.0 * 3 * S), 0.0);
-        // W = H X - X lam (sliced, exact blocks)
+        prof_end(ST_OA, nb * (nd * nd * 16.0 * 2.0 + nd * nd * 2.0 * 2 * S + nd * iud * (16.0 + 2.0 * 2 * S)), 0.0);
+        // W = H X - X lam (exact integer slices)
         prof_begin(ST_OA_GEMM);
-        for (int part = 0; part < 2; ++part) {
-            TcKMap ka, kb;
-            wmap(part, ka, kb);
-            TcOperand A{L.A, n, n, L.pitch, n * L.pitch, 2 * S};
-            TcOperand B{L.B, iu, n, L.pitch, iu * L.pitch, 3 * S};
-            FORGE_TRY((tc_gemm_tf32_mapped<OaWEpi, 8, true>(
-                st, A, ka, B, kb, 1, 0, OaWEpi{L.eA, L.eB, Xb, ldx, lamb, L.W, L.pitch, iu * L.pitch, part}, err)));
+        {
+            const OzOperand A{(const __nv_bfloat16*)L.A, n, n, L.pz, n * L.pz, nb * 2 * S, 2 * S};
+            const OzOperand B{(const __nv_bfloat16*)L.B, iu, n, L.pz, iu * L.pz, nb * 2 * S, 2 * S};
+            FORGE_TRY(oz_gemm<true>(st, A, 0, B, 0, n, oz_plans_complex(S, depth, n, false, false), nb, false,
+                                    OaWEpi{L.eA, L.eB, Xb, ldx, strideX, lamb, L.W, L.pitch, iu * L.pitch, n, iu, nall},
+                                    err));
         }
-        prof_end(ST_OA_GEMM, nd * iud * 16.0 * 2.0 + nd * nd * 16.0,
-                 (double)pairs.size() * 8.0 * nd * nd * iud);
+        prof_end(ST_OA_GEMM, nb * (nd * iud * 16.0 * 2.0 + nd * nd * 16.0),
+                 nb * 0.5 * (depth + 1) * (depth + 2) * 8.0 * nd * nd * iud);
         prof_begin(ST_OA);
-        k_oa_diag<<<(unsigned)iu, 256, 0, st>>>(Xb, ldx, n, L.W, L.pitch, iu * L.pitch, lamb, wb);
+        k_oa_diag<<<dim3((unsigned)iu, nbu), 256, 0, st>>>(Xb, ldx, n, L.W, L.pitch, iu * L.pitch, lamb, wb, strideX, nall,
+                                                           w_stride);
         FORGE_LAUNCH_CHECK();
         // C = X_all^H W -> E (separated pairs)
         {
             const int32_t za_r[6] = {0, 0, 2, 1, 1, 3}, zb_r[6] = {0, 1, 0, 2, 3, 2};
             const int32_t za_i[6] = {0, 0, 2, 1, 1, 3}, zb_i[6] = {2, 3, 2, 4, 5, 4};
-            TcOperand A{Xsb, nall, n, n4, n4 * nall, 4};
-            TcOperand B{L.W, iu, n, L.pitch, iu * L.pitch, 6};
+            TcOperand A{Xsb, nall, n, n4, n4 * nall, 4 * nb};
+            TcOperand B{L.W, iu, n, L.pitch, iu * L.pitch, 6 * nb};
             TcKMap ka, kb;
             cmap(za_r, zb_r, n, ka, kb);
-            FORGE_TRY(tc_gemm_tf32_mapped(st, A, ka, B, kb, 1, 0,
-                                          OaCEpi{lamb, delta, L.E, L.pitch, iu * L.pitch, 0}, err));
+            FORGE_TRY(tc_gemm_tf32_mapped(st, A, ka, B, kb, nb, 0,
+                                          OaCEpi{lamb, delta, L.E, L.pitch, iu * L.pitch, nall, 0}, err));
             cmap(za_i, zb_i, n, ka, kb);
-            FORGE_TRY(tc_gemm_tf32_mapped(st, A, ka, B, kb, 1, 0,
-                                          OaCEpi{lamb, delta, L.E, L.pitch, iu * L.pitch, 1}, err));
+            FORGE_TRY(tc_gemm_tf32_mapped(st, A, ka, B, kb, nb, 0,
+                                          OaCEpi{lamb, delta, L.E, L.pitch, iu * L.pitch, nall, 1}, err));
         }
-        k_oa_cluster<<<(unsigned)iu, 256, 0, st>>>(Xsb, n4, nall, n, lamb, delta, L.E, L.pitch, iu * L.pitch);
+        k_oa_cluster<<<dim3((unsigned)iu, nbu), 256, 0, st>>>(Xsb, n4, nall, n, lamb, delta, L.E, L.pitch, iu * L.pitch);
         FORGE_LAUNCH_CHECK();
         // X_j += X_all E
-        k_oa_transpose<<<dim3((unsigned)((nall + 31) / 32), nt), dim3(32, 8), 0, st>>>(Xsb, n4, nall, n, L.T,
+        k_oa_transpose<<<dim3((unsigned)((nall + 31) / 32), nt, nbu), dim3(32, 8), 0, st>>>(Xsb, n4, nall, n, L.T,
                                                                                        L.pitch);
         FORGE_LAUNCH_CHECK();
         {
             const int32_t za_r[6] = {0, 0, 2, 1, 1, 3}, zb_r[6] = {0, 1, 0, 4, 5, 4};
             const int32_t za_i[6] = {0, 0, 2, 1, 1, 3}, zb_i[6] = {2, 3, 2, 0, 1, 0};
-            TcOperand A{L.T, n, nall, L.pitch, n * L.pitch, 4};
-            TcOperand B{L.E, iu, nall, L.pitch, iu * L.pitch, 6};
+            TcOperand A{L.T, n, nall, L.pitch, n * L.pitch, 4 * nb};
+            TcOperand B{L.E, iu, nall, L.pitch, iu * L.pitch, 6 * nb};
             TcKMap ka, kb;
             cmap(za_r, zb_r, nall, ka, kb);
-            FORGE_TRY(tc_gemm_tf32_mapped(st, A, ka, B, kb, 1, 0, OaUEpi{Xb, ldx, 0}, err));
+            FORGE_TRY(tc_gemm_tf32_mapped(st, A, ka, B, kb, nb, 0, OaUEpi{Xb, ldx, strideX, 0}, err));
             cmap(za_i, zb_i, nall, ka, kb);
-            FORGE_TRY(tc_gemm_tf32_mapped(st, A, ka, B, kb, 1, 0, OaUEpi{Xb, ldx, 1}, err));
+            FORGE_TRY(tc_gemm_tf32_mapped(st, A, ka, B, kb, nb, 0, OaUEpi{Xb, ldx, strideX, 1}, err));
         }
-        k_normalize<<<(unsigned)iu, 256, 0, st>>>(Xb, n, ldx);
+        k_normalize<<<dim3((unsigned)iu, nbu), 256, 0, st>>>(Xb, n, ldx, strideX);
         FORGE_LAUNCH_CHECK();
-        prof_end(ST_OA, nd * nd * 4.0 * 4.0 * 2.0 + 2.0 * nd * iud * (16.0 + 24.0),
-                 2.0 * 3.0 * 8.0 * nd * nd * iud);
+        prof_end(ST_OA, nb * (nd * nd * 4.0 * 4.0 * 2.0 + 2.0 * nd * iud * (16.0 + 24.0)),
+                 nb * 2.0 * 3.0 * 8.0 * nd * nd * iud);
     }
     return 0;
 }

@@ -19,6 +19,7 @@
 namespace forge {
 
 constexpr int S7 = OZ_S;
+constexpr int OZ_REF_S = 4, OZ_REF_DEPTH = 3;   // projectors of refined eigenvectors
 
 int oz_make_tmap(CUtensorMap* map, const OzOperand& op) {
     return tc_make_tmap_bf16(map, op.ptr, op.cols, op.rows, op.nplanes, op.ld, op.plane, OZ_BK, OZ_T);
@@ -220,9 +221,9 @@ int her2k_oz(cudaStream_t st, TrdArgs<double>& a, int64_t p, int64_t w, int64_t 
     unsigned short* Zs = U + batch * P * plane;
     int *eU = g.oz_ex, *eZ = eU + batch * n;
     const dim3 gs(cdiv(m, 32), (unsigned)batch), bs(32, 8);
-    k_oz_rows<S7><<<gs, bs, 0, st>>>(LdPanel{a.A, a.W, a.lda, a.strideA, n, r0, p, w, 0}, m, 64, 64, U, 64, plane, eU, n);
+    k_oz_rows<S7><<<gs, bs, 0, st>>>(LdPanel{a.A, a.W, a.lda, a.strideA, n, r0, p, w, 0}, m, 64, 64, U, 64, plane, eU, n, nullptr);
     FORGE_LAUNCH_CHECK();
-    k_oz_rows<S7><<<gs, bs, 0, st>>>(LdPanel{a.A, a.W, a.lda, a.strideA, n, r0, p, w, 1}, m, 64, 64, Zs, 64, plane, eZ, n);
+    k_oz_rows<S7><<<gs, bs, 0, st>>>(LdPanel{a.A, a.W, a.lda, a.strideA, n, r0, p, w, 1}, m, 64, 64, Zs, 64, plane, eZ, n, nullptr);
     FORGE_LAUNCH_CHECK();
     const OzOperand A{(const __nv_bfloat16*)U, m, 64, 64, plane, batch * P, (int32_t)P};
     const OzOperand B{(const __nv_bfloat16*)Zs, m, 64, 64, plane, batch * P, (int32_t)P};
@@ -261,7 +262,7 @@ int backtransform_oz(cudaStream_t st, EigArgs& g) {
         k_oz_larft<<<(unsigned)zb, (unsigned)NB, smem, st>>>(g.oz_g, g.tau, n, j0c, (int)NB, batch, g.oz_t);
         FORGE_LAUNCH_CHECK();
         k_oz_rows<S7><<<dim3(cdiv(NB, 32), (unsigned)zb), dim3(32, 8), 0, st>>>(LdT{g.oz_t, NB}, NB, NB, NB, Ts, NB, pT, eT,
-                                                                                NB);
+                                                                                NB, nullptr);
         FORGE_LAUNCH_CHECK();
         for (int64_t blk = hi - 1; blk >= lo; --blk) {
             const int64_t j0 = blk * NB, q = blk - lo, K = n - j0;
@@ -288,7 +289,7 @@ int backtransform_oz(cudaStream_t st, EigArgs& g) {
                                                                                eW, iu);
             FORGE_LAUNCH_CHECK();
             k_oz_rows<S7><<<dim3(cdiv(K, 32), (unsigned)batch), dim3(32, 8), 0, st>>>(LdVr{v, j0}, K, NB, NB, Vr, NB, pR, eR,
-                                                                                      n);
+                                                                                      n, nullptr);
             FORGE_LAUNCH_CHECK();
             const OzOperand oR{(const __nv_bfloat16*)Vr, K, NB, NB, pR, batch * P, (int32_t)P};
             FORGE_TRY(oz_gemm(st, oR, 0, oW, 0, NB, oz_plans_complex(S7, OZ_DEPTH, NB, false, false), batch, false,
@@ -326,8 +327,10 @@ struct EpiProj {
 // P_c += sum over the items z of ph_c(z) C_z (C Hermitian, its lower triangle given): a CTA owns tile
 // (bi, bj) and its mirror image (bj, bi) of all four cells and adds the items in order, so that P
 // is read and written once.  HBM bound.
+// diag (or null): the diagonal of the C_z (nit x n), in place of C's own.
 __global__ void __launch_bounds__(256) k_proj_add(double2* __restrict__ P, const double* __restrict__ C,
-                                                  const ProjItem* __restrict__ it, int64_t nit, int64_t n) {
+                                                  const double* __restrict__ diag, const ProjItem* __restrict__ it,
+                                                  int64_t nit, int64_t n) {
     const int64_t bi = blockIdx.x, bj = blockIdx.y;
     if (bi < bj) return;
     __shared__ double sr[32][33], si[32][33];
@@ -372,10 +375,14 @@ __global__ void __launch_bounds__(256) k_proj_add(double2* __restrict__ P, const
                     cr = sr[tx][col];
                     ci = -si[tx][col];
                 }
+                if (diag && bi == bj && tx == col) {
+                    cr = i0 + tx < n ? diag[z * n + i0 + tx] : 0.0;
+                    ci = 0.0;
+                }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    acc[y][c].x = fma(ph[c].x, cr, fma(-ph[c].y, ci, acc[y][c].x));
-                    acc[y][c].y = fma(ph[c].x, ci, fma(ph[c].y, cr, acc[y][c].y));
+                    acc[y][c].x += ph[c].x * cr - ph[c].y * ci;
+                    acc[y][c].y += ph[c].x * ci + ph[c].y * cr;
                 }
             }
         }
@@ -391,42 +398,55 @@ __global__ void __launch_bounds__(256) k_proj_add(double2* __restrict__ P, const
 }  // namespace
 
 // items per launch: as many as fit in 2 GB of slices and products, at least one
-int64_t proj_oz_chunk(int64_t n, int64_t iu, int64_t nit) {
-    const int64_t per = 2 * S7 * n * up(iu, 8) * 2 + 2 * n * n * 8;
+static int64_t proj_oz_chunk(int64_t n, int64_t iu, int64_t nit, int S) {
+    const int64_t per = 2 * S * n * up(iu, 8) * 2 + 2 * n * n * 8;
     return std::max<int64_t>(1, std::min<int64_t>(nit, ((int64_t)2 << 30) / per));
 }
-size_t proj_oz_workspace_bytes(int64_t n, int64_t iu, int64_t nit) {
-    const int64_t ch = proj_oz_chunk(n, iu, nit);
-    return (size_t)ch * (2 * S7 * n * up(iu, 8) * 2 + 2 * n * n * 8 + up(n, 64) * 4) + (size_t)nit * sizeof(ProjItem) + 1024;
+size_t proj_oz_workspace_bytes(int64_t n, int64_t iu, int64_t nit, bool refined) {
+    const int S = refined ? OZ_REF_S : OZ_S;
+    const int64_t ch = proj_oz_chunk(n, iu, nit, S);
+    return (size_t)ch * (2 * S * n * up(iu, 8) * 2 + 2 * n * n * 8 + up(n, 64) * 12) + (size_t)nit * sizeof(ProjItem) + 1024;
 }
 
-// P_c += sum over items of ph_c conj(X) X^T over the first K columns of X at the item's slot
-int projectors_oz(cudaStream_t st, const double2* X, int64_t ldx, int64_t strideX, int64_t n, int64_t iu,
-                  const ProjItem* items, int64_t nit, double2* P, void* ws, int* err) {
+template <int S, int DEPTH, bool REF>
+static int projectors_cut(cudaStream_t st, const double2* X, int64_t ldx, int64_t strideX, int64_t n, int64_t iu,
+                          const ProjItem* items, int64_t nit, double2* P, void* ws, int* err) {
     if (nit <= 0) return 0;
     prof_begin(ST_PROJECTOR);
-    const int64_t ch = proj_oz_chunk(n, iu, nit), ldk = up(iu, 8), plane = n * ldk, PL = 2 * S7;
+    const int64_t ch = proj_oz_chunk(n, iu, nit, S), ldk = up(iu, 8), plane = n * ldk, PL = 2 * S;
     double* C = static_cast<double*>(ws);
     unsigned short* sl = reinterpret_cast<unsigned short*>(C + ch * 2 * n * n);
     int* e = reinterpret_cast<int*>(sl + ch * PL * plane);
-    ProjItem* dit = reinterpret_cast<ProjItem*>(((uintptr_t)(e + ch * n) + 255) & ~(uintptr_t)255);
+    double* dg = reinterpret_cast<double*>(((uintptr_t)(e + ch * n) + 255) & ~(uintptr_t)255);
+    ProjItem* dit = reinterpret_cast<ProjItem*>(((uintptr_t)(dg + ch * n) + 255) & ~(uintptr_t)255);
+    if (!REF) dg = nullptr;
     FORGE_CUDA(cudaMemcpyAsync(dit, items, nit * sizeof(ProjItem), cudaMemcpyHostToDevice, st));
     for (int64_t z0 = 0; z0 < nit; z0 += ch) {
         const int64_t nb = std::min(ch, nit - z0);
         int64_t K = 0;
         for (int64_t z = 0; z < nb; ++z) K = std::max(K, items[z0 + z].K);
         if (K <= 0) continue;
-        k_oz_rows<S7><<<dim3(cdiv(n, 32), (unsigned)nb), dim3(32, 8), 0, st>>>(LdProj{X, ldx, strideX, dit + z0}, n, K,
-                                                                               up(K, 8), sl, ldk, plane, e, n);
+        k_oz_rows<S, REF><<<dim3(cdiv(n, 32), (unsigned)nb), dim3(32, 8), 0, st>>>(
+            LdProj{X, ldx, strideX, dit + z0}, n, K, up(K, 8), sl, ldk, plane, e, n, dg);
         FORGE_LAUNCH_CHECK();
         const OzOperand op{(const __nv_bfloat16*)sl, n, K, ldk, plane, nb * PL, (int32_t)PL};
-        FORGE_TRY(oz_gemm(st, op, 0, op, 0, K, oz_plans_complex(S7, OZ_DEPTH, K, true, false), nb, true, EpiProj{C, n, e},
-                          err));
-        k_proj_add<<<dim3(cdiv(n, 32), cdiv(n, 32)), dim3(32, 8), 0, st>>>(P, C, dit + z0, nb, n);
+        FORGE_TRY(oz_gemm<REF>(st, op, 0, op, 0, K, oz_plans_complex(S, DEPTH, K, true, false), nb, true,
+                               EpiProj{C, n, e}, err));
+        k_proj_add<<<dim3(cdiv(n, 32), cdiv(n, 32)), dim3(32, 8), 0, st>>>(P, C, dg, dit + z0, nb, n);
         FORGE_LAUNCH_CHECK();
     }
     prof_end(ST_PROJECTOR, (double)n * iu * 16.0 * nit + 4.0 * 2.0 * n * n * 16.0, 4.0 * (double)n * n * (iu - 10) * nit);
     return 0;
+}
+
+// P_c += sum over items of ph_c conj(X) X^T over the first K columns of X at the item's slot.  refined: the
+// eigenvectors come from the refined mixed solve (errors of 1e-9): four slices taken from the top, ten
+// products in double-float sums (2^-48) and the diagonal (the site densities) in FP64.  Measured (TF32 slices, one
+// k a launch before): N = 364, 36 k 8.7 -> 0.9 ms; N = 1324, 16 k 11.0 -> 3.8 ms; N = 5044 19.1 -> 7.2 ms
+int projectors_oz(cudaStream_t st, const double2* X, int64_t ldx, int64_t strideX, int64_t n, int64_t iu,
+                  const ProjItem* items, int64_t nit, double2* P, void* ws, int* err, bool refined) {
+    return refined ? projectors_cut<OZ_REF_S, OZ_REF_DEPTH, true>(st, X, ldx, strideX, n, iu, items, nit, P, ws, err)
+                   : projectors_cut<OZ_S, OZ_DEPTH, false>(st, X, ldx, strideX, n, iu, items, nit, P, ws, err);
 }
 
 }  // namespace forge

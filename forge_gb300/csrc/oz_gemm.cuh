@@ -129,7 +129,12 @@ __device__ inline double oz_pow2(int k) {
 // lower: skip tiles whose rows all lie above the diagonal.  blockIdx.z = 2 z + part, z = b * ksplit + s; split
 // s takes K blocks [s kchunk, min(nkb, (s + 1) kchunk)) of every segment.
 // EPI: epi(z, part, row, col0, v[16], M, N) with the 16 columns' values before the 2^(eA + eB) scale.
-template <class EPI>
+// DF: the blocks of 256 are scaled by their level's power of two (exact) and added into double-float (hi, lo)
+// registers with an error-free TwoSum instead of int64; the epilogue gets hi + lo (about 48 bits) with the level scale
+// applied.  The refinement of the mixed solve uses it: its residual W enters FP32 products, whose rounding
+// noise reaches the refined density matrix at 1e-11 and the next iteration's at 1e-9, so its results are kept to the
+// last bit by keeping this order of additions.
+template <class EPI, bool DF>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     k_oz_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int64_t M, int64_t N,
               const __grid_constant__ OzPlans plans, int32_t nkb, int32_t koffA, int32_t koffB, int32_t zA, int32_t zB,
@@ -239,21 +244,30 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                     }
                 }
             }
+            // every commit's arrival lands before the CTA gives its shared memory back
             tc_commit(accum);
+            if (!*abort_flag && !mbar_wait(accum, 0, abort_flag)) *abort_flag = 1;
         }
+        __syncwarp();
     } else {
         const int quarter = warp & 3, half = (warp - 2) >> 2;
         const int64_t row = m0 + quarter * 32 + lane;
         const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 64);
         const uint32_t thi = tmem + ((uint32_t)(quarter * 32) << 16) + 256u + (uint32_t)(half * 128);
-        long long acc[64];
+        long long acc[DF ? 1 : 64];
+        float fh[DF ? 64 : 1], fl[DF ? 64 : 1];
+        if constexpr (DF) {
 #pragma unroll
-        for (int q = 0; q < 64; ++q) acc[q] = 0;
+            for (int q = 0; q < 64; ++q) fh[q] = fl[q] = 0.f;
+        } else {
+#pragma unroll
+            for (int q = 0; q < 64; ++q) acc[q] = 0;
+        }
         bool ok = true;
         int grp = 0;
         for (int l = 0; l < plan.nlev && ok; ++l) {
-            if (l > 0) {
-                if (l == plan.split) {
+            if constexpr (!DF) {
+                if (l > 0 && l == plan.split) {
                     // the first levels in FP64 (exact up to one rounding) to TMEM
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
@@ -265,14 +279,16 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                             r[2 * q + 1] = (uint32_t)__double2hiint(x);
                             acc[h * 16 + q] = 0;
                         }
+                        __syncwarp();
                         tmem_st32(thi + (uint32_t)(h * 32), r);
                     }
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                } else {
+                } else if (l > 0) {
 #pragma unroll
                     for (int q = 0; q < 64; ++q) acc[q] = (long long)((unsigned long long)acc[q] << 9);
                 }
             }
+            const float scl = __int_as_float((127 - (16 + 9 * l)) << 23);   // 2^-(16 + 9 l)
             const int ng = ((plan.first[l + 1] - plan.first[l]) * kn + 3) / 4;
             for (int g = 0; g < ng; ++g, ++grp) {
                 const int buf = grp & 1;
@@ -284,10 +300,22 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 #pragma unroll
                 for (int h = 0; h < 64; h += 32) {
                     float v[32];
+                    __syncwarp();
                     tmem_ld32(trow + (uint32_t)(buf * OZ_T + h), v);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if constexpr (DF) {
 #pragma unroll
-                    for (int q = 0; q < 32; ++q) acc[h + q] += (long long)__float2int_rn(v[q]);
+                        for (int q = 0; q < 32; ++q) {
+                            const float x = v[q] * scl;
+                            const float sm = fh[h + q] + x;
+                            const float bp = sm - fh[h + q];
+                            fl[h + q] += (fh[h + q] - (sm - bp)) + (x - bp);
+                            fh[h + q] = sm;
+                        }
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 32; ++q) acc[h + q] += (long long)__float2int_rn(v[q]);
+                    }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
@@ -303,8 +331,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
                 double d[16];
-                if (plan.split) {
+                if constexpr (DF) {
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) d[q] = (double)fh[h * 16 + q] + (double)fl[h * 16 + q];
+                } else if (plan.split) {
                     float r[32];
+                    __syncwarp();   // the epilogue functor may leave rows beyond M behind; tcgen05.ld is .aligned
                     tmem_ld32(thi + (uint32_t)(h * 32), r);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
@@ -319,6 +351,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             }
         }
     }
+    __syncwarp();
     __syncthreads();
     if (*abort_flag && threadIdx.x == 0) {
         atomicExch(err, 1);
@@ -330,6 +363,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
     }
@@ -344,7 +378,7 @@ inline int oz_ksplit_count(int64_t nkb, int64_t want) {
 
 // K: products per segment (from element koffA / koffB of the operands' rows; the offsets are multiples of
 // 8 elements, the 16 bytes TMA needs)
-template <class EPI>
+template <bool DF = false, class EPI>
 int oz_gemm(cudaStream_t st, const OzOperand& A, int64_t koffA, const OzOperand& B, int64_t koffB, int64_t K,
             const OzPlans& plans, int64_t batch, bool lower, const EPI& epi, int* err, int64_t want_split = 1) {
     if (A.rows <= 0 || B.rows <= 0 || batch <= 0 || K <= 0) return 0;
@@ -353,7 +387,12 @@ int oz_gemm(cudaStream_t st, const OzOperand& A, int64_t koffA, const OzOperand&
         set_error(FORGE_ERR_ARG, "oz_gemm: operands must be 16-byte aligned with pitches multiple of 8 elements");
         return FORGE_ERR_ARG;
     }
-    const int64_t nkb = (K + OZ_BK - 1) / OZ_BK;
+    // DF: whole blocks of 256 products per segment
+    const int64_t nkb = DF ? (K + 255) / 256 * 4 : (K + OZ_BK - 1) / OZ_BK;
+    if (DF && want_split != 1) {
+        set_error(FORGE_ERR_ARG, "oz_gemm: the double-float mode has no K split");
+        return FORGE_ERR_ARG;
+    }
     const int ks = oz_ksplit_count(nkb, want_split);
     if (2 * batch * ks > 65535) {
         set_error(FORGE_ERR_ARG, "oz_gemm: batch x K splits exceeds the grid's z extent");
@@ -366,10 +405,10 @@ int oz_gemm(cudaStream_t st, const OzOperand& A, int64_t koffA, const OzOperand&
     CUtensorMap ma, mb;
     FORGE_TRY(oz_make_tmap(&ma, A));
     FORGE_TRY(oz_make_tmap(&mb, B));
-    FORGE_CUDA(cudaFuncSetAttribute(k_oz_gemm<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+    FORGE_CUDA(cudaFuncSetAttribute(k_oz_gemm<EPI, DF>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
     const dim3 grd((unsigned)((A.rows + OZ_T - 1) / OZ_T), (unsigned)((B.rows + OZ_T - 1) / OZ_T),
                    (unsigned)(2 * batch * ks));
-    k_oz_gemm<EPI><<<grd, OZ_THREADS, OZ_SMEM, st>>>(ma, mb, A.rows, B.rows, plans, (int32_t)nkb, (int32_t)koffA,
+    k_oz_gemm<EPI, DF><<<grd, OZ_THREADS, OZ_SMEM, st>>>(ma, mb, A.rows, B.rows, plans, (int32_t)nkb, (int32_t)koffA,
                                                      (int32_t)koffB, A.zbatch, B.zbatch, lower ? 1 : 0, ks,
                                                      (int32_t)((nkb + ks - 1) / ks), epi, err);
     FORGE_LAUNCH_CHECK();
@@ -407,10 +446,45 @@ __device__ inline void oz_cut(double x, int e, unsigned short* out) {
     out[0] = (unsigned short)(__float_as_uint((float)(int)m) >> 16);
 }
 
+// The same slices taken from the top, each the nearest integer (ties to even) of what the slices before it left:
+// v_0 = rint(256 a), v_1 = rint(512 (256 a - v_0)), ...  (a = x 2^-e)
+template <int S>
+__device__ inline void oz_cut_rint(double x, int e, unsigned short* out) {
+    const long long bits = __double_as_longlong(x);
+    const int f = (int)(bits >> 52) & 0x7ff;
+    long long r = f ? (bits & 0xfffffffffffffLL) | (1LL << 52) : 0;
+    const int sh = f - 1013 - e;   // r 2^sh = |x| 2^(62 - e)
+    if (sh >= 0) {
+        r <<= sh;
+    } else if (sh < -54) {
+        r = r != 0;
+    } else {
+        const long long q = r >> -sh;
+        r = q | ((q << -sh) != r);   // what is cut off only breaks ties
+    }
+    if (bits < 0) r = -r;
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const int u = 54 - 9 * s;
+        const long long h = r + (1LL << (u - 1));
+        long long v = h >> u;
+        if ((h & ((1LL << u) - 1)) == 0) v &= ~1LL;
+        r -= v << u;
+        out[s] = (unsigned short)(__float_as_uint((float)(int)v) >> 16);
+    }
+}
+template <int S, bool RINT>
+__device__ inline void oz_cut_as(double x, int e, unsigned short* out) {
+    if constexpr (RINT)
+        oz_cut_rint<S>(x, e, out);
+    else
+        oz_cut<S>(x, e, out);
+}
+
 // Rows of the operand = columns of a column-major source: one CTA per (row, batch item).  LD: double2
 // ld(b, row, k).  Planes (0..S-1: real, S..2S-1: imaginary) of row `row` at
 // out + ((blockIdx.y * 2 S + p) * plane) + row * ldo + k; its scale to expo[b * estride + row].
-template <int S, class LD>
+template <int S, bool RINT = false, class LD>
 __global__ void __launch_bounds__(256) k_oz_cols(LD ld, int64_t k1, int64_t kpad, unsigned short* __restrict__ out,
                                                  int64_t ldo, int64_t plane, int* __restrict__ expo, int64_t estride) {
     const int64_t row = blockIdx.x, b = blockIdx.y;
@@ -433,10 +507,10 @@ __global__ void __launch_bounds__(256) k_oz_cols(LD ld, int64_t k1, int64_t kpad
     for (int64_t k = threadIdx.x; k < kpad; k += blockDim.x) {
         const double2 v = k < k1 ? ld(b, row, k) : make_double2(0.0, 0.0);
         unsigned short d[S];
-        oz_cut<S>(v.x, ec, d);
+        oz_cut_as<S, RINT>(v.x, ec, d);
 #pragma unroll
         for (int s = 0; s < S; ++s) o[s * plane + k] = d[s];
-        oz_cut<S>(v.y, ec, d);
+        oz_cut_as<S, RINT>(v.y, ec, d);
 #pragma unroll
         for (int s = 0; s < S; ++s) o[(S + s) * plane + k] = d[s];
     }
@@ -444,10 +518,11 @@ __global__ void __launch_bounds__(256) k_oz_cols(LD ld, int64_t k1, int64_t kpad
 
 // Rows of the operand = rows of a column-major source, K = its columns: a CTA (32 x 8) takes 32 rows and
 // transposes 32 x 32 tiles through shared memory.  Layout of the output as in k_oz_cols.
-template <int S, class LD>
+// diag (or null): sum of |v|^2 of every row in FP64, at diag[b * estride + row].
+template <int S, bool RINT = false, class LD>
 __global__ void __launch_bounds__(256) k_oz_rows(LD ld, int64_t rows, int64_t K, int64_t kpad,
                                                  unsigned short* __restrict__ out, int64_t ldo, int64_t plane,
-                                                 int* __restrict__ expo, int64_t estride) {
+                                                 int* __restrict__ expo, int64_t estride, double* __restrict__ diag) {
     const int64_t b = blockIdx.y, i0 = (int64_t)blockIdx.x * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int64_t Kb = ld.extent(b, K);   // columns of this batch item (the rest is zero)
@@ -470,28 +545,40 @@ __global__ void __launch_bounds__(256) k_oz_rows(LD ld, int64_t rows, int64_t K,
     }
     __syncthreads();
     unsigned short* o = out + b * 2 * S * plane;
+    __shared__ double dpart[8][32];
+    double dtot = 0.0;
     for (int64_t kt = 0; kt < kpad; kt += 32) {
+        double dsum = 0.0;
         for (int q = ty; q < 32; q += 8) {
             const int64_t k = kt + q;
-            tile[q][tx] = (i < rows && k < Kb) ? ld(b, i, k) : make_double2(0.0, 0.0);
+            const double2 x = (i < rows && k < Kb) ? ld(b, i, k) : make_double2(0.0, 0.0);
+            tile[q][tx] = x;
+            if (diag) dsum += x.x * x.x + x.y * x.y;
         }
+        if (diag) dpart[ty][tx] = dsum;
         __syncthreads();
+        if (diag && ty == 0) {
+            double t = 0.0;
+            for (int y = 0; y < 8; ++y) t += dpart[y][tx];
+            dtot += t;
+        }
         for (int q = ty; q < 32; q += 8) {
             const int64_t r = i0 + q, k = kt + tx;
             if (r < rows && k < kpad) {
                 const int e = red[0][q], ec = e == OZ_NAN ? 1025 : e;
                 const double2 v = tile[tx][q];
                 unsigned short d[S];
-                oz_cut<S>(v.x, ec, d);
+                oz_cut_as<S, RINT>(v.x, ec, d);
 #pragma unroll
                 for (int s = 0; s < S; ++s) o[s * plane + r * ldo + k] = d[s];
-                oz_cut<S>(v.y, ec, d);
+                oz_cut_as<S, RINT>(v.y, ec, d);
 #pragma unroll
                 for (int s = 0; s < S; ++s) o[(S + s) * plane + r * ldo + k] = d[s];
             }
         }
         __syncthreads();
     }
+    if (diag && ty == 0 && i < rows) diag[b * estride + i] = dtot;
 }
 
 }  // namespace forge

@@ -8,7 +8,9 @@
 //   Y = H X_w,  G = X_w^H Y,  S = X_w^H X_w,  S = L L^H,  L^{-1} G L^{-H} = U diag(theta) U^H,
 //   X_w <- X_w L^{-H} U,  w <- theta.
 // The FP64 H(k) of the batch is still resident; the three products are FP64 GEMMs on the CUDA
-// cores (8 N^2 nw FLOP per k for Y) and the nw x nw problem is solved on the host.
+// cores (8 N^2 nw FLOP per k for Y) and the nw x nw problem is solved on the host.  The products take 32 x 32
+// and 16 x 16 tiles: 64 x 64 ones computed a half of padding and left SMs idle (N = 5044, nw = 32: 26 -> 11 ms;
+// N = 1324, 16 k 21 -> 8.8 ms).
 #include <algorithm>
 #include <cmath>
 #include <thread>
@@ -232,12 +234,12 @@ int rr_window(cudaStream_t st, const double2* H, int64_t strideH, double2* X, in
     double2* Md = Sp + (size_t)kmax * nw * nw * batch;
     prof_begin(ST_REFINE);
     RrXcol xc{X, ldx, strideX, n, c0, nw};
-    FORGE_TRY((zgemm_launch<double2, IMAJOR, KMAJOR, false>(st, n, nw, n, batch, RrHermA{H, n, strideH}, xc,
+    FORGE_TRY((zgemm_launch<double2, IMAJOR, KMAJOR, false, 32>(st, n, nw, n, batch, RrHermA{H, n, strideH}, xc,
                                                             RrStoreY{Y, n, nw})));
     const int64_t ks = zg_ksplit_count(n, std::min<int64_t>(kmax, (n + 511) / 512));
-    FORGE_TRY((zgemm_launch_splitk<double2, KMAJOR, KMAJOR>(st, nw, nw, n, batch, ks, RrXcolConj{xc},
+    FORGE_TRY((zgemm_launch_splitk<double2, KMAJOR, KMAJOR, 16>(st, nw, nw, n, batch, ks, RrXcolConj{xc},
                                                             RrYcol{Y, n, nw}, RrStoreSmall{Gp, nw, batch})));
-    FORGE_TRY((zgemm_launch_splitk<double2, KMAJOR, KMAJOR>(st, nw, nw, n, batch, ks, RrXcolConj{xc}, xc,
+    FORGE_TRY((zgemm_launch_splitk<double2, KMAJOR, KMAJOR, 16>(st, nw, nw, n, batch, ks, RrXcolConj{xc}, xc,
                                                             RrStoreSmall{Sp, nw, batch})));
     const size_t nn = (size_t)nw * nw;
     std::vector<double2> gp(ks * batch * nn), sp(ks * batch * nn), M(batch * nn);
@@ -275,7 +277,7 @@ int rr_window(cudaStream_t st, const double2* H, int64_t strideH, double2* X, in
     FORGE_CUDA(cudaMemcpyAsync(Md, M.data(), M.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
     FORGE_CUDA(cudaMemcpyAsync(w, wh.data(), wh.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     // X_w <- X_w M (into T, then back into X)
-    FORGE_TRY((zgemm_launch<double2, IMAJOR, KMAJOR, false>(st, n, nw, nw, batch, RrXcolA{xc}, RrMB{Md, nw},
+    FORGE_TRY((zgemm_launch<double2, IMAJOR, KMAJOR, false, 32>(st, n, nw, nw, batch, RrXcolA{xc}, RrMB{Md, nw},
                                                             RrStoreY{T, n, nw})));
     k_rr_copyback<<<dim3(256, (unsigned)batch), 256, 0, st>>>(T, X, n, nw, c0, ldx, strideX);
     FORGE_LAUNCH_CHECK();
