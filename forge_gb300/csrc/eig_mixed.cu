@@ -48,7 +48,7 @@ __device__ inline void split2(float x, float& hi, float& lo) {
 struct MixedWs {
     int64_t n, iu, B, n4, Kp, nblk, nrb, pstride;
     float2* A32;
-    float2 *W, *Yrow, *Ycol, *Spart, *tau;
+    float2 *W, *Yrow, *Ycol, *Spart, *tau, *w0;
     double* part;
     double* scal;
     unsigned* cnt;
@@ -77,13 +77,14 @@ void carve(MixedWs& w, Carve& c) {
     w.Kp = (n + 31) / 32 * 32;
     w.nblk = (n + TRD_TILE - 1) / TRD_TILE;
     w.nrb = (n + 255) / 256;
-    w.pstride = 2 * ((n + 31) / 32) + 2;  // per-CTA partials of trd_col / trd_finish
+    w.pstride = 2 * ((n + 31) / 32) + 4 * ((n + 255) / 256);  // partial sums of trd_finish and trd_col
     w.A32 = c.take<float2>(B * n * n);
     w.W = c.take<float2>(B * n * TRD_NB);
     w.Yrow = c.take<float2>(B * w.nblk * n);
     w.Ycol = c.take<float2>(B * w.nblk * n);
     w.Spart = c.take<float2>(B * w.nrb * 2 * TRD_NB);
     w.tau = c.take<float2>(B * n);
+    w.w0 = c.take<float2>(B * n);
     w.part = c.take<double>(B * w.pstride);
     w.scal = c.take<double>(B * 16);
     w.cnt = c.take<unsigned>(B * 4);
@@ -597,6 +598,7 @@ int eig_mixed(cudaStream_t st, EigArgs& g, void* mixed_ws) {
     a.d = g.d;
     a.e = g.e;
     a.tau = ws.tau;
+    a.w0 = ws.w0;
     a.W = ws.W;
     a.Yrow = ws.Yrow;
     a.Ycol = ws.Ycol;

@@ -1,40 +1,18 @@
-// Batched Householder tridiagonalisation (see tridiag.cuh for the structure).
+// Batched Householder tridiagonalisation in FP32 (see tridiag.cuh for the structure).
 //
 // Bytes per column step (algorithmic): the trailing lower triangle, (n-col)^2/2
 // complex elements, read once by trd_hemv; the rank-2k update is GEMM-shaped.
+// What bounds a column besides trd_hemv's bytes is latency: kernel boundaries, and inside trd_col / trd_finish the
+// round trips to L2.  So the three kernels are launched programmatically, every thread's loads of a phase are in
+// flight together, and no CTA adds up partials one by one.  One matrix of n = 5044 (5043 columns), whole kernels:
+// trd_col 78 -> 58 ms, trd_hemv 91 -> 72 ms, trd_finish (with trd_fix, now once a panel) 116 -> 41 ms; n = 364, six
+// matrices: 5.4 -> 4.1, 4.2 -> 3.4, 5.4 -> 3.1 ms.
+// The order of every FP32 sum is part of the result: refined orbitals are compared to the last place.
 #include "tridiag.cuh"
 
 namespace forge {
 
 namespace {
-
-template <class V>
-__device__ inline V ldv(const V* p) {
-    return *p;
-}
-
-// Block-wide sum (blockDim.x == 256) in the working precision T: the FP32 path keeps its
-// per-element arithmetic off the FP64 pipe, which runs at 1/64 of the FP32 rate on this GPU.
-template <class T>
-__device__ inline T warp_sum_t(T v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-template <class T>
-__device__ inline T block_sum_256(T v, T* sh) {
-    v = warp_sum_t(v);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) sh[w] = v;
-    __syncthreads();
-    T r = (T)0;
-    if (threadIdx.x < 32) {
-        r = (l < 8) ? sh[l] : (T)0;
-        r = warp_sum_t(r);
-    }
-    __syncthreads();
-    return r;  // valid in thread 0
-}
 
 // "last CTA" detection for a per-batch counter; returns true in every thread of the last CTA.
 __device__ inline bool last_cta(unsigned* counter, unsigned total) {
@@ -50,29 +28,110 @@ __device__ inline bool last_cta(unsigned* counter, unsigned total) {
     return is_last;
 }
 
-}  // namespace
+
+constexpr int COL_ROWS = 64;   // rows (and threads) per CTA of k_trd_col: the panel's columns come in over many SMs
+constexpr int DOT_L = 8;       // reflectors per CTA of the panel dots
+
+// partial sums: [0, trd_col_parts) the norms of k_trd_col, one float a warp; then pairs w^H v of k_trd_finish
+__device__ inline int64_t trd_col_parts(int64_t n) { return (n + TRD_ROWS - 1) / TRD_ROWS * 4; }
+
+__device__ inline float warp_sum_f(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// alpha2 = -1/2 tau (w^H v) of the last column from the nd partials of k_trd_finish, by one warp
+__device__ inline float2 trd_alpha2(const TrdArgs<float>& a, int64_t b, int64_t nd) {
+    const double2* part = (const double2*)(a.part + b * a.pstride + trd_col_parts(a.n));
+    const double tr = a.scal[b * 16 + 4], ti = a.scal[b * 16 + 5];
+    double xr = 0.0, xi = 0.0;
+    for (int64_t q0 = threadIdx.x & 31; q0 < nd; q0 += 256) {
+        double2 t[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) t[q] = q0 + 32 * q < nd ? part[q0 + 32 * q] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            if (q0 + 32 * q >= nd) break;
+            xr += t[q].x;
+            xi += t[q].y;
+        }
+    }
+    xr = warp_sum_d(xr);
+    xi = warp_sum_d(xi);
+    return make_float2((float)(-0.5 * (tr * xr - ti * xi)), (float)(-0.5 * (tr * xi + ti * xr)));
+}
+
+// w + alpha2 v; the fused operations are spelled out because k_trd_col and k_trd_fix have to round alike
+__device__ inline float2 trd_corr(float2 w, float2 al, float2 v) {
+    return make_float2(__fadd_rn(w.x, fmaf(al.x, v.x, -__fmul_rn(al.y, v.y))),
+                       __fadd_rn(w.y, fmaf(al.y, v.x, __fmul_rn(al.x, v.y))));
+}
 
 // ---------------------------------------------------------------- trd_col (zlatrd column update + zlarfg)
-template <class T>
-__global__ void __launch_bounds__(TRD_ROWS) k_trd_col(TrdArgs<T> a, int64_t p, int ii, int64_t col, int has_refl) {
-    using V = typename CV<T>::type;
+// Adds alpha2 v to the last column's w (w0), then forms column col; the last CTA forms the reflector's scalars from
+// the partial norms.  The kernel is a chain of latencies (a column is a few hundred KB): all of a thread's panel
+// elements are loaded at once, half a panel a time, and the last CTA's four quotients sit in four lanes.
+__global__ void __launch_bounds__(COL_ROWS) k_trd_col(TrdArgs<float> a, int64_t p, int ii, int64_t col, int has_refl) {
     const int64_t b = blockIdx.y, n = a.n, lda = a.lda;
-    V* A = a.A + b * a.strideA;
-    V* W = a.W + b * (n * TRD_NB);
-    __shared__ V wrow[TRD_NB], arow[TRD_NB];
-    __shared__ T sh[8];
-    if (threadIdx.x < ii) {
-        wrow[threadIdx.x] = W[col + threadIdx.x * n];
-        arow[threadIdx.x] = A[col + (p + threadIdx.x) * lda];
+    float2* A = a.A + b * a.strideA;
+    float2* W = a.W + b * (n * TRD_NB);
+    const float2* w0 = a.w0 + b * n;
+    __shared__ float2 wrow[TRD_NB], arow[TRD_NB], s_al;
+    const int lane = threadIdx.x & 31;
+    const int64_t r = col + (int64_t)blockIdx.x * COL_ROWS + threadIdx.x;
+    const int lm = ii - 1;
+    const float2 z = make_float2(0.f, 0.f);
+    trd_chain_wait();
+    float2 x = z, wl = z, vl = z, av[16], wv[16];
+    if (r < n) {
+        x = A[r + col * lda];
+        if (ii > 0) {
+            wl = w0[r];
+            vl = A[r + (p + lm) * lda];
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+        av[q] = q < lm && r < n ? A[r + (p + q) * lda] : z;
+        wv[q] = q < lm && r < n ? W[r + q * n] : z;
+    }
+    if (threadIdx.x >= 32 && lane < ii) {
+        wrow[lane] = lane == lm ? w0[col] : W[col + lane * n];
+        arow[lane] = A[col + (p + lane) * lda];
+    }
+    if (ii > 0 && threadIdx.x < 32) {
+        const float2 al = trd_alpha2(a, b, (n - col + 31) / 32);
+        if (threadIdx.x == 0) s_al = al;
     }
     __syncthreads();
-    const int64_t r = col + (int64_t)blockIdx.x * TRD_ROWS + threadIdx.x;
-    T nrm = (T)0;
+    float nrm = 0.f;
     if (r < n) {
-        V x = A[r + col * lda];
-        for (int l = 0; l < ii; ++l) {
-            x = vsub(x, vmulcj(A[r + (p + l) * lda], wrow[l]));
-            x = vsub(x, vmulcj(W[r + l * n], arow[l]));
+#pragma unroll
+        for (int h = 0; h < TRD_NB; h += 16) {
+            if (h >= lm) break;
+            if (h > 0) {
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                    av[q] = h + q < lm ? A[r + (p + h + q) * lda] : z;
+                    wv[q] = h + q < lm ? W[r + (h + q) * n] : z;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                if (h + q < lm) {
+                    x = vsub(x, vmulcj(av[q], wrow[h + q]));
+                    x = vsub(x, vmulcj(wv[q], arow[h + q]));
+                }
+            }
+        }
+        if (ii > 0) {
+            // the last reflector, whose w takes its correction first
+            const float2 al = s_al, ar = arow[lm];
+            wl = trd_corr(wl, al, vl);
+            W[r + lm * n] = wl;
+            x = vsub(x, vmulcj(vl, trd_corr(wrow[lm], al, ar)));
+            x = vsub(x, vmulcj(wl, ar));
         }
         if (r == col) {
             x.y = 0;
@@ -86,68 +145,61 @@ __global__ void __launch_bounds__(TRD_ROWS) k_trd_col(TrdArgs<T> a, int64_t p, i
         }
         if (r >= col + 2) nrm = x.x * x.x + x.y * x.y;
     }
-    const T s = block_sum_256(nrm, sh);
-    double* part = a.part + b * a.pstride;
-    if (threadIdx.x == 0) part[blockIdx.x] = (double)s;
-    if (last_cta(a.cnt + b * 4, gridDim.x) && threadIdx.x == 0) {
-        double xn2 = 0.0;
-        for (unsigned q = 0; q < gridDim.x; ++q) xn2 += ((volatile double*)part)[q];
+    nrm = warp_sum_f(nrm);
+    float* part = (float*)(a.part + b * a.pstride);
+    const int64_t nw = (int64_t)gridDim.x * (COL_ROWS / 32);
+    if (lane == 0) part[(int64_t)blockIdx.x * (COL_ROWS / 32) + (threadIdx.x >> 5)] = nrm;
+    if (last_cta(a.cnt + b * 4, gridDim.x) && threadIdx.x < 32) {
+        // 256 rows in FP32 (eight warps as a tree), beyond that in FP64
         double* sc = a.scal + b * 16;
-        V* tau = a.tau + b * n;
-        if (!has_refl) {
-            tau[col] = vzero<V>();
-            sc[2] = 1.0;
-            sc[3] = 0.0;
-            sc[4] = 0.0;
-            sc[5] = 0.0;
-            return;
-        }
         const double ar = ((volatile double*)sc)[0], ai = ((volatile double*)sc)[1];
+        double xn2 = 0.0;
+        for (int64_t g = 8 * lane; g < nw; g += 256) {
+            float t[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) t[q] = g + q < nw ? ((volatile float*)part)[g + q] : 0.f;
+            xn2 += (double)(((t[0] + t[4]) + (t[2] + t[6])) + ((t[1] + t[5]) + (t[3] + t[7])));
+        }
+        xn2 = warp_sum_d(xn2);
+        float2* tau = a.tau + b * n;
         // zlarfg: beta = -sign(|(alpha, x)|, Re alpha), tau = (beta - alpha)/beta, x *= 1/(alpha - beta)
-        if (xn2 == 0.0 && ai == 0.0) {
-            tau[col] = vzero<V>();
+        if (!has_refl || (xn2 == 0.0 && ai == 0.0)) {
+            if (lane != 0) return;
+            tau[col] = make_float2(0.f, 0.f);
             sc[2] = 1.0;
             sc[3] = 0.0;
             sc[4] = 0.0;
             sc[5] = 0.0;
-            a.e[b * n + col] = ar;
+            if (has_refl) a.e[b * n + col] = ar;
         } else {
-            double beta = -copysign(sqrt(ar * ar + ai * ai + xn2), ar);
-            double tr = (beta - ar) / beta, ti = -ai / beta;
-            // 1/(alpha - beta)
-            double dr = ar - beta, di = ai;
-            double den = dr * dr + di * di;
-            sc[2] = dr / den;
-            sc[3] = -di / den;
-            sc[4] = tr;
-            sc[5] = ti;
-            tau[col] = vmake<V>((T)tr, (T)ti);
-            a.e[b * n + col] = beta;
+            const double beta = -copysign(sqrt(ar * ar + ai * ai + xn2), ar);
+            const double dr = ar - beta, di = ai, den = dr * dr + di * di;
+            // lanes 0, 1: 1 / (alpha - beta); lanes 2, 3: tau
+            const double num = lane == 0 ? dr : lane == 1 ? -di : lane == 2 ? beta - ar : -ai;
+            const double q = num / (lane < 2 ? den : beta);
+            if (lane < 4) sc[2 + lane] = q;
+            if (lane == 2) tau[col].x = (float)q;
+            if (lane == 3) tau[col].y = (float)q;
+            if (lane == 0) a.e[b * n + col] = beta;
         }
     }
 }
 
 // ---------------------------------------------------------------- trd_hemv (+ panel dots)
-template <class T>
-__device__ inline typename CV<T>::type trd_v(const typename CV<T>::type* A, int64_t lda, int64_t col, int64_t r,
-                                             double sr, double si) {
-    using V = typename CV<T>::type;
-    if (r == col + 1) return vmake<V>((T)1, (T)0);
-    const V x = A[r + col * lda];
-    const T tr = (T)sr, ti = (T)si;
-    return vmake<V>(x.x * tr - x.y * ti, x.x * ti + x.y * tr);
+// v = s x (1 in the first row); spelled out like trd_corr, so that the product and the stored v agree
+__device__ inline float2 trd_scale(float2 x, bool first, float tr, float ti) {
+    if (first) return make_float2(1.f, 0.f);
+    return make_float2(fmaf(x.x, tr, -__fmul_rn(x.y, ti)), fmaf(x.x, ti, __fmul_rn(x.y, tr)));
 }
 
-template <class T>
-__global__ void __launch_bounds__(256) k_trd_hemv(TrdArgs<T> a, int64_t p, int ii, int64_t col, int64_t ntiles) {
-    using V = typename CV<T>::type;
+__global__ void __launch_bounds__(256) k_trd_hemv(TrdArgs<float> a, int64_t p, int ii, int64_t col, int64_t ndc) {
+    using V = float2;
     const int64_t b = blockIdx.y, n = a.n, lda = a.lda;
     const V* A = a.A + b * a.strideA;
     const double* sc = a.scal + b * 16;
-    const double sr = sc[2], si = sc[3];
     const int64_t c0 = col + 1;
-    const int64_t t = blockIdx.x;
-    if (t < ntiles) {
+    const int64_t t = (int64_t)blockIdx.x - ndc;   // the dots' CTAs, the longer chains, go first
+    if (t >= 0) {
         // tile (bi, bj), bj <= bi, of the trailing matrix A(c0:n, c0:n): rows [64 bi, 64 bi + 64),
         // columns [64 bj, 64 bj + 64); t = bi (bi + 1) / 2 + bj
         int64_t bi = (int64_t)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);   // corrected below
@@ -159,22 +211,19 @@ __global__ void __launch_bounds__(256) k_trd_hemv(TrdArgs<T> a, int64_t p, int i
         __shared__ V rsum[4][HV_RB];
         __shared__ V cs[HV_RB][HV_CB + 1];
         __shared__ V cq[4][HV_CB];
-        if (threadIdx.x < HV_RB) {
-            const int64_t r = R0 + threadIdx.x;
-            vr[threadIdx.x] = (r < n) ? trd_v<T>(A, lda, col, r, sr, si) : vzero<V>();
-        } else if (threadIdx.x < HV_RB + HV_CB) {
-            const int64_t c = C0 + threadIdx.x - HV_RB;
-            vc[threadIdx.x - HV_RB] = (c < n) ? trd_v<T>(A, lda, col, c, sr, si) : vzero<V>();
-        }
         const int tr = threadIdx.x & 63, tg = threadIdx.x >> 6;
-        const int64_t r0 = R0 + tr;
+        const int64_t r0 = R0 + tr, rv = (tg == 0 ? R0 : C0) + tr;
+        trd_chain_wait();
         // 16 loads per thread (row r0, 16 columns) issued before any arithmetic
-        V a0[16];
+        const float sr = (float)sc[2], si = (float)sc[3];
+        V xv = vzero<V>(), a0[16];
+        if (tg < 2 && rv < n) xv = A[rv + col * lda];
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
             const int64_t c = C0 + tg * 16 + q;
             a0[q] = (r0 < n && c < n && c <= r0) ? A[r0 + c * lda] : vzero<V>();
         }
+        if (tg < 2) (tg == 0 ? vr : vc)[tr] = rv < n ? trd_scale(xv, rv == c0, sr, si) : vzero<V>();
         __syncthreads();
         V racc = vzero<V>();
         const V v0 = vr[tr];
@@ -212,134 +261,172 @@ __global__ void __launch_bounds__(256) k_trd_hemv(TrdArgs<T> a, int64_t p, int i
             if (c < n) Ycol[bi * n + c] = vadd(vadd(cq[0][q], cq[1][q]), vadd(cq[2][q], cq[3][q]));
         }
     } else {
-        // panel dots over rows [c0 + rb*256, ...): s1 = W^H v, s2 = V^H v
-        const int64_t rb = t - ntiles;
+        // panel dots over 256 rows and DOT_L reflectors: s1 = W^H v, s2 = V^H v.  The 32 sums of a warp (8 reflectors
+        // x 2 complex) are reduced together: each butterfly step halves what a lane carries, 31 shuffles, not 160.
+        const int64_t nlc = (ii + DOT_L - 1) / DOT_L, rb = blockIdx.x / nlc;
+        const int l0 = (int)(blockIdx.x - rb * nlc) * DOT_L;
         const int64_t r = c0 + rb * 256 + threadIdx.x;
         const V* W = a.W + b * (n * TRD_NB);
-        __shared__ V s1w[8][TRD_NB], s2w[8][TRD_NB];
-        V v = (r < n) ? trd_v<T>(A, lda, col, r, sr, si) : vzero<V>();
+        __shared__ float sw[8][32];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        for (int l = 0; l < ii; ++l) {
-            V x1 = vzero<V>(), x2 = vzero<V>();
-            if (r < n) {
-                x1 = vcjmul(W[r + l * n], v);
-                x2 = vcjmul(A[r + (p + l) * lda], v);
-            }
-            x1 = warp_sum(x1);
-            x2 = warp_sum(x2);
-            if (lane == 0) {
-                s1w[w][l] = x1;
-                s2w[w][l] = x2;
+        trd_chain_wait();
+        V v = vzero<V>(), xw[DOT_L], xa[DOT_L];
+        if (r < n) v = A[r + col * lda];
+#pragma unroll
+        for (int q = 0; q < DOT_L; ++q) {
+            const bool in = r < n && l0 + q < ii;
+            xw[q] = in ? W[r + (l0 + q) * n] : vzero<V>();
+            xa[q] = in ? A[r + (p + l0 + q) * lda] : vzero<V>();
+        }
+        v = r < n ? trd_scale(v, r == c0, (float)sc[2], (float)sc[3]) : v;
+        float m[32];
+#pragma unroll
+        for (int q = 0; q < DOT_L; ++q) {
+            const V x1 = vcjmul(xw[q], v), x2 = vcjmul(xa[q], v);
+            m[4 * q] = x1.x;
+            m[4 * q + 1] = x1.y;
+            m[4 * q + 2] = x2.x;
+            m[4 * q + 3] = x2.y;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int k = 0; k < o; ++k) {
+                const float give = up ? m[k] : m[k + o], keep = up ? m[k + o] : m[k];
+                m[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
             }
         }
+        sw[w][lane] = m[0];   // lane = 4 q + (part)
         __syncthreads();
-        V* S = a.Spart + b * a.sstride + rb * 2 * TRD_NB;
-        if (threadIdx.x < ii) {
-            V x1 = vzero<V>(), x2 = vzero<V>();
-            for (int q = 0; q < 8; ++q) {
-                x1 = vadd(x1, s1w[q][threadIdx.x]);
-                x2 = vadd(x2, s2w[q][threadIdx.x]);
-            }
-            S[threadIdx.x] = x1;
-            S[TRD_NB + threadIdx.x] = x2;
+        const int l = l0 + (threadIdx.x >> 2), c = threadIdx.x & 3;
+        if (threadIdx.x < 32 && l < ii) {
+            float x = 0.f;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) x += sw[q][threadIdx.x];
+            float* S = (float*)(a.Spart + b * a.sstride + rb * 2 * TRD_NB);
+            S[(c >> 1) * 2 * TRD_NB + 2 * l + (c & 1)] = x;
         }
     }
 }
 
 // ---------------------------------------------------------------- trd_finish
-template <class T>
-__global__ void __launch_bounds__(TRD_ROWS) k_trd_finish(TrdArgs<T> a, int64_t p, int ii, int64_t col, int64_t nb2,
+// y = A22 v - V (W^H v) - W (V^H v), w0 = tau y (w = w0 + alpha2 v follows in the next k_trd_col), v into A,
+// partial sums of w^H v.  32 rows per CTA; 8 threads a row share the partial slots and the reflectors, and load
+// theirs at once: like k_trd_col this is a chain of latencies.
+__global__ void __launch_bounds__(TRD_ROWS) k_trd_finish(TrdArgs<float> a, int64_t p, int ii, int64_t col, int64_t nb2,
                                                          int64_t nrb) {
-    using V = typename CV<T>::type;
+    using V = float2;
     const int64_t b = blockIdx.y, n = a.n, lda = a.lda;
     V* A = a.A + b * a.strideA;
-    V* W = a.W + b * (n * TRD_NB);
-    double* sc = a.scal + b * 16;
-    const double sr = sc[2], si = sc[3];
-    const V tau = vmake<V>((T)sc[4], (T)sc[5]);
+    const V* W = a.W + b * (n * TRD_NB);
     const int64_t c0 = col + 1;
     __shared__ V s1[TRD_NB], s2[TRD_NB];
-    __shared__ T sh[8];
-    if (threadIdx.x < ii) {
-        const V* S = a.Spart + b * a.sstride;
-        V x1 = vzero<V>(), x2 = vzero<V>();
-        for (int64_t q = 0; q < nrb; ++q) {
-            x1 = vadd(x1, S[q * 2 * TRD_NB + threadIdx.x]);
-            x2 = vadd(x2, S[q * 2 * TRD_NB + TRD_NB + threadIdx.x]);
-        }
-        s1[threadIdx.x] = x1;
-        s2[threadIdx.x] = x2;
-    }
-    // 32 rows per CTA, 8 threads per row share the sum over the Yrow / Ycol partial slots
     __shared__ V ysl[8][33];
     const int rr = threadIdx.x & 31, sl = threadIdx.x >> 5;
     const int64_t r = c0 + (int64_t)blockIdx.x * 32 + rr;
+    trd_chain_wait();
+    const double* sc = a.scal + b * 16;
+    const V s = make_float2((float)sc[2], (float)sc[3]), tau = make_float2((float)sc[4], (float)sc[5]);
+    V pa[4], pw[4], v = vzero<V>();
     if (r < n) {
-        // row part from the tiles (blk128(r), bj <= blk64(r)); column part from (bi >= blk128(r), blk64(r))
-        const int64_t Bc = (r - c0) / HV_CB, Br = (r - c0) / HV_RB;
-        const V* Yrow = a.Yrow + b * a.ystride;
-        const V* Ycol = a.Ycol + b * a.ystride;
+        if (sl == 0) v = A[r + col * lda];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int l = sl + 8 * q;
+            pa[q] = l < ii ? A[r + (p + l) * lda] : vzero<V>();
+            pw[q] = l < ii ? W[r + l * n] : vzero<V>();
+        }
+    }
+    if (threadIdx.x >= 192 && rr < ii) {
+        // warps 6 and 7 have the fewest slots: s1, s2 from the dots' partials
+        const V* S = a.Spart + b * a.sstride + (sl - 6) * TRD_NB + rr;
+        V x = vzero<V>();
+        for (int64_t q0 = 0; q0 < nrb; q0 += 8) {
+            V t[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) t[q] = q0 + q < nrb ? S[(q0 + q) * 2 * TRD_NB] : vzero<V>();
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (q0 + q < nrb) x = vadd(x, t[q]);
+        }
+        (sl == 6 ? s1 : s2)[rr] = x;
+    }
+    if (r < n) {
+        // row part from the tiles (blk64(r), bj <= blk64(r)); column part from (bi >= blk64(r), blk64(r))
+        const int64_t B = (r - c0) / HV_RB;
+        const V* Yrow = a.Yrow + b * a.ystride + r;
+        const V* Ycol = a.Ycol + b * a.ystride + r;
+        const int64_t nr = B >= sl ? (B - sl) / 8 + 1 : 0, nt = nr + (nb2 - B > sl ? (nb2 - B - sl + 7) / 8 : 0);
         V y = vzero<V>();
-        for (int64_t q = sl; q <= Bc; q += 8) y = vadd(y, Yrow[q * n + r]);
-        for (int64_t q = Br + sl; q < nb2; q += 8) y = vadd(y, Ycol[q * n + r]);
+        for (int64_t q0 = 0; q0 < nt; q0 += 12) {
+            V t[12];
+#pragma unroll
+            for (int q = 0; q < 12; ++q) {
+                const int64_t u = q0 + q;
+                t[q] = u < nr ? Yrow[(sl + 8 * u) * n] : u < nt ? Ycol[(B + sl + 8 * (u - nr)) * n] : vzero<V>();
+            }
+#pragma unroll
+            for (int q = 0; q < 12; ++q)
+                if (q0 + q < nt) y = vadd(y, t[q]);
+        }
         ysl[sl][rr] = y;
     }
-    __syncthreads();   // s1, s2 and the slot sums are in shared memory
+    __syncthreads();   // s1, s2 are in shared memory
     if (r < n) {
         // the panel corrections -V s1 - W s2, split over the 8 slices
         V y = ysl[sl][rr];
-        for (int l = sl; l < ii; l += 8) {
-            y = vsub(y, vmul(A[r + (p + l) * lda], s1[l]));
-            y = vsub(y, vmul(W[r + l * n], s2[l]));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int l = sl + 8 * q;
+            if (l < ii) {
+                y = vsub(y, vmul(pa[q], s1[l]));
+                y = vsub(y, vmul(pw[q], s2[l]));
+            }
         }
         ysl[sl][rr] = y;
     }
     __syncthreads();
-    T dre = (T)0, dim = (T)0;
-    if (sl == 0 && r < n) {
+    if (sl != 0) return;
+    float dre = 0.f, dim = 0.f;
+    if (r < n) {
         V y = vzero<V>();
 #pragma unroll
         for (int q = 0; q < 8; ++q) y = vadd(y, ysl[q][rr]);
         y = vmul(tau, y);
-        V v = trd_v<T>(A, lda, col, r, sr, si);
+        v = trd_scale(v, r == c0, s.x, s.y);
         A[r + col * lda] = v;
-        W[r + ii * n] = y;
+        a.w0[b * n + r] = y;
         // zdotc(w, v) = sum conj(w) v
-        V cv = vcjmul(y, v);
+        const V cv = vcjmul(y, v);
         dre = cv.x;
         dim = cv.y;
     }
-    const T s_re = block_sum_256(dre, sh);
-    const T s_im = block_sum_256(dim, sh);
-    double* part = a.part + b * a.pstride;
-    if (threadIdx.x == 0) {
-        part[2 * blockIdx.x] = (double)s_re;
-        part[2 * blockIdx.x + 1] = (double)s_im;
-    }
-    if (last_cta(a.cnt + b * 4 + 1, gridDim.x) && threadIdx.x == 0) {
-        double xr = 0.0, xi = 0.0;
-        for (unsigned q = 0; q < gridDim.x; ++q) {
-            xr += ((volatile double*)part)[2 * q];
-            xi += ((volatile double*)part)[2 * q + 1];
-        }
-        // alpha2 = -1/2 tau (w^H v)
-        const double tr = sc[4], ti = sc[5];
-        sc[6] = -0.5 * (tr * xr - ti * xi);
-        sc[7] = -0.5 * (tr * xi + ti * xr);
+    dre = warp_sum_f(dre);
+    dim = warp_sum_f(dim);
+    if (rr == 0) {
+        double* part = a.part + b * a.pstride + trd_col_parts(n) + 2 * blockIdx.x;
+        part[0] = (double)dre;
+        part[1] = (double)dim;
     }
 }
 
-template <class T>
-__global__ void __launch_bounds__(TRD_ROWS) k_trd_fix(TrdArgs<T> a, int ii, int64_t col) {
-    using V = typename CV<T>::type;
-    const int64_t b = blockIdx.y, n = a.n, lda = a.lda;
-    const V* A = a.A + b * a.strideA;
-    V* W = a.W + b * (n * TRD_NB);
-    const double* sc = a.scal + b * 16;
-    const V al = vmake<V>((T)sc[6], (T)sc[7]);
+// w += alpha2 v of the panel's last column (the rank-2k update reads W)
+__global__ void __launch_bounds__(TRD_ROWS) k_trd_fix(TrdArgs<float> a, int ii, int64_t col) {
+    const int64_t b = blockIdx.y, n = a.n;
+    __shared__ float2 s_al;
+    trd_chain_wait();
+    if (threadIdx.x < 32) {
+        const float2 al = trd_alpha2(a, b, (n - col - 1 + 31) / 32);
+        if (threadIdx.x == 0) s_al = al;
+    }
+    __syncthreads();
     const int64_t r = col + 1 + (int64_t)blockIdx.x * TRD_ROWS + threadIdx.x;
-    if (r < n) W[r + ii * n] = vadd(W[r + ii * n], vmul(al, A[r + col * lda]));
+    if (r < n)
+        a.W[b * (n * TRD_NB) + r + ii * n] = trd_corr(a.w0[b * n + r], s_al, a.A[b * a.strideA + r + col * a.lda]);
 }
+
+}  // namespace
 
 // ---------------------------------------------------------------- driver
 int tridiagonalize_f32(cudaStream_t st, TrdArgs<float>& a, int64_t batch) {
@@ -352,30 +439,27 @@ int tridiagonalize_f32(cudaStream_t st, TrdArgs<float>& a, int64_t batch) {
             const int64_t col = p + ii;
             const int has_refl = (col < n - 1) ? 1 : 0;
             const double esz = (double)sizeof(typename CV<T>::type);
-            dim3 ga((unsigned)((n - col + TRD_ROWS - 1) / TRD_ROWS), (unsigned)batch);
+            dim3 ga((unsigned)((n - col + COL_ROWS - 1) / COL_ROWS), (unsigned)batch);
             prof_begin(ST_TRD_COL);
-            k_trd_col<T><<<ga, TRD_ROWS, 0, st>>>(a, p, ii, col, has_refl);
-            FORGE_LAUNCH_CHECK();
+            FORGE_TRY(launch_chain(st, ga, COL_ROWS, k_trd_col, a, p, ii, col, has_refl));
             prof_end(ST_TRD_COL, batch * (double)(n - col) * (2.0 * ii + 2.0) * esz, 0.0);
             if (!has_refl) continue;
             ++nrefl;
             const int64_t n2 = n - col - 1;
             const int64_t nbr = (n2 + HV_RB - 1) / HV_RB;   // 64-row blocks (= 64-column blocks)
             const int64_t ntiles = nbr * (nbr + 1) / 2;     // row block bi holds bi + 1 tiles
-            const int64_t nrb = (n2 + 255) / 256;
-            dim3 gb((unsigned)(ntiles + (ii > 0 ? nrb : 0)), (unsigned)batch);
+            const int64_t nrb = ii > 0 ? (n2 + 255) / 256 : 0;
+            const int64_t ndc = nrb * ((ii + DOT_L - 1) / DOT_L);
+            dim3 gb((unsigned)(ntiles + ndc), (unsigned)batch);
             prof_begin(ST_HEMV);
-            k_trd_hemv<T><<<gb, 256, 0, st>>>(a, p, ii, col, ntiles);
-            FORGE_LAUNCH_CHECK();
+            FORGE_TRY(launch_chain(st, gb, 256, k_trd_hemv, a, p, ii, col, ndc));
             // algorithmic traffic: the trailing lower triangle read once
             prof_end(ST_HEMV, batch * 0.5 * (double)n2 * (double)(n2 + 1) * esz, batch * 8.0 * (double)n2 * n2);
             dim3 gf((unsigned)((n2 + 31) / 32), (unsigned)batch);
             dim3 gc((unsigned)((n2 + TRD_ROWS - 1) / TRD_ROWS), (unsigned)batch);
             prof_begin(ST_TRD_FINISH);
-            k_trd_finish<T><<<gf, TRD_ROWS, 0, st>>>(a, p, ii, col, nbr, ii > 0 ? nrb : 0);
-            FORGE_LAUNCH_CHECK();
-            k_trd_fix<T><<<gc, TRD_ROWS, 0, st>>>(a, ii, col);
-            FORGE_LAUNCH_CHECK();
+            FORGE_TRY(launch_chain(st, gf, TRD_ROWS, k_trd_finish, a, p, ii, col, nbr, nrb));
+            if (ii == w - 1 || col == n - 2) FORGE_TRY(launch_chain(st, gc, TRD_ROWS, k_trd_fix, a, ii, col));
             prof_end(ST_TRD_FINISH, batch * (double)n2 * (2.0 * ii + 4.0) * esz, 0.0);
         }
         if (nrefl > 0 && p + w < n) {

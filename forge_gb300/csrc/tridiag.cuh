@@ -3,15 +3,16 @@
 // LAPACK zhetrd/zlatrd (uplo = 'L') that the reference reaches through zheevr
 // (LapackRoutines.f90:414-426).
 //
-// Per column (all k of the batch in one launch each):
-//   trd_col   : update column col with the panel's previous reflectors, generate
-//               the reflector (zlarfg) in the last CTA (deterministic partials);
+// Per column (all k of the batch in one launch each; names of the FP32 kernels, FP64 has its own set):
+//   trd_col   : add alpha2 v to the last column's w, update column col with the
+//               panel's previous reflectors, generate the reflector (zlarfg) in the
+//               last CTA (deterministic partials);
 //   trd_hemv  : y = A22 v over 64x64 tiles of the trailing lower triangle, every
 //               element read once; row and column partials go to disjoint slots
 //               (Yrow / Ycol) so the reduction order is fixed; extra CTAs form
 //               the panel dots W^H v and V^H v;
-//   trd_finish: y -= V s1 + W s2, W(:,i) = tau y, v written back, alpha2 in the last CTA;
-//   trd_fix   : W(:,i) += alpha2 v.
+//   trd_finish: y -= V s1 + W s2, w0 = tau y, v written back, partials of w^H v.
+// One more launch a panel (trd_fix) adds alpha2 v to its last w.
 // After each panel of NB columns, the trailing matrix gets A22 -= V W^H + W V^H
 // (a rank-2k update on the tensor cores in the chosen precision).
 #pragma once
@@ -24,7 +25,7 @@ constexpr int TRD_NB = 32;      // panel width
 constexpr int TRD_TILE = 64;    // column granularity of the hemv partial slots (Yrow / Ycol)
 constexpr int HV_RB = 64;       // hemv tile rows
 constexpr int HV_CB = 64;       // hemv tile columns
-constexpr int TRD_ROWS = 256;   // rows per CTA in the column kernels
+constexpr int TRD_ROWS = 256;   // rows of one FP32 norm partial; threads per CTA of trd_finish / trd_fix
 
 template <class T>
 struct TrdArgs {
@@ -44,12 +45,35 @@ struct TrdArgs {
     int64_t pstride;
     double* scal;       // batch x 16
     unsigned* cnt;      // batch x 4
-    V* w0 = nullptr;    // batch x n: the last column's w before the alpha2 correction (FP64)
+    V* w0 = nullptr;    // batch x n: the last column's w before the alpha2 correction
     // trailing update on the tensor cores (her2k_oz in FP64, her2k_tc in the mixed path):
     // A(p+w:n, p+w:n) -= V W^H + W V^H for the panel [p, p+w)
     int (*her2k)(cudaStream_t st, TrdArgs<T>& a, int64_t p, int64_t w, int64_t batch, void* user) = nullptr;
     void* her2k_user = nullptr;
 };
+
+// The kernels of a column form one chain; each is launched programmatically (launch_chain) and may be scheduled
+// while its predecessor still runs.  It waits here for the predecessor's results; the next kernel's CTAs are
+// let in as soon as all of this grid's have started.
+__device__ __forceinline__ void trd_chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... Q>
+int launch_chain(cudaStream_t st, dim3 grid, unsigned threads, void (*k)(P...), Q... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+    FORGE_LAUNCH_CHECK();
+    return 0;
+}
 
 int tridiagonalize_f32(cudaStream_t st, TrdArgs<float>& a, int64_t batch);     // tridiag.cu
 int tridiagonalize_fp64(cudaStream_t st, TrdArgs<double>& a, int64_t batch);   // tridiag_fp64.cu

@@ -26,14 +26,6 @@ namespace forge {
 
 namespace {
 
-// The three kernels of a column form one chain; each is launched programmatically (launch_chain) and may be
-// scheduled while its predecessor still runs.  It waits here for the predecessor's results; the next
-// kernel's CTAs are let in as soon as all of this grid's have started.
-__device__ __forceinline__ void chain_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 constexpr int HT = 64;          // tile edge of k_hemv64
 constexpr int FR = 32;          // rows per CTA of k_col64 / k_finish64 (8 threads a row)
 // panel dots: a CTA takes 8 reflectors over 128 rows.  An FP64 instruction occupies a quarter of the SM's pipe
@@ -65,7 +57,7 @@ __global__ void __launch_bounds__(256) k_col64(TrdArgs<double> a, int64_t p, int
     const int rr = threadIdx.x & 31, sl = threadIdx.x >> 5;
     const int64_t r = col + (int64_t)blockIdx.x * FR + rr;
     const double2 z = make_double2(0.0, 0.0);
-    chain_wait();
+    trd_chain_wait();
     // the thread's reflectors l = sl + 8 q, loaded while warp 0 forms alpha2
     double2 x = z, x2 = z, v[4], w[4];
 #pragma unroll
@@ -133,7 +125,7 @@ __global__ void __launch_bounds__(256) k_col64(TrdArgs<double> a, int64_t p, int
 __global__ void __launch_bounds__(256) k_fix64(TrdArgs<double> a, int ii, int64_t col) {
     const int64_t b = blockIdx.y, n = a.n;
     __shared__ double2 s_al;
-    chain_wait();
+    trd_chain_wait();
     if (threadIdx.x < 32) {
         const double2 al = alpha2_of(a, b, (n - col - 1 + FR - 1) / FR);
         if (threadIdx.x == 0) s_al = al;
@@ -171,7 +163,7 @@ __global__ void __launch_bounds__(256, 2) k_hemv64(TrdArgs<double> a, int64_t p,
     const int64_t b = blockIdx.y, n = a.n, lda = a.lda, c0 = col + 1;
     const double2* __restrict__ A = a.A + b * a.strideA;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    chain_wait();
+    trd_chain_wait();
     // the scalars' CTA and the dots (chains of FP64 instructions) go first
     const int64_t t = (int64_t)blockIdx.x - 1 - ndot;
     if (t >= 0) {
@@ -375,7 +367,7 @@ __global__ void __launch_bounds__(256) k_finish64(TrdArgs<double> a, int64_t p, 
     const int rr = threadIdx.x & 31, sl = threadIdx.x >> 5;
     const int64_t r = c0 + (int64_t)blockIdx.x * FR + rr;
     const double2 z = make_double2(0.0, 0.0);
-    chain_wait();
+    trd_chain_wait();
     const double* sc = a.scal + b * 16;
     const double2 s = make_double2(sc[2], sc[3]), tau = make_double2(sc[4], sc[5]);
     // loads of the last steps first
@@ -472,22 +464,6 @@ __global__ void __launch_bounds__(256) k_finish64(TrdArgs<double> a, int64_t p, 
     }
 }
 
-template <class... P, class... Q>
-int launch_chain(cudaStream_t st, dim3 grid, void (*k)(P...), Q... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
-    FORGE_LAUNCH_CHECK();
-    return 0;
-}
-
 }  // namespace
 
 int tridiagonalize_fp64(cudaStream_t st, TrdArgs<double>& a, int64_t batch) {
@@ -499,7 +475,7 @@ int tridiagonalize_fp64(cudaStream_t st, TrdArgs<double>& a, int64_t batch) {
         for (int ii = 0; ii < w; ++ii) {
             const int64_t col = p + ii, n2 = n - col - 1;
             prof_begin(ST_TRD_COL);
-            FORGE_TRY(launch_chain(st, dim3((unsigned)((n - col + FR - 1) / FR), nbat), k_col64, a, p, ii, col));
+            FORGE_TRY(launch_chain(st, dim3((unsigned)((n - col + FR - 1) / FR), nbat), 256, k_col64, a, p, ii, col));
             prof_end(ST_TRD_COL, batch * (double)(n - col) * (2.0 * ii + 2.0) * 16.0, 0.0);
             if (n2 <= 0) {
                 // the last column has no reflector
@@ -511,13 +487,13 @@ int tridiagonalize_fp64(cudaStream_t st, TrdArgs<double>& a, int64_t batch) {
             const int64_t ndot = ii > 0 ? (n2 + DOT_ROWS - 1) / DOT_ROWS : 0;   // slots of the panel dots
             const int64_t ndc = ndot * ((ii + DOT_L - 1) / DOT_L);
             prof_begin(ST_HEMV);
-            FORGE_TRY(launch_chain(st, dim3((unsigned)(ntiles + ndc + 1), nbat), k_hemv64, a, p, ii, col, ndc));
+            FORGE_TRY(launch_chain(st, dim3((unsigned)(ntiles + ndc + 1), nbat), 256, k_hemv64, a, p, ii, col, ndc));
             // algorithmic traffic: the trailing lower triangle read once
             prof_end(ST_HEMV, batch * 0.5 * (double)n2 * (double)(n2 + 1) * 16.0, batch * 8.0 * (double)n2 * n2);
             prof_begin(ST_TRD_FINISH);
-            FORGE_TRY(launch_chain(st, dim3((unsigned)((n2 + FR - 1) / FR), nbat), k_finish64, a, p, ii, col, nb2, ndot));
+            FORGE_TRY(launch_chain(st, dim3((unsigned)((n2 + FR - 1) / FR), nbat), 256, k_finish64, a, p, ii, col, nb2, ndot));
             if (ii == w - 1 || col == n - 2) {
-                FORGE_TRY(launch_chain(st, dim3((unsigned)((n2 + 255) / 256), nbat), k_fix64, a, ii, col));
+                FORGE_TRY(launch_chain(st, dim3((unsigned)((n2 + 255) / 256), nbat), 256, k_fix64, a, ii, col));
             }
             prof_end(ST_TRD_FINISH, batch * (double)n2 * (2.0 * ii + 4.0) * 16.0, 0.0);
         }
