@@ -30,9 +30,8 @@ struct EigArgs {
     double* info;               // batch x 8
     int* clus;                  // batch x (iu + 2)
     double* Z;                  // batch x n x iu (row-major)
-    double* scr;                // 4 x n x (scr_stride * batch)
-    unsigned char* pivs;        // n x (scr_stride * batch)
-    int64_t scr_stride;         // >= iu
+    double* scr;                // 4 x n x (iu * batch)
+    unsigned char* pivs;        // n x (iu * batch)
     int* fail;                  // batch
     // FP64 products on the tensor cores (oz_fp64.cu): slices of X (and U, Z of the rank-2k update), V, V^H, W
     // and T; W and W2, the Gram matrices and T in FP64; row scales; error flag of the bounded waits

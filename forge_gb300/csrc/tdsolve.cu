@@ -162,19 +162,60 @@ __device__ inline int sturm(const T2* __restrict__ de, int n, T x) {
 // number of eigenpairs wanted of matrix b (a padded slot of a group wants its own nUpper)
 __device__ inline int64_t want_of(const int* lim, int64_t b, int64_t iu) { return lim ? (int64_t)lim[b] : iu; }
 
+// ---------------------------------------------------------------- division by FMAs
+// exponent of |x| (biased; 0 for zero and subnormals, 2047 for Inf and NaN)
+__device__ __forceinline__ int expo_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+// operands whose quotient, remainder and products of two neither over- nor underflow
+__device__ __forceinline__ bool mid_expo(double x) { return (unsigned)(expo_of(x) - 524) < 1000u; }
+// Reciprocal to about 2^-46: one Newton step on the hardware's approximation (2^-23).
+__device__ __forceinline__ double recip(double b) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+    return fma(r, fma(-b, r, 1.0), r);
+}
+// a / b from r = recip(b) for operands in mid-range: the remainder of a r brings the quotient to 2^-92 before its
+// one rounding (P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34 (1990)), so it is the rounded quotient but for one case in about 2^39.  Five FMAs with
+// recip: an FP64 instruction of a warp holds its scheduler's FP64 pipe for 64 clocks on this GPU, whatever the
+// number of lanes, so the count of them is what the serial chains below cost.
+__device__ __forceinline__ double quot(double a, double b, double r) {
+    const double q = a * r;
+    return fma(fma(-q, b, a), r, q);
+}
+
 // ---------------------------------------------------------------- quotient form (mixed precision)
-// number of eigenvalues <= x (dlaebz Sturm count)
-__device__ inline int sturm_q(const double* __restrict__ D, const double* __restrict__ E, int n, double x,
-                              double pivmin) {
-    double q = D[0] - x;
+// number of eigenvalues <= x (dlaebz Sturm count); t[i] = (d_i, e_{i-1}^2)
+__device__ inline int sturm_q(const double2* __restrict__ t, int n, double x, double pivmin) {
+    constexpr int U = 8;
+    double q = t[0].x - x;
     if (fabs(q) < pivmin) q = -pivmin;
     int cnt = (q <= 0.0) ? 1 : 0;
-#pragma unroll 4
-    for (int i = 1; i < n; ++i) {
-        const double e = E[i - 1];
-        q = D[i] - e * e / q - x;
-        if (fabs(q) < pivmin) q = -pivmin;
-        cnt += (q <= 0.0) ? 1 : 0;
+    const bool small_piv = expo_of(pivmin) < 524;
+    double2 nx[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) nx[u] = t[min(1 + u, n - 1)];
+    for (int i0 = 1; i0 < n; i0 += U) {
+        double2 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = nx[u];
+#pragma unroll
+        for (int u = 0; u < U; ++u) nx[u] = t[min(i0 + U + u, n - 1)];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i0 + u >= n) break;
+            double f;
+            if (mid_expo(q) && mid_expo(v[u].y))
+                f = quot(v[u].y, q, recip(q));
+            else
+                f = v[u].y / q;
+            q = v[u].x - f - x;
+            if (!(small_piv && mid_expo(q))) {
+                if (fabs(q) < pivmin) q = -pivmin;
+                cnt += (q <= 0.0) ? 1 : 0;
+            } else {
+                cnt += (int)((unsigned)__double2hiint(q) >> 31);
+            }
+        }
     }
     return cnt;
 }
@@ -192,120 +233,61 @@ __device__ inline int sturm_qf(const float* __restrict__ D, const float* __restr
     }
     return cnt;
 }
-// FP32 copies of the unscaled tridiagonal: tq[b][0..n) = d, tq[b][n..2n) = e^2
-__global__ void k_tri_to_f32(const double* __restrict__ d, const double* __restrict__ e, int64_t n,
-                             float* __restrict__ tq) {
+// The unscaled tridiagonal for the quotient form: t[b][i] = (d_i, e_{i-1}^2), and in FP32 tq[b][0..n) = d,
+// tq[b][n..2n) = e^2
+__global__ void k_tri_quot(const double* __restrict__ d, const double* __restrict__ e, int64_t n, double2* __restrict__ t,
+                           float* __restrict__ tq) {
     const int64_t b = blockIdx.y;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double em = (i > 0) ? e[b * n + i - 1] : 0.0;
+        t[b * n + i] = make_double2(d[b * n + i], em * em);
         tq[b * 2 * n + i] = (float)d[b * n + i];
         const double ei = (i < n - 1) ? e[b * n + i] : 0.0;
         tq[b * 2 * n + n + i] = (float)(ei * ei);
     }
 }
-// FP32 bisection of eigenvalue j in the quotient form, into w.  As in k_bisect_replay, a midpoint further
-// than 64 eps_32 |T| from the eigenvalue lam is decided without a count.
-__global__ void __launch_bounds__(32) k_bisect_qf(const float* __restrict__ tq, int64_t n, int64_t iu,
-                                                  const int* __restrict__ lim, const double* __restrict__ info,
-                                                  const double* __restrict__ lam, double* __restrict__ w) {
-    const int64_t b = blockIdx.y;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= want_of(lim, b, iu)) return;
-    const float* D = tq + b * 2 * n;
-    const float* E2 = D + n;
-    // Gershgorin bounds widened by the FP32 rounding of the counts
-    const float tn = (float)info[b * 8 + 4];
-    float lo = (float)info[b * 8 + 0] - 8.f * FLT_EPSILON * tn * 64.f, hi = (float)info[b * 8 + 1] + 8.f * FLT_EPSILON * tn * 64.f;
-    const float pivmin = fmaxf(1e-30f, (float)info[b * 8 + 3]);
-    const double l = lam[b * iu + j], far = 64.0 * (double)FLT_EPSILON * info[b * 8 + 4];
-    for (int it = 0; it < 64; ++it) {
-        const float width = hi - lo;
-        if (width <= 2.f * FLT_EPSILON * fmaxf(fabsf(lo), fabsf(hi)) || width <= pivmin) break;
-        const float mid = 0.5f * (lo + hi);
-        if (mid <= lo || mid >= hi) break;
-        const bool up = mid > l + far ? true : mid < l - far ? false : sturm_qf(D, E2, (int)n, mid, pivmin) >= j + 1;
-        if (up)
-            hi = mid;
-        else
-            lo = mid;
-    }
-    w[b * iu + j] = 0.5 * ((double)lo + (double)hi);
-}
-// The FP64 bisection of the mixed path, from the bracket x -/+ 8 eps_32 |T| of the FP32 estimate x when
-// the counts confirm it.  Its midpoints form a fixed dyadic sequence, and the quotient-form count decides
-// each: where a midpoint lies further from the eigenvalue that k_bisect found (lam) than 64 eps |T|,
-// many times the error of either count, the decision is known without a count; only the last few
-// are counted, several levels of the bisection tree at once (G lanes hold the 2^LEV - 1
-// midpoints of LEV levels).  Why not k_bisect's own result: the mixed path rounds the eigenvectors to
-// FP32 afterwards, and that rounding noise stays in the refined density matrix to second order
-// (3e-9 of its norm at N = 1324), so a last-place change of an eigenvalue would change the results by
-// as much; this keeps them bit for bit.  Bound: latency of the division chain, ~1300 clocks a step.
-// Measured, stage total with k_bisect: N = 5044, all eigenvalues 138 -> 51 ms; N = 1876, 9 k 46 -> 26 ms.
-template <int LEV>
-__global__ void __launch_bounds__(32) k_bisect_replay(const double* __restrict__ d, const double* __restrict__ e,
-                                                      int64_t n, int64_t iu, const int* __restrict__ lim,
-                                                      const double* __restrict__ info, const double* __restrict__ lam,
-                                                      double* __restrict__ w) {
+// Bisection of [lo, hi] while open(lo, hi), at most maxit halvings: where known(mid) is not 0 its sign is the decision
+// (+1: the eigenvalue is not above mid), elsewhere count(mid) is.  The 2^LEV - 1 midpoints of the next LEV
+// levels are counted at once by the G lanes of the eigenvalue's group.
+template <int LEV, class T, class Open, class Known, class Count>
+__device__ __forceinline__ void bisect_tree(T& lo, T& hi, bool live, int maxit, Open open, Known known, Count count) {
     constexpr int G = LEV == 1 ? 1 : 1 << LEV;
-    const int64_t b = blockIdx.y;
-    const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
     const int g = threadIdx.x % G, base = (threadIdx.x & 31) / G * G;
     const unsigned full = 0xffffffffu;
-    const bool live = j < want_of(lim, b, iu);
-    const double* D = d + b * n;
-    const double* E = e + b * n;
-    double lo = info[b * 8 + 0], hi = info[b * 8 + 1];
-    const double pivmin = info[b * 8 + 3], tnorm = info[b * 8 + 4];
-    const double l = live ? lam[b * iu + j] : 0.0, far = 64.0 * kEps * tnorm;
-    if (live) {
-        const double x = w[b * iu + j], delta = 8.0 * (double)FLT_EPSILON * tnorm;
-        const double l2 = fmax(lo, x - delta), h2 = fmin(hi, x + delta);
-        if (l2 < h2) {
-            const bool lok = l2 < l - far ? true : l2 > l + far ? false : sturm_q(D, E, (int)n, l2, pivmin) < j + 1;
-            const bool hok = h2 > l + far ? true : h2 < l - far ? false : sturm_q(D, E, (int)n, h2, pivmin) >= j + 1;
-            if (lok && hok) {
-                lo = l2;
-                hi = h2;
-            }
-        }
-    }
-    const double rtol = 4.0 * kEps;
-    auto open = [&](double a, double c) {
-        return c - a > fmax(fmax(kSafmin, pivmin), rtol * fmax(fabs(a), fabs(c)));
-    };
     int it = 0;
     for (;;) {
         // decisions that need no count
-        while (live && it < 256 && open(lo, hi)) {
-            const double mid = 0.5 * (lo + hi);
-            if (mid > l + far)
+        while (live && it < maxit && open(lo, hi)) {
+            const T mid = (T)0.5 * (lo + hi);
+            const int k = known(mid);
+            if (k == 0) break;
+            if (k > 0)
                 hi = mid;
-            else if (mid < l - far)
-                lo = mid;
             else
-                break;
+                lo = mid;
             ++it;
         }
-        const bool more = live && it < 256 && open(lo, hi);
+        const bool more = live && it < maxit && open(lo, hi);
         if (!__any_sync(full, more)) break;
         // lane g holds node g of the tree (1: root; children 2g, 2g + 1 = lower, upper half)
-        double a = lo, c = hi;
+        T a = lo, c = hi;
         if (G > 1)
             for (int bit = 30 - __clz(g > 0 ? g : 1); bit >= 0; --bit) {
-                const double mid = 0.5 * (a + c);
+                const T mid = (T)0.5 * (a + c);
                 if ((g >> bit) & 1)
                     a = mid;
                 else
                     c = mid;
             }
         bool up = false;
-        if (more && (G == 1 || g > 0)) up = sturm_q(D, E, (int)n, 0.5 * (a + c), pivmin) >= j + 1;
+        if (more && (G == 1 || g > 0)) up = count((T)0.5 * (a + c));
         const unsigned ups = __ballot_sync(full, up) >> base;
         if (more) {
             int node = G == 1 ? 0 : 1;
 #pragma unroll
             for (int q = 0; q < LEV; ++q) {
-                if (it < 256 && open(lo, hi)) {
-                    const double mid = 0.5 * (lo + hi);
+                if (it < maxit && open(lo, hi)) {
+                    const T mid = (T)0.5 * (lo + hi);
                     const bool u = (ups >> node) & 1u;
                     if (u)
                         hi = mid;
@@ -317,36 +299,119 @@ __global__ void __launch_bounds__(32) k_bisect_replay(const double* __restrict__
             }
         }
     }
-    if (g == 0 && j < iu) w[b * iu + j] = live ? 0.5 * (lo + hi) : 0.0;
+}
+// FP32 bisection of eigenvalue j in the quotient form, into w.  As in k_bisect_replay, a midpoint further
+// than 64 eps_32 |T| from the eigenvalue lam is decided without a count.
+template <int LEV>
+__global__ void __launch_bounds__(32) k_bisect_qf(const float* __restrict__ tq, int64_t n, int64_t iu,
+                                                  const int* __restrict__ lim, const double* __restrict__ info,
+                                                  const double* __restrict__ lam, double* __restrict__ w) {
+    constexpr int G = LEV == 1 ? 1 : 1 << LEV;
+    const int64_t b = blockIdx.y;
+    const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+    const bool live = j < want_of(lim, b, iu);
+    const float* D = tq + b * 2 * n;
+    const float* E2 = D + n;
+    // Gershgorin bounds widened by the FP32 rounding of the counts
+    const float tn = (float)info[b * 8 + 4];
+    float lo = (float)info[b * 8 + 0] - 8.f * FLT_EPSILON * tn * 64.f, hi = (float)info[b * 8 + 1] + 8.f * FLT_EPSILON * tn * 64.f;
+    const float pivmin = fmaxf(1e-30f, (float)info[b * 8 + 3]);
+    const double l = live ? lam[b * iu + j] : 0.0, far = 64.0 * (double)FLT_EPSILON * info[b * 8 + 4];
+    bisect_tree<LEV>(
+        lo, hi, live, 64,
+        [&](float a, float c) {
+            const float width = c - a, mid = 0.5f * (a + c);
+            return !(width <= 2.f * FLT_EPSILON * fmaxf(fabsf(a), fabsf(c)) || width <= pivmin || mid <= a || mid >= c);
+        },
+        [&](float mid) { return mid > l + far ? 1 : mid < l - far ? -1 : 0; },
+        [&](float mid) { return sturm_qf(D, E2, (int)n, mid, pivmin) >= j + 1; });
+    if (live && threadIdx.x % G == 0) w[b * iu + j] = 0.5 * ((double)lo + (double)hi);
+}
+// The FP64 bisection of the mixed path, from the bracket x -/+ 8 eps_32 |T| of the FP32 estimate x when
+// the counts confirm it.  Its midpoints form a fixed dyadic sequence, and the quotient-form count decides
+// each: where a midpoint lies further from the eigenvalue that k_bisect found (lam) than 64 eps |T|,
+// many times the error of either count, the decision is known without a count; only the last few
+// are counted, several levels of the bisection tree at once.  Why not k_bisect's own result: the mixed path rounds
+// the eigenvectors to FP32 afterwards, and that rounding noise stays in the refined density matrix to second order
+// (3e-9 of its norm at N = 1324), so a last-place change of an eigenvalue would change the results by
+// as much; this keeps them bit for bit.  Bound: the FP64 instructions of a step, seven.
+// Measured, kernel alone (a library division a step before): N = 5044, all eigenvalues 31 -> 17 ms; the whole stage
+// 51 -> 32 ms, N = 1324, 4 k 25 -> 16 ms, N = 1876, 9 k 26.5 -> 16 ms.
+template <int LEV>
+__global__ void __launch_bounds__(32) k_bisect_replay(const double2* __restrict__ de, int64_t n, int64_t iu,
+                                                      const int* __restrict__ lim, const double* __restrict__ info,
+                                                      const double* __restrict__ lam, double* __restrict__ w) {
+    constexpr int G = LEV == 1 ? 1 : 1 << LEV;
+    const int64_t b = blockIdx.y;
+    const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+    const bool live = j < want_of(lim, b, iu);
+    const double2* t = de + b * n;
+    double lo = info[b * 8 + 0], hi = info[b * 8 + 1];
+    const double pivmin = info[b * 8 + 3], tnorm = info[b * 8 + 4];
+    const double l = live ? lam[b * iu + j] : 0.0, far = 64.0 * kEps * tnorm;
+    auto known = [&](double mid) { return mid > l + far ? 1 : mid < l - far ? -1 : 0; };
+    auto count = [&](double mid) { return sturm_q(t, (int)n, mid, pivmin) >= j + 1; };
+    if (live) {
+        const double x = w[b * iu + j], delta = 8.0 * (double)FLT_EPSILON * tnorm;
+        const double l2 = fmax(lo, x - delta), h2 = fmin(hi, x + delta);
+        if (l2 < h2) {
+            const int kl = known(l2), kh = known(h2);
+            const bool lok = kl ? kl < 0 : !count(l2);
+            const bool hok = kh ? kh > 0 : count(h2);
+            if (lok && hok) {
+                lo = l2;
+                hi = h2;
+            }
+        }
+    }
+    const double rtol = 4.0 * kEps;
+    bisect_tree<LEV>(
+        lo, hi, live, 256,
+        [&](double a, double c) { return c - a > fmax(fmax(kSafmin, pivmin), rtol * fmax(fabs(a), fabs(c))); }, known, count);
+    if (threadIdx.x % G == 0 && j < iu) w[b * iu + j] = live ? 0.5 * (lo + hi) : 0.0;
 }
 
 // ---------------------------------------------------------------- multisection (minors)
-// eigenvalue j of the scaled T by bisection to FP32 accuracy, into w (scaled)
-__global__ void k_bisect_f32(const float2* __restrict__ tf, int64_t n, int64_t iu, const int* __restrict__ lim,
-                             const double* __restrict__ info, double* __restrict__ w) {
+// Eigenvalue j of the scaled T to FP32 accuracy, into w (scaled): multisection by G lanes as in k_bisect.
+template <int G>
+__global__ void __launch_bounds__(32) k_bisect_f32(const float2* __restrict__ tf, int64_t n, int64_t iu,
+                                                   const int* __restrict__ lim, const double* __restrict__ info,
+                                                   double* __restrict__ w) {
     const int64_t b = blockIdx.y;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= want_of(lim, b, iu)) return;
+    const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+    const int g = threadIdx.x % G, base = (threadIdx.x & 31) / G * G;
+    const bool live = j < want_of(lim, b, iu);
+    const unsigned full = 0xffffffffu;
+    const unsigned gmask = (unsigned)(((1ull << G) - 1ull) << base);
     const double s = tri_scale(info + b * 8);
     // Gershgorin bounds widened by the FP32 rounding of the counts
     float lo = (float)(info[b * 8 + 0] * s) - 512.f * FLT_EPSILON, hi = (float)(info[b * 8 + 1] * s) + 512.f * FLT_EPSILON;
     for (int it = 0; it < 64; ++it) {
         // the counts are good to a few FP32 ulps of |T| <= 1
-        if (!(hi - lo > FLT_EPSILON)) break;
-        const float mid = 0.5f * (lo + hi);
-        if (mid <= lo || mid >= hi) break;
-        if (sturm<float>(tf + b * n, (int)n, mid) >= j + 1)
-            hi = mid;
-        else
-            lo = mid;
+        const float width = hi - lo;
+        const bool open = live && width > FLT_EPSILON;
+        if (!__any_sync(full, open)) break;
+        const float x = lo + width * ((float)(g + 1) / (float)(G + 1));
+        bool up = true;
+        if (open) up = sturm<float>(tf + b * n, (int)n, x) >= j + 1;
+        const unsigned ups = (__ballot_sync(full, up) & gmask) >> base;
+        const int f = ups ? __ffs(ups) - 1 : G;
+        const float xf = __shfl_sync(full, x, base + (f < G ? f : G - 1));
+        const float xp = __shfl_sync(full, x, base + (f > 0 ? f - 1 : 0));
+        if (open) {
+            if (f < G) hi = fminf(hi, xf);
+            if (f > 0) lo = fmaxf(lo, xp);
+            // no representable point inside the bracket
+            if (!(hi - lo < width)) lo = hi = 0.5f * (lo + hi);
+        }
     }
-    w[b * iu + j] = 0.5 * ((double)lo + (double)hi);
+    if (live && g == 0) w[b * iu + j] = 0.5 * ((double)lo + (double)hi);
 }
 
 // Eigenvalue j in FP64 by multisection: G lanes evaluate the Sturm counts at G equally spaced points of
 // the bracket, which shrinks by G + 1 a round.  The bracket starts from the FP32 estimate in w: it is
 // widened by 16 until the FP64 counts confirm it, at last to the Gershgorin interval.  Stops at the
-// reference's 4 eps |lambda|.  G (launch rule in tridiag_eigvecs): a round costs the latency of n
+// reference's 4 eps |lambda|, or at abstol (scaled) where that is wider.  G (launch rule in tridiag_eigvecs): a round costs the latency of n
 // dependent steps as long as the FP64 pipes are not full, so few eigenvalues take many lanes each.
 // Bound: FP64 pipe (three slots a step) or, below ~19000 lanes, the latency of the chain.  Measured,
 // FP64 stage total (quotient-form bisection by one lane before): N = 1324, 16 k 47.9 -> 6.4 ms;
@@ -354,7 +419,7 @@ __global__ void k_bisect_f32(const float2* __restrict__ tf, int64_t n, int64_t i
 template <int G>
 __global__ void __launch_bounds__(32) k_bisect(const double2* __restrict__ de, int64_t n, int64_t iu,
                                                 const int* __restrict__ lim, const double* __restrict__ info,
-                                                double* w) {
+                                                double abstol, double* w) {
     const int64_t b = blockIdx.y;
     const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
     const int g = threadIdx.x % G;
@@ -391,7 +456,7 @@ __global__ void __launch_bounds__(32) k_bisect(const double2* __restrict__ de, i
     const double rtol = 4.0 * kEps;
     for (int it = 0; it < 256; ++it) {
         const double width = hi - lo;
-        const double tol = fmax(8.636168555094445e-78, rtol * fmax(fabs(lo), fabs(hi)));   // >= 2^-256
+        const double tol = fmax(abstol, rtol * fmax(fabs(lo), fabs(hi)));
         const bool open = live && width > tol;
         if (!__any_sync(full, open)) break;
         const double x = lo + width * ((double)(g + 1) / (double)(G + 1));
@@ -449,144 +514,245 @@ __device__ inline uint64_t mix64(uint64_t x) {
     return x;
 }
 
-// a / b from r = RN(1 / b), correctly rounded for operands whose quotient and remainder neither over- nor
-// underflow (P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", IBM J. Res. Dev. 34 (1990)): three dependent FMAs once r is known.
-__device__ __forceinline__ double quot(double a, double b, double r) {
-    const double q = a * r;
-    return fma(fma(-q, b, a), r, q);
-}
-// exponent of |x| (biased; 0 for zero and subnormals, 2047 for Inf and NaN)
-__device__ __forceinline__ int expo_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+// |x| as an integer: absolute values compare as their bit patterns, off the FP64 pipe
+__device__ __forceinline__ uint64_t abs_bits(double x) { return (uint64_t)__double_as_longlong(x) & 0x7fffffffffffffffULL; }
 
-// Inverse iteration, one thread per cluster.  Scratch per thread (strided by 'stride' threads): a, b, c, dd
-// (doubles), piv (bytes).  Every pass is a serial chain over the rows (a division a row in the
-// factorization and the back-substitution), so the rows' loads are issued IV_U rows ahead of their use
-// and the reciprocals of everything that is known before the chain gets there (the pivots of the
-// back-substitution; scale and off-diagonal of the factorization) are formed off the chain.  Measured:
-// N = 5044, all eigenvectors, some clusters of two 80 -> 39 ms; N = 1876, 9 k 16.9 -> 6.9 ms.
+// Inverse iteration (dstein).  What bounds it is the count of FP64 instructions along the serial chains over the
+// rows (see quot): twelve a row for a factorization, nine for a solve; comparisons and maxima go by bit patterns, the
+// pivot is chosen by cross products unless the two quotients agree to 2^-48, and a row's one quotient is
+// that of the chosen branch.  Rows are loaded IV_U ahead.  Only the orthogonalisation inside a cluster has to go
+// member by member: k_invit_lu factorizes for every eigenvalue at once, k_invit<0> does the whole iteration for
+// the first member of each cluster and the first solve for the others, k_invit<1> the rest of these with eight lanes a
+// cluster.  Scratch (rows of pitch S = batch iu): diagonal, first and second superdiagonal
+// of U, multipliers, pivots; the last row's free multiplier slot holds the tolerance of the tiny pivots.
+// Measured (stage, one thread a cluster and a division a row before): N = 5044, all eigenvectors of one matrix 18.4 ->
+// 12 ms without clusters, 64 -> 29 ms with one of about five; N = 1324, 4 k, some clusters 24 -> 12 ms; N = 1876, 9 k
+// 6.9 -> 4.6 ms.
 constexpr int IV_U = 8;
-__global__ void __launch_bounds__(32)
-    k_invit(const double* __restrict__ d, const double* __restrict__ e, int64_t n_, int64_t iu,
-            const double* __restrict__ w, const int* __restrict__ lim, const double* __restrict__ info, double ortol_rel,
-            const int* __restrict__ clus, double* Z /* batch x (n x iu) row-major */, double* scr, unsigned char* pivs,
-            int64_t stride, int* __restrict__ fail) {
-    const int64_t b = blockIdx.y;
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int* C = clus + b * (iu + 2);
-    const int ncl = C[0];
-    if (t >= ncl) return;
-    const int n = (int)n_;
-    const double* __restrict__ D = d + b * n_;
-    const double* __restrict__ E = e + b * n_;
-    const double* Wb = w + b * iu;
-    double* Zb = Z + b * n_ * iu;
-    const int64_t S = stride * gridDim.y;           // scratch row pitch
-    double* ua = scr + b * stride + t;              // diag of U
-    double* ub = ua + n_ * S;                       // first super-diag of U
-    double* uc = ub + n_ * S;                       // multipliers
-    double* ud = uc + n_ * S;                       // second super-diag of U
-    unsigned char* up = pivs + b * stride + t;
-    const double onenrm = info[b * 8 + 2];
-    const int js = C[1 + t];
-    const int64_t nw = want_of(lim, b, iu);
-    int je = js + 1;
-    while (je < nw && !(Wb[je] - Wb[je - 1] > ortol_rel * onenrm)) ++je;
-    if (onenrm == 0.0) {
-        // T = 0: any orthonormal basis (the scaled right-hand sides below would vanish)
-        for (int j = js; j < je; ++j)
-            for (int i = 0; i < n; ++i) Zb[i * iu + j] = (i == j) ? 1.0 : 0.0;
-        return;
+
+struct InvitArgs {
+    const double *d, *e, *w, *info;
+    const int *lim, *clus;
+    int64_t n, iu;
+    double ortol_rel;
+    double* Z;   // batch x (n x iu) row-major
+    double* scr;
+    unsigned char* pivs;
+    int* fail;
+};
+__device__ __forceinline__ bool starts_cluster(const double* W, int64_t j, double ortol) {
+    return j == 0 || W[j] - W[j - 1] > ortol;
+}
+
+// dlagtf: T - xj I = P L U; tol: dlagts tolerance for job = -1
+__global__ void __launch_bounds__(32) k_invit_lu(InvitArgs g) {
+    const int64_t b = blockIdx.y, j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const double onenrm = g.info[b * 8 + 2];
+    if (j >= want_of(g.lim, b, g.iu) || onenrm == 0.0) return;
+    const int n = (int)g.n;
+    const double* __restrict__ D = g.d + b * n;
+    const double* __restrict__ E = g.e + b * n;
+    const double* Wb = g.w + b * g.iu;
+    const int64_t S = g.iu * gridDim.y;
+    double* ua = g.scr + b * g.iu + j;
+    double* ub = ua + n * S;
+    double* uc = ub + n * S;
+    double* ud = uc + n * S;
+    unsigned char* up = g.pivs + b * g.iu + j;
+    // close eigenvalues of a cluster are moved apart
+    int64_t js = j;
+    while (!starts_cluster(Wb, js, g.ortol_rel * onenrm)) --js;
+    double xj = Wb[js];
+    for (int64_t q = js + 1; q <= j; ++q) {
+        const double xm = xj, pertol = 10.0 * fabs(kEps * Wb[q]);
+        xj = Wb[q];
+        if (xj - xm < pertol) xj = xm + pertol;
     }
-    double xjm = 0.0;
-    for (int j = js; j < je; ++j) {
-        double xj = Wb[j];
-        if (j > js) {
-            double pertol = 10.0 * fabs(kEps * xj);
-            if (xj - xjm < pertol) xj = xjm + pertol;
+    double ak = D[0] - xj, bk = (n > 1) ? E[0] : 0.0;
+    double scale1 = fabs(ak) + ((n > 1) ? fabs(E[0]) : 0.0);
+    uint64_t big = 0;
+    double nd[IV_U], ne[IV_U];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < IV_U; ++q) {
+            nd[q] = D[min(k0 + q + 1, n - 1)];
+            ne[q] = k0 + q + 1 < n - 1 ? E[k0 + q + 1] : 0.0;
         }
-        xjm = xj;
-        double* z = Zb + j;
-        // ---- dlagtf: T - xj I = P L U; tol: dlagts tolerance for job = -1
-        double tol, unn;
-        {
-            double ak = D[0] - xj, bk = (n > 1) ? E[0] : 0.0;
-            double scale1 = fabs(ak) + ((n > 1) ? fabs(E[0]) : 0.0), rs1 = 1.0 / scale1;
-            tol = 0.0;
-#pragma unroll 4
-            for (int k = 0; k < n - 1; ++k) {
-                const double ck = E[k];
-                double ak1 = D[k + 1] - xj;
-                double bk1 = (k < n - 2) ? E[k + 1] : 0.0;
-                double scale2 = fabs(ck) + fabs(ak1);
-                if (k < n - 2) scale2 += fabs(bk1);
-                // off the chain: 1 / scale2, 1 / ck; the quotients by them need operands in mid-range
-                const double rs2 = 1.0 / scale2, rc = 1.0 / ck;
-                const int ea = expo_of(ak), ec = expo_of(ck), e1 = expo_of(scale1), e2 = expo_of(scale2);
-                const bool mid = min(min(ea, ec), min(e1, e2)) > 512 && max(max(ea, ec), max(e1, e2)) < 1536;
-                double qa, qc, m1;
-                const double m0 = ck / ak;
-                if (mid) {
-                    qa = quot(fabs(ak), scale1, rs1);
-                    qc = quot(fabs(ck), scale2, rs2);
-                    m1 = quot(ak, ck, rc);
-                } else {
-                    qa = fabs(ak) / scale1;
-                    qc = fabs(ck) / scale2;
-                    m1 = ak / ck;
-                }
-                const double piv1 = (ak == 0.0) ? 0.0 : qa;
-                unsigned char pv = 0;
-                double dk = 0.0, a = ak, bb = bk, c = 0.0;
-                if (ck == 0.0) {
-                    scale1 = scale2;
-                    rs1 = rs2;
-                } else {
-                    const double piv2 = qc;
-                    if (piv2 <= piv1) {
-                        scale1 = scale2;
-                        rs1 = rs2;
-                        const double m = m0;
-                        c = m;
-                        ak1 = ak1 - m * bk;
-                    } else {
-                        pv = 1;
-                        const double mult = m1;
-                        a = ck;
-                        const double temp = ak1;
-                        ak1 = bk - mult * temp;
-                        if (k < n - 2) {
-                            dk = bk1;
-                            bk1 = -mult * dk;
-                        }
-                        bb = temp;
-                        c = mult;
-                    }
-                }
-                const int64_t o = (int64_t)k * S;
-                ua[o] = a;
-                ub[o] = bb;
-                uc[o] = c;
-                ud[o] = dk;
-                up[o] = pv;
-                tol = fmax(tol, fmax(fabs(a), fmax(fabs(bb), fabs(dk))));
-                ak = ak1;
-                bk = bk1;
+    };
+    fetch(0);
+    double ck = bk;   // E[k]
+    for (int k0 = 0; k0 < n - 1; k0 += IV_U) {
+        double cd[IV_U], ce[IV_U];
+#pragma unroll
+        for (int q = 0; q < IV_U; ++q) {
+            cd[q] = nd[q];
+            ce[q] = ne[q];
+        }
+        fetch(k0 + IV_U);
+#pragma unroll
+        for (int q = 0; q < IV_U; ++q) {
+            const int k = k0 + q;
+            if (k >= n - 1) break;
+            double ak1 = cd[q] - xj, bk1 = ce[q];
+            const double scale2 = k < n - 2 ? fabs(ck) + fabs(ak1) + fabs(bk1) : fabs(ck) + fabs(ak1);
+            double a = ak, bb = bk, c = 0.0, dk = 0.0;
+            unsigned char pv = 0;
+            const bool mid = mid_expo(ak) && mid_expo(ck) && mid_expo(scale1) && mid_expo(scale2);
+            const int64_t dx = mid ? __double_as_longlong(fabs(ck) * scale1) - __double_as_longlong(fabs(ak) * scale2) : 0;
+            bool swap;
+            if (mid && (dx > 16 || dx < -16)) {
+                swap = dx > 0;
+            } else {
+                const double piv1 = (ak == 0.0) ? 0.0 : fabs(ak) / scale1, piv2 = fabs(ck) / scale2;
+                swap = !(ck == 0.0) && !(piv2 <= piv1);
             }
-            unn = ak;
-            ua[(int64_t)(n - 1) * S] = ak;
-            tol = fmax(tol, fabs(ak));
+            if (ck == 0.0) {
+                scale1 = scale2;
+            } else {
+                const double num = swap ? ak : ck, den = swap ? ck : ak;
+                c = mid ? quot(num, den, recip(den)) : num / den;
+                // without / with exchange: ak1 - c bk and bk1, or bk - c ak1 and -c bk1
+                const double x = swap ? bk : ak1, y = swap ? ak1 : bk;
+                ak1 = fma(-c, y, x);
+                if (swap) {
+                    pv = 1;
+                    a = ck;
+                    bb = y;
+                    if (k < n - 2) {
+                        dk = bk1;
+                        bk1 = -c * dk;
+                    }
+                } else {
+                    scale1 = scale2;
+                }
+            }
+            const int64_t o = (int64_t)k * S;
+            ua[o] = a;
+            ub[o] = bb;
+            uc[o] = c;
+            ud[o] = dk;
+            up[o] = pv;
+            big = max(max(big, abs_bits(a)), max(abs_bits(bb), abs_bits(dk)));
+            ak = ak1;
+            bk = bk1;
+            ck = ce[q];
         }
-        tol *= kEps;
-        if (tol == 0.0) tol = kEps;
-        // ---- starting vector in Z(:, j)
-        uint64_t seed = mix64(((uint64_t)b << 40) ^ ((uint64_t)j * 0x9e3779b97f4a7c15ULL) ^ 0x1234567ULL);
+    }
+    ua[(int64_t)(n - 1) * S] = ak;
+    big = max(big, abs_bits(ak));
+    double tol = __longlong_as_double((long long)big) * kEps;
+    if (tol == 0.0) tol = kEps;
+    uc[(int64_t)(n - 1) * S] = tol;
+}
+
+// One pass over z by the IV_G lanes of a cluster: z -= dot u (u may be null), *dot_next = sum z un over the rows in
+// order (un may be null) and the largest |z|, as bits.  The update is one instruction for IV_G rows; the sum's
+// operands go round by shuffles, so that its chain of FMAs is all that a row costs.
+constexpr int IV_G = 8;
+__device__ __forceinline__ void mgs_pass(unsigned mask, int n, int64_t iu, double* z, const double* u, double dot,
+                                         const double* un, double* dot_next, uint64_t* top) {
+    const int g = threadIdx.x % IV_G;
+    double acc = 0.0;
+    uint64_t big = 0;
+    auto at = [&](const double* x, int i) { return x && i < n ? x[(int64_t)i * iu] : 0.0; };
+    constexpr int U = 4;   // IV_G U rows in flight ahead of their use
+    double zv[U], uv[U], nv[U];
+    auto fetch = [&](int i0) {
+#pragma unroll
+        for (int p = 0; p < U; ++p) {
+            zv[p] = at(z, i0 + p * IV_G);
+            uv[p] = at(u, i0 + p * IV_G);
+            nv[p] = at(un, i0 + p * IV_G);
+        }
+    };
+    fetch(g);
+    for (int i0 = 0; i0 < n; i0 += U * IV_G) {
+        double v[U], uc[U], w[U];
+#pragma unroll
+        for (int p = 0; p < U; ++p) {
+            v[p] = zv[p];
+            uc[p] = uv[p];
+            w[p] = nv[p];
+        }
+        fetch(i0 + U * IV_G + g);
+#pragma unroll
+        for (int p = 0; p < U; ++p) {
+            const int i = i0 + p * IV_G + g;
+            if (u) {
+                v[p] = fma(-dot, uc[p], v[p]);
+                if (i < n) z[(int64_t)i * iu] = v[p];
+            }
+            if (i < n) big = max(big, abs_bits(v[p]));
+        }
+        if (un) {
+#pragma unroll
+            for (int p = 0; p < U; ++p)
+#pragma unroll
+                for (int q = 0; q < IV_G; ++q) {
+                    const double x = __shfl_sync(mask, v[p], q, IV_G), c = __shfl_sync(mask, w[p], q, IV_G);
+                    if (i0 + p * IV_G + q < n) acc = fma(x, c, acc);
+                }
+        }
+    }
+    *dot_next = acc;
+#pragma unroll
+    for (int o = IV_G / 2; o > 0; o >>= 1) big = max(big, (uint64_t)__shfl_xor_sync(mask, (unsigned long long)big, o, IV_G));
+    *top = big;
+}
+
+// REST = 0: a thread per eigenvalue, 1: IV_G lanes per cluster (members after the first; the solves are lane 0's)
+template <int REST>
+__global__ void __launch_bounds__(32) k_invit(InvitArgs g) {
+    const int64_t b = blockIdx.y;
+    const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / (REST ? IV_G : 1);
+    const int lane = REST ? threadIdx.x % IV_G : 0;
+    const unsigned mask = ((1u << IV_G) - 1u) << (threadIdx.x & 31) / IV_G * IV_G;   // of a cluster's lanes
+    const int n = (int)g.n;
+    const int64_t iu = g.iu;
+    const double onenrm = g.info[b * 8 + 2], ortol = g.ortol_rel * onenrm;
+    const double* Wb = g.w + b * iu;
+    double* Zb = g.Z + b * n * iu;
+    const int64_t S = iu * gridDim.y;
+    const int64_t nw = want_of(g.lim, b, iu);
+    int js, je;
+    bool first = true;   // the first member of its cluster
+    if (REST) {
+        const int* C = g.clus + b * (iu + 2);
+        if (t >= C[0] || onenrm == 0.0) return;
+        js = C[1 + t];
+        je = js + 1;
+        while (je < nw && !starts_cluster(Wb, je, ortol)) ++je;
+    } else {
+        if (t >= nw) return;
+        js = (int)t;
+        je = js + 1;
+        if (onenrm == 0.0) {
+            // T = 0: any orthonormal basis (the scaled right-hand sides below would vanish)
+            for (int i = 0; i < n; ++i) Zb[i * iu + js] = (i == js) ? 1.0 : 0.0;
+            return;
+        }
+        first = starts_cluster(Wb, js, ortol);
+    }
+    for (int j = REST ? js + 1 : js; j < je; ++j) {
+        double* z = Zb + j;
+        const double* ua = g.scr + b * iu + j;
+        const double* ub = ua + n * S;
+        const double* uc = ub + n * S;
+        const double* ud = uc + n * S;
+        const unsigned char* up = g.pivs + b * iu + j;
+        const double unn = ua[(int64_t)(n - 1) * S], tol = uc[(int64_t)(n - 1) * S];
         double bmax = 0.0;
-        for (int i = 0; i < n; ++i) {
-            seed = mix64(seed + 0x9e3779b97f4a7c15ULL);
-            const double v = (double)(seed >> 11) * (2.0 / 9007199254740992.0) - 1.0;
-            z[i * iu] = v;
-            bmax = fmax(bmax, fabs(v));
+        if (!REST) {
+            // ---- starting vector in Z(:, j)
+            uint64_t seed = mix64(((uint64_t)b << 40) ^ ((uint64_t)j * 0x9e3779b97f4a7c15ULL) ^ 0x1234567ULL);
+            uint64_t big = 0;
+            for (int i = 0; i < n; ++i) {
+                seed = mix64(seed + 0x9e3779b97f4a7c15ULL);
+                const double v = (double)(seed >> 11) * (2.0 / 9007199254740992.0) - 1.0;
+                z[i * iu] = v;
+                big = max(big, abs_bits(v));
+            }
+            bmax = __longlong_as_double((long long)big);
         }
         const int maxits = 5, extra = 2;
         const double dtpcrt = sqrt(0.1 / (double)n);
@@ -594,57 +760,52 @@ __global__ void __launch_bounds__(32)
         bool ok = false;
         while (its < maxits) {
             ++its;
-            // scale: scl = n * onenrm * max(eps, |u_nn|) / ||b||_inf
-            double scl = (double)n * onenrm * fmax(kEps, fabs(unn)) / bmax;
-            // forward: apply P and L
-            {
-                double yprev = z[0] * scl;
-                double rz[IV_U], rm[IV_U];
-                unsigned char rp[IV_U];
-                auto fetch = [&](int k0) {
+            double nrm = 0.0;
+            if (!REST || (its > 1 && lane == 0)) {
+                // scale: scl = n * onenrm * max(eps, |u_nn|) / ||b||_inf
+                const double scl = (double)n * onenrm * fmax(kEps, fabs(unn)) / bmax;
+                // forward: apply P and L
+                {
+                    double yprev = z[0] * scl;
+                    double rz[IV_U], rm[IV_U];
+                    unsigned char rp[IV_U];
+                    auto fetch = [&](int k0) {
 #pragma unroll
-                    for (int q = 0; q < IV_U; ++q) {
-                        const int k = min(k0 + q, n - 1);
-                        const int64_t o = (int64_t)(k > 0 ? k - 1 : 0) * S;
-                        rz[q] = z[k * iu];
-                        rm[q] = uc[o];
-                        rp[q] = up[o];
-                    }
-                };
-                fetch(1);
-                for (int k0 = 1; k0 < n; k0 += IV_U) {
-                    double cz[IV_U], cm[IV_U];
-                    unsigned char cp[IV_U];
+                        for (int q = 0; q < IV_U; ++q) {
+                            const int k = min(k0 + q, n - 1);
+                            const int64_t o = (int64_t)(k > 0 ? k - 1 : 0) * S;
+                            rz[q] = z[k * iu];
+                            rm[q] = uc[o];
+                            rp[q] = up[o];
+                        }
+                    };
+                    fetch(1);
+                    for (int k0 = 1; k0 < n; k0 += IV_U) {
+                        double cz[IV_U], cm[IV_U];
+                        unsigned char cp[IV_U];
 #pragma unroll
-                    for (int q = 0; q < IV_U; ++q) {
-                        cz[q] = rz[q];
-                        cm[q] = rm[q];
-                        cp[q] = rp[q];
-                    }
-                    if (k0 + IV_U < n) fetch(k0 + IV_U);
+                        for (int q = 0; q < IV_U; ++q) {
+                            cz[q] = rz[q];
+                            cm[q] = rm[q];
+                            cp[q] = rp[q];
+                        }
+                        if (k0 + IV_U < n) fetch(k0 + IV_U);
 #pragma unroll
-                    for (int q = 0; q < IV_U; ++q) {
-                        const int k = k0 + q;
-                        if (k < n) {
-                            double yk = cz[q] * scl;
-                            const double m = cm[q];
-                            if (cp[q] == 0) {
-                                yk = yk - m * yprev;
-                            } else {
-                                const double temp = yprev;
-                                yprev = yk;
-                                yk = temp - m * yk;
+                        for (int q = 0; q < IV_U; ++q) {
+                            const int k = k0 + q;
+                            if (k < n) {
+                                const double yk = __dmul_rn(cz[q], scl);
+                                const bool sw = cp[q] != 0;
+                                const double top = sw ? yk : yprev;
+                                yprev = fma(-cm[q], top, sw ? yprev : yk);
+                                z[(k - 1) * iu] = top;
                             }
-                            z[(k - 1) * iu] = yprev;
-                            yprev = yk;
                         }
                     }
+                    z[(n - 1) * iu] = yprev;
                 }
-                z[(n - 1) * iu] = yprev;
-            }
-            // backward with perturbation of tiny pivots
-            double nrm = 0.0;
-            {
+                // backward with perturbation of tiny pivots
+                uint64_t big = 0;
                 double y1 = 0.0, y2 = 0.0;  // y(k+1), y(k+2)
                 double rz[IV_U], ra[IV_U], rb[IV_U], rd[IV_U];
                 auto fetch = [&](int k0) {
@@ -667,7 +828,7 @@ __global__ void __launch_bounds__(32)
                         ca[q] = ra[q];
                         cb[q] = rb[q];
                         cd[q] = rd[q];
-                        cr[q] = 1.0 / ca[q];
+                        cr[q] = recip(ca[q]);   // of use for mid-range pivots only
                     }
                     if (k0 - IV_U >= 0) fetch(k0 - IV_U);
 #pragma unroll
@@ -675,13 +836,10 @@ __global__ void __launch_bounds__(32)
                         const int k = k0 - q;
                         if (k >= 0) {
                             double temp = cz[q];
-                            if (k <= n - 3)
-                                temp = temp - cb[q] * y1 - cd[q] * y2;
-                            else if (k == n - 2)
-                                temp = temp - cb[q] * y1;
+                            if (k <= n - 2) temp = fma(-cb[q], y1, temp);
+                            if (k <= n - 3) temp = fma(-cd[q], y2, temp);
                             double ak = ca[q], yk;
-                            const int ea = expo_of(ak), et = expo_of(temp);
-                            if (min(ea, et) > 512 && max(ea, et) < 1536) {
+                            if (mid_expo(ak) && mid_expo(temp)) {
                                 // mid-range operands: no scaling or perturbation applies
                                 yk = quot(temp, ak, cr[q]);
                             } else {
@@ -708,55 +866,60 @@ __global__ void __launch_bounds__(32)
                                 yk = temp / ak;
                             }
                             z[k * iu] = yk;
-                            nrm = fmax(nrm, fabs(yk));
+                            big = max(big, abs_bits(yk));
                             y2 = y1;
                             y1 = yk;
                         }
                     }
                 }
+                nrm = __longlong_as_double((long long)big);
             }
-            // modified Gram-Schmidt against earlier cluster members
-            if (j > js) {
-                for (int q = js; q < j; ++q) {
-                    double dot = 0.0;
-                    const double* zq = Zb + q;
-#pragma unroll 16
-                    for (int i = 0; i < n; ++i) dot += z[i * iu] * zq[i * iu];
-                    nrm = 0.0;
-                    for (int i = 0; i < n; i += 16) {
-                        double v[16], u[16];
-#pragma unroll
-                        for (int p = 0; p < 16; ++p) {
-                            const int64_t o = (int64_t)min(i + p, n - 1) * iu;
-                            v[p] = z[o];
-                            u[p] = zq[o];
-                        }
-#pragma unroll
-                        for (int p = 0; p < 16; ++p)
-                            if (i + p < n) {
-                                v[p] -= dot * u[p];
-                                z[(int64_t)(i + p) * iu] = v[p];
-                                nrm = fmax(nrm, fabs(v[p]));
-                            }
-                    }
-                }
+            if (!first) break;   // the other members go on in k_invit<1>
+            if (REST) {
+                // modified Gram-Schmidt against earlier cluster members
+                __syncwarp(mask);
+                double dot = 0.0;
+                uint64_t big = 0;
+                mgs_pass(mask, n, iu, z, nullptr, 0.0, Zb + js, &dot, &big);
+                for (int q = js; q < j; ++q) mgs_pass(mask, n, iu, z, Zb + q, dot, q + 1 < j ? Zb + q + 1 : nullptr, &dot, &big);
+                __syncwarp(mask);
+                nrm = __longlong_as_double((long long)big);
             }
             bmax = nrm;
-            if (nrm < dtpcrt) continue;
+            if (!(nrm >= dtpcrt)) continue;
             ++nrmchk;
             if (nrmchk < extra + 1) continue;
             ok = true;
             break;
         }
-        if (!ok) atomicAdd(fail + b, 1);
+        if (!first) return;
+        if (!ok && lane == 0) atomicAdd(g.fail + b, 1);
         // normalise (2-norm), largest component positive
-        double s2 = 0.0, big = 0.0, bigv = 0.0;
+        if (REST) {
+            double s2 = 0.0;
+            uint64_t big = 0;
+            mgs_pass(mask, n, iu, z, nullptr, 0.0, z, &s2, &big);
+            // the first row that holds the largest component
+            int at = n;
+            for (int i = lane; i < n && at == n; i += IV_G)
+                if (abs_bits(z[(int64_t)i * iu]) == big) at = i;
+#pragma unroll
+            for (int o = IV_G / 2; o > 0; o >>= 1) at = min(at, __shfl_xor_sync(mask, at, o, IV_G));
+            double scl = 1.0 / sqrt(s2);
+            if (at < n && z[(int64_t)at * iu] < 0.0) scl = -scl;
+            __syncwarp(mask);
+            for (int i = lane; i < n; i += IV_G) z[(int64_t)i * iu] *= scl;
+            __syncwarp(mask);
+            continue;
+        }
+        double s2 = 0.0, bigv = 0.0;
+        uint64_t big = 0;
 #pragma unroll 16
         for (int i = 0; i < n; ++i) {
-            double v = z[i * iu];
+            const double v = z[i * iu];
             s2 += v * v;
-            if (fabs(v) > big) {
-                big = fabs(v);
+            if (abs_bits(v) > big) {
+                big = abs_bits(v);
                 bigv = v;
             }
         }
@@ -845,38 +1008,44 @@ int tridiag_eigvecs(cudaStream_t st, EigArgs& g) {
         g.d, g.e, n, g.info, g.de, g.tf);
     FORGE_LAUNCH_CHECK();
     double* lam = g.replay ? g.scr : g.w;   // the scratch of the eigenvectors is free until k_invit
-    k_bisect_f32<<<dim3((unsigned)((iu + 31) / 32), (unsigned)batch), 32, 0, st>>>(g.tf, n, iu, g.iu_lim, g.info, lam);
+    const unsigned by = (unsigned)batch;
+    auto grid = [&](int G) { return dim3((unsigned)((iu * G + 31) / 32), by); };   // one warp a CTA: spread over the SMs
+    // FP32 counts are latency-bound up to four warps a scheduler
+    const bool wide32 = iu * batch * 8 <= 152 * 4 * 4 * 32;
+    if (wide32)
+        k_bisect_f32<8><<<grid(8), 32, 0, st>>>(g.tf, n, iu, g.iu_lim, g.info, lam);
+    else
+        k_bisect_f32<4><<<grid(4), 32, 0, st>>>(g.tf, n, iu, g.iu_lim, g.info, lam);
     FORGE_LAUNCH_CHECK();
-    // full FP64 accuracy in both precisions: the eigenvectors of close eigenvalues need it.  Lanes per
-    // eigenvalue: four warps fill the FP64 pipes of an SM (152 x 128 lanes); beyond that more
-    // points a round only add work
+    // full FP64 accuracy in both precisions: the eigenvectors of close eigenvalues need it (where k_bisect_replay
+    // follows, to 4 eps |T|).  Lanes per eigenvalue: four warps fill the FP64 pipes of an SM (152 x 128 lanes);
+    // beyond that more points a round only add work
     const int64_t lanes = 152 * 128;
     const int G = iu * batch * 8 <= lanes ? 8 : iu * batch * 4 <= lanes + lanes / 4 ? 4 : iu * batch <= lanes ? 2 : 1;
-    const dim3 gb((unsigned)((iu * G + 31) / 32), (unsigned)batch);   // one warp a CTA: spread over the SMs
+    const double abstol = g.replay ? 4.0 * kEps : 8.636168555094445e-78;   // at least 2^-256
     if (G == 8)
-        k_bisect<8><<<gb, 32, 0, st>>>(g.de, n, iu, g.iu_lim, g.info, lam);
+        k_bisect<8><<<grid(8), 32, 0, st>>>(g.de, n, iu, g.iu_lim, g.info, abstol, lam);
     else if (G == 4)
-        k_bisect<4><<<gb, 32, 0, st>>>(g.de, n, iu, g.iu_lim, g.info, lam);
+        k_bisect<4><<<grid(4), 32, 0, st>>>(g.de, n, iu, g.iu_lim, g.info, abstol, lam);
     else if (G == 2)
-        k_bisect<2><<<gb, 32, 0, st>>>(g.de, n, iu, g.iu_lim, g.info, lam);
+        k_bisect<2><<<grid(2), 32, 0, st>>>(g.de, n, iu, g.iu_lim, g.info, abstol, lam);
     else
-        k_bisect<1><<<gb, 32, 0, st>>>(g.de, n, iu, g.iu_lim, g.info, lam);
+        k_bisect<1><<<grid(1), 32, 0, st>>>(g.de, n, iu, g.iu_lim, g.info, abstol, lam);
     FORGE_LAUNCH_CHECK();
     if (g.replay) {
-        const unsigned by = (unsigned)batch;
-        k_tri_to_f32<<<dim3((unsigned)std::min<int64_t>((n + 255) / 256, 64), by), 256, 0, st>>>(g.d, g.e, n, g.tq);
+        k_tri_quot<<<dim3((unsigned)std::min<int64_t>((n + 255) / 256, 64), by), 256, 0, st>>>(g.d, g.e, n, g.de, g.tq);
         FORGE_LAUNCH_CHECK();
-        k_bisect_qf<<<dim3((unsigned)((iu + 31) / 32), by), 32, 0, st>>>(g.tq, n, iu, g.iu_lim, g.info, lam, g.w);
+        if (wide32)
+            k_bisect_qf<3><<<grid(8), 32, 0, st>>>(g.tq, n, iu, g.iu_lim, g.info, lam, g.w);
+        else
+            k_bisect_qf<2><<<grid(4), 32, 0, st>>>(g.tq, n, iu, g.iu_lim, g.info, lam, g.w);
         FORGE_LAUNCH_CHECK();
         if (G == 8)
-            k_bisect_replay<3><<<dim3((unsigned)((iu * 8 + 31) / 32), by), 32, 0, st>>>(g.d, g.e, n, iu, g.iu_lim, g.info,
-                                                                                        lam, g.w);
+            k_bisect_replay<3><<<grid(8), 32, 0, st>>>(g.de, n, iu, g.iu_lim, g.info, lam, g.w);
         else if (G == 4)
-            k_bisect_replay<2><<<dim3((unsigned)((iu * 4 + 31) / 32), by), 32, 0, st>>>(g.d, g.e, n, iu, g.iu_lim, g.info,
-                                                                                        lam, g.w);
+            k_bisect_replay<2><<<grid(4), 32, 0, st>>>(g.de, n, iu, g.iu_lim, g.info, lam, g.w);
         else
-            k_bisect_replay<1><<<dim3((unsigned)((iu + 31) / 32), by), 32, 0, st>>>(g.d, g.e, n, iu, g.iu_lim, g.info,
-                                                                                    lam, g.w);
+            k_bisect_replay<1><<<grid(1), 32, 0, st>>>(g.de, n, iu, g.iu_lim, g.info, lam, g.w);
         FORGE_LAUNCH_CHECK();
     }
     prof_end(ST_BISECT, batch * 16.0 * n, batch * 10.0 * 60.0 * (double)n * iu);
@@ -886,8 +1055,25 @@ int tridiag_eigvecs(cudaStream_t st, EigArgs& g) {
     if (g.iu_lim) FORGE_CUDA(cudaMemsetAsync(g.Z, 0, sizeof(double) * (size_t)batch * n * iu, st));
     k_clusters<<<(unsigned)batch, 256, 0, st>>>(g.w, iu, g.iu_lim, g.info, g.ortol_rel, g.clus);
     FORGE_LAUNCH_CHECK();
-    k_invit<<<dim3((unsigned)((g.scr_stride + 31) / 32), (unsigned)batch), 32, 0, st>>>(
-        g.d, g.e, n, iu, g.w, g.iu_lim, g.info, g.ortol_rel, g.clus, g.Z, g.scr, g.pivs, g.scr_stride, g.fail);
+    InvitArgs v;
+    v.d = g.d;
+    v.e = g.e;
+    v.w = g.w;
+    v.info = g.info;
+    v.lim = g.iu_lim;
+    v.clus = g.clus;
+    v.n = n;
+    v.iu = iu;
+    v.ortol_rel = g.ortol_rel;
+    v.Z = g.Z;
+    v.scr = g.scr;
+    v.pivs = g.pivs;
+    v.fail = g.fail;
+    k_invit_lu<<<grid(1), 32, 0, st>>>(v);
+    FORGE_LAUNCH_CHECK();
+    k_invit<0><<<grid(1), 32, 0, st>>>(v);
+    FORGE_LAUNCH_CHECK();
+    k_invit<1><<<grid(IV_G), 32, 0, st>>>(v);
     FORGE_LAUNCH_CHECK();
     prof_end(ST_INVIT, batch * 8.0 * (double)n * iu, 0.0);
     return 0;
@@ -916,7 +1102,6 @@ void carve(EigArgs& g, Carve& c) {
     g.ystride = nblk * n;
     g.sstride = nrb * 2 * TRD_NB;
     g.pstride = 3 * ((n + 31) / 32) + 1;  // per-CTA partials of k_col64 and k_finish64
-    g.scr_stride = iu;
     g.d = c.take<double>(B * n);
     g.e = c.take<double>(B * n);
     g.tau = c.take<double2>(B * n);
