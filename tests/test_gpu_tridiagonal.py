@@ -1,5 +1,4 @@
-"""Eigenvalues and eigenvectors of the tridiagonal solver (multisection, twisted factorizations, inverse
-iteration of clusters) through the allocation-free entry point, against LAPACK.
+"""Eigenvalues and eigenvectors of the tridiagonal solver (multisection, inverse iteration, clusters) through the allocation-free entry point, against LAPACK.
 
 Bounds: eigenvalues to a few n eps |A| (backward error of the reduction), residuals likewise; the
 vectors of eigenvalues apart by more than ortol = 1e-7 |T|_1 are orthogonal to eps / 1e-7 with a
@@ -20,6 +19,8 @@ def _matrix(kind, n, rng):
     H = (G + G.conj().T) / 2
     if kind == "random":
         return H
+    if kind in ("tiny", "huge"):   # products of two elements beyond the range of the division by FMAs
+        return H * {"tiny": 1e-100, "huge": 1e100}[kind]
     Q, _ = np.linalg.qr(G)
     if kind == "pairs":          # every eigenvalue twice: clusters
         w = np.repeat(np.linspace(-1.0, 2.0, (n + 1) // 2), 2)[:n]
@@ -60,3 +61,9 @@ def test_tridiagonal_solver(kind, n, iu):
     assert np.max(np.abs(w - ref)) <= 8 * n * EPS * scale
     assert np.max(np.abs(H @ X - X * w)) <= 16 * n * EPS * scale
     assert np.max(np.abs(X.conj().T @ X - np.eye(iu))) <= 64 * EPS / 1e-7
+
+
+@pytest.mark.parametrize("kind", ["tiny", "huge"])
+@pytest.mark.parametrize("n,iu", [(5, 4), (33, 32), (130, 65)])
+def test_tridiagonal_solver_far_scales(kind, n, iu):
+    test_tridiagonal_solver(kind, n, iu)
