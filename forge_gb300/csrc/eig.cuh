@@ -38,6 +38,9 @@ struct EigArgs {
     void *oz_xs, *oz_vr, *oz_vh, *oz_ws, *oz_ts;
     double2 *oz_wp, *oz_g, *oz_t;
     int* oz_ex;
+    int4* limbs;                // of the tridiagonalisation; shares oz_vh
+    int* limb_f;
+    int64_t limb_tiles;
     int* oz_err;
     float2* tf;                 // batch x n: T scaled to |T| <= 1, (d_i, e_{i-1}^2) in FP32 (FP32 bisection)
     double2* de;                // the same in FP64

@@ -167,16 +167,16 @@ __device__ inline int64_t want_of(const int* lim, int64_t b, int64_t iu) { retur
 __device__ __forceinline__ int expo_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 // operands whose quotient, remainder and products of two neither over- nor underflow
 __device__ __forceinline__ bool mid_expo(double x) { return (unsigned)(expo_of(x) - 524) < 1000u; }
-// Reciprocal to about 2^-46: one Newton step on the hardware's approximation (2^-23).
+// Reciprocal to 2^-40: one Newton step on the hardware's approximation (2^-20).
 __device__ __forceinline__ double recip(double b) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
     return fma(r, fma(-b, r, 1.0), r);
 }
-// a / b from r = recip(b) for operands in mid-range: the remainder of a r brings the quotient to 2^-92 before its
+// a / b from r = recip(b) for operands in mid-range: the remainder of a r brings the quotient to 2^-80 before its
 // one rounding (P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
-// IBM J. Res. Dev. 34 (1990)), so it is the rounded quotient but for one case in about 2^39.  Five FMAs with
-// recip: an FP64 instruction of a warp holds its scheduler's FP64 pipe for 64 clocks on this GPU, whatever the
+// IBM J. Res. Dev. 34 (1990)), so it is the rounded quotient but for one case in 2^27 or fewer (none of 1.5e9
+// random ones).  Five FMAs with recip: an FP64 instruction of a warp holds its scheduler's FP64 pipe for 64 clocks on this GPU, whatever the
 // number of lanes, so the count of them is what the serial chains below cost.
 __device__ __forceinline__ double quot(double a, double b, double r) {
     const double q = a * r;
@@ -976,6 +976,9 @@ int eig_fp64(cudaStream_t st, EigArgs& g) {
     a.scal = g.scal;
     a.cnt = g.cnt;
     a.w0 = g.w0;
+    a.limbs = g.limbs;
+    a.limb_f = g.limb_f;
+    a.limb_tiles = g.limb_tiles;
     a.her2k = her2k_oz;
     a.her2k_user = &g;
     FORGE_CUDA(cudaMemsetAsync(g.oz_err, 0, sizeof(int), st));
@@ -1098,10 +1101,10 @@ struct Carve {
 void carve(EigArgs& g, Carve& c) {
     const int64_t n = g.n, iu = g.iu, B = g.batch;
     const int64_t nblk = (n + TRD_TILE - 1) / TRD_TILE;
-    const int64_t nrb = (n + 127) / 128;   // slots of the panel dots
+    const int64_t nrb = 4;   // slots of the panel dots
     g.ystride = nblk * n;
     g.sstride = nrb * 2 * TRD_NB;
-    g.pstride = 3 * ((n + 31) / 32) + 1;  // per-CTA partials of k_col64 and k_finish64
+    g.pstride = 3 * ((n + 15) / 16);  // per-CTA partials of k_col64 and k_finish64
     g.d = c.take<double>(B * n);
     g.e = c.take<double>(B * n);
     g.tau = c.take<double2>(B * n);
@@ -1125,7 +1128,11 @@ void carve(EigArgs& g, Carve& c) {
     g.oz_xs = g.scr;
     g.pivs = c.take<unsigned char>(n * iu * B);
     g.fail = c.take<int>(B);
-    g.oz_vh = c.take<char>(2 * z.vh);
+    // the trailing matrix in limbs (tridiagonalisation) shares the space of V^H (back-transformation)
+    g.limb_tiles = nblk * (nblk + 1) / 2;
+    g.oz_vh = c.take<char>(std::max<size_t>(2 * z.vh, sizeof(int4) * B * g.limb_tiles * TRD_TILE * TRD_TILE));
+    g.limbs = (int4*)g.oz_vh;
+    g.limb_f = c.take<int>(B * g.limb_tiles);
     g.oz_ws = c.take<char>(2 * z.ws);
     g.oz_ts = c.take<char>(2 * z.ts);
     g.oz_wp = c.take<double2>(z.wp);

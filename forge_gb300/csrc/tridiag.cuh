@@ -46,6 +46,10 @@ struct TrdArgs {
     double* scal;       // batch x 16
     unsigned* cnt;      // batch x 4
     V* w0 = nullptr;    // batch x n: the last column's w before the alpha2 correction
+    // FP64: the trailing triangle as integer limbs, batch x limb_tiles tiles of 64 x 64, and the tiles' exponents
+    int4* limbs = nullptr;
+    int* limb_f = nullptr;
+    int64_t limb_tiles = 0;
     // trailing update on the tensor cores (her2k_oz in FP64, her2k_tc in the mixed path):
     // A(p+w:n, p+w:n) -= V W^H + W V^H for the panel [p, p+w)
     int (*her2k)(cudaStream_t st, TrdArgs<T>& a, int64_t p, int64_t w, int64_t batch, void* user) = nullptr;
@@ -59,9 +63,22 @@ __device__ __forceinline__ void trd_chain_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// Loads ahead of trd_chain_wait: of what the predecessor's own predecessor, or an older kernel, wrote (the predecessor
+// has started all of its CTAs past its wait by then, so those results are in memory); from L2.
+__device__ __forceinline__ double2 ld_early(const double2* p) {
+    double2 v;
+    asm volatile("ld.global.cg.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 ld_early(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
 template <class... P, class... Q>
-int launch_chain(cudaStream_t st, dim3 grid, unsigned threads, void (*k)(P...), Q... args) {
+int launch_chain_smem(cudaStream_t st, dim3 grid, unsigned threads, size_t smem, void (*k)(P...), Q... args) {
     cudaLaunchConfig_t cfg = {};
+    cfg.dynamicSmemBytes = smem;
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.stream = st;
@@ -73,6 +90,11 @@ int launch_chain(cudaStream_t st, dim3 grid, unsigned threads, void (*k)(P...), 
     cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
     FORGE_LAUNCH_CHECK();
     return 0;
+}
+
+template <class... P, class... Q>
+int launch_chain(cudaStream_t st, dim3 grid, unsigned threads, void (*k)(P...), Q... args) {
+    return launch_chain_smem(st, grid, threads, 0, k, args...);
 }
 
 int tridiagonalize_f32(cudaStream_t st, TrdArgs<float>& a, int64_t batch);     // tridiag.cu
