@@ -3,7 +3,8 @@
 // Bytes per column step (algorithmic): the trailing lower triangle, (n-col)^2/2
 // complex elements, read once by trd_hemv; the rank-2k update is GEMM-shaped.
 // What bounds a column besides trd_hemv's bytes is latency: kernel boundaries, and inside trd_col / trd_finish the
-// round trips to L2.  So the three kernels are launched programmatically, every thread's loads of a phase are in
+// round trips to L2.  So the three kernels are launched programmatically and load what older kernels left (the panel,
+// the trailing matrix) before they wait for their predecessor, every thread's loads of a phase are in
 // flight together, and no CTA adds up partials one by one.  One matrix of n = 5044 (5043 columns), whole kernels:
 // trd_col 78 -> 58 ms, trd_hemv 91 -> 72 ms, trd_finish (with trd_fix, now once a panel) 116 -> 41 ms; n = 364, six
 // matrices: 5.4 -> 4.1, 4.2 -> 3.4, 5.4 -> 3.1 ms.
@@ -29,7 +30,7 @@ __device__ inline bool last_cta(unsigned* counter, unsigned total) {
 }
 
 
-constexpr int COL_ROWS = 64;   // rows (and threads) per CTA of k_trd_col: the panel's columns come in over many SMs
+constexpr int COL_ROWS = 64;   // rows per CTA of k_trd_col (and one warp for alpha2): the panel's columns come in over many SMs
 constexpr int DOT_L = 8;       // reflectors per CTA of the panel dots
 
 // partial sums: [0, trd_col_parts) the norms of k_trd_col, one float a warp; then pairs w^H v of k_trd_finish
@@ -41,25 +42,27 @@ __device__ inline float warp_sum_f(float v) {
     return v;
 }
 
-// alpha2 = -1/2 tau (w^H v) of the last column from the nd partials of k_trd_finish, by one warp
-__device__ inline float2 trd_alpha2(const TrdArgs<float>& a, int64_t b, int64_t nd) {
-    const double2* part = (const double2*)(a.part + b * a.pstride + trd_col_parts(a.n));
+// alpha2 = -1/2 tau (w^H v) of the last column from the nd partials of k_trd_finish, by one warp: lanes below 16 the real
+// part, the others the imaginary part (an FP64 instruction of a warp takes 64 clocks, however many lanes are active)
+__device__ inline float trd_alpha2(const TrdArgs<float>& a, int64_t b, int64_t nd) {
+    const double* part = a.part + b * a.pstride + trd_col_parts(a.n);
+    const int lane = threadIdx.x & 31, im = lane >> 4;
     const double tr = a.scal[b * 16 + 4], ti = a.scal[b * 16 + 5];
-    double xr = 0.0, xi = 0.0;
-    for (int64_t q0 = threadIdx.x & 31; q0 < nd; q0 += 256) {
-        double2 t[8];
+    double s = 0.0;
+    for (int64_t q0 = lane & 15; q0 < nd; q0 += 160) {
+        double t[10];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) t[q] = q0 + 32 * q < nd ? part[q0 + 32 * q] : make_double2(0.0, 0.0);
+        for (int q = 0; q < 10; ++q) t[q] = q0 + 16 * q < nd ? part[2 * (q0 + 16 * q) + im] : 0.0;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            if (q0 + 32 * q >= nd) break;
-            xr += t[q].x;
-            xi += t[q].y;
+        for (int q = 0; q < 10; ++q) {
+            if (q0 - (lane & 15) + 16 * q >= nd) break;
+            s += t[q];
         }
     }
-    xr = warp_sum_d(xr);
-    xi = warp_sum_d(xi);
-    return make_float2((float)(-0.5 * (tr * xr - ti * xi)), (float)(-0.5 * (tr * xi + ti * xr)));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const double o = __shfl_xor_sync(0xffffffffu, s, 16);
+    return (float)(-0.5 * (im ? tr * s + ti * o : tr * s - ti * o));
 }
 
 // w + alpha2 v; the fused operations are spelled out because k_trd_col and k_trd_fix have to round alike
@@ -72,7 +75,7 @@ __device__ inline float2 trd_corr(float2 w, float2 al, float2 v) {
 // Adds alpha2 v to the last column's w (w0), then forms column col; the last CTA forms the reflector's scalars from
 // the partial norms.  The kernel is a chain of latencies (a column is a few hundred KB): all of a thread's panel
 // elements are loaded at once, half a panel a time, and the last CTA's four quotients sit in four lanes.
-__global__ void __launch_bounds__(COL_ROWS) k_trd_col(TrdArgs<float> a, int64_t p, int ii, int64_t col, int has_refl) {
+__global__ void __launch_bounds__(COL_ROWS + 32) k_trd_col(TrdArgs<float> a, int64_t p, int ii, int64_t col, int has_refl) {
     const int64_t b = blockIdx.y, n = a.n, lda = a.lda;
     float2* A = a.A + b * a.strideA;
     float2* W = a.W + b * (n * TRD_NB);
@@ -82,31 +85,34 @@ __global__ void __launch_bounds__(COL_ROWS) k_trd_col(TrdArgs<float> a, int64_t 
     const int64_t r = col + (int64_t)blockIdx.x * COL_ROWS + threadIdx.x;
     const int lm = ii - 1;
     const float2 z = make_float2(0.f, 0.f);
-    trd_chain_wait();
+    const bool mine = threadIdx.x < COL_ROWS && r < n, alpha_warp = threadIdx.x >= COL_ROWS;
+    // what older kernels left: the raw column, the panel but for its last reflector
     float2 x = z, wl = z, vl = z, av[16], wv[16];
-    if (r < n) {
-        x = A[r + col * lda];
-        if (ii > 0) {
-            wl = w0[r];
-            vl = A[r + (p + lm) * lda];
-        }
-    }
+    if (mine) x = ld_early(A + r + col * lda);
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
-        av[q] = q < lm && r < n ? A[r + (p + q) * lda] : z;
-        wv[q] = q < lm && r < n ? W[r + q * n] : z;
+        av[q] = q < lm && mine ? ld_early(A + r + (p + q) * lda) : z;
+        wv[q] = q < lm && mine ? ld_early(W + r + q * n) : z;
     }
-    if (threadIdx.x >= 32 && lane < ii) {
-        wrow[lane] = lane == lm ? w0[col] : W[col + lane * n];
-        arow[lane] = A[col + (p + lane) * lda];
+    if (alpha_warp && lane < lm) {
+        wrow[lane] = ld_early(W + col + lane * n);
+        arow[lane] = ld_early(A + col + (p + lane) * lda);
     }
-    if (ii > 0 && threadIdx.x < 32) {
-        const float2 al = trd_alpha2(a, b, (n - col + 31) / 32);
-        if (threadIdx.x == 0) s_al = al;
+    trd_chain_wait();
+    if (mine && ii > 0) {
+        wl = w0[r];
+        vl = A[r + (p + lm) * lda];
     }
     __syncthreads();
-    float nrm = 0.f;
-    if (r < n) {
+    if (alpha_warp && ii > 0) {
+        if (lane == 0) {
+            wrow[lm] = w0[col];
+            arow[lm] = A[col + (p + lm) * lda];
+        }
+        const float al = trd_alpha2(a, b, (n - col + 31) / 32);
+        if ((lane & 15) == 0) reinterpret_cast<float*>(&s_al)[lane >> 4] = al;
+    }
+    if (mine) {
 #pragma unroll
         for (int h = 0; h < TRD_NB; h += 16) {
             if (h >= lm) break;
@@ -125,6 +131,10 @@ __global__ void __launch_bounds__(COL_ROWS) k_trd_col(TrdArgs<float> a, int64_t 
                 }
             }
         }
+    }
+    __syncthreads();
+    float nrm = 0.f;
+    if (mine) {
         if (ii > 0) {
             // the last reflector, whose w takes its correction first
             const float2 al = s_al, ar = arow[lm];
@@ -148,19 +158,21 @@ __global__ void __launch_bounds__(COL_ROWS) k_trd_col(TrdArgs<float> a, int64_t 
     nrm = warp_sum_f(nrm);
     float* part = (float*)(a.part + b * a.pstride);
     const int64_t nw = (int64_t)gridDim.x * (COL_ROWS / 32);
-    if (lane == 0) part[(int64_t)blockIdx.x * (COL_ROWS / 32) + (threadIdx.x >> 5)] = nrm;
+    if (lane == 0 && !alpha_warp) part[(int64_t)blockIdx.x * (COL_ROWS / 32) + (threadIdx.x >> 5)] = nrm;
     if (last_cta(a.cnt + b * 4, gridDim.x) && threadIdx.x < 32) {
         // 256 rows in FP32 (eight warps as a tree), beyond that in FP64
         double* sc = a.scal + b * 16;
         const double ar = ((volatile double*)sc)[0], ai = ((volatile double*)sc)[1];
-        double xn2 = 0.0;
-        for (int64_t g = 8 * lane; g < nw; g += 256) {
+        double xn2 = 0.0;   // summed in order: a last place of beta is a last place of eigenvalues
+        for (int64_t g0 = 0; g0 < nw; g0 += 256) {
+            const int64_t g = g0 + 8 * lane;
             float t[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) t[q] = g + q < nw ? ((volatile float*)part)[g + q] : 0.f;
-            xn2 += (double)(((t[0] + t[4]) + (t[2] + t[6])) + ((t[1] + t[5]) + (t[3] + t[7])));
+            const float t8 = ((t[0] + t[4]) + (t[2] + t[6])) + ((t[1] + t[5]) + (t[3] + t[7]));
+            const int m = (int)min((int64_t)32, (nw - g0 + 7) / 8);
+            for (int q = 0; q < m; ++q) xn2 += (double)__shfl_sync(0xffffffffu, t8, q);
         }
-        xn2 = warp_sum_d(xn2);
         float2* tau = a.tau + b * n;
         // zlarfg: beta = -sign(|(alpha, x)|, Re alpha), tau = (beta - alpha)/beta, x *= 1/(alpha - beta)
         if (!has_refl || (xn2 == 0.0 && ai == 0.0)) {
@@ -213,16 +225,16 @@ __global__ void __launch_bounds__(256) k_trd_hemv(TrdArgs<float> a, int64_t p, i
         __shared__ V cq[4][HV_CB];
         const int tr = threadIdx.x & 63, tg = threadIdx.x >> 6;
         const int64_t r0 = R0 + tr, rv = (tg == 0 ? R0 : C0) + tr;
-        trd_chain_wait();
-        // 16 loads per thread (row r0, 16 columns) issued before any arithmetic
-        const float sr = (float)sc[2], si = (float)sc[3];
+        // 16 loads per thread (row r0, 16 columns) before the column is known: a panel leaves A22 as it is
         V xv = vzero<V>(), a0[16];
-        if (tg < 2 && rv < n) xv = A[rv + col * lda];
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
             const int64_t c = C0 + tg * 16 + q;
-            a0[q] = (r0 < n && c < n && c <= r0) ? A[r0 + c * lda] : vzero<V>();
+            a0[q] = (r0 < n && c < n && c <= r0) ? ld_early(A + r0 + c * lda) : vzero<V>();
         }
+        trd_chain_wait();
+        const float sr = (float)sc[2], si = (float)sc[3];
+        if (tg < 2 && rv < n) xv = A[rv + col * lda];
         if (tg < 2) (tg == 0 ? vr : vc)[tr] = rv < n ? trd_scale(xv, rv == c0, sr, si) : vzero<V>();
         __syncthreads();
         V racc = vzero<V>();
@@ -269,14 +281,19 @@ __global__ void __launch_bounds__(256) k_trd_hemv(TrdArgs<float> a, int64_t p, i
         const V* W = a.W + b * (n * TRD_NB);
         __shared__ float sw[8][32];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        trd_chain_wait();
         V v = vzero<V>(), xw[DOT_L], xa[DOT_L];
-        if (r < n) v = A[r + col * lda];
 #pragma unroll
         for (int q = 0; q < DOT_L; ++q) {
-            const bool in = r < n && l0 + q < ii;
-            xw[q] = in ? W[r + (l0 + q) * n] : vzero<V>();
-            xa[q] = in ? A[r + (p + l0 + q) * lda] : vzero<V>();
+            // W's last column is the predecessor's
+            xw[q] = r < n && l0 + q < ii - 1 ? ld_early(W + r + (l0 + q) * n) : vzero<V>();
+            xa[q] = r < n && l0 + q < ii ? ld_early(A + r + (p + l0 + q) * lda) : vzero<V>();
+        }
+        trd_chain_wait();
+        if (r < n) {
+            v = A[r + col * lda];
+#pragma unroll
+            for (int q = 0; q < DOT_L; ++q)
+                if (l0 + q == ii - 1) xw[q] = W[r + (l0 + q) * n];
         }
         v = r < n ? trd_scale(v, r == c0, (float)sc[2], (float)sc[3]) : v;
         float m[32];
@@ -325,19 +342,20 @@ __global__ void __launch_bounds__(TRD_ROWS) k_trd_finish(TrdArgs<float> a, int64
     __shared__ V ysl[8][33];
     const int rr = threadIdx.x & 31, sl = threadIdx.x >> 5;
     const int64_t r = c0 + (int64_t)blockIdx.x * 32 + rr;
-    trd_chain_wait();
-    const double* sc = a.scal + b * 16;
-    const V s = make_float2((float)sc[2], (float)sc[3]), tau = make_float2((float)sc[4], (float)sc[5]);
+    // what older kernels left: the panel, the raw column and its scalars
     V pa[4], pw[4], v = vzero<V>();
     if (r < n) {
-        if (sl == 0) v = A[r + col * lda];
+        if (sl == 0) v = ld_early(A + r + col * lda);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int l = sl + 8 * q;
-            pa[q] = l < ii ? A[r + (p + l) * lda] : vzero<V>();
-            pw[q] = l < ii ? W[r + l * n] : vzero<V>();
+            pa[q] = l < ii ? ld_early(A + r + (p + l) * lda) : vzero<V>();
+            pw[q] = l < ii ? ld_early(W + r + l * n) : vzero<V>();
         }
     }
+    trd_chain_wait();
+    const double* sc = a.scal + b * 16;
+    const V s = make_float2((float)sc[2], (float)sc[3]), tau = make_float2((float)sc[4], (float)sc[5]);
     if (threadIdx.x >= 192 && rr < ii) {
         // warps 6 and 7 have the fewest slots: s1, s2 from the dots' partials
         const V* S = a.Spart + b * a.sstride + (sl - 6) * TRD_NB + rr;
@@ -417,8 +435,8 @@ __global__ void __launch_bounds__(TRD_ROWS) k_trd_fix(TrdArgs<float> a, int ii, 
     __shared__ float2 s_al;
     trd_chain_wait();
     if (threadIdx.x < 32) {
-        const float2 al = trd_alpha2(a, b, (n - col - 1 + 31) / 32);
-        if (threadIdx.x == 0) s_al = al;
+        const float al = trd_alpha2(a, b, (n - col - 1 + 31) / 32);
+        if ((threadIdx.x & 15) == 0) reinterpret_cast<float*>(&s_al)[threadIdx.x >> 4] = al;
     }
     __syncthreads();
     const int64_t r = col + 1 + (int64_t)blockIdx.x * TRD_ROWS + threadIdx.x;
@@ -441,7 +459,7 @@ int tridiagonalize_f32(cudaStream_t st, TrdArgs<float>& a, int64_t batch) {
             const double esz = (double)sizeof(typename CV<T>::type);
             dim3 ga((unsigned)((n - col + COL_ROWS - 1) / COL_ROWS), (unsigned)batch);
             prof_begin(ST_TRD_COL);
-            FORGE_TRY(launch_chain(st, ga, COL_ROWS, k_trd_col, a, p, ii, col, has_refl));
+            FORGE_TRY(launch_chain(st, ga, COL_ROWS + 32, k_trd_col, a, p, ii, col, has_refl));
             prof_end(ST_TRD_COL, batch * (double)(n - col) * (2.0 * ii + 2.0) * esz, 0.0);
             if (!has_refl) continue;
             ++nrefl;
