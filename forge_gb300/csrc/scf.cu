@@ -84,19 +84,62 @@ struct SortArgs {
     ScfScalars* sc;
 };
 
-__global__ void k_sort_fermi(SortArgs a) {
+// Energies as integers of the same order; NaN has none.
+__device__ inline long long sort_key(double e) {
+    const long long b = __double_as_longlong(e == 0.0 ? 0.0 : e);
+    return b < 0 ? b ^ 0x7fffffffffffffffLL : b;
+}
+
+// Different energies have one order: every state counts the states below it.  Equal energies (or NaN) are put in the
+// order that SortEnergies_1Spin's heap sort gives them, by that sort, which is a serial chain of one thread.
+// Measured, 720 states: 0.97 -> 0.17 ms; 180 states: 0.20 -> 0.02 ms.
+constexpr int SORT_T = 1024;
+__global__ void __launch_bounds__(SORT_T) k_sort_fermi(SortArgs a) {
     extern __shared__ double sm[];
     const int64_t n = a.numb * a.Nk;
     double* e = sm;
     double* ix = sm + n;
+    bool odd = false;
     for (int64_t ic = threadIdx.x; ic < n; ic += blockDim.x) {
         // SortEnergies_1Spin: icount = (band-1)*Nk + k, energies(icount) = Bands(band, k)
         int64_t band = ic / a.Nk, k = ic - band * a.Nk;
-        e[ic] = a.w[k * a.iu + (a.nLower - 1) + band];
-        ix[ic] = (double)(ic + 1);
+        const double v = a.w[k * a.iu + (a.nLower - 1) + band];
+        e[ic] = v;
+        odd |= v != v;
+    }
+    odd = __syncthreads_or(odd);
+    // ranks (exchanged through ix), unless two energies are equal
+    if (!odd) {
+        for (int64_t ic = threadIdx.x; ic < n; ic += blockDim.x) {
+            const long long key = sort_key(e[ic]);
+            int64_t below = 0, same = 0;
+#pragma unroll 8
+            for (int64_t q = 0; q < n; ++q) {
+                const long long o = sort_key(e[q]);
+                below += o < key;
+                same += o == key;
+            }
+            odd |= same > 1;
+            ix[ic] = (double)below;
+        }
+    }
+    odd = __syncthreads_or(odd);
+    if (!odd) {
+        // into the rank's place: the energies are read again from the bands
+        for (int64_t ic = threadIdx.x; ic < n; ic += blockDim.x) {
+            const int64_t band = ic / a.Nk, k = ic - band * a.Nk;
+            e[(int64_t)ix[ic]] = a.w[k * a.iu + (a.nLower - 1) + band];
+        }
+    } else {
+        for (int64_t ic = threadIdx.x; ic < n; ic += blockDim.x) ix[ic] = (double)(ic + 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0 && n > 1) {
+    if (!odd) {
+        // ix is the rank of state ic; its inverse goes out through the result array and back
+        for (int64_t ic = threadIdx.x; ic < n; ic += blockDim.x) a.sorted_idx[(int64_t)ix[ic]] = ic + 1;
+        __syncthreads();
+        for (int64_t q = threadIdx.x; q < n; q += blockDim.x) ix[q] = (double)((volatile int64_t*)a.sorted_idx)[q];
+    } else if (threadIdx.x == 0 && n > 1) {
         // heap sort of rows (e, ix) on e, 1-based as in dsort_lists
         double* E = e - 1;
         double* I = ix - 1;
@@ -142,21 +185,32 @@ __global__ void k_sort_fermi(SortArgs a) {
     }
     __shared__ int64_t s_nocc, s_npart;
     __shared__ double s_ef, s_deg;
-    if (threadIdx.x == 0) {
-        // Main.f90:400-412 (Fortran nint: half away from zero)
-        double x = (double)(a.Nk * a.NP) + (double)a.Nk / 2.0 * a.nfilling;
-        int64_t nF = a.numS * (int64_t)((x >= 0) ? floor(x + 0.5) : -floor(-x + 0.5));
-        double ef = 0.0;
-        if (nF >= 1 && nF < n) ef = (e[nF - 1] + e[nF]) / 2.0;
-        int64_t nocc = 0, npart = 0;
-        for (int64_t q = 0; q < n; ++q) {
-            if ((e[q] - ef) < -a.tol) {
-                ++nocc;
-            } else if (fabs(e[q] - ef) < a.tol) {
-                ++nocc;
-                ++npart;
-            }
+    __shared__ int s_cnt[2];
+    // Main.f90:400-412 (Fortran nint: half away from zero)
+    const double x = (double)(a.Nk * a.NP) + (double)a.Nk / 2.0 * a.nfilling;
+    const int64_t nF = a.numS * (int64_t)((x >= 0) ? floor(x + 0.5) : -floor(-x + 0.5));
+    double ef = 0.0;
+    if (nF >= 1 && nF < n) ef = (e[nF - 1] + e[nF]) / 2.0;
+    if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
+    __syncthreads();
+    int occ = 0, part = 0;
+    for (int64_t q = threadIdx.x; q < n; q += blockDim.x) {
+        if ((e[q] - ef) < -a.tol) {
+            ++occ;
+        } else if (fabs(e[q] - ef) < a.tol) {
+            ++occ;
+            ++part;
         }
+    }
+    occ = __reduce_add_sync(0xffffffffu, occ);
+    part = __reduce_add_sync(0xffffffffu, part);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&s_cnt[0], occ);
+        atomicAdd(&s_cnt[1], part);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int64_t nocc = s_cnt[0], npart = s_cnt[1];
         double deg = 1.0 / (double)npart * (double)(nF + npart - nocc);
         a.sc->EF = ef;
         a.sc->DegFactor = deg;
@@ -215,7 +269,7 @@ int launch_sort_fermi(Context& c, const double* w, double nfilling, double* sort
     }
     FORGE_CUDA(cudaFuncSetAttribute(k_sort_fermi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     prof_begin(ST_SORT);
-    k_sort_fermi<<<1, 256, smem, c.stream>>>(a);
+    k_sort_fermi<<<1, SORT_T, smem, c.stream>>>(a);
     FORGE_LAUNCH_CHECK();
     prof_end(ST_SORT, (double)(c.numb * c.Nk) * 32.0, 0.0);
     return 0;
@@ -249,26 +303,41 @@ __device__ inline double block_max(double v, double* sh) {
     return r;
 }
 
-// partials: RED_CTAS x 8 : Kin_a, Kin_b, Qaa, Qab, Qbb, Mres
+// partials: RED_CTAS x 8 : Kin_a, Kin_b, Qaa, Qab, Qbb, Mres.  SAME: Pa is Pb, and the forms of b are those of a.
+// Bound: FP64 pipe (two lanes a clock and SM) with two states, 18 instructions an element; a square root an element
+// would double that, so it is taken only where the squared difference exceeds the thread's largest so far.
+// Measured, N = 5044 (10^8 elements): two states 6.0 -> 4.0 ms,
+// one 6.0 -> 0.8 ms.
+template <bool SAME>
 __global__ void __launch_bounds__(256) k_energy_pass(const double* __restrict__ te, const double2* __restrict__ Pa,
                                                      const double2* __restrict__ Pb, int64_t N, double alpha,
                                                      double* __restrict__ partials) {
     const size_t NN = (size_t)N * N, total = 4 * NN;
     const size_t chunk = (total + gridDim.x - 1) / gridDim.x;
     const size_t beg = blockIdx.x * chunk, end = (beg + chunk < total) ? beg + chunk : total;
-    double ka = 0, kb = 0, qaa = 0, qab = 0, qbb = 0, mres = 0;
+    double ka = 0, kb = 0, qaa = 0, qab = 0, qbb = 0, mres = 0, m2 = 0;
     for (size_t q = beg + threadIdx.x; q < end; q += blockDim.x) {
         const size_t c = q / NN, o = q - c * NN;
         const double wk = te[c * NN + o], wf = te[(4 + c) * NN + o];
-        const double2 a = Pa[q], b = Pb[q];
+        const double2 a = Pa[q];
         ka += wk * a.x;
-        kb += wk * b.x;
         qaa += wf * (a.x * a.x + a.y * a.y);
+        if (SAME) continue;
+        const double2 b = Pb[q];
+        kb += wk * b.x;
         qab += wf * (a.x * b.x + a.y * b.y);
         qbb += wf * (b.x * b.x + b.y * b.y);
         const double dx = b.x - a.x, dy = b.y - a.y;
-        const double wmag = (c == 0) ? fabs(wf) : 0.5 * fabs(wf);
-        mres = fmax(mres, alpha * wmag * sqrt(dx * dx + dy * dy));
+        const double d2 = dx * dx + dy * dy, t = (c == 0 ? 4.0 * wf : wf) * wf * d2;   // (2 wmag)^2 d2
+        if (t > m2) {
+            m2 = t;
+            const double wmag = (c == 0) ? fabs(wf) : 0.5 * fabs(wf);
+            mres = fmax(mres, alpha * wmag * sqrt(d2));
+        }
+    }
+    if (SAME) {
+        kb = ka;
+        qab = qbb = qaa;
     }
     __shared__ double sh[32];
     double r0 = block_sum(ka, sh), r1 = block_sum(kb, sh), r2 = block_sum(qaa, sh), r3 = block_sum(qab, sh),
@@ -284,14 +353,17 @@ __global__ void __launch_bounds__(256) k_energy_pass(const double* __restrict__ 
     }
 }
 
-__global__ void k_reduce_forms(const double* __restrict__ partials, int nparts, ScfScalars* sc) {
-    if (threadIdx.x != 0) return;
-    double s[6] = {0, 0, 0, 0, 0, 0};
-    for (int q = 0; q < nparts; ++q) {
-        for (int t = 0; t < 5; ++t) s[t] += partials[q * 8 + t];
-        s[5] = fmax(s[5], partials[q * 8 + 5]);
+// a warp a form (one thread, one partial after the other: 0.4 ms)
+__global__ void __launch_bounds__(192) k_reduce_forms(const double* __restrict__ partials, int nparts, ScfScalars* sc) {
+    const int t = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double s = 0.0;
+#pragma unroll 8
+    for (int q = lane; q < nparts; q += 32) {
+        const double v = partials[q * 8 + t];
+        s = t < 5 ? s + v : fmax(s, v);
     }
-    for (int t = 0; t < 6; ++t) sc->forms[t] = s[t];
+    s = t < 5 ? warp_sum_d(s) : warp_max_d(s);
+    if (lane == 0) sc->forms[t] = s;
 }
 
 // y_a = LR dn_a, y_b = LR dn_b ; partial over column chunks: part[chunk][2N]
@@ -496,9 +568,12 @@ int scf_energy_forms(Context& c, const double* te, const double2* Pa, const doub
     const int64_t N = c.N;
     const double NN = (double)N * N;
     prof_begin(ST_ENERGY);
-    k_energy_pass<<<RED_CTAS, 256, 0, c.stream>>>(te, Pa, Pb, N, c.s.alpha, work);
+    if (Pa == Pb)
+        k_energy_pass<true><<<RED_CTAS, 256, 0, c.stream>>>(te, Pa, Pb, N, c.s.alpha, work);
+    else
+        k_energy_pass<false><<<RED_CTAS, 256, 0, c.stream>>>(te, Pa, Pb, N, c.s.alpha, work);
     FORGE_LAUNCH_CHECK();
-    k_reduce_forms<<<1, 32, 0, c.stream>>>(work, RED_CTAS, sc);
+    k_reduce_forms<<<1, 192, 0, c.stream>>>(work, RED_CTAS, sc);
     FORGE_LAUNCH_CHECK();
     // 8 tables + two 4-cell complex states read once
     prof_end(ST_ENERGY, 8.0 * NN * 8.0 + 2.0 * 4.0 * NN * 16.0, 4.0 * NN * 14.0);
@@ -555,6 +630,14 @@ int scf_combine(Context& c, double2* win, const double2* bulk) {
 // their FP32 rounding is relative to their own size; x and r themselves stay FP64.
 constexpr int DIIS_CTAS = 1216;
 
+// (double)x by integer operations: the conversion instruction runs on the FP64 pipe (two lanes a clock and SM), which
+// bounds the two kernels below.  Measured, N = 5044, six slots: k_diis_update 11.0 -> 6.2 ms.
+__device__ __forceinline__ double f2d(float x) {
+    const unsigned b = __float_as_uint(x), m = b & 0x7fffffffu;
+    if (m - 0x00800000u < 0x7f000000u) return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(m << 29));
+    return m == 0 ? __hiloint2double((int)b, 0) : (double)x;   // zero; subnormal, Inf, NaN
+}
+
 // dR_new = (Pn - P) - rprev into slot snew; a_i = Re<dR_i, dR_new>, b_i = Re<dR_i, r> for the
 // slots in the list (snew included, with the value just stored); per-CTA partials [2 x DIIS_MAX].
 __global__ void __launch_bounds__(256) k_diis_dots(DiisArgs d) {
@@ -566,14 +649,16 @@ __global__ void __launch_bounds__(256) k_diis_dots(DiisArgs d) {
         const double2 x = d.P[q], y = d.Pn[q];
         const double rr = y.x - x.x, ri = y.y - x.y;
         const float2 rp = d.rprev[q];
-        const float2 dn = make_float2((float)(rr - (double)rp.x), (float)(ri - (double)rp.y));
+        const float2 dn = make_float2((float)(rr - f2d(rp.x)), (float)(ri - f2d(rp.y)));
         dRnew[q] = dn;
+        const double dnx = f2d(dn.x), dny = f2d(dn.y);
 #pragma unroll
         for (int i = 0; i < DIIS_MAX; ++i) {
             if (i < d.nslots) {
                 const float2 v = (d.slots[i] == d.snew) ? dn : d.hist[(size_t)(2 * d.slots[i] + 1) * d.nn4 + q];
-                a[i] += (double)v.x * dn.x + (double)v.y * dn.y;
-                bb[i] += (double)v.x * rr + (double)v.y * ri;
+                const double vx = f2d(v.x), vy = f2d(v.y);
+                a[i] += vx * dnx + vy * dny;
+                bb[i] += vx * rr + vy * ri;
             }
         }
     }
@@ -601,8 +686,8 @@ __global__ void __launch_bounds__(256) k_diis_update(DiisArgs d) {
             if (i < d.nslots) {
                 const float2 dx = d.hist[(size_t)(2 * d.slots[i]) * d.nn4 + q];
                 const float2 dr = d.hist[(size_t)(2 * d.slots[i] + 1) * d.nn4 + q];
-                nx -= d.gamma[i] * ((double)dx.x + d.beta * (double)dr.x);
-                ny -= d.gamma[i] * ((double)dx.y + d.beta * (double)dr.y);
+                nx -= d.gamma[i] * (f2d(dx.x) + d.beta * f2d(dr.x));
+                ny -= d.gamma[i] * (f2d(dx.y) + d.beta * f2d(dr.y));
             }
         }
         dXp[q] = make_float2((float)(nx - x.x), (float)(ny - x.y));
