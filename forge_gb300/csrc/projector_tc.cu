@@ -18,9 +18,9 @@ __device__ inline float tf32_hi_p(float x) {
 }
 
 // X (n x K columns of X_k, column-major, FP64) -> 6 planes (n rows x ldk, band contiguous).
-// Also adds sum_k |X_ik|^2 of its 32 columns, in FP64, into diag[i]: the diagonal of C (the site
+// Also the sum of |X_ik|^2 over its 32 columns, in FP64, to diag[blockIdx.y * n + i]: the diagonal of C (the site
 // densities, which drive the long-range Hartree potential) is taken from there, not from the
-// tensor-core product.
+// tensor-core product.  The partial sums are added in order (k_proj_accum), so that two runs agree.
 __global__ void k_stage_proj(const double2* __restrict__ X, int64_t ldx, int64_t n, int64_t K, int64_t ldk,
                              float* __restrict__ Xt, double* __restrict__ diag) {
     __shared__ double2 tile[32][33];
@@ -38,7 +38,7 @@ __global__ void k_stage_proj(const double2* __restrict__ X, int64_t ldx, int64_t
     if (threadIdx.y == 0 && i0 + threadIdx.x < n) {
         double t = 0.0;
         for (int y = 0; y < (int)blockDim.y; ++y) t += dpart[y][threadIdx.x];
-        atomicAdd(diag + i0 + threadIdx.x, t);
+        diag[blockIdx.y * n + i0 + threadIdx.x] = t;
     }
     const size_t P = (size_t)n * ldk;
     for (int q = threadIdx.y; q < 32; q += blockDim.y) {
@@ -78,7 +78,7 @@ struct ProjStoreEpi {
 // Hermitian C of which only the lower triangle (Cr, Ci) was formed; 32 x 32 tiles, coalesced.
 __global__ void __launch_bounds__(256) k_proj_accum(double2* __restrict__ P, const float* __restrict__ Cr,
                                                     const float* __restrict__ Ci, const double* __restrict__ diag,
-                                                    int64_t n, double2 ph0, double2 ph1, double2 ph2, double2 ph3) {
+                                                    int64_t ndiag, int64_t n, double2 ph0, double2 ph1, double2 ph2, double2 ph3) {
     const int64_t bi = blockIdx.x, bj = blockIdx.y;
     if (bi < bj) return;
     __shared__ float sr[32][33], si[32][33];
@@ -98,8 +98,9 @@ __global__ void __launch_bounds__(256) k_proj_accum(double2* __restrict__ P, con
         if (i >= n || j >= n) continue;
         double cr, ci;
         if (i == j) {
-            cr = diag[i];
-            ci = 0.0;
+            cr = ci = 0.0;
+#pragma unroll 8
+            for (int64_t q = 0; q < ndiag; ++q) cr += diag[q * n + i];
         } else if (i > j) {
             cr = sr[y][threadIdx.x];
             ci = si[y][threadIdx.x];
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(256) k_proj_accum(double2* __restrict__ P, con
 }
 
 size_t proj_tc_workspace_floats(int64_t n, int64_t iu) {
-    return 6 * (size_t)n * ((iu + 3) / 4 * 4) + 2 * (size_t)n * n + 2 * (size_t)n + 256;
+    return 6 * (size_t)n * ((iu + 3) / 4 * 4) + 2 * (size_t)n * n + 2 * (size_t)n * ((iu + 31) / 32) + 256;
 }
 
 // P_c += ph_c * conj(X) X^T over the first K columns of X (n x K, ldx) on the tensor cores.
@@ -147,7 +148,6 @@ int bulk_projector_tc(cudaStream_t st, const double2* X, int64_t ldx, int64_t n,
     Cr = (float*)(((uintptr_t)Cr + 255) & ~(uintptr_t)255);
     float* Ci = Cr + (size_t)n * n;
     double* diag = (double*)(((uintptr_t)(Ci + (size_t)n * n) + 255) & ~(uintptr_t)255);
-    FORGE_CUDA(cudaMemsetAsync(diag, 0, n * sizeof(double), st));
     dim3 g((unsigned)((n + 31) / 32), (unsigned)((K + 31) / 32));
     k_stage_proj<<<g, dim3(32, 8), 0, st>>>(X, ldx, n, K, ldk, ws, diag);
     FORGE_LAUNCH_CHECK();
@@ -168,7 +168,7 @@ int bulk_projector_tc(cudaStream_t st, const double2* X, int64_t ldx, int64_t n,
     FORGE_TRY(tc_gemm_tf32_mapped(st, op, mk(za), op, mk(zbr), 1, 1, ProjStoreEpi{Cr, n}, err));
     FORGE_TRY(tc_gemm_tf32_mapped(st, op, mk(za), op, mk(zbi), 1, 1, ProjStoreEpi{Ci, n}, err));
     const unsigned nt = (unsigned)((n + 31) / 32);
-    k_proj_accum<<<dim3(nt, nt), dim3(32, 8), 0, st>>>(P, Cr, Ci, diag, n, ph[0], ph[1], ph[2], ph[3]);
+    k_proj_accum<<<dim3(nt, nt), dim3(32, 8), 0, st>>>(P, Cr, Ci, diag, nkp, n, ph[0], ph[1], ph[2], ph[3]);
     FORGE_LAUNCH_CHECK();
     const double nd = (double)n;
     prof_end(ST_PROJECTOR, nd * K * 16.0 + 2.0 * 4.0 * 2.0 * nd * nd * 16.0, 2.0 * 2.0 * nd * nd * 6.0 * K / 2.0);
