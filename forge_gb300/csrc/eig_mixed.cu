@@ -98,8 +98,9 @@ void carve(MixedWs& w, Carve& c) {
     bt_split_caps(n, iu, B, ksg, ksw);
     w.Wb = c.take<float2>(ksw * B * BT_NB * iu);
     w.W2 = c.take<float2>(B * BT_NB * iu);
-    w.G = c.take<float2>(ksg * B * BT_NB * BT_NB);
-    w.T = c.take<float2>(B * BT_NB * BT_NB);
+    const int64_t nbt = std::max<int64_t>(1, (n - 1 + BT_NB - 1) / BT_NB);   // blocks of the back-transformation
+    w.G = c.take<float2>(nbt * ksg * B * BT_NB * BT_NB);
+    w.T = c.take<float2>(nbt * B * BT_NB * BT_NB);
     w.err = c.take<int>(1);
 }
 }  // namespace
@@ -358,12 +359,21 @@ struct TWb {
     }
 };
 
-// T of the compact-WY form from the Gram matrix G = V^H V, given as ks K-split partials
-// (partial s of batch item b at G + (s * batch + b) * BT_NB^2).  blockDim.x = BT_NB.
-__global__ void k_larft32(const float2* __restrict__ G, int64_t ks, int64_t batch, const float2* __restrict__ tau,
-                          int64_t n, int64_t j0, int64_t nbk, float2* __restrict__ T) {
-    const int64_t b = blockIdx.x;
-    float2* Tb = T + b * BT_NB * BT_NB;
+// K splits of the Gram matrix of block blk
+__host__ __device__ inline int64_t bt_gram_want(int64_t n, int64_t blk, int64_t cap) {
+    const int64_t want = (n - blk * BT_NB + 255) / 256;
+    return want < cap ? want : cap;
+}
+// T of the compact-WY form from the Gram matrices G = V^H V of all blocks, given as K-split partials (partial s of
+// batch item b of block blk at G + ((blk * cap + s) * batch + b) * BT_NB^2).  blockDim.x = BT_NB, grid (batch, blocks).
+// One block is a chain of BT_NB steps on one SM (170 us), so all blocks go side by side.  Measured, the whole
+// back-transformation: N = 5044, one matrix (79 blocks) 43.7 -> 34.1 ms; N = 1324, 16 matrices 12.5 -> 10.4 ms.
+__global__ void k_larft32(const float2* __restrict__ G, int64_t cap, int64_t batch, const float2* __restrict__ tau,
+                          int64_t n, float2* __restrict__ T) {
+    const int64_t b = blockIdx.x, blk = blockIdx.y, j0 = blk * BT_NB;
+    const int64_t nbk = n - 1 - j0 < BT_NB ? n - 1 - j0 : BT_NB, ks = zg_ksplit_count(n - j0, bt_gram_want(n, blk, cap));
+    G += blk * cap * batch * BT_NB * BT_NB;
+    float2* Tb = T + (blk * batch + b) * BT_NB * BT_NB;
     const float2* tb = tau + b * n;
     __shared__ float2 tmp[BT_NB];
     __shared__ float2 Gs[BT_NB][BT_NB + 1];   // Gs[i][r] = G(r, i), upper part r < i
@@ -522,6 +532,17 @@ int backtransform_tc(cudaStream_t st, MixedWs& ws, int64_t batch) {
     const int64_t lda = n, strideA = n * n;
     int64_t ksg_cap, ksw_cap;
     bt_split_caps(n, iu, batch, ksg_cap, ksw_cap);
+    if (nblocks <= 0) return 0;
+    // Gram matrices (CUDA cores, FP32, split over K to fill the GPU) and compact-WY factors of all blocks
+    for (int64_t blk = 0; blk < nblocks; ++blk) {
+        const int64_t j0 = blk * BT_NB, nbk = std::min<int64_t>(nrefl - j0, BT_NB);
+        FORGE_TRY((zgemm_launch_splitk<float2, KMAJOR, KMAJOR>(
+            st, BT_NB, BT_NB, n - j0, batch, bt_gram_want(n, blk, ksg_cap), BtGA{ws.A32, lda, strideA, n, j0, nbk},
+            BtGB{ws.A32, lda, strideA, n, j0, nbk},
+            StoreGramSplit{ws.G + blk * ksg_cap * batch * BT_NB * BT_NB, batch})));
+    }
+    k_larft32<<<dim3((unsigned)batch, (unsigned)nblocks), BT_NB, 0, st>>>(ws.G, ksg_cap, batch, ws.tau, n, ws.T);
+    FORGE_LAUNCH_CHECK();
     for (int64_t blk = nblocks - 1; blk >= 0; --blk) {
         const int64_t j0 = blk * BT_NB;
         const int64_t nbk = (nrefl - j0 < BT_NB) ? (nrefl - j0) : BT_NB;
@@ -529,14 +550,6 @@ int backtransform_tc(cudaStream_t st, MixedWs& ws, int64_t batch) {
         const int64_t nkp = (Krows + 31) / 32;
         const int64_t Kp = nkp * 32;
         int64_t ksw = 1;
-        // Gram (CUDA cores, FP32, split over K to fill the GPU) and compact-WY factor
-        const int64_t kg_want = std::min<int64_t>(ksg_cap, (Krows + 255) / 256);
-        const int64_t ksg = zg_ksplit_count(Krows, kg_want);
-        FORGE_TRY((zgemm_launch_splitk<float2, KMAJOR, KMAJOR>(
-            st, BT_NB, BT_NB, Krows, batch, kg_want, BtGA{ws.A32, lda, strideA, n, j0, nbk},
-            BtGB{ws.A32, lda, strideA, n, j0, nbk}, StoreGramSplit{ws.G, batch})));
-        k_larft32<<<(unsigned)batch, BT_NB, 0, st>>>(ws.G, ksg, batch, ws.tau, n, j0, nbk, ws.T);
-        FORGE_LAUNCH_CHECK();
         // W = V^H X  (tensor cores)
         k_stage_bt1<<<dim3((unsigned)((Kp + 255) / 256), BT_NB, (unsigned)batch), 256, 0, st>>>(
             ws.A32, lda, strideA, n, j0, nbk, Kp, ws.A1, 2 * BT_NB * 6 * ws.Kp);
@@ -558,7 +571,8 @@ int backtransform_tc(cudaStream_t st, MixedWs& ws, int64_t batch) {
             FORGE_TRY(tc_gemm_tf32_mapped(st, A, ka, B, kb, batch, 0, BtW1Epi{ws.Wb, nbk, iu}, ws.err, want));
         }
         // W2 = T W (CUDA cores; W summed over its K-split partials on load)
-        FORGE_TRY((zgemm_launch<float2, IMAJOR, KMAJOR, false>(st, BT_NB, iu, BT_NB, batch, TWa{ws.T, nbk},
+        FORGE_TRY((zgemm_launch<float2, IMAJOR, KMAJOR, false>(st, BT_NB, iu, BT_NB, batch,
+                                                                TWa{ws.T + blk * batch * BT_NB * BT_NB, nbk},
                                                                 TWb{ws.Wb, nbk, iu, ksw},
                                                                 StoreF2{ws.W2, BT_NB, BT_NB * iu})));
         // X(j0:, :) -= V W2  (tensor cores)

@@ -127,7 +127,7 @@ inline int zgemm_launch(cudaStream_t st, int64_t M, int64_t N, int64_t K, int64_
 }
 
 // Number of K splits zgemm_launch_splitk runs for a K extent when `want` are asked for (none empty).
-inline int64_t zg_ksplit_count(int64_t K, int64_t want) {
+__host__ __device__ inline int64_t zg_ksplit_count(int64_t K, int64_t want) {
     if (want <= 1 || K <= ZG_BK) return 1;
     int64_t chunk = (K + want - 1) / want;
     chunk = (chunk + ZG_BK - 1) / ZG_BK * ZG_BK;
