@@ -6,8 +6,8 @@
 // round trips to L2.  So the three kernels are launched programmatically and load what older kernels left (the panel,
 // the trailing matrix) before they wait for their predecessor, every thread's loads of a phase are in
 // flight together, and no CTA adds up partials one by one.  One matrix of n = 5044 (5043 columns), whole kernels:
-// trd_col 78 -> 58 ms, trd_hemv 91 -> 72 ms, trd_finish (with trd_fix, now once a panel) 116 -> 41 ms; n = 364, six
-// matrices: 5.4 -> 4.1, 4.2 -> 3.4, 5.4 -> 3.1 ms.
+// trd_col 78 -> 55 ms, trd_hemv 91 -> 62 ms, trd_finish (with trd_fix, now once a panel) 116 -> 42 ms; n = 364, 36
+// matrices: 5.4 -> 3.9, 4.2 -> 3.2, 5.4 -> 3.1 ms.
 // The order of every FP32 sum is part of the result: refined orbitals are compared to the last place.
 #include "tridiag.cuh"
 
@@ -225,12 +225,18 @@ __global__ void __launch_bounds__(256) k_trd_hemv(TrdArgs<float> a, int64_t p, i
         __shared__ V cq[4][HV_CB];
         const int tr = threadIdx.x & 63, tg = threadIdx.x >> 6;
         const int64_t r0 = R0 + tr, rv = (tg == 0 ? R0 : C0) + tr;
-        // 16 loads per thread (row r0, 16 columns) before the column is known: a panel leaves A22 as it is
+        // 16 loads per thread (row r0, 16 columns) before the column is known: a panel leaves A22 as it is.  Most tiles are
+        // whole and below the diagonal: no bounds, no conjugates of the diagonal there (a third of the instructions).
+        const bool whole = bi > bj && R0 + HV_RB <= n;
         V xv = vzero<V>(), a0[16];
+        const V* pa = A + r0 + (C0 + tg * 16) * lda;
+        if (whole) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int64_t c = C0 + tg * 16 + q;
-            a0[q] = (r0 < n && c < n && c <= r0) ? ld_early(A + r0 + c * lda) : vzero<V>();
+            for (int q = 0; q < 16; ++q, pa += lda) a0[q] = ld_early(pa);
+        } else {
+            const int cn = (int)min(n - (C0 + tg * 16), (int64_t)16), cd = (int)min(r0 - (C0 + tg * 16), (int64_t)16);
+#pragma unroll
+            for (int q = 0; q < 16; ++q, pa += lda) a0[q] = (r0 < n && q < cn && q <= cd) ? ld_early(pa) : vzero<V>();
         }
         trd_chain_wait();
         const float sr = (float)sc[2], si = (float)sc[3];
@@ -239,15 +245,23 @@ __global__ void __launch_bounds__(256) k_trd_hemv(TrdArgs<float> a, int64_t p, i
         __syncthreads();
         V racc = vzero<V>();
         const V v0 = vr[tr];
+        if (whole) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int64_t c = C0 + tg * 16 + q;
-            V x0 = a0[q];
-            const bool d0 = (c == r0);
-            if (d0) x0.y = 0;
-            racc = vadd(racc, vmul(x0, vc[tg * 16 + q]));
-            // column part: conj(A(r, c)) v_r for r > c (the diagonal belongs to the row part only)
-            cs[tr][tg * 16 + q] = d0 ? vzero<V>() : vcjmul(x0, v0);
+            for (int q = 0; q < 16; ++q) {
+                racc = vadd(racc, vmul(a0[q], vc[tg * 16 + q]));
+                cs[tr][tg * 16 + q] = vcjmul(a0[q], v0);
+            }
+        } else {
+            const int dq = (int)max(min(r0 - (C0 + tg * 16), (int64_t)16), (int64_t)-1);   // the diagonal's column
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                V x0 = a0[q];
+                const bool d0 = q == dq;
+                if (d0) x0.y = 0;
+                racc = vadd(racc, vmul(x0, vc[tg * 16 + q]));
+                // column part: conj(A(r, c)) v_r for r > c (the diagonal belongs to the row part only)
+                cs[tr][tg * 16 + q] = d0 ? vzero<V>() : vcjmul(x0, v0);
+            }
         }
         rsum[tg][tr] = racc;
         __syncthreads();
