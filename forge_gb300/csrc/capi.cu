@@ -342,12 +342,26 @@ int project_items(forge_ctx* x, const std::vector<ProjItem>& items, double2* out
     return 0;
 }
 
+// whether a bounded wait of the projectors' products gave up (waits for the stream)
+int projector_status(forge_ctx* x) {
+    if (!x->tcerr.ptr) return 0;
+    int herr = 0;
+    FORGE_CUDA(cudaMemcpyAsync(&herr, x->tcerr.ptr, sizeof(int), cudaMemcpyDeviceToHost, x->c.stream));
+    FORGE_CUDA(cudaStreamSynchronize(x->c.stream));
+    if (herr) {
+        set_error(FORGE_ERR_TIMEOUT, "tcgen05 projector: a bounded mbarrier wait gave up");
+        return FORGE_ERR_TIMEOUT;
+    }
+    return 0;
+}
+
 // the zFockBulk sum over the local k points: bands 1..nLower-1 of every k
 int project_bulk(forge_ctx* x, double2* out) {
     const int64_t kb = x->k_begin, ke = (x->k_end > 0) ? x->k_end : x->c.Nk;
     std::vector<ProjItem> items;
     for (int64_t k = kb; k < ke; ++k) add_projector(x, k, x->c.nLower - 1, &x->h_bph[k * 4], items);
-    return project_items(x, items, out);
+    FORGE_TRY(project_items(x, items, out));
+    return projector_status(x);
 }
 
 // window states with the C3 average: a state at a C3-invariant k becomes itself and its two
@@ -488,15 +502,7 @@ int project_fused_once(forge_ctx* x) {
     }
     FORGE_CUDA(cudaMemsetAsync(c.bulk.ptr, 0, 4 * NN * sizeof(double2), c.stream));
     FORGE_TRY(scf_combine(c, x->Pn.as<double2>(), c.bulk.as<double2>()));
-    if (x->tcerr.ptr) {
-        int herr = 0;
-        FORGE_CUDA(cudaMemcpyAsync(&herr, x->tcerr.ptr, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-        FORGE_CUDA(cudaStreamSynchronize(c.stream));
-        if (herr) {
-            set_error(FORGE_ERR_TIMEOUT, "tcgen05 projector: a bounded mbarrier wait gave up");
-            return FORGE_ERR_TIMEOUT;
-        }
-    }
+    FORGE_TRY(projector_status(x));
     x->have_pnew = true;
     return 0;
 }
@@ -594,15 +600,7 @@ int project_valley_once(forge_ctx* x) {
     FORGE_TRY(valley_window(x, st));
     FORGE_CUDA(cudaMemsetAsync(c.bulk.ptr, 0, 4 * NN * sizeof(double2), c.stream));
     FORGE_TRY(scf_combine(c, x->Pn.as<double2>(), c.bulk.as<double2>()));
-    if (x->tcerr.ptr) {
-        int herr = 0;
-        FORGE_CUDA(cudaMemcpyAsync(&herr, x->tcerr.ptr, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-        FORGE_CUDA(cudaStreamSynchronize(c.stream));
-        if (herr) {
-            set_error(FORGE_ERR_TIMEOUT, "tcgen05 projector: a bounded mbarrier wait gave up");
-            return FORGE_ERR_TIMEOUT;
-        }
-    }
+    FORGE_TRY(projector_status(x));
     x->have_pnew = true;
     return 0;
 }
