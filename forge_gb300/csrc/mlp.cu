@@ -3,8 +3,10 @@
 //
 // Forward: one CTA of 128 threads per 32 samples; activations of the 32 samples stay in shared
 // memory, thread t computes hidden unit t for all of them (weights read as bf16 pairs).
-// Backward: the same tiling in reverse; per-CTA weight gradients are reduced in shared memory and
-// added to the FP32 gradient buffers with atomics.  Adam updates the FP32 masters and refreshes
+// Backward: the same tiling in reverse; per-CTA weight gradients are summed over the 32 samples by a thread each and
+// added to the FP32 gradient buffers with atomics, a warp's 32 in one line.  Bound: FP32 FMAs fed by shared-memory
+// broadcasts, so those are float4 (rows of MLP_P floats), four FMAs a load.  Measured, gradient of 14560 samples
+// with its copies: 520 -> 275 us.  Adam updates the FP32 masters and refreshes
 // the BF16 copies used by the next forward pass.
 // No counterpart in the reference (FORGE starts from the non-interacting guess or a checkpoint).
 #include <cuda_bf16.h>
@@ -21,6 +23,8 @@ constexpr int MLP_W = 128;     // hidden width
 constexpr int MLP_S = 32;      // samples per CTA
 constexpr int MLP_MAXIN = 64;  // max input features
 constexpr int MLP_MAXOUT = 8;  // max outputs
+constexpr int MLP_P = MLP_W + 4;      // row pitches in shared memory (float4)
+constexpr int MLP_XP = MLP_MAXIN + 4;
 
 struct MlpDims {
     int din, dout;
@@ -49,17 +53,34 @@ __device__ inline float dsilu(float x) {
     return s * (1.f + x * (1.f - s));
 }
 
+// acc[s] += w . v[s][f .. f + 3], in the order of f
+template <int P>
+__device__ __forceinline__ void fma4(float* acc, const float (*v)[P], int f, float4 w) {
+#pragma unroll
+    for (int s = 0; s < MLP_S; ++s) {
+        const float4 x = *reinterpret_cast<const float4*>(&v[s][f]);
+        acc[s] = fmaf(w.w, x.w, fmaf(w.z, x.z, fmaf(w.y, x.y, fmaf(w.x, x.x, acc[s]))));
+    }
+}
+// four consecutive bf16 weights (8-byte aligned)
+__device__ __forceinline__ float4 weights4(const __nv_bfloat16* p) {
+    const uint2 q = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xffff0000u), __uint_as_float(q.y << 16),
+                       __uint_as_float(q.y & 0xffff0000u));
+}
+
 // pre-activations are stored (Z0, Z1, Z2: B x 128) for the backward pass
 __global__ void __launch_bounds__(MLP_W) k_mlp_forward(MlpDims d, const __nv_bfloat16* __restrict__ W,
                                                        const float* __restrict__ X, int64_t n, float* __restrict__ Y,
                                                        float* __restrict__ Z) {
-    __shared__ float h[MLP_S][MLP_W + 1];
-    __shared__ float xin[MLP_S][MLP_MAXIN + 1];
+    __shared__ __align__(16) float h[MLP_S][MLP_P];
+    __shared__ __align__(16) float xin[MLP_S][MLP_XP];
     const int t = threadIdx.x;
     const int64_t s0 = (int64_t)blockIdx.x * MLP_S;
-    for (int q = t; q < MLP_S * d.din; q += MLP_W) {
-        const int s = q / d.din, f = q - s * d.din;
-        xin[s][f] = (s0 + s < n) ? X[(s0 + s) * d.din + f] : 0.f;
+    const int din4 = (d.din + 3) / 4 * 4;
+    for (int q = t; q < MLP_S * din4; q += MLP_W) {
+        const int s = q / din4, f = q - s * din4;
+        xin[s][f] = (s0 + s < n && f < d.din) ? X[(s0 + s) * d.din + f] : 0.f;
     }
     __syncthreads();
     float acc[MLP_S];
@@ -68,11 +89,9 @@ __global__ void __launch_bounds__(MLP_W) k_mlp_forward(MlpDims d, const __nv_bfl
         const float bias = __bfloat162float(W[d.b0 + t]);
 #pragma unroll
         for (int s = 0; s < MLP_S; ++s) acc[s] = bias;
-        for (int f = 0; f < d.din; ++f) {
-            const float w = __bfloat162float(W[d.w0 + (int64_t)t * d.din + f]);
-#pragma unroll
-            for (int s = 0; s < MLP_S; ++s) acc[s] = fmaf(w, xin[s][f], acc[s]);
-        }
+        const __nv_bfloat16* w0 = W + d.w0 + (int64_t)t * d.din;
+        auto wt0 = [&](int f) { return f < d.din ? __bfloat162float(w0[f]) : 0.f; };
+        for (int f = 0; f < din4; f += 4) fma4<MLP_XP>(acc, xin, f, make_float4(wt0(f), wt0(f + 1), wt0(f + 2), wt0(f + 3)));
 #pragma unroll
         for (int s = 0; s < MLP_S; ++s) {
             if (Z && s0 + s < n) Z[(s0 + s) * 3 * MLP_W + t] = acc[s];
@@ -86,11 +105,7 @@ __global__ void __launch_bounds__(MLP_W) k_mlp_forward(MlpDims d, const __nv_bfl
         const float bias = __bfloat162float(W[bo + t]);
 #pragma unroll
         for (int s = 0; s < MLP_S; ++s) acc[s] = bias;
-        for (int f = 0; f < MLP_W; ++f) {
-            const float w = __bfloat162float(W[wo + (int64_t)t * MLP_W + f]);
-#pragma unroll
-            for (int s = 0; s < MLP_S; ++s) acc[s] = fmaf(w, h[s][f], acc[s]);
-        }
+        for (int f = 0; f < MLP_W; f += 4) fma4<MLP_P>(acc, h, f, weights4(W + wo + (int64_t)t * MLP_W + f));
         __syncthreads();
 #pragma unroll
         for (int s = 0; s < MLP_S; ++s) {
@@ -114,10 +129,10 @@ __global__ void __launch_bounds__(MLP_W) k_mlp_backward(MlpDims d, const __nv_bf
                                                         const float* __restrict__ Tgt, const float* __restrict__ wt,
                                                         const float* __restrict__ Z, int64_t n,
                                                         float* __restrict__ G, float* __restrict__ loss) {
-    __shared__ float a[MLP_S][MLP_W + 1];   // activations of the current layer input
-    __shared__ float g[MLP_S][MLP_W + 1];   // gradient w.r.t. pre-activations of the current layer
+    __shared__ __align__(16) float a[MLP_S][MLP_P];   // activations of the current layer input
+    __shared__ __align__(16) float g[MLP_S][MLP_P];   // gradient w.r.t. pre-activations of the current layer
     __shared__ float dy[MLP_S][MLP_MAXOUT];
-    __shared__ float xin[MLP_S][MLP_MAXIN + 1];
+    __shared__ __align__(16) float xin[MLP_S][MLP_XP];
     const int t = threadIdx.x;
     const int64_t s0 = (int64_t)blockIdx.x * MLP_S;
     float lsum = 0.f;
@@ -166,12 +181,27 @@ __global__ void __launch_bounds__(MLP_W) k_mlp_backward(MlpDims d, const __nv_bf
         for (int s = 0; s < MLP_S; ++s)
             a[s][t] = (s0 + s < n) ? silu(Z[(s0 + s) * 3 * MLP_W + (layer - 1) * MLP_W + t]) : 0.f;
         __syncthreads();
-        // dW[t][f] for fixed t (output unit) over f: thread t owns row t
-        for (int f = 0; f < MLP_W; ++f) {
-            float gw = 0.f;
-#pragma unroll 8
-            for (int s = 0; s < MLP_S; ++s) gw = fmaf(g[s][t], a[s][f], gw);
-            atomicAdd(&G[wo + (int64_t)t * MLP_W + f], gw);
+        // dW[u][t]: thread t owns input t (a warp's 32 atomics fall in one line), four output units u at a time
+        {
+            float as[MLP_S];
+#pragma unroll
+            for (int s = 0; s < MLP_S; ++s) as[s] = a[s][t];
+            for (int u = 0; u < MLP_W; u += 4) {
+                float4 gw = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int s = 0; s < MLP_S; ++s) {
+                    const float4 x = *reinterpret_cast<const float4*>(&g[s][u]);
+                    gw.x = fmaf(x.x, as[s], gw.x);
+                    gw.y = fmaf(x.y, as[s], gw.y);
+                    gw.z = fmaf(x.z, as[s], gw.z);
+                    gw.w = fmaf(x.w, as[s], gw.w);
+                }
+                float* o = &G[wo + (int64_t)u * MLP_W + t];
+                atomicAdd(o, gw.x);
+                atomicAdd(o + MLP_W, gw.y);
+                atomicAdd(o + 2 * MLP_W, gw.z);
+                atomicAdd(o + 3 * MLP_W, gw.w);
+            }
         }
         {
             float gb = 0.f;
@@ -182,10 +212,10 @@ __global__ void __launch_bounds__(MLP_W) k_mlp_backward(MlpDims d, const __nv_bf
         float gp[MLP_S];
 #pragma unroll
         for (int s = 0; s < MLP_S; ++s) gp[s] = 0.f;
-        for (int u = 0; u < MLP_W; ++u) {
-            const float w = __bfloat162float(W[wo + (int64_t)u * MLP_W + t]);
-#pragma unroll
-            for (int s = 0; s < MLP_S; ++s) gp[s] = fmaf(w, g[s][u], gp[s]);
+        for (int u = 0; u < MLP_W; u += 4) {
+            const __nv_bfloat16* w = W + wo + (int64_t)u * MLP_W + t;
+            fma4<MLP_P>(gp, g, u, make_float4(__bfloat162float(w[0]), __bfloat162float(w[MLP_W]),
+                                              __bfloat162float(w[2 * MLP_W]), __bfloat162float(w[3 * MLP_W])));
         }
         __syncthreads();
 #pragma unroll
@@ -194,10 +224,12 @@ __global__ void __launch_bounds__(MLP_W) k_mlp_backward(MlpDims d, const __nv_bf
         __syncthreads();
     }
     // first layer: dW0[t][f] = sum_s g[s][t] x[s][f]
-    for (int f = 0; f < d.din; ++f) {
+    for (int q = t; q < MLP_W * d.din; q += MLP_W) {
+        const int u = q / d.din, f = q - u * d.din;
         float gw = 0.f;
-        for (int s = 0; s < MLP_S; ++s) gw = fmaf(g[s][t], xin[s][f], gw);
-        atomicAdd(&G[d.w0 + (int64_t)t * d.din + f], gw);
+#pragma unroll 8
+        for (int s = 0; s < MLP_S; ++s) gw = fmaf(g[s][u], xin[s][f], gw);
+        atomicAdd(&G[d.w0 + q], gw);
     }
     {
         float gb = 0.f;
