@@ -86,7 +86,9 @@ __global__ void __launch_bounds__(COL_ROWS + 32) k_trd_col(TrdArgs<float> a, int
     const int lm = ii - 1;
     const float2 z = make_float2(0.f, 0.f);
     const bool mine = threadIdx.x < COL_ROWS && r < n, alpha_warp = threadIdx.x >= COL_ROWS;
-    // what older kernels left: the raw column, the panel but for its last reflector
+    // A panel's first column follows the kernel that updated the matrix.  Later ones load ahead what older kernels left:
+    // the raw column, the panel but for its last reflector.
+    if (ii == 0) trd_chain_wait();
     float2 x = z, wl = z, vl = z, av[16], wv[16];
     if (mine) x = ld_early(A + r + col * lda);
 #pragma unroll
@@ -98,7 +100,7 @@ __global__ void __launch_bounds__(COL_ROWS + 32) k_trd_col(TrdArgs<float> a, int
         wrow[lane] = ld_early(W + col + lane * n);
         arow[lane] = ld_early(A + col + (p + lane) * lda);
     }
-    trd_chain_wait();
+    if (ii > 0) trd_chain_wait();
     if (mine && ii > 0) {
         wl = w0[r];
         vl = A[r + (p + lm) * lda];

@@ -64,7 +64,8 @@ __device__ __forceinline__ void trd_chain_wait() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 // Loads ahead of trd_chain_wait: of what the predecessor's own predecessor, or an older kernel, wrote (the predecessor
-// has started all of its CTAs past its wait by then, so those results are in memory); from L2.
+// has started all of its CTAs past its wait by then, so those results are in memory); from L2.  The predecessor's own
+// results, and those of a kernel that was not launched by launch_chain, are not: they come after the wait.
 __device__ __forceinline__ double2 ld_early(const double2* p) {
     double2 v;
     asm volatile("ld.global.cg.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));

@@ -58,8 +58,8 @@ __device__ __forceinline__ double xor16(double v) { return __shfl_xor_sync(0xfff
 // partial sums: [0, np) norm of the column (k_col64), then np pairs w^H v (k_finish64)
 __device__ inline int64_t parts_of(int64_t n, int fr) { return (n + fr - 1) / fr; }
 
-// alpha2 = -1/2 tau (w^H v) of the last column from the nd partials of k_finish64, (rows rows, fr a partial), by one warp; lanes below 16 the
-// real part, the others the imaginary part
+// alpha2 = -1/2 tau (w^H v) of the last column from the partials of k_finish64 (rows rows, fr a partial), by one warp;
+// lanes below 16 the real part, the others the imaginary part
 __device__ inline double alpha2_of(const TrdArgs<double>& a, int64_t b, int64_t rows, int fr) {
     const double* part = a.part + b * a.pstride + parts_of(a.n, fr);
     const int64_t nd = parts_of(rows, fr);
