@@ -73,8 +73,7 @@ int scf_diis_dens(Context& c, const double2* P, double* dens, double* work, ScfS
 int scf_diis_commit(Context& c, ScfScalars* sc);
 size_t scf_diis_parts();
 // mixed-precision eigen-solver (eig_mixed.cu) and its FP64 window refinement (rr_window.cu)
-int eig_mixed(cudaStream_t st, EigArgs& g, void* mixed_ws);
-size_t eig_mixed_workspace_bytes(int64_t n, int64_t iu, int64_t batch);
+int eig_mixed(cudaStream_t st, EigArgs& g, void* mixed_ws, size_t ws_bytes);
 int rr_window(cudaStream_t st, const double2* H, int64_t strideH, double2* X, int64_t ldx, int64_t strideX, double* w,
               int64_t iu, int64_t n, int64_t c0, int64_t nw, int64_t batch, void* ws);
 size_t rr_window_workspace_bytes(int64_t n, int64_t batch);
@@ -253,10 +252,10 @@ int eig_batch_run(forge_ctx* x, int64_t k0, int64_t nb, int* info, double2* Xdst
         g.iu_out = iu;
         g.w = x->w_all.as<double>();
     }
-    eig_bind_workspace(g, x->eigws.ptr);
+    FORGE_TRY(eig_bind_workspace(g, x->eigws.ptr, x->eigws.bytes));
     if (c.precision == FORGE_PREC_MIXED) {
         auto solve = [&]() -> int {
-            int r = eig_mixed(c.stream, g, x->mixws.ptr);
+            int r = eig_mixed(c.stream, g, x->mixws.ptr, x->mixws.bytes);
             if (r || !oa) return r;
             // FP64-accurate eigenpairs 1..iu from the mixed ones (tensor-core refinement)
             int64_t n4 = 0;
@@ -928,8 +927,8 @@ int solve_group_device(forge_ctx** xs, int64_t nctx, int* infos) {
         for (int64_t q = 0; q < nb; ++q) lims[q] = (int)xs[items[q0 + q].first]->c.nUpper;
         FORGE_CUDA(cudaMemcpyAsync(x0->g_lim.ptr, lims.data(), nb * sizeof(int), cudaMemcpyHostToDevice, st));
         g.iu_lim = x0->g_lim.as<int>();
-        eig_bind_workspace(g, x0->g_eigws.ptr);
-        FORGE_TRY(mixed ? eig_mixed(st, g, x0->g_mixws.ptr) : eig_fp64(st, g));
+        FORGE_TRY(eig_bind_workspace(g, x0->g_eigws.ptr, x0->g_eigws.bytes));
+        FORGE_TRY(mixed ? eig_mixed(st, g, x0->g_mixws.ptr, x0->g_mixws.bytes) : eig_fp64(st, g));
         if (mixed && x0->rr_width > 0)
             for (int64_t q = 0; q < nb; ++q) {
                 const int64_t iub = xs[items[q0 + q].first]->c.nUpper;
@@ -1605,8 +1604,8 @@ int forge_gpu_zheevr_batch(forge_ctx* x, int64_t nb, const double* A, int64_t iu
         g.iu_out = iu;
         g.w = wall.as<double>();
     }
-    eig_bind_workspace(g, ws.ptr);
-    rc = (c.precision == FORGE_PREC_MIXED) ? eig_mixed(c.stream, g, mws.ptr) : eig_fp64(c.stream, g);
+    rc = eig_bind_workspace(g, ws.ptr, ws.bytes);
+    if (!rc) rc = (c.precision == FORGE_PREC_MIXED) ? eig_mixed(c.stream, g, mws.ptr, mws.bytes) : eig_fp64(c.stream, g);
     if (!rc && oa) {
         int64_t n4 = 0;
         const float* planes = eig_mixed_planes(mws.ptr, N, N, nb, &n4);

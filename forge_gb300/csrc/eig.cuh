@@ -51,10 +51,14 @@ struct EigArgs {
     int64_t iu_out = 0;         // mixed solver: FP64 columns written to X (0: all iu)
 };
 
-// workspace sizes (bytes) for a given problem
+// workspace sizes (bytes) for a given problem; they serve every smaller batch as well
 size_t eig_workspace_bytes(int64_t n, int64_t iu, int64_t batch);
-// carve the workspace out of one device buffer
-void eig_bind_workspace(EigArgs& g, void* base);
+// carve the workspace out of one device buffer; FORGE_ERR_ARG if the batch needs more than the bytes given
+int eig_bind_workspace(EigArgs& g, void* base, size_t bytes);
+
+size_t eig_mixed_workspace_bytes(int64_t n, int64_t iu, int64_t batch);
+// K-split partial products of a batch and the room for them: Gram matrices (used, room), V^H X (used, room)
+void eig_mixed_splits(int64_t n, int64_t iu, int64_t batch, int64_t* out);
 
 int eig_fp64(cudaStream_t st, EigArgs& g);
 int tridiag_eigvecs(cudaStream_t st, EigArgs& g);

@@ -33,6 +33,13 @@ inline void bt_split_caps(int64_t n, int64_t iu, int64_t batch, int64_t& ksg, in
                             std::max<int64_t>(1, 6 * ((n + 31) / 32) / 8));
     ksg = std::max<int64_t>(1, ksg);
 }
+// The most that ksg x batch and ksw x batch reach for any batch up to the given one: a smaller batch takes more splits
+// (ceil(target / (t b)) b <= target / t + b), and a workspace sized once serves every batch below its own.
+inline void bt_split_room(int64_t n, int64_t iu, int64_t batch, int64_t& roomg, int64_t& roomw) {
+    const int64_t t = (iu + TC_BN - 1) / TC_BN;
+    roomg = std::min(std::min<int64_t>(32, (n + 255) / 256) * batch, BT_CTA_TARGET + batch);
+    roomw = std::min(std::min<int64_t>(16, std::max<int64_t>(1, 6 * ((n + 31) / 32) / 8)) * batch, BT_CTA_TARGET / t + batch);
+}
 constexpr int HK = 384;     // K'' of the split rank-2k update: 3 splits x (re, im) x 2 x TRD_NB
 
 __device__ inline float tf32_hi(float x) {
@@ -94,16 +101,24 @@ void carve(MixedWs& w, Carve& c) {
     w.A1 = c.take<float>(B * 2 * BT_NB * 6 * w.Kp);
     w.A2 = c.take<float>(B * 2 * n * 6 * BT_NB);
     w.B2 = c.take<float>(B * iu * 6 * BT_NB);
-    int64_t ksg, ksw;
-    bt_split_caps(n, iu, B, ksg, ksw);
-    w.Wb = c.take<float2>(ksw * B * BT_NB * iu);
+    int64_t roomg, roomw;
+    bt_split_room(n, iu, B, roomg, roomw);
+    w.Wb = c.take<float2>(roomw * BT_NB * iu);
     w.W2 = c.take<float2>(B * BT_NB * iu);
     const int64_t nbt = std::max<int64_t>(1, (n - 1 + BT_NB - 1) / BT_NB);   // blocks of the back-transformation
-    w.G = c.take<float2>(nbt * ksg * B * BT_NB * BT_NB);
+    w.G = c.take<float2>(nbt * roomg * BT_NB * BT_NB);
     w.T = c.take<float2>(nbt * B * BT_NB * BT_NB);
     w.err = c.take<int>(1);
 }
 }  // namespace
+
+void eig_mixed_splits(int64_t n, int64_t iu, int64_t batch, int64_t* out) {
+    int64_t ksg, ksw;
+    bt_split_caps(n, iu, batch, ksg, ksw);
+    out[0] = ksg * batch;
+    out[2] = ksw * batch;
+    bt_split_room(n, iu, batch, out[1], out[3]);
+}
 
 // the TF32 hi / lo eigenvector planes of the last eig_mixed call on this workspace (four planes of
 // n4 x iu floats per matrix: hi.re, hi.im, lo.re, lo.im, column-major)
@@ -593,13 +608,17 @@ int backtransform_tc(cudaStream_t st, MixedWs& ws, int64_t batch) {
 }
 
 // ---------------------------------------------------------------- driver
-int eig_mixed(cudaStream_t st, EigArgs& g, void* mixed_ws) {
+int eig_mixed(cudaStream_t st, EigArgs& g, void* mixed_ws, size_t ws_bytes) {
     MixedWs ws{};
     ws.n = g.n;
     ws.iu = g.iu;
     ws.B = g.batch;
     Carve c{static_cast<char*>(mixed_ws)};
     carve(ws, c);
+    if (c.off > ws_bytes) {
+        set_error(FORGE_ERR_ARG, "mixed eigen-solver: %zu bytes of workspace for a batch that needs %zu", ws_bytes, c.off);
+        return FORGE_ERR_ARG;
+    }
     const int64_t n = g.n, iu = g.iu, batch = g.batch;
     FORGE_CUDA(cudaMemsetAsync(ws.err, 0, sizeof(int), st));
     k_h_to_f32<<<1216, 256, 0, st>>>(g.A, ws.A32, (size_t)batch * n * n);

@@ -88,8 +88,8 @@ extern "C" int forge_gpu_zheevr_noalloc(double* A, int64_t n, int64_t iu, double
     g.strideX = n * iu;
     g.w = w;
     g.ortol_rel = 1e-7;
-    eig_bind_workspace(g, g_noalloc_ptr[dev]);
-    int rc = eig_fp64(st, g);
+    int rc = eig_bind_workspace(g, g_noalloc_ptr[dev], kNoAllocBytes);
+    if (!rc) rc = eig_fp64(st, g);
     int fail = 0;
     if (rc == 0) {
         cudaError_t e = cudaMemcpyAsync(&fail, g.fail, sizeof(int), cudaMemcpyDeviceToHost, st);

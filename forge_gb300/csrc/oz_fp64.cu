@@ -217,14 +217,17 @@ void oz_sizes(int64_t n, int64_t iu, int64_t batch, OzSizes& z) {
     z.mb = n > 512 ? std::max<int64_t>(1, (z.nblk + 1) / 2) : n > 384 ? 1 : z.nblk;
     z.ldx = up(n, 8);
     // K splits of V^H X: enough CTAs for the GPU, no split shorter than 256 rows
-    const int64_t tiles = std::max<int64_t>(1, (iu + OZ_T - 1) / OZ_T * 2 * batch);
-    z.ks = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(n > 512 ? 8 : 1, (152 + tiles - 1) / tiles), n / 256));
+    const int64_t t = (iu + OZ_T - 1) / OZ_T * 2, tiles = t * batch;
+    const int64_t most = std::max<int64_t>(1, std::min<int64_t>(n > 512 ? 8 : 1, n / 256));
+    z.ks = std::min(most, (152 + tiles - 1) / tiles);
     const int64_t P = 2 * S7;
     z.xs = batch * P * iu * z.ldx;
     z.vr = batch * P * n * z.NB;
     z.uz = batch * 2 * P * n * 64;   // U and Z of the rank-2k update
     z.vh = z.mb * batch * P * z.NB * z.ldx;
-    z.wp = z.ks * batch * iu * z.NB;
+    // the most that ks x batch reaches for any batch up to this one (a smaller batch takes more splits): the workspace
+    // serves every batch below the one it was sized for
+    z.wp = std::min(most * batch, 152 / t + batch) * iu * z.NB;
     z.ws = batch * P * iu * z.NB;
     z.g = z.mb * batch * z.NB * z.NB;
     z.ts = z.mb * batch * P * z.NB * z.NB;

@@ -1156,9 +1156,34 @@ size_t eig_workspace_bytes(int64_t n, int64_t iu, int64_t batch) {
     return c.off;
 }
 
-void eig_bind_workspace(EigArgs& g, void* base) {
+int eig_bind_workspace(EigArgs& g, void* base, size_t bytes) {
     Carve c{static_cast<char*>(base)};
     carve(g, c);
+    if (c.off > bytes) {
+        set_error(FORGE_ERR_ARG, "eigen-solver: %zu bytes of workspace for a batch that needs %zu", bytes, c.off);
+        return FORGE_ERR_ARG;
+    }
+    return 0;
 }
 
 }  // namespace forge
+
+extern "C" int forge_selftest_eig_workspace(int64_t n, int64_t iu, int64_t batch, int mixed, int64_t* out) {
+    using namespace forge;
+    if (n < 2 || iu < 1 || iu > n || batch < 1 || !out) {
+        set_error(FORGE_ERR_ARG, "selftest_eig_workspace: bad arguments");
+        return FORGE_ERR_ARG;
+    }
+    if (mixed) {
+        eig_mixed_splits(n, iu, batch, out + 1);
+        out[0] = (int64_t)eig_mixed_workspace_bytes(n, iu, batch);
+        return 0;
+    }
+    OzSizes z;
+    oz_sizes(n, iu, batch, z);
+    out[0] = (int64_t)eig_workspace_bytes(n, iu, batch);
+    out[1] = z.ks * batch;
+    out[2] = z.wp / (iu * z.NB);
+    out[3] = out[4] = 0;
+    return 0;
+}
