@@ -193,13 +193,15 @@ __global__ void __launch_bounds__(256) k_fix64(TrdArgs<double> a, int ii, int64_
 
 // ---------------------------------------------------------------- block floating point
 __device__ inline int field_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
-// x = (hi 2^28 + lo) 2^(fs - 1022 - 55) up to a unit, |hi| <= 2^27, |lo| <= 2^27, for field_of(x) <= fs and
-// 64 <= fs (zeros and values below 2^-1022 then shift out)
+// x = (hi 2^28 + lo) 2^(fs - 1022 - 55) up to half a unit, |hi| <= 2^27, |lo| <= 2^27, for field_of(x) <= fs and
+// 64 <= fs (zeros and values below 2^-1022 then shift out).  Nearest, ties to even: cut off towards zero, the errors of a
+// row of elements of one sign add up (the lowest band of a lattice, n = 364: 1.4e-14 instead of 2e-15).
 __device__ __forceinline__ void limbs(double x, int fs, int& hi, int& lo) {
     const int h = __double2hiint(x), s = h >> 31;
     const unsigned long long m =
         (((unsigned long long)((h & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(x)) << 2;
-    const unsigned long long v = m >> min(fs - ((h >> 20) & 0x7ff), 63);
+    const int sh = min(fs - ((h >> 20) & 0x7ff), 63);
+    const unsigned long long v = (m + (((1ULL << sh) - 1) >> 1) + ((m >> sh) & 1)) >> sh;
     const int l = (int)((unsigned)v & 0xfffffff), c = l >> 27;   // balanced low limb
     hi = (((int)(v >> 28) + c) ^ s) - s;
     lo = ((l - (c << 28)) ^ s) - s;
