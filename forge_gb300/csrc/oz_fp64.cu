@@ -78,25 +78,23 @@ struct LdT {  // rows l of T (upper triangular, column-major NB x NB)
     }
 };
 
-// Exponent of the largest |W| of a panel's trailing rows (biased), by atomicMax.  V and W share the scale of a row in
-// the rank-2k update, and |V| <= 1 while |W| is of the matrix' norm: V takes 2^k ~ max |W| along, so that neither
-// loses digits to the other whatever unit the matrix is in.
-__global__ void __launch_bounds__(256) k_oz_panel_max(const double2* __restrict__ W, int64_t n, int64_t r0, int64_t w,
+// Exponents of the largest |W| of a panel's columns (rows below the reduced one; biased), by atomicMax.  V and W share the scale
+// of a row in the rank-2k update, and |v_l| <= 1 while |w_l| is of the size of what column l reduced: v_l takes
+// 2^s ~ sqrt(max |w_l|) along and w_l 2^-s, so that neither loses digits to the other, nor a column to an earlier one,
+// whatever unit the matrix is in and however it is graded.
+__global__ void __launch_bounds__(256) k_oz_panel_max(const double2* __restrict__ W, int64_t n, int64_t p, int64_t w,
                                                       int* __restrict__ wmax) {
-    const int64_t b = blockIdx.y, r = r0 + (int64_t)blockIdx.x * 64 + (threadIdx.x & 63);
-    int f = 0;
-    if (r < n)
-        for (int64_t l = threadIdx.x >> 6; l < w; l += 4) {
-            const double2 x = W[b * n * TRD_NB + r + l * n];
-            f = max(f, max(oz_field(x.x), oz_field(x.y)));
-        }
-    f = __reduce_max_sync(0xffffffffu, f);
-    if ((threadIdx.x & 31) == 0 && f > 0) atomicMax(wmax + b, f);
+    const int64_t b = blockIdx.y, r = p + 1 + (int64_t)blockIdx.x * 64 + (threadIdx.x & 63);
+    for (int64_t l = threadIdx.x >> 6; l < w; l += 4) {
+        const double2 x = r < n && r > p + l ? W[b * n * TRD_NB + r + l * n] : make_double2(0.0, 0.0);
+        const int f = __reduce_max_sync(0xffffffffu, max(oz_field(x.x), oz_field(x.y)));
+        if ((threadIdx.x & 31) == 0 && f > 0) atomicMax(wmax + b * TRD_NB + l, f);
+    }
 }
-// k of the panel: 0 where W vanishes or holds a non-finite value
-__device__ inline int panel_expo(int f) { return f == 0 || f == 2047 ? 0 : f - 1023; }
+// s of a column: 0 where w vanishes or holds a non-finite value
+__device__ inline int panel_expo(int f) { return f == 0 || f == 2047 ? 0 : (f - 1023) >> 1; }
 
-struct LdPanel {  // rows i of [2^k V W] (swap = 0) or [W 2^k V] (swap = 1) of a panel of w columns, 32 slots each
+struct LdPanel {  // rows i of [2^s V  2^-s W] (swap = 0) or [2^-s W  2^s V] (swap = 1), a panel of w columns, 32 slots each
     const double2 *A, *W;
     const int* wmax;
     int64_t lda, strideA, n, r0, p, w;
@@ -105,9 +103,10 @@ struct LdPanel {  // rows i of [2^k V W] (swap = 0) or [W 2^k V] (swap = 1) of a
     __device__ double2 operator()(int64_t b, int64_t i, int64_t k) const {
         const int64_t l = k & (TRD_NB - 1);
         if (l >= w) return make_double2(0.0, 0.0);
-        if ((k >> 5) ^ swap) return W[b * n * TRD_NB + r0 + i + l * n];
-        const double2 v = A[b * strideA + r0 + i + (p + l) * lda];
-        const double s = oz_pow2(panel_expo(wmax[b]));
+        const bool ofw = (k >> 5) ^ swap;
+        const double2 v = ofw ? W[b * n * TRD_NB + r0 + i + l * n] : A[b * strideA + r0 + i + (p + l) * lda];
+        const int e = panel_expo(wmax[b * TRD_NB + l]);
+        const double s = oz_pow2(ofw ? -e : e);
         return make_double2(v.x * s, v.y * s);
     }
 };
@@ -152,12 +151,12 @@ struct EpiSubX {
 struct EpiHer2k {
     double2* A;
     int64_t lda, stride;
-    const int *eA, *eB, *wmax;
+    const int *eA, *eB;
     int64_t se;
     __device__ void operator()(int64_t b, int part, int64_t row, int64_t col0, const double* v, int64_t M,
                                int64_t N) const {
         if (row >= M || col0 > row) return;
-        const int ea = eA[b * se + row] - panel_expo(wmax[b]);
+        const int ea = eA[b * se + row];
         double* o = reinterpret_cast<double*>(A + b * stride + row + col0 * lda) + part;
         double x[16];
 #pragma unroll
@@ -231,7 +230,7 @@ void oz_sizes(int64_t n, int64_t iu, int64_t batch, OzSizes& z) {
     z.ws = batch * P * iu * z.NB;
     z.g = z.mb * batch * z.NB * z.NB;
     z.ts = z.mb * batch * P * z.NB * z.NB;
-    z.ex = batch * (2 * iu + 2 * n) + 2 * z.mb * batch * z.NB;
+    z.ex = batch * (2 * iu + 3 * n + TRD_NB) + 2 * z.mb * batch * z.NB;
 }
 
 // ---------------------------------------------------------------- rank-2k update
@@ -245,9 +244,9 @@ int her2k_oz(cudaStream_t st, TrdArgs<double>& a, int64_t p, int64_t w, int64_t 
     unsigned short* U = reinterpret_cast<unsigned short*>(g.oz_xs);
     unsigned short* Zs = U + batch * P * plane;
     int *eU = g.oz_ex, *eZ = eU + batch * n;
-    int* wmax = eZ + batch * n + p / TRD_NB * batch;   // one a panel, in the scales that the back-transformation uses later
-    if (p == 0) FORGE_CUDA(cudaMemsetAsync(wmax, 0, sizeof(int) * batch * cdiv(n, TRD_NB), st));
-    k_oz_panel_max<<<dim3(cdiv(m, 64), (unsigned)batch), 256, 0, st>>>(a.W, n, r0, w, wmax);
+    int* wmax = eZ + batch * n + p * batch;   // one a column, in the scales that the back-transformation uses later
+    if (p == 0) FORGE_CUDA(cudaMemsetAsync(wmax, 0, sizeof(int) * batch * up(n, TRD_NB), st));
+    k_oz_panel_max<<<dim3(cdiv(n - p - 1, 64), (unsigned)batch), 256, 0, st>>>(a.W, n, p, w, wmax);
     FORGE_LAUNCH_CHECK();
     const dim3 gs(cdiv(m, 32), (unsigned)batch), bs(32, 8);
     k_oz_rows<S7><<<gs, bs, 0, st>>>(LdPanel{a.A, a.W, wmax, a.lda, a.strideA, n, r0, p, w, 0}, m, 64, 64, U, 64, plane, eU, n, nullptr);
@@ -257,7 +256,7 @@ int her2k_oz(cudaStream_t st, TrdArgs<double>& a, int64_t p, int64_t w, int64_t 
     const OzOperand A{(const __nv_bfloat16*)U, m, 64, 64, plane, batch * P, (int32_t)P};
     const OzOperand B{(const __nv_bfloat16*)Zs, m, 64, 64, plane, batch * P, (int32_t)P};
     return oz_gemm(st, A, 0, B, 0, 64, oz_plans_complex(S7, OZ_DEPTH, 64, false, true), batch, true,
-                   EpiHer2k{a.A + r0 + r0 * a.lda, a.lda, a.strideA, eU, eZ, wmax, n}, g.oz_err);
+                   EpiHer2k{a.A + r0 + r0 * a.lda, a.lda, a.strideA, eU, eZ, n}, g.oz_err);
 }
 
 // ---------------------------------------------------------------- back-transformation

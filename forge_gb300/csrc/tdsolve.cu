@@ -1132,7 +1132,7 @@ void carve(EigArgs& g, Carve& c) {
     g.limb_tiles = nblk * (nblk + 1) / 2;
     g.oz_vh = c.take<char>(std::max<size_t>(2 * z.vh, sizeof(int4) * B * g.limb_tiles * TRD_TILE * TRD_TILE));
     g.limbs = (int4*)g.oz_vh;
-    g.limb_f = c.take<int>(B * g.limb_tiles);
+    g.limb_f = c.take<int>(B * g.limb_tiles * 2 * TRD_TILE);
     g.oz_ws = c.take<char>(2 * z.ws);
     g.oz_ts = c.take<char>(2 * z.ts);
     g.oz_wp = c.take<double2>(z.wp);

@@ -46,7 +46,8 @@ struct TrdArgs {
     double* scal;       // batch x 16
     unsigned* cnt;      // batch x 4
     V* w0 = nullptr;    // batch x n: the last column's w before the alpha2 correction
-    // FP64: the trailing triangle as integer limbs, batch x limb_tiles tiles of 64 x 64, and the tiles' exponents
+    // FP64: the trailing triangle as integer limbs, batch x limb_tiles tiles of 64 x 64, and the exponents of
+    // their rows and columns, 128 a tile
     int4* limbs = nullptr;
     int* limb_f = nullptr;
     int64_t limb_tiles = 0;

@@ -10,12 +10,15 @@
 //
 // k_hemv64 has eight FP64 FMAs per element to do, four clocks an element on an SM with two FP64 lanes a clock,
 // where HBM delivers an element in 0.7 clocks and the integer pipe does 64 32 x 32 + 64 bit
-// multiply-adds a clock.  So the product runs in integers: the tile and the two segments of x
-// are block floating point (one power of two for each tile and each segment, 55 bits below it), every
+// multiply-adds a clock.  So the product runs in integers: a tile is scaled by a power of two for each of its rows and
+// columns, so that the largest element of every row and column is about one, a segment of x takes the
+// tile's scales along, and both are block floating point (55 bits below the maximum).  Every
 // value is two 28-bit limbs and a product three multiply-adds, summed exactly in int64; only the
-// 128 results of a tile are converted to FP64.  An element keeps 2^-55 of its tile's maximum (FP64
+// 128 results of a tile are converted to FP64.  A scaled element keeps 2^-55 of one (FP64
 // keeps 2^-53 of its own value); the dropped low x low limb products are below 2^-56 of the two maxima
-// each, of random sign.  |hi|, |lo| <= 2^27 and at most 256 products a sum stay below 2^62.  The trailing matrix does
+// each, of random sign.  The scales make the error of a row follow the row's size, as FP64's does: a graded matrix
+// D B D keeps the relative accuracy of its small eigenvalues (with one scale a tile, 1e-10 instead of 1e-13 at a
+// ratio of 1e-8, and nothing left at 1e-20).  |hi|, |lo| <= 2^27 and at most 256 products a sum stay below 2^62.  The trailing matrix does
 // not change inside a panel (V and W carry its update), so k_limbs64 cuts it once for 32 columns, into as
 // many bytes as it had, in the order in which k_hemv64's threads read it.  Bound: integer multiply-adds (24 an element).
 // Measured (stage; cut anew in every column before): N = 1324, 16 k 57.6 -> 41 ms, N = 3268, one k 64 -> 53 ms.  What
@@ -193,14 +196,14 @@ __global__ void __launch_bounds__(256) k_fix64(TrdArgs<double> a, int ii, int64_
 
 // ---------------------------------------------------------------- block floating point
 __device__ inline int field_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
-// x = (hi 2^28 + lo) 2^(fs - 1022 - 55) up to half a unit, |hi| <= 2^27, |lo| <= 2^27, for field_of(x) <= fs and
-// 64 <= fs (zeros and values below 2^-1022 then shift out).  Nearest, ties to even: cut off towards zero, the errors of a
+// x = (hi 2^28 + lo) 2^(f - 1022 - 55) up to half a unit, |hi| <= 2^27, |lo| <= 2^27, for sh = f - field_of(x) >= 0;
+// values below 2^-1022 are zero.  Nearest, ties to even: cut off towards zero, the errors of a
 // row of elements of one sign add up (the lowest band of a lattice, n = 364: 1.4e-14 instead of 2e-15).
-__device__ __forceinline__ void limbs(double x, int fs, int& hi, int& lo) {
+__device__ __forceinline__ void limbs(double x, int sh, int& hi, int& lo) {
     const int h = __double2hiint(x), s = h >> 31;
     const unsigned long long m =
         (((unsigned long long)((h & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(x)) << 2;
-    const int sh = min(fs - ((h >> 20) & 0x7ff), 63);
+    sh = (h >> 20) & 0x7ff ? (int)min((unsigned)sh, 63u) : 63;
     const unsigned long long v = (m + (((1ULL << sh) - 1) >> 1) + ((m >> sh) & 1)) >> sh;
     const int l = (int)((unsigned)v & 0xfffffff), c = l >> 27;   // balanced low limb
     hi = (((int)(v >> 28) + c) ^ s) - s;
@@ -209,15 +212,24 @@ __device__ __forceinline__ void limbs(double x, int fs, int& hi, int& lo) {
 __device__ __forceinline__ void mad(long long& acc, int x, int y) { acc += (long long)x * y; }
 __device__ __forceinline__ long long shfl_xor64(long long v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
 
+// Exponents (as biased fields) of a tile's row or column without a nonzero element, and of operands that are not finite
+constexpr int NO_EXPO = -8192, NAN_EXPO = 1 << 20;
+// exponent of x 2^e
+__device__ inline int scaled_field(double x, int e) {
+    const int f = field_of(x);
+    return f == 2047 ? NAN_EXPO : f ? f + e : 2 * NO_EXPO;
+}
 // scale 2^(fa + fv - 2 * 1022 - 82) of H 2^28 + M, a sum of limb products; NaN if an operand was not finite
 __device__ inline double limb_scale(int fa, int fv) {
-    if (fa == 2047 || fv == 2047) return __longlong_as_double(0x7ff8000000000000LL);
+    if (max(fa, fv) >= NAN_EXPO / 2) return __longlong_as_double(0x7ff8000000000000LL);
     const int k = fa + fv - 2044 - 82;
     return k > -1022 && k < 1023 ? __hiloint2double((1023 + k) << 20, 0) : ldexp(1.0, k);
 }
 
 // The strict lower triangle of A(p:n, p:n) in limbs, 64 x 64 tiles (bi, bj), bj <= bi, t = bi (bi + 1) / 2 + bj: element
-// (tr + 16 i, 8 tc + j) at (4 j + i) 128 + 16 tc + tr; the tile's exponent to limb_f.
+// (tr + 16 i, 8 tc + j) at (4 j + i) 128 + 16 tc + tr.  To limb_f, 128 a tile: r_i, the exponent of row i's largest
+// element, and c_j <= 0, that of column j's largest once the rows are scaled; element (i, j) is in units of
+// 2^(r_i + c_j - 1022 - 55).
 __device__ inline int64_t tile_row(int64_t t) {
     int64_t bi = (int64_t)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);   // corrected below
     while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
@@ -228,10 +240,9 @@ __global__ void __launch_bounds__(256) k_limbs64(TrdArgs<double> a, int64_t p) {
     const int64_t b = blockIdx.y, n = a.n, lda = a.lda, t = blockIdx.x, bi = tile_row(t), bj = t - bi * (bi + 1) / 2;
     const double2* __restrict__ A = a.A + b * a.strideA;
     const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
-    __shared__ int red[8];
+    __shared__ int red[8][HT], rexp[HT];
     // thread: rows tr + 16 i, columns tc + 16 q
     double2 e[4][4];
-    int f = 0;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -239,16 +250,45 @@ __global__ void __launch_bounds__(256) k_limbs64(TrdArgs<double> a, int64_t p) {
             const int64_t r = p + bi * HT + tr + 16 * i, c = p + bj * HT + tc + 16 * q;
             e[i][q] = (r < n && c < r) ? A[r + c * lda] : make_double2(0.0, 0.0);
         }
+    int fe[4][4], r[4], cm[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int i = 0; i < 4; ++i) {
+        int f = 2 * NO_EXPO;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) f = max(f, max(field_of(e[i][q].x), field_of(e[i][q].y)));
-    f = __reduce_max_sync(0xffffffffu, f);
-    if ((tid & 31) == 0) red[tid >> 5] = f;
+        for (int q = 0; q < 4; ++q) {
+            fe[i][q] = max(scaled_field(e[i][q].x, 0), scaled_field(e[i][q].y, 0));
+            f = max(f, fe[i][q]);
+        }
+        f = max(f, __shfl_xor_sync(0xffffffffu, f, 16));
+        if ((tid & 16) == 0) red[tid >> 5][tr + 16 * i] = f;
+    }
     __syncthreads();
-    int fa = 64;
+    if (tid < HT) {
+        int f = NO_EXPO;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) fa = max(fa, red[q]);
+        for (int q = 0; q < 8; ++q) f = max(f, red[q][tid]);
+        rexp[tid] = f;
+    }
+    // an element that is not finite spoils the tile's rows and columns
+    const bool bad = __syncthreads_or(tid < HT && rexp[tid] >= NAN_EXPO);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = rexp[tr + 16 * i];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        int f = NO_EXPO;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (fe[i][q] > NO_EXPO) f = max(f, fe[i][q] - r[i]);
+#pragma unroll
+        for (int k = 8; k > 0; k >>= 1) f = max(f, __shfl_xor_sync(0xffffffffu, f, k));
+        cm[q] = f;
+    }
+    int* ex = a.limb_f + (b * a.limb_tiles + t) * (2 * HT);
+    if (tid < HT) ex[tid] = bad ? NAN_EXPO : rexp[tid];
+    if (tr == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ex[HT + tc + 16 * q] = bad ? NAN_EXPO : cm[q];
+    }
     int4* o = a.limbs + (b * a.limb_tiles + t) * (HT * HT);
 #pragma unroll
     for (int q = 0; q < 4; ++q)
@@ -256,11 +296,10 @@ __global__ void __launch_bounds__(256) k_limbs64(TrdArgs<double> a, int64_t p) {
         for (int i = 0; i < 4; ++i) {
             const int c = tc + 16 * q;
             int4 x;
-            limbs(e[i][q].x, fa, x.x, x.y);
-            limbs(e[i][q].y, fa, x.z, x.w);
+            limbs(e[i][q].x, r[i] + cm[q] - field_of(e[i][q].x), x.x, x.y);
+            limbs(e[i][q].y, r[i] + cm[q] - field_of(e[i][q].y), x.z, x.w);
             o[(4 * (c & 7) + i) * 128 + 16 * (c >> 3) + tr] = x;
         }
-    if (tid == 0) a.limb_f[b * a.limb_tiles + t] = fa;
 }
 
 constexpr int HV_T = 128;   // threads of k_hemv64
@@ -293,29 +332,35 @@ __global__ void __launch_bounds__(HV_T, 4) k_hemv64(TrdArgs<double> a, int64_t p
         };
 #pragma unroll
         for (int q = 0; q < 4; ++q) fetch(q);
+        // r_i of the tile's rows (threads 0 .. 63) and c_j of its columns
+        const int ex = __ldcg(a.limb_f + (b * a.limb_tiles + t) * (2 * HT) + tid);
         // tile (bi, bj), bj <= bi, from row and column p on; x vanishes up to c0
         const int64_t bi = tile_row(t), bj = t - bi * (bi + 1) / 2;
         trd_chain_wait();
         const int64_t R0 = p + bi * HT, C0 = p + bj * HT;
         __shared__ int4 vr[HT], vc[HT];              // limbs (re hi, re lo, im hi, im lo) of x
-        __shared__ int redV[4];
+        __shared__ int redV[4], exps[2 * HT];
         __shared__ long long rs[4][4][HT], cs[4][HT];   // sums: H re, H im, M re, M im
         const int tr = tid & 15, tc = tid >> 4;
-        const int fa = a.limb_f[b * a.limb_tiles + t];
         double2 xv = make_double2(0.0, 0.0);
         {
             const int64_t r = tid < HT ? R0 + tid : C0 + tid - HT;
             if (r < n && r > c0) xv = A[r + col * lda];
-            const int g = __reduce_max_sync(0xffffffffu, max(field_of(xv.x), field_of(xv.y)));
+        }
+        // x with the scales of the rows (for the sums over them) and of the columns
+        const int xs = tid < HT ? ex - 1022 : ex;
+        {
+            const int g = __reduce_max_sync(0xffffffffu, max(scaled_field(xv.x, xs), scaled_field(xv.y, xs)));
             if (lane == 0) redV[warp] = g;
+            exps[tid] = ex;
         }
         __syncthreads();
-        const int fr = max(max(redV[0], redV[1]), 64), fc = max(max(redV[2], redV[3]), 64);
+        const int fr = max(redV[0], redV[1]), fc = max(redV[2], redV[3]);
         {
             int4 l;
-            const int fx = tid < HT ? fr : fc;
-            limbs(xv.x, fx, l.x, l.y);
-            limbs(xv.y, fx, l.z, l.w);
+            const int fx = (tid < HT ? fr : fc) - xs;
+            limbs(xv.x, fx - field_of(xv.x), l.x, l.y);
+            limbs(xv.y, fx - field_of(xv.y), l.z, l.w);
             (tid < HT ? vr[tid] : vc[tid - HT]) = l;
         }
         __syncthreads();
@@ -389,10 +434,10 @@ __global__ void __launch_bounds__(HV_T, 4) k_hemv64(TrdArgs<double> a, int64_t p
         const long long M = (rs[0][2 + im][v] + rs[1][2 + im][v]) + (rs[2][2 + im][v] + rs[3][2 + im][v]);
         if (R0 + v < n)
             reinterpret_cast<double*>(a.Yrow + b * a.ystride + bj * n + R0 + v)[im] =
-                fma((double)H, 268435456.0, (double)M) * limb_scale(fa, fc);
+                fma((double)H, 268435456.0, (double)M) * limb_scale(exps[v], fc);
         if (C0 + v < n)
             reinterpret_cast<double*>(a.Ycol + b * a.ystride + bi * n + C0 + v)[im] =
-                fma((double)cs[im][v], 268435456.0, (double)cs[2 + im][v]) * limb_scale(fa, fr);
+                fma((double)cs[im][v], 268435456.0, (double)cs[2 + im][v]) * limb_scale(exps[HT + v] + 1022, fr);
     } else if (blockIdx.x > 0) {
         // panel dots: warp <-> reflector, lanes over the rows
         const int ng = (ii + DOT_L - 1) / DOT_L;

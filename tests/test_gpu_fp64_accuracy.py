@@ -39,3 +39,58 @@ def test_lattice_eigenvalues(ntheta):
         h = _hermitian(H[:, :, b])
         e, X = np.linalg.eigh(h)
         assert np.max(np.abs(w[pick, b] - _quotients(h, X[:, pick]))) <= 3 * EPS * np.max(np.abs(e))
+
+
+def _graded(n, ratio, rng):
+    """A = D B D with a well conditioned B and the entries of D falling from 1 to sqrt(ratio)."""
+    G = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    B = np.eye(n) + 0.1 * (G + G.conj().T) / np.sqrt(n)
+    d = np.exp2(np.round(np.log2(np.logspace(0, np.log10(ratio) / 2, n))))
+    return d[:, None] * B * d[None, :], np.linalg.cond(B)
+
+
+def _positive_eigenvalues(A):
+    """Of a positive definite matrix, each to a few eps cond(B) of itself: one-sided Jacobi on the Cholesky factor
+    (J. Demmel and K. Veselic, Jacobi's method is more accurate than QR, SIAM J. Matrix Anal. Appl. 13, 1992)."""
+    L = np.linalg.cholesky(A)
+    n = L.shape[0]
+    for _ in range(30):
+        worst = 0.0
+        for p in range(n - 1):
+            for q in range(p + 1, n):
+                a, b, g = np.vdot(L[:, p], L[:, p]).real, np.vdot(L[:, q], L[:, q]).real, np.vdot(L[:, p], L[:, q])
+                off = abs(g) / np.sqrt(a * b)
+                if off <= EPS:
+                    continue
+                worst = max(worst, off)
+                z = (b - a) / (2 * abs(g))
+                t = (1.0 if z >= 0 else -1.0) / (abs(z) + np.hypot(1.0, z))
+                c = 1 / np.hypot(1.0, t)
+                x, y = L[:, p].copy(), L[:, q] * (g.conjugate() / abs(g))
+                L[:, p], L[:, q] = c * x - c * t * y, c * t * x + c * y
+        if worst <= 8 * EPS:
+            break
+    return np.sort(np.sum(np.abs(L) ** 2, 0))
+
+
+@pytest.mark.parametrize("n,ratio", [(7, 1e-8), (40, 1e-8), (40, 1e-20), (66, 1e-16), (100, 1e-12)])
+@pytest.mark.parametrize("unit", [1.0, 1e-60])
+def test_graded_matrix(n, ratio, unit):
+    """Small eigenvalues of a graded matrix keep their relative accuracy, n^2 eps cond(B) with a factor of four
+    (J. Barlow and J. Demmel, Computing accurate eigensystems of scaled diagonally dominant matrices, 1990)."""
+    import ctypes as C
+
+    import torch
+
+    import forge_gb300 as fg
+    A, cond = _graded(n, ratio, np.random.default_rng(n))
+    f = fg.load_library().forge_gpu_zheevr_noalloc
+    f.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]
+    f.restype = C.c_int
+    dA = torch.from_numpy(np.ascontiguousarray(A.T * unit)).cuda()
+    w = torch.empty(n, dtype=torch.float64, device="cuda")
+    Z = torch.empty(n, n, dtype=torch.complex128, device="cuda")
+    torch.cuda.synchronize()
+    assert f(dA.data_ptr(), n, n, w.data_ptr(), Z.data_ptr(), None) == 0
+    ref = _positive_eigenvalues(A)
+    assert np.max(np.abs(w.cpu().numpy() / unit / ref - 1)) <= 4 * n * n * EPS * cond
