@@ -408,6 +408,39 @@ __global__ void __launch_bounds__(32) k_bisect_f32(const float2* __restrict__ tf
     if (live && g == 0) w[b * iu + j] = 0.5 * ((double)lo + (double)hi);
 }
 
+// Eigenvalue j of the scaled T if it is below TINY: bisection with the quotients (dlaebz), whose smallest pivot is
+// kSafmin for |T| <= 1.  A minor's replacement by 2^-160 of its predecessor is a change of d_i by that much, so the
+// multisection's counts place an eigenvalue to 2^-159: nothing to one above 2^-106, everything to one below.
+constexpr double TINY = 7.888609052210118e-31;   // 2^-100
+__device__ __noinline__ double bisect_tiny(const double2* __restrict__ t, int n, int64_t j, double glo, double ghi) {
+    auto count = [&](double x) {
+        double q = t[0].x - x;
+        if (fabs(q) < kSafmin) q = -kSafmin;
+        int64_t cnt = q <= 0.0;
+        for (int i = 1; i < n; ++i) {
+            const double2 v = t[i];
+            q = v.x - v.y / q - x;
+            if (fabs(q) < kSafmin) q = -kSafmin;
+            cnt += q <= 0.0;
+        }
+        return cnt;
+    };
+    double lo = fmax(glo, -2.0 * TINY), hi = fmin(ghi, 2.0 * TINY);
+    if (!(lo < hi && count(lo) < j + 1 && count(hi) >= j + 1)) {
+        lo = glo;
+        hi = ghi;
+    }
+    for (int it = 0; it < 256; ++it) {
+        if (!(hi - lo > fmax(kSafmin, 4.0 * kEps * fmax(fabs(lo), fabs(hi))))) break;
+        const double mid = 0.5 * (lo + hi);
+        if (count(mid) >= j + 1)
+            hi = mid;
+        else
+            lo = mid;
+    }
+    return 0.5 * (lo + hi);
+}
+
 // Eigenvalue j in FP64 by multisection: G lanes evaluate the Sturm counts at G equally spaced points of
 // the bracket, which shrinks by G + 1 a round.  The bracket starts from the FP32 estimate in w: it is
 // widened by 16 until the FP64 counts confirm it, at last to the Gershgorin interval.  Stops at the
@@ -474,7 +507,12 @@ __global__ void __launch_bounds__(32) k_bisect(const double2* __restrict__ de, i
             if (!(hi - lo < width)) lo = hi = 0.5 * (lo + hi);
         }
     }
-    if (live && g == 0) w[b * iu + j] = 0.5 * (lo + hi) / s;
+    if (live && g == 0) {
+        double lam = 0.5 * (lo + hi);
+        // abstol is wider where k_bisect_replay follows, which has quotients of its own
+        if (abstol < TINY && fabs(lam) < TINY) lam = bisect_tiny(t, (int)n, j, glo, ghi);
+        w[b * iu + j] = lam / s;
+    }
     if (!live && g == 0 && j < iu) w[b * iu + j] = 0.0;
 }
 

@@ -94,3 +94,36 @@ def test_graded_matrix(n, ratio, unit):
     assert f(dA.data_ptr(), n, n, w.data_ptr(), Z.data_ptr(), None) == 0
     ref = _positive_eigenvalues(A)
     assert np.max(np.abs(w.cpu().numpy() / unit / ref - 1)) <= 4 * n * n * EPS * cond
+
+
+def _eigenvalues(A):
+    import ctypes as C
+
+    import torch
+
+    import forge_gb300 as fg
+    f = fg.load_library().forge_gpu_zheevr_noalloc
+    f.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]
+    f.restype = C.c_int
+    n = A.shape[0]
+    dA = torch.from_numpy(np.ascontiguousarray(A.T)).cuda()
+    w = torch.empty(n, dtype=torch.float64, device="cuda")
+    Z = torch.empty(n, n, dtype=torch.complex128, device="cuda")
+    torch.cuda.synchronize()
+    assert f(dA.data_ptr(), n, n, w.data_ptr(), Z.data_ptr(), None) == 0
+    return w.cpu().numpy()
+
+
+@pytest.mark.parametrize("ratio", [1e-40, 1e-50, 1e-60])
+def test_eigenvalues_far_below_the_norm(ratio):
+    """As test_graded_matrix, past the 2^-106 of the norm to which minors with replacements place an eigenvalue."""
+    n = 40
+    A, cond = _graded(n, ratio, np.random.default_rng(n))
+    assert np.max(np.abs(_eigenvalues(A) / _positive_eigenvalues(A) - 1)) <= 4 * n * n * EPS * cond
+
+
+def test_diagonal_over_many_orders():
+    """Eigenvalues that stand on the diagonal come back to the bisection's 2 EPS |lambda|."""
+    d = np.array([1e-33, 4.0, -3e-58, 1e-12, 0.0, -2e-31, 7e-31, 5e-45, -1.0, 6e-55])
+    w = _eigenvalues(np.diag(d).astype(complex))
+    assert np.all(np.abs(w - np.sort(d)) <= np.maximum(2 * EPS * np.abs(np.sort(d)), 1e-75))
