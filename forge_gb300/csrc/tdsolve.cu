@@ -17,6 +17,8 @@
 // eps*||T||/gap stays below 1e-8 outside clusters.
 #include <algorithm>
 #include <cfloat>
+#include <vector>
+
 #include "cvec.cuh"
 #include "eig.cuh"
 
@@ -96,19 +98,23 @@ __global__ void k_tri_scale(const double* __restrict__ d, const double* __restri
 // A minor below 2^-THR of its predecessor is replaced by -2^-THR of it (the quotient form's
 // |q| < pivmin -> -pivmin), and every fourth step both are rescaled by a power of two, so nothing
 // under- or overflows: |T - x I| <= 4 grows a minor by less than 2^8 in four steps, and four
-// replacements shrink it by 2^-4 THR.  Sign and exponent are handled as integers.
+// replacements, with one carried over the rescale, leave it at 2^-5 THR of the larger, which has to be a normal number
+// whose own predecessor is above 2^THR times the smallest (5 THR < BIAS).  In FP32 2^-25 is below the rounding of
+// d_i.  Sign and exponent are handled as integers.
 template <class T>
 struct Minor;
 template <>
 struct Minor<double> {
     static constexpr int THR = 160, MB = 20, BIAS = 1023;
+    static_assert(5 * THR < BIAS, "five replacements stay normal");
     __device__ static int hi(double x) { return __double2hiint(x); }
     __device__ static double add_hi(double x, int dh) { return __hiloint2double(__double2hiint(x) + dh, __double2loint(x)); }
     __device__ static double neg(double x) { return __hiloint2double(__double2hiint(x) ^ 0x80000000, __double2loint(x)); }
 };
 template <>
 struct Minor<float> {
-    static constexpr int THR = 28, MB = 23, BIAS = 127;
+    static constexpr int THR = 25, MB = 23, BIAS = 127;
+    static_assert(5 * THR < BIAS, "five replacements stay normal");
     __device__ static int hi(float x) { return __float_as_int(x); }
     __device__ static float add_hi(float x, int dh) { return __int_as_float(__float_as_int(x) + dh); }
     __device__ static float neg(float x) { return __int_as_float(__float_as_int(x) ^ 0x80000000); }
@@ -1205,6 +1211,52 @@ int eig_bind_workspace(EigArgs& g, void* base, size_t bytes) {
 }
 
 }  // namespace forge
+
+namespace forge {
+namespace {
+__global__ void k_selftest_sturm(const double2* de, const float2* tf, int n, int64_t nx, const double* x, int* c64, int* c32) {
+    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (q >= nx) return;
+    c64[q] = sturm<double>(de, n, x[q]);
+    c32[q] = sturm<float>(tf, n, (float)x[q]);
+}
+}  // namespace
+}  // namespace forge
+
+extern "C" int forge_gpu_selftest_sturm(int64_t n, const double* d, const double* e, int64_t nx, const double* x, int* c64,
+                                        int* c32) {
+    using namespace forge;
+    if (n < 1 || nx < 1 || !d || !x || !c64 || !c32 || (n > 1 && !e)) {
+        set_error(FORGE_ERR_ARG, "selftest_sturm: bad arguments");
+        return FORGE_ERR_ARG;
+    }
+    std::vector<double2> de(n);
+    std::vector<float2> tf(n);
+    for (int64_t i = 0; i < n; ++i) {
+        const double em = i > 0 ? e[i - 1] : 0.0;
+        de[i] = make_double2(d[i], em * em);
+        tf[i] = make_float2((float)d[i], (float)(em * em));
+    }
+    DevBuf a, b, p, c;
+    int rc = 0;
+    if (!(rc = a.ensure(n * sizeof(double2))) && !(rc = b.ensure(n * sizeof(float2))) && !(rc = p.ensure(nx * 8)) &&
+        !(rc = c.ensure(nx * 8))) {
+        int *g64 = c.as<int>(), *g32 = g64 + nx;
+        cudaMemcpy(a.ptr, de.data(), n * sizeof(double2), cudaMemcpyHostToDevice);
+        cudaMemcpy(b.ptr, tf.data(), n * sizeof(float2), cudaMemcpyHostToDevice);
+        cudaMemcpy(p.ptr, x, nx * 8, cudaMemcpyHostToDevice);
+        k_selftest_sturm<<<(unsigned)((nx + 63) / 64), 64>>>(a.as<double2>(), b.as<float2>(), (int)n, nx, p.as<double>(), g64, g32);
+        cudaMemcpy(c64, g64, nx * 4, cudaMemcpyDeviceToHost);
+        cudaMemcpy(c32, g32, nx * 4, cudaMemcpyDeviceToHost);
+        const cudaError_t err = cudaGetLastError();
+        if (err != cudaSuccess) {
+            set_error(FORGE_ERR_CUDA, "selftest_sturm: %s", cudaGetErrorString(err));
+            rc = FORGE_ERR_CUDA;
+        }
+    }
+    for (DevBuf* q : {&a, &b, &p, &c}) q->release();
+    return rc;
+}
 
 extern "C" int forge_selftest_eig_workspace(int64_t n, int64_t iu, int64_t batch, int mixed, int64_t* out) {
     using namespace forge;

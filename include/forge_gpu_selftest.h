@@ -31,6 +31,11 @@ int forge_gpu_selftest_tc_gemm_timeout(int64_t M, int64_t N, int64_t K, int64_t 
  * M^H S M = I.  Returns 1 if S is not positive definite. */
 int forge_selftest_rr_small(int64_t n, const double* G, const double* S, double* theta, double* M);
 
+/* Numbers of eigenvalues <= x[q] of the tridiagonal (d, e), |T| <= 1, by the minors' Sturm counts of
+ * the tridiagonal solver in FP64 and in FP32. */
+int forge_gpu_selftest_sturm(int64_t n, const double* d, const double* e, int64_t nx, const double* x, int* c64,
+                             int* c32);
+
 /* Host only: workspace of a batched eigen-solve.  out[0]: bytes; out[1], out[2]: K-split partial
  * products that a solve of this batch forms and the room for them; out[3], out[4]: the same of the
  * mixed solver's second split product (0 in FP64). */
