@@ -181,8 +181,8 @@ __device__ __forceinline__ double recip(double b) {
 }
 // a / b from r = recip(b) for operands in mid-range: the remainder of a r brings the quotient to 2^-80 before its
 // one rounding (P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
-// IBM J. Res. Dev. 34 (1990)), so it is the rounded quotient but for one case in 2^27 or fewer (none of 1.5e9
-// random ones).  Five FMAs with recip: an FP64 instruction of a warp holds its scheduler's FP64 pipe for 64 clocks on this GPU, whatever the
+// IBM J. Res. Dev. 34 (1990)), so it is the rounded quotient but for one case in 2^27 or fewer, a
+// unit in the last place then (forge_gpu_selftest_quot counts them).  Five FMAs with recip: an FP64 instruction of a warp holds its scheduler's FP64 pipe for 64 clocks on this GPU, whatever the
 // number of lanes, so the count of them is what the serial chains below cost.
 __device__ __forceinline__ double quot(double a, double b, double r) {
     const double q = a * r;
@@ -1220,6 +1220,26 @@ __global__ void k_selftest_sturm(const double2* de, const float2* tf, int n, int
     c64[q] = sturm<double>(de, n, x[q]);
     c32[q] = sturm<float>(tf, n, (float)x[q]);
 }
+// counts of quot(a, b) that differ from a / b, and of those that differ by more than a unit in the last place
+__global__ void k_selftest_quot(uint64_t seed, int64_t per_thread, unsigned long long* bad) {
+    uint64_t s = mix64(seed ^ ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) * 0x9e3779b97f4a7c15ULL));
+    unsigned long long off = 0, far = 0, seen = 0;
+    for (int64_t i = 0; i < per_thread; ++i) {
+        const uint64_t x = mix64(s += 0x9e3779b97f4a7c15ULL), y = mix64(s += 0x9e3779b97f4a7c15ULL);
+        // exponents over the range that mid_expo admits, and in half of the cases close to each other
+        const int ex = 524 + (int)(mix64(x ^ 1) % 1000), ey = i & 1 ? 524 + (int)(mix64(y ^ 1) % 1000) : ex;
+        const double a = __longlong_as_double((long long)((x & 0x800fffffffffffffULL) | (uint64_t)ex << 52));
+        const double b = __longlong_as_double((long long)((y & 0x800fffffffffffffULL) | (uint64_t)ey << 52));
+        if (!mid_expo(a) || !mid_expo(b)) continue;
+        ++seen;
+        const long long d = __double_as_longlong(quot(a, b, recip(b))) - __double_as_longlong(a / b);
+        off += d != 0;
+        far += d > 1 || d < -1;
+    }
+    atomicAdd(bad, seen);
+    atomicAdd(bad + 1, off);
+    atomicAdd(bad + 2, far);
+}
 }  // namespace
 }  // namespace forge
 
@@ -1256,6 +1276,26 @@ extern "C" int forge_gpu_selftest_sturm(int64_t n, const double* d, const double
     }
     for (DevBuf* q : {&a, &b, &p, &c}) q->release();
     return rc;
+}
+
+extern "C" int forge_gpu_selftest_quot(int64_t seed, int64_t count, int64_t* out) {
+    using namespace forge;
+    if (count < 1 || !out) {
+        set_error(FORGE_ERR_ARG, "selftest_quot: bad arguments");
+        return FORGE_ERR_ARG;
+    }
+    constexpr int64_t threads = 1216 * 128;
+    DevBuf c;
+    FORGE_TRY(c.ensure(3 * sizeof(int64_t)));
+    cudaMemset(c.ptr, 0, 3 * sizeof(int64_t));
+    k_selftest_quot<<<1216, 128>>>((uint64_t)seed, (count + threads - 1) / threads, c.as<unsigned long long>());
+    const cudaError_t err = cudaMemcpy(out, c.ptr, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost);
+    c.release();
+    if (err != cudaSuccess) {
+        set_error(FORGE_ERR_CUDA, "selftest_quot: %s", cudaGetErrorString(err));
+        return FORGE_ERR_CUDA;
+    }
+    return 0;
 }
 
 extern "C" int forge_selftest_eig_workspace(int64_t n, int64_t iu, int64_t batch, int mixed, int64_t* out) {

@@ -36,6 +36,11 @@ int forge_selftest_rr_small(int64_t n, const double* G, const double* S, double*
 int forge_gpu_selftest_sturm(int64_t n, const double* d, const double* e, int64_t nx, const double* x, int* c64,
                              int* c32);
 
+/* The tridiagonal solver's division by FMAs against the compiler's on at least `count` pairs of random
+ * operands over the exponents that it admits: out[0] pairs tried, out[1] different results, out[2]
+ * results off by more than a unit in the last place. */
+int forge_gpu_selftest_quot(int64_t seed, int64_t count, int64_t* out);
+
 /* Host only: workspace of a batched eigen-solve.  out[0]: bytes; out[1], out[2]: K-split partial
  * products that a solve of this batch forms and the room for them; out[3], out[4]: the same of the
  * mixed solver's second split product (0 in FP64). */

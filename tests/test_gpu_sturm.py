@@ -38,3 +38,14 @@ def test_counts_of_a_coupled_matrix(n):
     c = _counts(d, e, x)
     ref = np.sum(w[None, :] <= x[:, None], 1)
     assert np.array_equal(c[0], ref) and np.array_equal(c[1], ref)
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_division_by_fmas(seed):
+    """quot(a, b) against a / b: never off by more than a unit in the last place.  The remainder step leaves the
+    quotient within 2^-80 before its rounding, so it rounds the other way for at most one pair in 2^26."""
+    import forge_gb300 as fg
+    out = (C.c_int64 * 3)()
+    assert fg.load_library().forge_gpu_selftest_quot(C.c_int64(seed), C.c_int64(1 << 29), out) == 0
+    assert out[0] >= 1 << 29
+    assert out[2] == 0 and out[1] <= out[0] >> 26
