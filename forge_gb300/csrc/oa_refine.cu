@@ -324,10 +324,10 @@ OaLayout oa_layout(int64_t n, int64_t iu, int64_t nb, void* base) {
     return L;
 }
 
-// matrices refined together: what fits in 4 GB, at least one (one matrix of N = 364 has nine tiles)
+// matrices refined together: what fits in 4 GB and in a launch's grid, at least one (one matrix of N = 364 has nine tiles)
 int64_t oa_chunk(int64_t n, int64_t iu, int64_t batch) {
     const int64_t per = (int64_t)oa_layout(n, iu, 1, nullptr).bytes;
-    return std::max<int64_t>(1, std::min<int64_t>(batch, ((int64_t)4 << 30) / per));
+    return std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(batch, OZ_GRID_Z), ((int64_t)4 << 30) / per));
 }
 
 }  // namespace

@@ -19,6 +19,7 @@
 namespace forge {
 
 constexpr int S7 = OZ_S;
+constexpr int64_t GRID_Y = 65535;
 constexpr int OZ_REF_S = 4, OZ_REF_DEPTH = 3;   // projectors of refined eigenvectors
 
 int oz_make_tmap(CUtensorMap* map, const OzOperand& op) {
@@ -213,7 +214,10 @@ void oz_sizes(int64_t n, int64_t iu, int64_t batch, OzSizes& z) {
     z.nblk = (std::max<int64_t>(1, n - 1) + z.NB - 1) / z.NB;
     // blocks whose V^H and T are formed together: half of them (14 n^2 bytes); the allocation-free entry's
     // 16 MiB array (n <= 512) holds all blocks up to 384 and single ones above
-    z.mb = n > 512 ? std::max<int64_t>(1, (z.nblk + 1) / 2) : n > 384 ? 1 : z.nblk;
+    const int64_t mb = n > 512 ? std::max<int64_t>(1, (z.nblk + 1) / 2) : n > 384 ? 1 : z.nblk;
+    // blocks x matrices in a grid's y extent; room: the most that mb x batch reaches for any batch up to this one
+    z.mb = std::max<int64_t>(1, std::min<int64_t>(mb, GRID_Y / batch));
+    const int64_t room = std::min(mb * batch, std::max<int64_t>(batch, GRID_Y));
     z.ldx = up(n, 8);
     // K splits of V^H X: enough CTAs for the GPU, no split shorter than 256 rows
     const int64_t t = (iu + OZ_T - 1) / OZ_T * 2, tiles = t * batch;
@@ -223,14 +227,14 @@ void oz_sizes(int64_t n, int64_t iu, int64_t batch, OzSizes& z) {
     z.xs = batch * P * iu * z.ldx;
     z.vr = batch * P * n * z.NB;
     z.uz = batch * 2 * P * n * 64;   // U and Z of the rank-2k update
-    z.vh = z.mb * batch * P * z.NB * z.ldx;
+    z.vh = room * P * z.NB * z.ldx;
     // the most that ks x batch reaches for any batch up to this one (a smaller batch takes more splits): the workspace
     // serves every batch below the one it was sized for
     z.wp = std::min(most * batch, 152 / t + batch) * iu * z.NB;
     z.ws = batch * P * iu * z.NB;
-    z.g = z.mb * batch * z.NB * z.NB;
-    z.ts = z.mb * batch * P * z.NB * z.NB;
-    z.ex = batch * (2 * iu + 3 * n + TRD_NB) + 2 * z.mb * batch * z.NB;
+    z.g = room * z.NB * z.NB;
+    z.ts = room * P * z.NB * z.NB;
+    z.ex = batch * (2 * iu + 3 * n + TRD_NB) + 2 * room * z.NB;
 }
 
 // ---------------------------------------------------------------- rank-2k update
@@ -425,10 +429,10 @@ __global__ void __launch_bounds__(256) k_proj_add(double2* __restrict__ P, const
 }
 }  // namespace
 
-// items per launch: as many as fit in 2 GB of slices and products, at least one
+// items per launch: as many as fit in 2 GB of slices and products and in a launch's grid, at least one
 static int64_t proj_oz_chunk(int64_t n, int64_t iu, int64_t nit, int S) {
     const int64_t per = 2 * S * n * up(iu, 8) * 2 + 2 * n * n * 8;
-    return std::max<int64_t>(1, std::min<int64_t>(nit, ((int64_t)2 << 30) / per));
+    return std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nit, OZ_GRID_Z), ((int64_t)2 << 30) / per));
 }
 size_t proj_oz_workspace_bytes(int64_t n, int64_t iu, int64_t nit, bool refined) {
     const int S = refined ? OZ_REF_S : OZ_S;

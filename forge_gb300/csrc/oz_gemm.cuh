@@ -23,6 +23,8 @@
 // the previous one is added up; columns 256..511 hold the FP64 value of the first levels when all
 // levels together exceed 63 bits.
 #pragma once
+#include <algorithm>
+
 #include <cuda_bf16.h>
 
 #include "tc_gemm.cuh"
@@ -33,6 +35,7 @@ constexpr int OZ_T = 128, OZ_BK = 64, OZ_STAGES = 6, OZ_THREADS = 320;
 constexpr int OZ_TILE_BYTES = OZ_T * OZ_BK * 2;   // 16 KB per operand and stage
 constexpr int OZ_SMEM = OZ_STAGES * 2 * OZ_TILE_BYTES + 1024 + 256;
 constexpr int OZ_MAXSEG = 64, OZ_MAXLEV = 8;
+constexpr int OZ_GRID_Z = 32767;                  // products of a batch (times K splits) per launch
 constexpr int OZ_S = 7, OZ_DEPTH = 6;             // FP64-equivalent: 28 slice products
 constexpr int OZ_NAN = 1 << 24;                   // exponent of a row that holds a non-finite value
 
@@ -126,7 +129,7 @@ __device__ inline double oz_pow2(int k) {
     return k > OZ_NAN / 2 ? __longlong_as_double(0x7ff8000000000000LL) : ldexp(1.0, k);
 }
 
-// lower: skip tiles whose rows all lie above the diagonal.  blockIdx.z = 2 z + part, z = b * ksplit + s; split
+// lower: skip tiles whose rows all lie above the diagonal.  blockIdx.z = 2 (z - z0) + part, z = b * ksplit + s; split
 // s takes K blocks [s kchunk, min(nkb, (s + 1) kchunk)) of every segment.
 // EPI: epi(z, part, row, col0, v[16], M, N) with the 16 columns' values before the 2^(eA + eB) scale.
 // DF: the blocks of 256 are scaled by their level's power of two (exact) and added into double-float (hi, lo)
@@ -138,7 +141,7 @@ template <class EPI, bool DF>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     k_oz_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int64_t M, int64_t N,
               const __grid_constant__ OzPlans plans, int32_t nkb, int32_t koffA, int32_t koffB, int32_t zA, int32_t zB,
-              int lower, int32_t ksplit, int32_t kchunk, EPI epi, int* err) {
+              int lower, int32_t ksplit, int32_t kchunk, int32_t z0, EPI epi, int* err) {
     const int64_t m0 = (int64_t)blockIdx.x * OZ_T, n0 = (int64_t)blockIdx.y * OZ_T;
     if (lower && m0 + OZ_T - 1 < n0) return;
     extern __shared__ __align__(1024) unsigned char oz_smem_raw[];
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     volatile int* n_consumed = abort_flag + 2;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int part = blockIdx.z & 1, z = blockIdx.z >> 1;
+    const int part = blockIdx.z & 1, z = (int)(blockIdx.z >> 1) + z0;
     const OzPlan& plan = plans.part[part];
     const int b = z / ksplit;
     const int klo = (z - b * ksplit) * kchunk;
@@ -394,10 +397,6 @@ int oz_gemm(cudaStream_t st, const OzOperand& A, int64_t koffA, const OzOperand&
         return FORGE_ERR_ARG;
     }
     const int ks = oz_ksplit_count(nkb, want_split);
-    if (2 * batch * ks > 65535) {
-        set_error(FORGE_ERR_ARG, "oz_gemm: batch x K splits exceeds the grid's z extent");
-        return FORGE_ERR_ARG;
-    }
     if (!plans.part[0].nlev || !plans.part[1].nlev) {
         set_error(FORGE_ERR_ARG, "oz_gemm: K = %lld exceeds the exact integer sums", (long long)K);
         return FORGE_ERR_ARG;
@@ -406,12 +405,15 @@ int oz_gemm(cudaStream_t st, const OzOperand& A, int64_t koffA, const OzOperand&
     FORGE_TRY(oz_make_tmap(&ma, A));
     FORGE_TRY(oz_make_tmap(&mb, B));
     FORGE_CUDA(cudaFuncSetAttribute(k_oz_gemm<EPI, DF>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
-    const dim3 grd((unsigned)((A.rows + OZ_T - 1) / OZ_T), (unsigned)((B.rows + OZ_T - 1) / OZ_T),
-                   (unsigned)(2 * batch * ks));
-    k_oz_gemm<EPI, DF><<<grd, OZ_THREADS, OZ_SMEM, st>>>(ma, mb, A.rows, B.rows, plans, (int32_t)nkb, (int32_t)koffA,
-                                                     (int32_t)koffB, A.zbatch, B.zbatch, lower ? 1 : 0, ks,
-                                                     (int32_t)((nkb + ks - 1) / ks), epi, err);
-    FORGE_LAUNCH_CHECK();
+    // the grid's z extent holds both parts of 32767 products
+    for (int64_t z0 = 0; z0 < batch * ks; z0 += OZ_GRID_Z) {
+        const dim3 grd((unsigned)((A.rows + OZ_T - 1) / OZ_T), (unsigned)((B.rows + OZ_T - 1) / OZ_T),
+                       (unsigned)(2 * std::min<int64_t>(OZ_GRID_Z, batch * ks - z0)));
+        k_oz_gemm<EPI, DF><<<grd, OZ_THREADS, OZ_SMEM, st>>>(ma, mb, A.rows, B.rows, plans, (int32_t)nkb, (int32_t)koffA,
+                                                         (int32_t)koffB, A.zbatch, B.zbatch, lower ? 1 : 0, ks,
+                                                         (int32_t)((nkb + ks - 1) / ks), (int32_t)z0, epi, err);
+        FORGE_LAUNCH_CHECK();
+    }
     return 0;
 }
 
