@@ -1566,6 +1566,92 @@ int forge_gpu_hamiltonian(forge_ctx* x, const double* Potential, const double* z
     return rc;
 }
 
+// matrices of a caller's batch solved together: all of them unless the workspace does not fit beside them
+static int64_t zheevr_chunk(forge_ctx* x, int64_t iu, int64_t nb) {
+    const int64_t N = x->c.N;
+    const bool mixed = x->c.precision == FORGE_PREC_MIXED, oa = mixed && x->oa_mode != 0;
+    const int64_t iu_solve = oa ? N : iu;
+    size_t per = eig_workspace_bytes(N, iu_solve, 1);
+    if (mixed) per += eig_mixed_workspace_bytes(N, iu_solve, 1);
+    if (mixed && x->rr_width > 0) per += rr_window_workspace_bytes(N, 1);
+    if (oa) per += (size_t)N * sizeof(double);
+    size_t freeb = 0, totalb = 0;
+    cudaMemGetInfo(&freeb, &totalb);
+    const size_t reserve = ((size_t)256 << 20) + (oa ? oa_workspace_bytes(N, iu, nb) : 0);
+    int64_t b = std::max<int64_t>(1, freeb > reserve ? (int64_t)((freeb - reserve) / per) : 1);
+    if (const char* env = std::getenv("FORGE_EIG_BATCH")) {
+        const long cap = std::strtol(env, nullptr, 10);
+        if (cap > 0 && cap < b) b = cap;
+    }
+    if (b >= nb) return nb;
+    const int64_t launches = (nb + b - 1) / b;
+    return (nb + launches - 1) / launches;
+}
+
+namespace {
+struct ZheevrBufs {
+    DevBuf A, X, w, ws, mws, wall, ows, oerr, rws;
+    ~ZheevrBufs() {
+        for (DevBuf* b : {&A, &X, &w, &ws, &mws, &wall, &ows, &oerr, &rws}) b->release();
+    }
+};
+
+// matrices [b0, b0 + nb) of the batch, in place
+int zheevr_solve(forge_ctx* x, ZheevrBufs& d, int64_t b0, int64_t nb, int64_t iu, int* fails) {
+    Context& c = x->c;
+    const int64_t N = c.N;
+    const bool oa = c.precision == FORGE_PREC_MIXED && x->oa_mode != 0;
+    EigArgs g{};
+    g.n = N;
+    g.iu = iu;
+    g.batch = nb;
+    g.A = d.A.as<double2>() + b0 * N * N;
+    g.lda = N;
+    g.strideA = N * N;
+    g.X = d.X.as<double2>() + b0 * N * iu;
+    g.ldx = N;
+    g.strideX = N * iu;
+    double* w = d.w.as<double>() + b0 * iu;
+    g.w = w;
+    g.ortol_rel = 1e-7;
+    if (oa) {
+        g.iu = N;
+        g.iu_out = iu;
+        g.w = d.wall.as<double>();
+    }
+    FORGE_TRY(eig_bind_workspace(g, d.ws.ptr, d.ws.bytes));
+    if (c.precision != FORGE_PREC_MIXED) {
+        FORGE_TRY(eig_fp64(c.stream, g));
+    } else {
+        FORGE_TRY(eig_mixed(c.stream, g, d.mws.ptr, d.mws.bytes));
+        if (oa) {
+            int64_t n4 = 0;
+            const float* planes = eig_mixed_planes(d.mws.ptr, N, N, nb, &n4);
+            FORGE_CUDA(cudaMemsetAsync(d.oerr.ptr, 0, sizeof(int), c.stream));
+            FORGE_TRY(oa_refine(c.stream, g.A, g.strideA, planes, n4, N, g.w, N, iu, nb, g.X, g.ldx, g.strideX, w, iu,
+                                d.ows.ptr, d.oerr.as<int>(), x->oa_delta, x->oa_depth));
+            int herr = 0;
+            if (cudaMemcpyAsync(&herr, d.oerr.ptr, sizeof(int), cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
+                cudaStreamSynchronize(c.stream) != cudaSuccess || herr) {
+                set_error(FORGE_ERR_TIMEOUT, "eigenpair refinement: tensor-core wait gave up or CUDA error");
+                return FORGE_ERR_TIMEOUT;
+            }
+            g.w = w;
+            g.iu = iu;
+        }
+        if (x->rr_width > 0) {
+            // the same FP64 window refinement as the SCF's solves
+            const int64_t nw = std::min<int64_t>(x->rr_width, iu);
+            FORGE_TRY(d.rws.ensure(rr_window_workspace_bytes(N, nb)));
+            FORGE_TRY(rr_window(c.stream, g.A, g.strideA, g.X, g.ldx, g.strideX, g.w, iu, N, iu - nw, nw, nb, d.rws.ptr));
+        }
+    }
+    FORGE_CUDA(cudaMemcpyAsync(fails, g.fail, nb * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    FORGE_CUDA(cudaStreamSynchronize(c.stream));
+    return 0;
+}
+}  // namespace
+
 int forge_gpu_zheevr_batch(forge_ctx* x, int64_t nb, const double* A, int64_t iu, double* w, double* Z) {
     FORGE_TRY(check_ctx(x));
     Context& c = x->c;
@@ -1575,77 +1661,27 @@ int forge_gpu_zheevr_batch(forge_ctx* x, int64_t nb, const double* A, int64_t iu
         return FORGE_ERR_ARG;
     }
     const size_t NN = (size_t)N * N;
-    const bool oa = c.precision == FORGE_PREC_MIXED && x->oa_mode != 0;
+    const bool mixed = c.precision == FORGE_PREC_MIXED, oa = mixed && x->oa_mode != 0;
     const int64_t iu_solve = oa ? N : iu;
-    DevBuf dA, dX, dw, ws, mws, wall, ows, oerr;
-    int rc = 0;
-    if ((rc = dA.ensure(nb * NN * sizeof(double2))) || (rc = dX.ensure(nb * N * iu * sizeof(double2))) ||
-        (rc = dw.ensure(nb * iu * sizeof(double))) || (rc = ws.ensure(eig_workspace_bytes(N, iu_solve, nb))))
-        return rc;
-    if (c.precision == FORGE_PREC_MIXED && (rc = mws.ensure(eig_mixed_workspace_bytes(N, iu_solve, nb)))) return rc;
-    if (oa && ((rc = wall.ensure(nb * N * sizeof(double))) || (rc = ows.ensure(oa_workspace_bytes(N, iu, nb))) ||
-               (rc = oerr.ensure(sizeof(int)))))
-        return rc;
-    FORGE_CUDA(cudaMemcpyAsync(dA.ptr, A, nb * NN * sizeof(double2), cudaMemcpyHostToDevice, c.stream));
-    EigArgs g{};
-    g.n = N;
-    g.iu = iu;
-    g.batch = nb;
-    g.A = dA.as<double2>();
-    g.lda = N;
-    g.strideA = N * N;
-    g.X = dX.as<double2>();
-    g.ldx = N;
-    g.strideX = N * iu;
-    g.w = dw.as<double>();
-    g.ortol_rel = 1e-7;
+    ZheevrBufs d;
+    FORGE_TRY(d.A.ensure(nb * NN * sizeof(double2)));
+    FORGE_TRY(d.X.ensure(nb * N * iu * sizeof(double2)));
+    FORGE_TRY(d.w.ensure(nb * iu * sizeof(double)));
+    const int64_t B = zheevr_chunk(x, iu, nb);
+    FORGE_TRY(d.ws.ensure(eig_workspace_bytes(N, iu_solve, B)));
+    if (mixed) FORGE_TRY(d.mws.ensure(eig_mixed_workspace_bytes(N, iu_solve, B)));
     if (oa) {
-        g.iu = N;
-        g.iu_out = iu;
-        g.w = wall.as<double>();
+        FORGE_TRY(d.wall.ensure(B * N * sizeof(double)));
+        FORGE_TRY(d.ows.ensure(oa_workspace_bytes(N, iu, B)));
+        FORGE_TRY(d.oerr.ensure(sizeof(int)));
     }
-    rc = eig_bind_workspace(g, ws.ptr, ws.bytes);
-    if (!rc) rc = (c.precision == FORGE_PREC_MIXED) ? eig_mixed(c.stream, g, mws.ptr, mws.bytes) : eig_fp64(c.stream, g);
-    if (!rc && oa) {
-        int64_t n4 = 0;
-        const float* planes = eig_mixed_planes(mws.ptr, N, N, nb, &n4);
-        cudaMemsetAsync(oerr.ptr, 0, sizeof(int), c.stream);
-        rc = oa_refine(c.stream, g.A, g.strideA, planes, n4, N, g.w, N, iu, nb, g.X, g.ldx, g.strideX, dw.as<double>(),
-                       iu, ows.ptr, oerr.as<int>(), x->oa_delta, x->oa_depth);
-        int herr = 0;
-        if (!rc && (cudaMemcpyAsync(&herr, oerr.ptr, sizeof(int), cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
-                    cudaStreamSynchronize(c.stream) != cudaSuccess || herr)) {
-            set_error(FORGE_ERR_TIMEOUT, "eigenpair refinement: tensor-core wait gave up or CUDA error");
-            rc = FORGE_ERR_TIMEOUT;
-        }
-        g.w = dw.as<double>();
-        g.iu = iu;
-    }
-    DevBuf rws;
-    if (!rc && c.precision == FORGE_PREC_MIXED && x->rr_width > 0) {
-        // the same FP64 window refinement as the SCF's solves
-        const int64_t nw = std::min<int64_t>(x->rr_width, iu);
-        rc = rws.ensure(rr_window_workspace_bytes(N, nb));
-        if (!rc)
-            rc = rr_window(c.stream, g.A, g.strideA, g.X, g.ldx, g.strideX, g.w, iu, N, iu - nw, nw, nb, rws.ptr);
-    }
+    FORGE_CUDA(cudaMemcpyAsync(d.A.ptr, A, nb * NN * sizeof(double2), cudaMemcpyHostToDevice, c.stream));
     std::vector<int> fails(nb);
-    if (!rc) {
-        FORGE_CUDA(cudaMemcpyAsync(w, dw.ptr, nb * iu * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-        if (Z) FORGE_CUDA(cudaMemcpyAsync(Z, dX.ptr, nb * N * iu * sizeof(double2), cudaMemcpyDeviceToHost, c.stream));
-        FORGE_CUDA(cudaMemcpyAsync(fails.data(), g.fail, nb * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-        FORGE_CUDA(cudaStreamSynchronize(c.stream));
-    }
-    dA.release();
-    dX.release();
-    dw.release();
-    ws.release();
-    mws.release();
-    wall.release();
-    ows.release();
-    oerr.release();
-    rws.release();
-    if (rc) return rc;
+    for (int64_t b0 = 0; b0 < nb; b0 += B)
+        FORGE_TRY(zheevr_solve(x, d, b0, std::min(B, nb - b0), iu, fails.data() + b0));
+    FORGE_CUDA(cudaMemcpyAsync(w, d.w.ptr, nb * iu * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    if (Z) FORGE_CUDA(cudaMemcpyAsync(Z, d.X.ptr, nb * N * iu * sizeof(double2), cudaMemcpyDeviceToHost, c.stream));
+    FORGE_CUDA(cudaStreamSynchronize(c.stream));
     int bad = 0;
     for (int64_t b = 0; b < nb; ++b) bad += fails[b] ? 1 : 0;
     return bad;

@@ -122,7 +122,9 @@ int forge_gpu_hamiltonian(forge_ctx* ctx, const double* Potential, const double*
 
 /* zdiagRed (LapackRoutines.f90:381-433) on a batch of nb Hermitian matrices given in the
  * lower triangle (ndim x ndim complex each, column-major, host): eigenvalues 1..iu in
- * ascending order into w (iu x nb) and eigenvectors into Z (ndim x iu x nb). */
+ * ascending order into w (iu x nb) and eigenvectors into Z (ndim x iu x nb).  The matrices and
+ * vectors of the whole batch are on the device; the solver's workspace serves as many of them at a
+ * time as fit beside them (or FORGE_EIG_BATCH of the environment, if that is less). */
 int forge_gpu_zheevr_batch(forge_ctx* ctx, int64_t nb, const double* A, int64_t iu, double* w, double* Z);
 
 /* Solve (HartreeFock.f90:402-483): H(k) for all k, eigenpairs 1..nUpper, window bands and
