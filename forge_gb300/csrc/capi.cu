@@ -108,6 +108,8 @@ struct forge_ctx {
     int oa_depth = 4;
     bool oa_active = false, oa_latched = false;
     double last_residual = INFINITY;
+    // test hook: the next FP64 solves / projector batches that report a bounded wait that gave up
+    int fail_solves = 0, fail_projectors = 0;
     DevBuf oaws, w_all;
     // group solve led by this context (forge_gpu_solve_group): padded H slots, eigenpairs, workspaces
     DevBuf g_H, g_X, g_w, g_eigws, g_mixws, g_tmp, g_rows, g_sig, g_rr, g_lim;
@@ -227,9 +229,30 @@ int upload_state(forge_ctx* x, const double* Potential, const double* zFock) {
     return 0;
 }
 
-// eigen-solve of the batch of H already assembled in c.H for k in [k0, k0+nb); the eigenpairs go to
+int injected_timeout(int& left) {
+    if (left <= 0) return 0;
+    --left;
+    set_error(FORGE_ERR_TIMEOUT, "injected: a bounded wait gave up");
+    return FORGE_ERR_TIMEOUT;
+}
+
+// solve(), and once more after again() if a bounded tensor-core wait gave up (the kernel drained and freed its TMEM);
+// again() restores the matrices, which the FP64 reduction overwrites
+template <class Solve, class Again>
+int solve_twice(const Solve& solve, const Again& again) {
+    int rc = solve();
+    if (rc != FORGE_ERR_TIMEOUT) return rc;
+    std::fprintf(stderr, "forge: %s; solving the batch again\n", forge_gpu_last_error());
+    FORGE_TRY(again());
+    return solve();
+}
+
+// eigen-solve of the batch of H that assemble() puts into c.H for k in [k0, k0+nb); the eigenpairs go to
 // the slots of those k, or to Xdst / wdst when given
-int eig_batch_run(forge_ctx* x, int64_t k0, int64_t nb, int* info, double2* Xdst = nullptr, double* wdst = nullptr) {
+template <class Assemble>
+int eig_batch_run(forge_ctx* x, int64_t k0, int64_t nb, int* info, const Assemble& assemble, double2* Xdst = nullptr,
+                  double* wdst = nullptr) {
+    FORGE_TRY(assemble());
     Context& c = x->c;
     const int64_t N = c.N, iu = c.nUpper;
     EigArgs g{};
@@ -273,15 +296,8 @@ int eig_batch_run(forge_ctx* x, int64_t k0, int64_t nb, int* info, double2* Xdst
             }
             return 0;
         };
-        int rc = solve();
-        if (rc == FORGE_ERR_TIMEOUT) {
-            // a bounded tensor-core wait gave up (the kernel drained and freed its TMEM): the
-            // input H(k) is unchanged (the refinement only mirrors its lower triangle), so the
-            // batch is solved again once
-            std::fprintf(stderr, "forge: %s; solving the batch again\n", forge_gpu_last_error());
-            rc = solve();
-        }
-        FORGE_TRY(rc);
+        // the input H(k) is unchanged (the refinement only mirrors its lower triangle)
+        FORGE_TRY(solve_twice(solve, []() { return 0; }));
         g.w = w_iu;
         g.iu = iu;
         if (x->rr_width > 0) {
@@ -292,7 +308,12 @@ int eig_batch_run(forge_ctx* x, int64_t k0, int64_t nb, int* info, double2* Xdst
                                 x->rrws.ptr));
         }
     } else {
-        FORGE_TRY(eig_fp64(c.stream, g));
+        FORGE_TRY(solve_twice(
+            [&]() -> int {
+                FORGE_TRY(eig_fp64(c.stream, g));
+                return injected_timeout(x->fail_solves);
+            },
+            assemble));
     }
     std::vector<int> fails(nb);
     FORGE_CUDA(cudaMemcpyAsync(fails.data(), g.fail, nb * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
@@ -351,14 +372,21 @@ int projector_status(forge_ctx* x) {
         set_error(FORGE_ERR_TIMEOUT, "tcgen05 projector: a bounded mbarrier wait gave up");
         return FORGE_ERR_TIMEOUT;
     }
-    return 0;
+    return injected_timeout(x->fail_projectors);
 }
 
-// the zFockBulk sum over the local k points: bands 1..nLower-1 of every k
+// the zFockBulk sum over the local k points, bands 1..nLower-1 of every k, into out (zero on entry); formed again
+// once if a bounded wait gave up, which leaves the eigenvectors as they are
 int project_bulk(forge_ctx* x, double2* out) {
     const int64_t kb = x->k_begin, ke = (x->k_end > 0) ? x->k_end : x->c.Nk;
     std::vector<ProjItem> items;
     for (int64_t k = kb; k < ke; ++k) add_projector(x, k, x->c.nLower - 1, &x->h_bph[k * 4], items);
+    FORGE_TRY(project_items(x, items, out));
+    int rc = projector_status(x);
+    if (rc != FORGE_ERR_TIMEOUT) return rc;
+    std::fprintf(stderr, "forge: %s; forming the projector again\n", forge_gpu_last_error());
+    FORGE_CUDA(cudaMemsetAsync(out, 0, 4 * (size_t)x->c.N * x->c.N * sizeof(double2), x->c.stream));
+    FORGE_CUDA(cudaMemsetAsync(x->tcerr.ptr, 0, sizeof(int), x->c.stream));
     FORGE_TRY(project_items(x, items, out));
     return projector_status(x);
 }
@@ -421,10 +449,13 @@ int solve_device(forge_ctx* x, int* info, bool with_projector = true) {
         const int64_t N_ = c.N, iu = c.nUpper, nr = (int64_t)x->c3t.reps.size();
         for (int64_t r0 = 0; r0 < nr; r0 += B) {
             const int64_t nb = (nr - r0 < B) ? nr - r0 : B;
-            for (int64_t b = 0; b < nb; ++b)
-                FORGE_TRY(launch_assemble(c, c.V.as<double>(), c.P.as<double2>(), x->c3t.reps[r0 + b], 1,
-                                          c.H.as<double2>() + (size_t)b * NN));
-            FORGE_TRY(eig_batch_run(x, r0, nb, info, x->c3_Xr.as<double2>() + (size_t)r0 * N_ * iu,
+            auto assemble = [&]() -> int {
+                for (int64_t b = 0; b < nb; ++b)
+                    FORGE_TRY(launch_assemble(c, c.V.as<double>(), c.P.as<double2>(), x->c3t.reps[r0 + b], 1,
+                                              c.H.as<double2>() + (size_t)b * NN));
+                return 0;
+            };
+            FORGE_TRY(eig_batch_run(x, r0, nb, info, assemble, x->c3_Xr.as<double2>() + (size_t)r0 * N_ * iu,
                                     x->c3_wr.as<double>() + (size_t)r0 * iu));
         }
         FORGE_TRY(launch_c3_rotate(c.stream, x->c3_Xr.as<double2>(), x->c3_wr.as<double>(), N_, iu, x->c3t.nslots,
@@ -438,8 +469,9 @@ int solve_device(forge_ctx* x, int* info, bool with_projector = true) {
     }
     for (int64_t k0 = kb; k0 < ke; k0 += B) {
         const int64_t nb = (ke - k0 < B) ? ke - k0 : B;
-        FORGE_TRY(launch_assemble(c, c.V.as<double>(), c.P.as<double2>(), k0, nb, c.H.as<double2>()));
-        FORGE_TRY(eig_batch_run(x, k0, nb, info));
+        FORGE_TRY(eig_batch_run(x, k0, nb, info, [&]() {
+            return launch_assemble(c, c.V.as<double>(), c.P.as<double2>(), k0, nb, c.H.as<double2>());
+        }));
     }
     if (with_projector) FORGE_TRY(project_bulk(x, c.bulk.as<double2>()));
     x->have_solve = true;
@@ -899,17 +931,21 @@ int solve_group_device(forge_ctx** xs, int64_t nctx, int* infos) {
     double* gw = x0->g_w.as<double>();
     for (size_t q0 = 0; q0 < items.size(); q0 += (size_t)B) {
         const int64_t nb = std::min<int64_t>(B, (int64_t)(items.size() - q0));
-        for (int64_t q = 0; q < nb; ++q) {
-            Context& cb = xs[items[q0 + q].first]->c;
-            const cudaStream_t own = cb.stream;
-            cb.stream = st;   // the assembly of every member on the group's stream
-            const int rc = launch_assemble(cb, cb.V.as<double>(), cb.P.as<double2>(), items[q0 + q].second, 1,
-                                           x0->g_tmp.as<double2>());
-            cb.stream = own;
-            FORGE_TRY(rc);
-            FORGE_TRY(launch_pad_slot(st, x0->g_tmp.as<double2>(), cb.N, gH + q * slot, nmax, x0->g_rows.as<double>(),
-                                      x0->g_sig.as<double>()));
-        }
+        auto assemble = [&]() -> int {
+            for (int64_t q = 0; q < nb; ++q) {
+                Context& cb = xs[items[q0 + q].first]->c;
+                const cudaStream_t own = cb.stream;
+                cb.stream = st;   // the assembly of every member on the group's stream
+                const int rc = launch_assemble(cb, cb.V.as<double>(), cb.P.as<double2>(), items[q0 + q].second, 1,
+                                               x0->g_tmp.as<double2>());
+                cb.stream = own;
+                FORGE_TRY(rc);
+                FORGE_TRY(launch_pad_slot(st, x0->g_tmp.as<double2>(), cb.N, gH + q * slot, nmax, x0->g_rows.as<double>(),
+                                          x0->g_sig.as<double>()));
+            }
+            return 0;
+        };
+        FORGE_TRY(assemble());
         EigArgs g{};
         g.n = nmax;
         g.iu = iumax;
@@ -928,7 +964,12 @@ int solve_group_device(forge_ctx** xs, int64_t nctx, int* infos) {
         FORGE_CUDA(cudaMemcpyAsync(x0->g_lim.ptr, lims.data(), nb * sizeof(int), cudaMemcpyHostToDevice, st));
         g.iu_lim = x0->g_lim.as<int>();
         FORGE_TRY(eig_bind_workspace(g, x0->g_eigws.ptr, x0->g_eigws.bytes));
-        FORGE_TRY(mixed ? eig_mixed(st, g, x0->g_mixws.ptr, x0->g_mixws.bytes) : eig_fp64(st, g));
+        FORGE_TRY(solve_twice(
+            [&]() -> int {
+                FORGE_TRY(mixed ? eig_mixed(st, g, x0->g_mixws.ptr, x0->g_mixws.bytes) : eig_fp64(st, g));
+                return mixed ? 0 : injected_timeout(x0->fail_solves);
+            },
+            assemble));
         if (mixed && x0->rr_width > 0)
             for (int64_t q = 0; q < nb; ++q) {
                 const int64_t iub = xs[items[q0 + q].first]->c.nUpper;
@@ -1596,8 +1637,8 @@ struct ZheevrBufs {
     }
 };
 
-// matrices [b0, b0 + nb) of the batch, in place
-int zheevr_solve(forge_ctx* x, ZheevrBufs& d, int64_t b0, int64_t nb, int64_t iu, int* fails) {
+// matrices [b0, b0 + nb) of the batch A, in place of their copies in d.A
+int zheevr_solve(forge_ctx* x, ZheevrBufs& d, const double* A, int64_t b0, int64_t nb, int64_t iu, int* fails) {
     Context& c = x->c;
     const int64_t N = c.N;
     const bool oa = c.precision == FORGE_PREC_MIXED && x->oa_mode != 0;
@@ -1621,7 +1662,16 @@ int zheevr_solve(forge_ctx* x, ZheevrBufs& d, int64_t b0, int64_t nb, int64_t iu
     }
     FORGE_TRY(eig_bind_workspace(g, d.ws.ptr, d.ws.bytes));
     if (c.precision != FORGE_PREC_MIXED) {
-        FORGE_TRY(eig_fp64(c.stream, g));
+        FORGE_TRY(solve_twice(
+            [&]() -> int {
+                FORGE_TRY(eig_fp64(c.stream, g));
+                return injected_timeout(x->fail_solves);
+            },
+            [&]() -> int {
+                FORGE_CUDA(cudaMemcpyAsync(g.A, A + 2 * b0 * N * N, nb * N * N * sizeof(double2), cudaMemcpyHostToDevice,
+                                           c.stream));
+                return 0;
+            }));
     } else {
         FORGE_TRY(eig_mixed(c.stream, g, d.mws.ptr, d.mws.bytes));
         if (oa) {
@@ -1678,13 +1728,20 @@ int forge_gpu_zheevr_batch(forge_ctx* x, int64_t nb, const double* A, int64_t iu
     FORGE_CUDA(cudaMemcpyAsync(d.A.ptr, A, nb * NN * sizeof(double2), cudaMemcpyHostToDevice, c.stream));
     std::vector<int> fails(nb);
     for (int64_t b0 = 0; b0 < nb; b0 += B)
-        FORGE_TRY(zheevr_solve(x, d, b0, std::min(B, nb - b0), iu, fails.data() + b0));
+        FORGE_TRY(zheevr_solve(x, d, A, b0, std::min(B, nb - b0), iu, fails.data() + b0));
     FORGE_CUDA(cudaMemcpyAsync(w, d.w.ptr, nb * iu * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     if (Z) FORGE_CUDA(cudaMemcpyAsync(Z, d.X.ptr, nb * N * iu * sizeof(double2), cudaMemcpyDeviceToHost, c.stream));
     FORGE_CUDA(cudaStreamSynchronize(c.stream));
     int bad = 0;
     for (int64_t b = 0; b < nb; ++b) bad += fails[b] ? 1 : 0;
     return bad;
+}
+
+int forge_gpu_selftest_timeouts(forge_ctx* x, int64_t solves, int64_t projectors) {
+    FORGE_TRY(check_ctx(x));
+    x->fail_solves = (int)solves;
+    x->fail_projectors = (int)projectors;
+    return 0;
 }
 
 int forge_gpu_solve(forge_ctx* x, const double* Potential, const double* zFock, double* Bands, double* zEigenvectors,

@@ -339,7 +339,8 @@ int forge_gpu_mlp_train(forge_mlp* mlp, const float* X, const float* targets, in
  * address.  Every call ends by synchronising `stream` to read the solver's convergence flag, so
  * the call blocks the host until its work is done and cannot be recorded into a CUDA graph.
  * Calls share the array: calls whose work overlaps on the GPU race.  Returns 0, 1 (inverse
- * iteration did not converge) or FORGE_ERR_*.  The solver is the FP64 path of
+ * iteration did not converge) or FORGE_ERR_*; A is overwritten in any case, so a caller that gets
+ * FORGE_ERR_TIMEOUT tries again with a fresh copy of the matrix.  The solver is the FP64 path of
  * forge_gpu_zheevr_batch. */
 #define FORGE_NOALLOC_MAX_N 512
 #define FORGE_NOALLOC_SCRATCH_BYTES (16u * 1024u * 1024u)

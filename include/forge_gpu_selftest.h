@@ -9,6 +9,8 @@
 
 #include <stdint.h>
 
+#include "forge_gpu.h"
+
 #ifdef __cplusplus
 extern "C" {
 #endif
@@ -30,6 +32,10 @@ int forge_gpu_selftest_tc_gemm_timeout(int64_t M, int64_t N, int64_t K, int64_t 
  * with S = L L^H and L^{-1} G L^{-H} = U diag(theta) U^H, so that G M = S M diag(theta) and
  * M^H S M = I.  Returns 1 if S is not positive definite. */
 int forge_selftest_rr_small(int64_t n, const double* G, const double* S, double* theta, double* M);
+
+/* The context's next `solves` FP64 eigen-solves and `projectors` batches of projectors report, once their work is
+ * done, that a bounded wait gave up (FORGE_ERR_TIMEOUT); each is tried a second time. */
+int forge_gpu_selftest_timeouts(forge_ctx* ctx, int64_t solves, int64_t projectors);
 
 /* Numbers of eigenvalues <= x[q] of the tridiagonal (d, e), |T| <= 1, by the minors' Sturm counts of
  * the tridiagonal solver in FP64 and in FP32. */
