@@ -161,7 +161,7 @@ int choose_batch(forge_ctx* x) {
     const int64_t N = c.N, iu = c.nUpper;
     const bool oa = c.precision == FORGE_PREC_MIXED && x->oa_mode != 0;
     const int64_t iu_solve = oa ? N : iu;   // the refinement needs every eigenpair of the mixed solve
-    size_t per_k = (size_t)N * N * 16 + eig_workspace_bytes(N, iu_solve, 1);
+    size_t per_k = (size_t)N * N * 16 + eig_workspace_bytes(N, iu_solve, 1, c.precision == FORGE_PREC_MIXED);
     if (c.precision == FORGE_PREC_MIXED) per_k += eig_mixed_workspace_bytes(N, iu_solve, 1);
     if (oa) per_k += (size_t)N * 8;
     size_t freeb = 0, totalb = 0;
@@ -207,7 +207,7 @@ int ensure_solve_buffers(forge_ctx* x) {
     }
     const bool oa = c.precision == FORGE_PREC_MIXED && x->oa_mode != 0;
     const int64_t iu_solve = oa ? N : iu;
-    FORGE_TRY(x->eigws.ensure(eig_workspace_bytes(N, iu_solve, B)));
+    FORGE_TRY(x->eigws.ensure(eig_workspace_bytes(N, iu_solve, B, c.precision == FORGE_PREC_MIXED)));
     if (c.precision == FORGE_PREC_MIXED) FORGE_TRY(x->mixws.ensure(eig_mixed_workspace_bytes(N, iu_solve, B)));
     if (oa) {
         FORGE_TRY(x->w_all.ensure((size_t)B * N * sizeof(double)));
@@ -275,6 +275,7 @@ int eig_batch_run(forge_ctx* x, int64_t k0, int64_t nb, int* info, const Assembl
         g.iu_out = iu;
         g.w = x->w_all.as<double>();
     }
+    g.mixed = c.precision == FORGE_PREC_MIXED;
     FORGE_TRY(eig_bind_workspace(g, x->eigws.ptr, x->eigws.bytes));
     if (c.precision == FORGE_PREC_MIXED) {
         auto solve = [&]() -> int {
@@ -908,7 +909,7 @@ int solve_group_device(forge_ctx** xs, int64_t nctx, int* infos) {
     }
     const bool mixed = c0.precision == FORGE_PREC_MIXED;
     const size_t slot = (size_t)nmax * nmax;
-    size_t per_item = slot * 16 + eig_workspace_bytes(nmax, iumax, 1) + (size_t)nmax * iumax * 16 + iumax * 8;
+    size_t per_item = slot * 16 + eig_workspace_bytes(nmax, iumax, 1, mixed) + (size_t)nmax * iumax * 16 + iumax * 8;
     if (mixed) per_item += eig_mixed_workspace_bytes(nmax, iumax, 1);
     size_t freeb = 0, totalb = 0;
     cudaMemGetInfo(&freeb, &totalb);
@@ -918,7 +919,7 @@ int solve_group_device(forge_ctx** xs, int64_t nctx, int* infos) {
     FORGE_TRY(x0->g_H.ensure((size_t)B * slot * sizeof(double2)));
     FORGE_TRY(x0->g_X.ensure((size_t)B * nmax * iumax * sizeof(double2)));
     FORGE_TRY(x0->g_w.ensure((size_t)B * iumax * sizeof(double)));
-    FORGE_TRY(x0->g_eigws.ensure(eig_workspace_bytes(nmax, iumax, B)));
+    FORGE_TRY(x0->g_eigws.ensure(eig_workspace_bytes(nmax, iumax, B, mixed)));
     if (mixed) FORGE_TRY(x0->g_mixws.ensure(eig_mixed_workspace_bytes(nmax, iumax, B)));
     FORGE_TRY(x0->g_tmp.ensure(slot * sizeof(double2)));
     FORGE_TRY(x0->g_rows.ensure(nmax * sizeof(double)));
@@ -963,6 +964,7 @@ int solve_group_device(forge_ctx** xs, int64_t nctx, int* infos) {
         for (int64_t q = 0; q < nb; ++q) lims[q] = (int)xs[items[q0 + q].first]->c.nUpper;
         FORGE_CUDA(cudaMemcpyAsync(x0->g_lim.ptr, lims.data(), nb * sizeof(int), cudaMemcpyHostToDevice, st));
         g.iu_lim = x0->g_lim.as<int>();
+        g.mixed = mixed;
         FORGE_TRY(eig_bind_workspace(g, x0->g_eigws.ptr, x0->g_eigws.bytes));
         FORGE_TRY(solve_twice(
             [&]() -> int {
@@ -1612,7 +1614,7 @@ static int64_t zheevr_chunk(forge_ctx* x, int64_t iu, int64_t nb) {
     const int64_t N = x->c.N;
     const bool mixed = x->c.precision == FORGE_PREC_MIXED, oa = mixed && x->oa_mode != 0;
     const int64_t iu_solve = oa ? N : iu;
-    size_t per = eig_workspace_bytes(N, iu_solve, 1);
+    size_t per = eig_workspace_bytes(N, iu_solve, 1, mixed);
     if (mixed) per += eig_mixed_workspace_bytes(N, iu_solve, 1);
     if (mixed && x->rr_width > 0) per += rr_window_workspace_bytes(N, 1);
     if (oa) per += (size_t)N * sizeof(double);
@@ -1660,6 +1662,7 @@ int zheevr_solve(forge_ctx* x, ZheevrBufs& d, const double* A, int64_t b0, int64
         g.iu_out = iu;
         g.w = d.wall.as<double>();
     }
+    g.mixed = c.precision == FORGE_PREC_MIXED;
     FORGE_TRY(eig_bind_workspace(g, d.ws.ptr, d.ws.bytes));
     if (c.precision != FORGE_PREC_MIXED) {
         FORGE_TRY(solve_twice(
@@ -1718,7 +1721,7 @@ int forge_gpu_zheevr_batch(forge_ctx* x, int64_t nb, const double* A, int64_t iu
     FORGE_TRY(d.X.ensure(nb * N * iu * sizeof(double2)));
     FORGE_TRY(d.w.ensure(nb * iu * sizeof(double)));
     const int64_t B = zheevr_chunk(x, iu, nb);
-    FORGE_TRY(d.ws.ensure(eig_workspace_bytes(N, iu_solve, B)));
+    FORGE_TRY(d.ws.ensure(eig_workspace_bytes(N, iu_solve, B, mixed)));
     if (mixed) FORGE_TRY(d.mws.ensure(eig_mixed_workspace_bytes(N, iu_solve, B)));
     if (oa) {
         FORGE_TRY(d.wall.ensure(B * N * sizeof(double)));

@@ -26,7 +26,6 @@ struct EigArgs {
     double* part;
     int64_t pstride;
     double* scal;               // batch x 16
-    unsigned* cnt;              // batch x 4
     double* info;               // batch x 8
     int* clus;                  // batch x (iu + 2)
     double* Z;                  // batch x n x iu (row-major)
@@ -45,6 +44,7 @@ struct EigArgs {
     float2* tf;                 // batch x n: T scaled to |T| <= 1, (d_i, e_{i-1}^2) in FP32 (FP32 bisection)
     double2* de;                // the same in FP64
     float* tq;                  // batch x 2n: unscaled T in FP32, d and e^2 (mixed precision)
+    bool mixed = false;         // workspace of the mixed solver (set before it is bound)
     int replay = 0;             // 1 (mixed precision): eigenvalues as the quotient-form bisection gives them
     double ortol_rel;
     const int* iu_lim = nullptr;  // device: eigenpairs wanted of each matrix (nullptr: iu of every one)
@@ -52,7 +52,8 @@ struct EigArgs {
 };
 
 // workspace sizes (bytes) for a given problem; they serve every smaller batch as well
-size_t eig_workspace_bytes(int64_t n, int64_t iu, int64_t batch);
+// (mixed: what the mixed solver shares with the FP64 one; the rest of its workspace is eig_mixed_workspace_bytes)
+size_t eig_workspace_bytes(int64_t n, int64_t iu, int64_t batch, bool mixed);
 // carve the workspace out of one device buffer; FORGE_ERR_ARG if the batch needs more than the bytes given
 int eig_bind_workspace(EigArgs& g, void* base, size_t bytes);
 

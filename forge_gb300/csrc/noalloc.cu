@@ -10,8 +10,8 @@
 // (FORGE_NOALLOC_SCRATCH_BYTES) until the process exits.
 //
 // The array is shared by every call on a device and keeps the contents of the last call; the
-// solver clears what must start at zero (its CTA counters and the failure flags) at the start of
-// each call.  Calls whose work overlaps on the GPU race on the array, so callers must order
+// solver clears what must start at zero (the failure and error flags, the panels' largest exponents)
+// in each call.  Calls whose work overlaps on the GPU race on the array, so callers must order
 // them (one stream, or events).  Host code only uses the array through the device address
 // obtained with cudaGetSymbolAddress, once per device with that device current, during the
 // first call on that device (std::call_once per device: concurrent first calls from several
@@ -50,7 +50,7 @@ extern "C" int forge_gpu_zheevr_noalloc(double* A, int64_t n, int64_t iu, double
                   (long long)n, (long long)kNoAllocMaxN);
         return FORGE_ERR_ARG;
     }
-    const size_t need = eig_workspace_bytes(n, iu, 1);
+    const size_t need = eig_workspace_bytes(n, iu, 1, false);
     if (need > kNoAllocBytes) {
         set_error(FORGE_ERR_ARG, "zheevr_noalloc: workspace of %zu bytes exceeds the %zu-byte static array", need,
                   kNoAllocBytes);

@@ -1018,7 +1018,6 @@ int eig_fp64(cudaStream_t st, EigArgs& g) {
     a.part = g.part;
     a.pstride = g.pstride;
     a.scal = g.scal;
-    a.cnt = g.cnt;
     a.w0 = g.w0;
     a.limbs = g.limbs;
     a.limb_f = g.limb_f;
@@ -1151,6 +1150,19 @@ void carve(EigArgs& g, Carve& c) {
     g.pstride = 3 * ((n + 15) / 16);  // per-CTA partials of k_col64 and k_finish64
     g.d = c.take<double>(B * n);
     g.e = c.take<double>(B * n);
+    g.info = c.take<double>(B * 8);
+    g.clus = c.take<int>(B * (iu + 2));
+    g.pivs = c.take<unsigned char>(n * iu * B);
+    g.fail = c.take<int>(B);
+    g.tf = c.take<float2>(B * n);
+    g.de = c.take<double2>(B * n);
+    if (g.mixed) {
+        // the reduction and the back-transformation have their own workspace (eig_mixed.cu)
+        g.Z = c.take<double>(B * n * iu);
+        g.scr = c.take<double>(4 * n * iu * B);
+        g.tq = c.take<float>(B * 2 * n);
+        return;
+    }
     g.tau = c.take<double2>(B * n);
     g.Wp = c.take<double2>(B * n * TRD_NB);
     g.w0 = c.take<double2>(B * n);
@@ -1159,9 +1171,6 @@ void carve(EigArgs& g, Carve& c) {
     g.Spart = c.take<double2>(B * g.sstride);
     g.part = c.take<double>(B * g.pstride);
     g.scal = c.take<double>(B * 16);
-    g.cnt = c.take<unsigned>(B * 4);
-    g.info = c.take<double>(B * 8);
-    g.clus = c.take<int>(B * (iu + 2));
     OzSizes z;
     oz_sizes(n, iu, B, z);
     // the slices of X (and of the rank-2k update) share the scratch of the inverse iteration, those of V its
@@ -1170,8 +1179,6 @@ void carve(EigArgs& g, Carve& c) {
     g.oz_vr = g.Z;
     g.scr = (double*)c.take<char>(std::max<size_t>(sizeof(double) * 4 * n * iu * B, 2 * std::max(z.xs, z.uz)));
     g.oz_xs = g.scr;
-    g.pivs = c.take<unsigned char>(n * iu * B);
-    g.fail = c.take<int>(B);
     // the trailing matrix in limbs (tridiagonalisation) shares the space of V^H (back-transformation)
     g.limb_tiles = nblk * (nblk + 1) / 2;
     g.oz_vh = c.take<char>(std::max<size_t>(2 * z.vh, sizeof(int4) * B * g.limb_tiles * TRD_TILE * TRD_TILE));
@@ -1184,14 +1191,12 @@ void carve(EigArgs& g, Carve& c) {
     g.oz_t = c.take<double2>(z.g);
     g.oz_ex = c.take<int>(z.ex);
     g.oz_err = c.take<int>(1);
-    g.tf = c.take<float2>(B * n);
-    g.de = c.take<double2>(B * n);
-    g.tq = c.take<float>(B * 2 * n);
 }
 }  // namespace
 
-size_t eig_workspace_bytes(int64_t n, int64_t iu, int64_t batch) {
+size_t eig_workspace_bytes(int64_t n, int64_t iu, int64_t batch, bool mixed) {
     EigArgs g{};
+    g.mixed = mixed;
     g.n = n;
     g.iu = iu;
     g.batch = batch;
@@ -1306,12 +1311,12 @@ extern "C" int forge_selftest_eig_workspace(int64_t n, int64_t iu, int64_t batch
     }
     if (mixed) {
         eig_mixed_splits(n, iu, batch, out + 1);
-        out[0] = (int64_t)eig_mixed_workspace_bytes(n, iu, batch);
+        out[0] = (int64_t)(eig_mixed_workspace_bytes(n, iu, batch) + eig_workspace_bytes(n, iu, batch, true));
         return 0;
     }
     OzSizes z;
     oz_sizes(n, iu, batch, z);
-    out[0] = (int64_t)eig_workspace_bytes(n, iu, batch);
+    out[0] = (int64_t)eig_workspace_bytes(n, iu, batch, false);
     out[1] = z.ks * batch;
     out[2] = z.wp / (iu * z.NB);
     out[3] = out[4] = 0;

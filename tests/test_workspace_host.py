@@ -21,3 +21,10 @@ def test_workspace_serves_every_smaller_batch(lib, n, iu, mixed):
         assert need >= last, batch
         assert g <= groom and w <= wroom, batch
         last = need
+
+
+@pytest.mark.parametrize("n", [3268, 5044, 11908])
+def test_mixed_workspace_holds_nothing_of_the_fp64_path(lib, n):
+    """All pairs of one matrix: Z, the factors and pivots (41 n^2 bytes), the FP32 matrix (8), two planes' pairs (16),
+    and panels and partial products that fall off as 1 / n."""
+    assert _need(lib, n, n, 1, 1)[0] <= (65 + 36000 / n) * n * n
