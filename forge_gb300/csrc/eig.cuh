@@ -45,6 +45,7 @@ struct EigArgs {
     double2* de;                // the same in FP64
     float* tq;                  // batch x 2n: unscaled T in FP32, d and e^2 (mixed precision)
     bool mixed = false;         // workspace of the mixed solver (set before it is bound)
+    bool lean = false;          // FP64 workspace of the allocation-free entry (n <= 512, set before it is bound)
     int replay = 0;             // 1 (mixed precision): eigenvalues as the quotient-form bisection gives them
     double ortol_rel;
     const int* iu_lim = nullptr;  // device: eigenpairs wanted of each matrix (nullptr: iu of every one)
@@ -53,7 +54,7 @@ struct EigArgs {
 
 // workspace sizes (bytes) for a given problem; they serve every smaller batch as well
 // (mixed: what the mixed solver shares with the FP64 one; the rest of its workspace is eig_mixed_workspace_bytes)
-size_t eig_workspace_bytes(int64_t n, int64_t iu, int64_t batch, bool mixed);
+size_t eig_workspace_bytes(int64_t n, int64_t iu, int64_t batch, bool mixed, bool lean = false);
 // carve the workspace out of one device buffer; FORGE_ERR_ARG if the batch needs more than the bytes given
 int eig_bind_workspace(EigArgs& g, void* base, size_t bytes);
 
@@ -69,7 +70,7 @@ struct OzSizes {
     int64_t NB, nblk, mb, ks, ldx;        // block width, blocks, blocks per chunk, K splits of V^H X, slice pitch
     int64_t xs, vr, vh, uz, wp, ws, g, ts, ex;
 };
-void oz_sizes(int64_t n, int64_t iu, int64_t batch, OzSizes& z);
+void oz_sizes(int64_t n, int64_t iu, int64_t batch, bool lean, OzSizes& z);
 int her2k_oz(cudaStream_t st, TrdArgs<double>& a, int64_t p, int64_t w, int64_t batch, void* user);
 int backtransform_oz(cudaStream_t st, EigArgs& g);
 

@@ -50,7 +50,7 @@ extern "C" int forge_gpu_zheevr_noalloc(double* A, int64_t n, int64_t iu, double
                   (long long)n, (long long)kNoAllocMaxN);
         return FORGE_ERR_ARG;
     }
-    const size_t need = eig_workspace_bytes(n, iu, 1, false);
+    const size_t need = eig_workspace_bytes(n, iu, 1, false, true);
     if (need > kNoAllocBytes) {
         set_error(FORGE_ERR_ARG, "zheevr_noalloc: workspace of %zu bytes exceeds the %zu-byte static array", need,
                   kNoAllocBytes);
@@ -88,6 +88,7 @@ extern "C" int forge_gpu_zheevr_noalloc(double* A, int64_t n, int64_t iu, double
     g.strideX = n * iu;
     g.w = w;
     g.ortol_rel = 1e-7;
+    g.lean = true;
     int rc = eig_bind_workspace(g, g_noalloc_ptr[dev], kNoAllocBytes);
     if (!rc) rc = eig_fp64(st, g);
     int fail = 0;

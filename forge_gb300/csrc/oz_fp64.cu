@@ -209,19 +209,19 @@ __global__ void k_oz_larft(const double2* __restrict__ G, const double2* __restr
 // 64 (half of the tile is padding, but T costs an eighth and the workspace half).
 int oz_bt_nb(int64_t n) { return n > 512 ? 128 : 64; }
 
-void oz_sizes(int64_t n, int64_t iu, int64_t batch, OzSizes& z) {
+void oz_sizes(int64_t n, int64_t iu, int64_t batch, bool lean, OzSizes& z) {
     z.NB = oz_bt_nb(n);
     z.nblk = (std::max<int64_t>(1, n - 1) + z.NB - 1) / z.NB;
-    // blocks whose V^H and T are formed together: half of them (14 n^2 bytes); the allocation-free entry's
-    // 16 MiB array (n <= 512) holds all blocks up to 384 and single ones above
-    const int64_t mb = n > 512 ? std::max<int64_t>(1, (z.nblk + 1) / 2) : n > 384 ? 1 : z.nblk;
+    // blocks whose V^H and T are formed together: T is a serial chain a block, so all of them up to 512, half of them
+    // (14 n^2 bytes) above; the allocation-free entry's 16 MiB array holds all up to 384 and single ones above
+    const int64_t mb = n > 512 ? std::max<int64_t>(1, (z.nblk + 1) / 2) : lean && n > 384 ? 1 : z.nblk;
     // blocks x matrices in a grid's y extent; room: the most that mb x batch reaches for any batch up to this one
     z.mb = std::max<int64_t>(1, std::min<int64_t>(mb, GRID_Y / batch));
     const int64_t room = std::min(mb * batch, std::max<int64_t>(batch, GRID_Y));
     z.ldx = up(n, 8);
     // K splits of V^H X: enough CTAs for the GPU, no split shorter than 256 rows
     const int64_t t = (iu + OZ_T - 1) / OZ_T * 2, tiles = t * batch;
-    const int64_t most = std::max<int64_t>(1, std::min<int64_t>(n > 512 ? 8 : 1, n / 256));
+    const int64_t most = std::max<int64_t>(1, std::min<int64_t>(lean ? 1 : 8, n / 256));
     z.ks = std::min(most, (152 + tiles - 1) / tiles);
     const int64_t P = 2 * S7;
     z.xs = batch * P * iu * z.ldx;
@@ -268,7 +268,7 @@ int backtransform_oz(cudaStream_t st, EigArgs& g) {
     const int64_t n = g.n, iu = g.iu, batch = g.batch, nrefl = n - 1;
     if (nrefl <= 0) return 0;
     OzSizes z;
-    oz_sizes(n, iu, batch, z);
+    oz_sizes(n, iu, batch, g.lean, z);
     const int64_t NB = z.NB, P = 2 * S7;
     const Refl v{g.A, g.lda, g.strideA, n};
     unsigned short *Xs = (unsigned short*)g.oz_xs, *Vr = (unsigned short*)g.oz_vr, *VH = (unsigned short*)g.oz_vh;

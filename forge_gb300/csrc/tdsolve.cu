@@ -1172,7 +1172,7 @@ void carve(EigArgs& g, Carve& c) {
     g.part = c.take<double>(B * g.pstride);
     g.scal = c.take<double>(B * 16);
     OzSizes z;
-    oz_sizes(n, iu, B, z);
+    oz_sizes(n, iu, B, g.lean, z);
     // the slices of X (and of the rank-2k update) share the scratch of the inverse iteration, those of V its
     // vectors: both are free before it, and again once Z has been copied to X
     g.Z = (double*)c.take<char>(std::max<size_t>(sizeof(double) * B * n * iu, 2 * z.vr));
@@ -1194,9 +1194,10 @@ void carve(EigArgs& g, Carve& c) {
 }
 }  // namespace
 
-size_t eig_workspace_bytes(int64_t n, int64_t iu, int64_t batch, bool mixed) {
+size_t eig_workspace_bytes(int64_t n, int64_t iu, int64_t batch, bool mixed, bool lean) {
     EigArgs g{};
     g.mixed = mixed;
+    g.lean = lean;
     g.n = n;
     g.iu = iu;
     g.batch = batch;
@@ -1315,7 +1316,7 @@ extern "C" int forge_selftest_eig_workspace(int64_t n, int64_t iu, int64_t batch
         return 0;
     }
     OzSizes z;
-    oz_sizes(n, iu, batch, z);
+    oz_sizes(n, iu, batch, false, z);
     out[0] = (int64_t)eig_workspace_bytes(n, iu, batch, false);
     out[1] = z.ks * batch;
     out[2] = z.wp / (iu * z.NB);

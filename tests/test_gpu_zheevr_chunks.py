@@ -34,3 +34,22 @@ def test_batch_in_parts(mode, cap, monkeypatch):
         nrm = np.linalg.norm(H[:, :, b], 2)
         assert np.max(np.abs(w[:, b] - np.linalg.eigvalsh(H[:, :, b])[:iu])) <= eps * nrm
         assert np.max(np.abs(H[:, :, b] @ X[:, :, b] - X[:, :, b] * w[:, b])) <= eps * nrm
+
+
+def test_blocks_of_reflectors_formed_together():
+    """N = 508: a caller's batch forms V^H and T of all eight blocks in one launch (the allocation-free entry, whose
+    array is small, one at a time)."""
+    import forge_gb300 as fg
+    with fg.HartreeFock(fg.Setup(ntheta=6, numk=1)) as hf:
+        n, nb = hf.N, 3
+        iu = n // 2 + 10
+        rng = np.random.default_rng(6)
+        G = rng.standard_normal((n, n, nb)) + 1j * rng.standard_normal((n, n, nb))
+        H = np.asfortranarray((G + G.conj().transpose(1, 0, 2)) / 2)
+        w, X, info = hf.zheevr_batch(H, iu)
+    assert info == 0
+    for b in range(nb):
+        nrm = np.linalg.norm(H[:, :, b], 2)
+        assert np.max(np.abs(w[:, b] - np.linalg.eigvalsh(H[:, :, b])[:iu])) <= 8 * n * EPS * nrm
+        assert np.max(np.abs(H[:, :, b] @ X[:, :, b] - X[:, :, b] * w[:, b])) <= 16 * n * EPS * nrm
+        assert np.max(np.abs(X[:, :, b].conj().T @ X[:, :, b] - np.eye(iu))) <= 64 * EPS / 1e-7
