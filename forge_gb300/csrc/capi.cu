@@ -78,12 +78,12 @@ int rr_window(cudaStream_t st, const double2* H, int64_t strideH, double2* X, in
               int64_t iu, int64_t n, int64_t c0, int64_t nw, int64_t batch, void* ws);
 size_t rr_window_workspace_bytes(int64_t n, int64_t batch);
 const float* eig_mixed_planes(void* mixed_ws, int64_t n, int64_t iu, int64_t batch, int64_t* n4);
-size_t oa_workspace_bytes(int64_t n, int64_t iu, int64_t batch);
+size_t oa_workspace_bytes(int64_t n, int64_t iu, int64_t batch, int64_t cap);
 int launch_pad_slot(cudaStream_t st, const double2* src, int64_t nb, double2* dst, int64_t n, double* rowsum,
                     double* sigma);
 int oa_refine(cudaStream_t st, double2* H, int64_t strideH, const float* Xs, int64_t n4, int64_t nall,
               const double* lam, int64_t n, int64_t iu, int64_t batch, double2* X, int64_t ldx, int64_t strideX,
-              double* w_out, int64_t w_stride, void* ws, int* err, double delta, int depth);
+              double* w_out, int64_t w_stride, void* ws, int64_t cap, int* err, double delta, int depth);
 
 }  // namespace forge
 
@@ -110,6 +110,8 @@ struct forge_ctx {
     double last_residual = INFINITY;
     // test hook: the next FP64 solves / projector batches that report a bounded wait that gave up
     int fail_solves = 0, fail_projectors = 0;
+    // bytes of the matrices refined, and of the projectors formed, by one launch
+    int64_t oa_cap = (int64_t)4 << 30, proj_cap = (int64_t)2 << 30;
     DevBuf oaws, w_all;
     // group solve led by this context (forge_gpu_solve_group): padded H slots, eigenpairs, workspaces
     DevBuf g_H, g_X, g_w, g_eigws, g_mixws, g_tmp, g_rows, g_sig, g_rr, g_lim;
@@ -173,7 +175,7 @@ int choose_batch(forge_ctx* x) {
     // cells) is allocated at the first mixing step, after this choice
     const size_t diis = x->mix_mode == FORGE_MIX_PULAY ? ((size_t)(2 * (x->diis_depth + 1) + 1) * 4 * N * N * 8) : 0;
     const size_t reserve = ((size_t)8 << 30) + (size_t)xslots * N * iu * 16 + (size_t)10 * N * N * 16 +
-                           (oa ? oa_workspace_bytes(N, iu, c.Nk) : 0) + diis;
+                           (oa ? oa_workspace_bytes(N, iu, c.Nk, x->oa_cap) : 0) + diis;
     const size_t budget = freeb > reserve ? freeb - reserve : freeb / 4;
     int64_t b = (int64_t)(budget / per_k);
     // FORGE_EIG_BATCH caps the number of k points solved per launch (memory control)
@@ -211,7 +213,7 @@ int ensure_solve_buffers(forge_ctx* x) {
     if (c.precision == FORGE_PREC_MIXED) FORGE_TRY(x->mixws.ensure(eig_mixed_workspace_bytes(N, iu_solve, B)));
     if (oa) {
         FORGE_TRY(x->w_all.ensure((size_t)B * N * sizeof(double)));
-        FORGE_TRY(x->oaws.ensure(oa_workspace_bytes(N, iu, B)));
+        FORGE_TRY(x->oaws.ensure(oa_workspace_bytes(N, iu, B, x->oa_cap)));
         FORGE_TRY(x->tcerr.ensure(sizeof(int)));
     }
     FORGE_TRY(c.bulk.ensure(4 * NN * sizeof(double2)));
@@ -286,7 +288,7 @@ int eig_batch_run(forge_ctx* x, int64_t k0, int64_t nb, int* info, const Assembl
             const float* planes = eig_mixed_planes(x->mixws.ptr, N, N, nb, &n4);
             FORGE_CUDA(cudaMemsetAsync(x->tcerr.ptr, 0, sizeof(int), c.stream));
             r = oa_refine(c.stream, g.A, g.strideA, planes, n4, N, g.w, N, iu, nb, g.X, g.ldx, g.strideX, w_iu, iu,
-                          x->oaws.ptr, x->tcerr.as<int>(), x->oa_delta, x->oa_depth);
+                          x->oaws.ptr, x->oa_cap, x->tcerr.as<int>(), x->oa_delta, x->oa_depth);
             if (r) return r;
             int herr = 0;
             FORGE_CUDA(cudaMemcpyAsync(&herr, x->tcerr.ptr, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
@@ -351,9 +353,9 @@ int project_items(forge_ctx* x, const std::vector<ProjItem>& items, double2* out
     }
     const bool refined = c.precision == FORGE_PREC_MIXED && x->oa_active;
     if (c.precision != FORGE_PREC_MIXED || refined) {
-        FORGE_TRY(x->projws.ensure(proj_oz_workspace_bytes(N, iu, nit, refined)));
+        FORGE_TRY(x->projws.ensure(proj_oz_workspace_bytes(N, iu, nit, refined, x->proj_cap)));
         return projectors_oz(c.stream, c.X.as<double2>(), N, N * iu, N, iu, items.data(), nit, out, x->projws.ptr,
-                             x->tcerr.as<int>(), refined);
+                             x->tcerr.as<int>(), refined, x->proj_cap);
     }
     for (const ProjItem& p : items) {
         const double2* Xk = c.X.as<double2>() + (size_t)p.slot * N * iu;
@@ -1620,7 +1622,7 @@ static int64_t zheevr_chunk(forge_ctx* x, int64_t iu, int64_t nb) {
     if (oa) per += (size_t)N * sizeof(double);
     size_t freeb = 0, totalb = 0;
     cudaMemGetInfo(&freeb, &totalb);
-    const size_t reserve = ((size_t)256 << 20) + (oa ? oa_workspace_bytes(N, iu, nb) : 0);
+    const size_t reserve = ((size_t)256 << 20) + (oa ? oa_workspace_bytes(N, iu, nb, x->oa_cap) : 0);
     int64_t b = std::max<int64_t>(1, freeb > reserve ? (int64_t)((freeb - reserve) / per) : 1);
     if (const char* env = std::getenv("FORGE_EIG_BATCH")) {
         const long cap = std::strtol(env, nullptr, 10);
@@ -1682,7 +1684,7 @@ int zheevr_solve(forge_ctx* x, ZheevrBufs& d, const double* A, int64_t b0, int64
             const float* planes = eig_mixed_planes(d.mws.ptr, N, N, nb, &n4);
             FORGE_CUDA(cudaMemsetAsync(d.oerr.ptr, 0, sizeof(int), c.stream));
             FORGE_TRY(oa_refine(c.stream, g.A, g.strideA, planes, n4, N, g.w, N, iu, nb, g.X, g.ldx, g.strideX, w, iu,
-                                d.ows.ptr, d.oerr.as<int>(), x->oa_delta, x->oa_depth));
+                                d.ows.ptr, x->oa_cap, d.oerr.as<int>(), x->oa_delta, x->oa_depth));
             int herr = 0;
             if (cudaMemcpyAsync(&herr, d.oerr.ptr, sizeof(int), cudaMemcpyDeviceToHost, c.stream) != cudaSuccess ||
                 cudaStreamSynchronize(c.stream) != cudaSuccess || herr) {
@@ -1725,7 +1727,7 @@ int forge_gpu_zheevr_batch(forge_ctx* x, int64_t nb, const double* A, int64_t iu
     if (mixed) FORGE_TRY(d.mws.ensure(eig_mixed_workspace_bytes(N, iu_solve, B)));
     if (oa) {
         FORGE_TRY(d.wall.ensure(B * N * sizeof(double)));
-        FORGE_TRY(d.ows.ensure(oa_workspace_bytes(N, iu, B)));
+        FORGE_TRY(d.ows.ensure(oa_workspace_bytes(N, iu, B, x->oa_cap)));
         FORGE_TRY(d.oerr.ensure(sizeof(int)));
     }
     FORGE_CUDA(cudaMemcpyAsync(d.A.ptr, A, nb * NN * sizeof(double2), cudaMemcpyHostToDevice, c.stream));
@@ -1738,6 +1740,17 @@ int forge_gpu_zheevr_batch(forge_ctx* x, int64_t nb, const double* A, int64_t iu
     int bad = 0;
     for (int64_t b = 0; b < nb; ++b) bad += fails[b] ? 1 : 0;
     return bad;
+}
+
+int forge_gpu_selftest_launch_bytes(forge_ctx* x, int64_t refinement, int64_t projectors) {
+    FORGE_TRY(check_ctx(x));
+    if (refinement < 1 || projectors < 1) {
+        set_error(FORGE_ERR_ARG, "selftest_launch_bytes: bad arguments");
+        return FORGE_ERR_ARG;
+    }
+    x->oa_cap = refinement;
+    x->proj_cap = projectors;
+    return 0;
 }
 
 int forge_gpu_selftest_timeouts(forge_ctx* x, int64_t solves, int64_t projectors) {

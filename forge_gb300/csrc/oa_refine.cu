@@ -324,16 +324,16 @@ OaLayout oa_layout(int64_t n, int64_t iu, int64_t nb, void* base) {
     return L;
 }
 
-// matrices refined together: what fits in 4 GB and in a launch's grid, at least one (one matrix of N = 364 has nine tiles)
-int64_t oa_chunk(int64_t n, int64_t iu, int64_t batch) {
+// matrices refined together: what fits in cap bytes and in a launch's grid, at least one (one matrix of N = 364 has nine tiles)
+int64_t oa_chunk(int64_t n, int64_t iu, int64_t batch, int64_t cap) {
     const int64_t per = (int64_t)oa_layout(n, iu, 1, nullptr).bytes;
-    return std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(batch, OZ_GRID_Z), ((int64_t)4 << 30) / per));
+    return std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(batch, OZ_GRID_Z), cap / per));
 }
 
 }  // namespace
 
-size_t oa_workspace_bytes(int64_t n, int64_t iu, int64_t batch) {
-    return oa_layout(n, iu, oa_chunk(n, iu, batch), nullptr).bytes + 256;
+size_t oa_workspace_bytes(int64_t n, int64_t iu, int64_t batch, int64_t cap) {
+    return oa_layout(n, iu, oa_chunk(n, iu, batch, cap), nullptr).bytes + 256;
 }
 
 // Refines columns 0..iu-1 of X (FP64, unit-normalised, ldx, strideX per matrix) and their eigenvalues
@@ -343,7 +343,7 @@ size_t oa_workspace_bytes(int64_t n, int64_t iu, int64_t batch) {
 // w_out + b * w_stride.  depth: slice products s + t <= depth of the residual (3 or 4).
 int oa_refine(cudaStream_t st, double2* H, int64_t strideH, const float* Xs, int64_t n4, int64_t nall,
               const double* lam, int64_t n, int64_t iu, int64_t batch, double2* X, int64_t ldx, int64_t strideX,
-              double* w_out, int64_t w_stride, void* ws, int* err, double delta, int depth) {
+              double* w_out, int64_t w_stride, void* ws, int64_t cap, int* err, double delta, int depth) {
     if (iu <= 0 || batch <= 0) return 0;
     if (nall != n || iu > nall || depth < 1 || depth > OA_SLICES - 1 || n4 < n || (n4 % 4)) {
         set_error(FORGE_ERR_ARG, "oa_refine: needs all n eigenvectors (nall=%lld n=%lld), iu <= n, depth 1..%d",
@@ -351,7 +351,7 @@ int oa_refine(cudaStream_t st, double2* H, int64_t strideH, const float* Xs, int
         return FORGE_ERR_ARG;
     }
     constexpr int S = OA_SLICES;
-    const int64_t chunk = oa_chunk(n, iu, batch);
+    const int64_t chunk = oa_chunk(n, iu, batch, cap);
     const OaLayout L = oa_layout(n, iu, chunk, ws);
     auto cmap = [&](const int32_t* za, const int32_t* zb, int64_t K, TcKMap& ka, TcKMap& kb) {
         ka = TcKMap{};

@@ -429,23 +429,23 @@ __global__ void __launch_bounds__(256) k_proj_add(double2* __restrict__ P, const
 }
 }  // namespace
 
-// items per launch: as many as fit in 2 GB of slices and products and in a launch's grid, at least one
-static int64_t proj_oz_chunk(int64_t n, int64_t iu, int64_t nit, int S) {
+// items per launch: as many as fit in cap bytes of slices and products and in a launch's grid, at least one
+static int64_t proj_oz_chunk(int64_t n, int64_t iu, int64_t nit, int S, int64_t cap) {
     const int64_t per = 2 * S * n * up(iu, 8) * 2 + 2 * n * n * 8;
-    return std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nit, OZ_GRID_Z), ((int64_t)2 << 30) / per));
+    return std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nit, OZ_GRID_Z), cap / per));
 }
-size_t proj_oz_workspace_bytes(int64_t n, int64_t iu, int64_t nit, bool refined) {
+size_t proj_oz_workspace_bytes(int64_t n, int64_t iu, int64_t nit, bool refined, int64_t cap) {
     const int S = refined ? OZ_REF_S : OZ_S;
-    const int64_t ch = proj_oz_chunk(n, iu, nit, S);
+    const int64_t ch = proj_oz_chunk(n, iu, nit, S, cap);
     return (size_t)ch * (2 * S * n * up(iu, 8) * 2 + 2 * n * n * 8 + up(n, 64) * 12) + (size_t)nit * sizeof(ProjItem) + 1024;
 }
 
 template <int S, int DEPTH, bool REF>
 static int projectors_cut(cudaStream_t st, const double2* X, int64_t ldx, int64_t strideX, int64_t n, int64_t iu,
-                          const ProjItem* items, int64_t nit, double2* P, void* ws, int* err) {
+                          const ProjItem* items, int64_t nit, double2* P, void* ws, int* err, int64_t cap) {
     if (nit <= 0) return 0;
     prof_begin(ST_PROJECTOR);
-    const int64_t ch = proj_oz_chunk(n, iu, nit, S), ldk = up(iu, 8), plane = n * ldk, PL = 2 * S;
+    const int64_t ch = proj_oz_chunk(n, iu, nit, S, cap), ldk = up(iu, 8), plane = n * ldk, PL = 2 * S;
     double* C = static_cast<double*>(ws);
     unsigned short* sl = reinterpret_cast<unsigned short*>(C + ch * 2 * n * n);
     int* e = reinterpret_cast<int*>(sl + ch * PL * plane);
@@ -476,9 +476,9 @@ static int projectors_cut(cudaStream_t st, const double2* X, int64_t ldx, int64_
 // products in double-float sums (2^-48) and the diagonal (the site densities) in FP64.  Measured (TF32 slices, one
 // k a launch before): N = 364, 36 k 8.7 -> 0.9 ms; N = 1324, 16 k 11.0 -> 3.8 ms; N = 5044 19.1 -> 7.2 ms
 int projectors_oz(cudaStream_t st, const double2* X, int64_t ldx, int64_t strideX, int64_t n, int64_t iu,
-                  const ProjItem* items, int64_t nit, double2* P, void* ws, int* err, bool refined) {
-    return refined ? projectors_cut<OZ_REF_S, OZ_REF_DEPTH, true>(st, X, ldx, strideX, n, iu, items, nit, P, ws, err)
-                   : projectors_cut<OZ_S, OZ_DEPTH, false>(st, X, ldx, strideX, n, iu, items, nit, P, ws, err);
+                  const ProjItem* items, int64_t nit, double2* P, void* ws, int* err, bool refined, int64_t cap) {
+    return refined ? projectors_cut<OZ_REF_S, OZ_REF_DEPTH, true>(st, X, ldx, strideX, n, iu, items, nit, P, ws, err, cap)
+                   : projectors_cut<OZ_S, OZ_DEPTH, false>(st, X, ldx, strideX, n, iu, items, nit, P, ws, err, cap);
 }
 
 }  // namespace forge

@@ -17,9 +17,10 @@ struct ProjItem {
     int64_t slot, K;
     double2 ph[4];
 };
-size_t proj_oz_workspace_bytes(int64_t n, int64_t iu, int64_t nit, bool refined);
+// cap: bytes of slices and products per launch (the result does not depend on it)
+size_t proj_oz_workspace_bytes(int64_t n, int64_t iu, int64_t nit, bool refined, int64_t cap);
 int projectors_oz(cudaStream_t st, const double2* X, int64_t ldx, int64_t strideX, int64_t n, int64_t iu,
-                  const ProjItem* items, int64_t nit, double2* P, void* ws, int* err, bool refined);
+                  const ProjItem* items, int64_t nit, double2* P, void* ws, int* err, bool refined, int64_t cap);
 int window_projector_fp64(cudaStream_t st, const WinState* states, int64_t nstates, const double2* X, int64_t ldx,
                           int64_t strideX, int64_t N, double2* P);
 size_t proj_tc_workspace_floats(int64_t n, int64_t iu);

@@ -33,6 +33,10 @@ int forge_gpu_selftest_tc_gemm_timeout(int64_t M, int64_t N, int64_t K, int64_t 
  * M^H S M = I.  Returns 1 if S is not positive definite. */
 int forge_selftest_rr_small(int64_t n, const double* G, const double* S, double* theta, double* M);
 
+/* Bytes that one launch of the eigenpair refinement and one of the sliced projectors may take (4 GB and 2 GB by
+ * default), so that small cases run several; results do not depend on them. */
+int forge_gpu_selftest_launch_bytes(forge_ctx* ctx, int64_t refinement, int64_t projectors);
+
 /* The context's next `solves` FP64 eigen-solves and `projectors` batches of projectors report, once their work is
  * done, that a bounded wait gave up (FORGE_ERR_TIMEOUT); each is tried a second time. */
 int forge_gpu_selftest_timeouts(forge_ctx* ctx, int64_t solves, int64_t projectors);
