@@ -53,12 +53,13 @@ CONFIGS = {
 METRIC = "time-to-SCF (s) and SCF iters, 1.05deg TBG: net+mixed vs plain FP64, same accuracy"
 
 # Plain FP64 GPU SCF runs measured to convergence with `--mode plain --converge` (Pulay depth 6,
-# beta 0.7, corrected DegFactor).  They are reported in the labelled field plain_fp64_recorded and
-# give the reference arm its iteration count; they never enter `value`.
+# beta 0.7, corrected DegFactor).  They are reported in the labelled fields plain_fp64_recorded and
+# plain_fp64_measured and give the reference arm its iteration count; they never enter `value`.
 PLAIN_FP64_RECORDED = {
-    # 1.05 deg: a plain FP64 SCF (about 70 minutes) does not fit one GPU lease, so the count is that of
-    # the FP64-equivalent trajectory (every mixed solve refined to FP64 accuracy: the same iterates
-    # to 1e-9) and the time per iteration is the measured FP64 one
+    # 1.05 deg, an estimate for the FP64 kernels of its date (products and reduction on the FP64 pipe), which have been
+    # replaced since; PLAIN_FP64_MEASURED holds the present ones.  A plain FP64 SCF took about 70 minutes and
+    # did not fit one GPU lease, so the count is that of the FP64-equivalent trajectory (every mixed solve refined
+    # to FP64 accuracy: the same iterates to 1e-9) and the time per iteration is the measured FP64 one
     "tbg_m31_N11908_4x4_nu+2_eps10_1.05deg": {
         "iterations": 11, "converged": None, "estimated": True, "final_residual": 4.19e-07,
         "ms_per_iter": 347800.0, "guess_s": 300.0, "time_to_scf_s": 300.0 + 11 * 347.8,
@@ -68,16 +69,24 @@ PLAIN_FP64_RECORDED = {
                    "python3 bench.py --gpus 1 --steps 20 --warmup 5 (FP64 iterations 22-25 of its run); "
                    "FP64 guess = one FP64 solve of the 16 k points (16 x 18.7 s, forge_gb300.eigbench)"},
     "tbg_m10_N1324_12x12_nu+2_eps10": {
-        "iterations": 6, "time_to_scf_s": 36.1, "ms_per_iter": 5160.0, "converged": True,
-        "final_residual": 1.0e-07, "date": "2026-12-03",
+        "iterations": 6, "time_to_scf_s": 6.07, "ms_per_iter": 870.7, "converged": True,
+        "final_residual": 1.02e-07, "date": "2026-12-05",
         "command": "python bench.py --config 1 --mode plain --converge"},
+}
+# The same, measured to convergence with the present kernels
+PLAIN_FP64_MEASURED = {
+    "tbg_m31_N11908_4x4_nu+2_eps10_1.05deg": {
+        "iterations": 11, "time_to_scf_s": 434.3, "ms_per_iter": 36214.5, "guess_s": 35.9, "converged": True,
+        "final_residual": 4.186e-07, "date": "2026-12-05",
+        "command": "python bench.py --config 4 --mode plain --converge --itmax 20 --warmup 1"},
 }
 
 # DRAM traffic of the dominant kernels from ncu captures small enough for the profiler
 # (dram__bytes_read.sum + dram__bytes_write.sum), per unit of the work model: per algorithmic byte
 # for the streaming kernels, per algorithmic flop for the sliced residual product (its DRAM bytes
 # are panel re-reads, which grow with the tile-K products, i.e. with the flops, not with the
-# operand bytes).
+# operand bytes).  The residual product's ratio is of the TF32 kernel that was captured; the bf16 slice kernel
+# (k_oz_gemm) in its place has twice the tile width and half the operand bytes, and has not been captured.
 NCU_TRAFFIC_RATIO = {
     "hemv": (1.044, "bytes", "ncu --set full of k_trd_hemv<float> at N=5044, column 1501 (n'=3543): 52.25 MB "
                              "read + 0.19 MB written against 50.23 MB algorithmic (trailing lower triangle, "
@@ -627,6 +636,8 @@ def main():
     rec = PLAIN_FP64_RECORDED.get(cfg["name"])
     if rec:
         line["plain_fp64_recorded"] = rec
+    if cfg["name"] in PLAIN_FP64_MEASURED:
+        line["plain_fp64_measured"] = PLAIN_FP64_MEASURED[cfg["name"]]
     if args.save_state and r["state"] is not None:
         np.savez_compressed(args.save_state, residuals=np.array([h["residual"] for h in hist]),
                             energies=np.array([h["TotalEnergy"] for h in hist]),

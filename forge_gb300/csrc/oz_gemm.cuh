@@ -9,8 +9,12 @@
 // of 256 of them below 2^24, so the FP32 accumulation in TMEM is exact; every 256 products the epilogue
 // warps add the block to int64 accumulators, and each level d = s + t weighs 2^9 less than the one
 // before, so a level is a shift.  Nothing is rounded until the sum is converted to FP64.  With
-// seven slices and depth 6 the operands keep 62 bits below their row's maximum and the neglected
-// products are below 2^-62 of the two maxima: less than the rounding of an FP64 GEMM over the same K.
+// seven slices and depth 6 the operands keep 62 bits below their row's maximum.  A slice s is at most 2^-9s of the
+// row's scale, so the neglected pairs of a real product (six with s + t = 7, the next ones 2^-9 of these) are below
+// 6 x 2^-63 = 2^-60.4 of the two maxima, twice that for a component of a complex product, and about 2^-63 for digits of
+// random sign: small beside the rounding of an FP64 product of the row maxima, 2^-53.  An element below 2^-9 of its
+// row's maximum has fewer than FP64's 53 bits; the callers scale their operands so that a row's elements matter by
+// its maximum (oz_fp64.cu).
 //
 // Why: this GPU's FP64 pipe does 1.2 TFLOP/s (two FMA lanes a clock and SM); 28 slice products at the
 // measured bf16 rate are 1938 / 28 = 69 TFLOP/s of FP64-accurate work.

@@ -5,11 +5,13 @@
 // eigenvalues by bisection (dstebz) and the vectors by inverse iteration (zstein);
 // this file restates that route for the GPU:
 //   k_gersh     : Gershgorin interval, 1-norm and pivmin per matrix;
-//   k_bisect*   : eigenvalues by Sturm counts, an FP32 bracket and FP64 multisection;
+//   k_bisect*   : eigenvalues by Sturm counts, an FP32 bracket and FP64 multisection
+//                 (eigenvalues near zero by bisection with quotients);
 //   k_clusters  : groups consecutive eigenvalues closer than ortol;
-//   k_invit     : one thread per cluster: LU of T - lambda I with partial pivoting
-//                 (dlagtf), perturbed back-substitution (dlagts, job=-1), modified
-//                 Gram-Schmidt against the earlier members of the cluster;
+//   k_invit_lu  : LU of T - lambda I with partial pivoting (dlagtf), a thread an eigenvalue;
+//   k_invit     : perturbed back-substitution (dlagts, job=-1): a thread an eigenvalue for the first members
+//                 of the clusters and the first solve of the others, then eight lanes a cluster for the others'
+//                 modified Gram-Schmidt against the earlier members and further solves;
 //   back-transform: Q applied in compact-WY blocks (zlarft forward/columnwise) on the tensor
 //                 cores (oz_fp64.cu; eig_mixed.cu for the mixed path).
 // ortol is tighter than zstein's 1e-3*||T||_1 (which groups a whole dense spectrum

@@ -21,7 +21,8 @@
 // ratio of 1e-8, and nothing left at 1e-20).  |hi|, |lo| <= 2^27 and at most 256 products a sum stay below 2^62.  The trailing matrix does
 // not change inside a panel (V and W carry its update), so k_limbs64 cuts it once for 32 columns, into as
 // many bytes as it had, in the order in which k_hemv64's threads read it.  Bound: integer multiply-adds (24 an element).
-// Measured (stage; cut anew in every column before): N = 1324, 16 k 57.6 -> 41 ms, N = 3268, one k 64 -> 53 ms.  What
+// Measured (stage; cut anew in every column before): N = 1324, 16 k 57.6 -> 41 ms, N = 3268, one k 64 -> 53 ms; with an
+// exponent for each row and column of a tile, not one for all, 43 and 55 ms.  What
 // keeps it from the multiply-adds' rate is their latency: 16 warps an SM (registers) issue on 36% of the clocks.
 // k_col64 and k_finish64, with FP64 instructions shared by more lanes and the loads of older results ahead of the
 // predecessor's end: the whole reduction N = 3268, one k 103 -> 79 ms; N = 76, nine k 1.5 -> 1.3 ms.

@@ -1,5 +1,5 @@
-"""The FP64 window Rayleigh-Ritz on the device (products on the tensor cores, Jacobi in one CTA) for every parity
-of the window's width, and batches larger than one launch, against LAPACK."""
+"""The FP64 window Rayleigh-Ritz (products in FP64 tiles on the CUDA cores, the small problem on the host) for every
+parity of the window's width, on three matrices in one launch, against LAPACK."""
 import numpy as np
 import pytest
 
