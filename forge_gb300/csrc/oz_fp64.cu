@@ -173,7 +173,8 @@ struct EpiHer2k {
 
 // T of the compact-WY form from G = V^H V (zlarft, forward columnwise): T(0:i, i) = -tau_i T(0:i, 0:i) G(0:i, i),
 // T(i, i) = tau_i.  One CTA per (block, matrix), thread l owns row l; T packed by columns in shared memory.
-// FP64 pipe bound (NB^3 / 6 complex products on one SM), so all blocks of a chunk run side by side.
+// FP64 pipe bound (NB^3 / 6 complex products on one SM), so all blocks of a chunk run side by side; the last block's
+// chain ends with its last reflector (n = 2: 338 us for all 64 steps).
 __global__ void k_oz_larft(const double2* __restrict__ G, const double2* __restrict__ tau, int64_t n, int64_t j0, int NB,
                            int64_t batch, double2* __restrict__ T) {
     extern __shared__ double2 lt_sm[];
@@ -182,9 +183,10 @@ __global__ void k_oz_larft(const double2* __restrict__ G, const double2* __restr
     const int64_t z = blockIdx.x, q = z / batch, b = z - q * batch, jb = j0 + q * NB;
     const double2* g = G + z * NB * NB;
     double2* To = T + z * NB * NB;
-    const int l = threadIdx.x;
-    for (int i = 0; i < NB; ++i) {
-        const double2 ti = jb + i < n - 1 ? tau[b * n + jb + i] : make_double2(0.0, 0.0);
+    const int l = threadIdx.x, nrefl = (int)min((int64_t)NB, n - 1 - jb);
+    for (int i = nrefl; i < NB; ++i) To[l + i * NB] = make_double2(0.0, 0.0);
+    for (int i = 0; i < nrefl; ++i) {
+        const double2 ti = tau[b * n + jb + i];
         if (l < i) tmp[l] = cmul(cmake(-ti.x, -ti.y), g[l + i * NB]);
         __syncthreads();
         double2 acc = make_double2(0.0, 0.0);

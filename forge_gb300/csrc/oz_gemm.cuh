@@ -259,6 +259,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     } else {
         const int quarter = warp & 3, half = (warp - 2) >> 2;
         const int64_t row = m0 + quarter * 32 + lane;
+        // 16-column groups of the warp's part that hold results: the conversions run on the FP64 pipe and are most of a
+        // small product's time (n = 2: 65 us a product with the whole tile converted)
+        const int64_t cols = m0 + quarter * 32 < M ? N - (n0 + half * 64) : 0;
+        const int live = (int)min((int64_t)4, max((int64_t)0, (cols + 15) / 16));
         const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 64);
         const uint32_t thi = tmem + ((uint32_t)(quarter * 32) << 16) + 256u + (uint32_t)(half * 128);
         long long acc[DF ? 1 : 64];
@@ -278,6 +282,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                     // the first levels in FP64 (exact up to one rounding) to TMEM
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
+                        if (h >= live) break;
                         uint32_t r[32];
 #pragma unroll
                         for (int q = 0; q < 16; ++q) {
@@ -306,6 +311,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                 for (int h = 0; h < 64; h += 32) {
+                    if (h / 16 >= live) break;
                     float v[32];
                     __syncwarp();
                     tmem_ld32(trow + (uint32_t)(buf * OZ_T + h), v);
@@ -337,6 +343,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             const double c1 = plan.split ? oz_pow2(-(16 + 9 * (plan.split - 1))) : 0.0;
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
+                if (h >= live) break;
                 double d[16];
                 if constexpr (DF) {
 #pragma unroll

@@ -127,3 +127,31 @@ def test_diagonal_over_many_orders():
     d = np.array([1e-33, 4.0, -3e-58, 1e-12, 0.0, -2e-31, 7e-31, 5e-45, -1.0, 6e-55])
     w = _eigenvalues(np.diag(d).astype(complex))
     assert np.all(np.abs(w - np.sort(d)) <= np.maximum(2 * EPS * np.abs(np.sort(d)), 1e-75))
+
+
+@pytest.mark.parametrize("n", [2, 4, 8, 9, 15, 16, 17, 18, 32, 33, 47, 48, 49, 50, 81])
+def test_small_matrices(n):
+    """The last (here only) block of reflectors ends with its last reflector, and a product's epilogue with the last row
+    and column: every pair of matrices around the 16 columns and 32 rows that it goes by.  LAPACK's bounds."""
+    import ctypes as C
+
+    import torch
+
+    import forge_gb300 as fg
+    f = fg.load_library().forge_gpu_zheevr_noalloc
+    f.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]
+    f.restype = C.c_int
+    rng = np.random.default_rng(n)
+    G = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    H = (G + G.conj().T) / 2
+    nrm = np.linalg.norm(H, 2)
+    for iu in sorted({1, n // 2, n - 1, n} - {0}):
+        dA = torch.from_numpy(np.ascontiguousarray(H.T)).cuda()
+        w = torch.empty(iu, dtype=torch.float64, device="cuda")
+        Z = torch.empty(iu, n, dtype=torch.complex128, device="cuda")
+        torch.cuda.synchronize()
+        assert f(dA.data_ptr(), n, iu, w.data_ptr(), Z.data_ptr(), None) == 0
+        w, X = w.cpu().numpy(), Z.cpu().numpy().T
+        assert np.max(np.abs(w - np.linalg.eigvalsh(H)[:iu])) <= 8 * n * EPS * nrm
+        assert np.max(np.abs(H @ X - X * w)) <= 16 * n * EPS * nrm
+        assert np.max(np.abs(X.conj().T @ X - np.eye(iu))) <= 64 * EPS / 1e-7
