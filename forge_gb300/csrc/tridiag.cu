@@ -493,7 +493,7 @@ int tridiagonalize_f32(cudaStream_t st, TrdArgs<float>& a, int64_t batch) {
             dim3 gc((unsigned)((n2 + TRD_ROWS - 1) / TRD_ROWS), (unsigned)batch);
             prof_begin(ST_TRD_FINISH);
             FORGE_TRY(launch_chain(st, gf, TRD_ROWS, k_trd_finish, a, p, ii, col, nbr, nrb));
-            if (ii == w - 1 || col == n - 2) FORGE_TRY(launch_chain(st, gc, TRD_ROWS, k_trd_fix, a, ii, col));
+            if (ii == w - 1) FORGE_TRY(launch_chain(st, gc, TRD_ROWS, k_trd_fix, a, ii, col));
             prof_end(ST_TRD_FINISH, batch * (double)n2 * (2.0 * ii + 4.0) * esz, 0.0);
         }
         if (nrefl > 0 && p + w < n) {

@@ -660,9 +660,7 @@ static int tridiagonalize_rows(cudaStream_t st, TrdArgs<double>& a, int64_t batc
             prof_end(ST_HEMV, batch * 0.5 * (double)n2 * (double)(n2 + 1) * 16.0, batch * 8.0 * (double)n2 * n2);
             prof_begin(ST_TRD_FINISH);
             FORGE_TRY(launch_chain(st, dim3((unsigned)((n2 + fr - 1) / fr), nbat), 256, k_finish64<RW>, a, p, ii, col, nb2, ndot));
-            if (ii == w - 1 || col == n - 2) {
-                FORGE_TRY(launch_chain(st, dim3((unsigned)((n2 + 255) / 256), nbat), 256, k_fix64, a, ii, col, fr));
-            }
+            if (ii == w - 1) FORGE_TRY(launch_chain(st, dim3((unsigned)((n2 + 255) / 256), nbat), 256, k_fix64, a, ii, col, fr));
             prof_end(ST_TRD_FINISH, batch * (double)n2 * (2.0 * ii + 4.0) * 16.0, 0.0);
         }
         if (nrefl > 0 && p + w < n) {
