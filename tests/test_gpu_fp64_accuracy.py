@@ -129,7 +129,7 @@ def test_diagonal_over_many_orders():
     assert np.all(np.abs(w - np.sort(d)) <= np.maximum(2 * EPS * np.abs(np.sort(d)), 1e-75))
 
 
-@pytest.mark.parametrize("n", [2, 4, 8, 9, 15, 16, 17, 18, 32, 33, 47, 48, 49, 50, 81])
+@pytest.mark.parametrize("n", [2, 4, 8, 9, 15, 16, 17, 18, 32, 33, 34, 47, 48, 49, 50, 81])
 def test_small_matrices(n):
     """The last (here only) block of reflectors ends with its last reflector, and a product's epilogue with the last row
     and column: every pair of matrices around the 16 columns and 32 rows that it goes by.  LAPACK's bounds."""
